@@ -216,3 +216,50 @@ def test_mixed_fill_matches_fp64_fill(gpu_pkg, with_images):
           ", ".join(f"{k[0]} {k[1]} {v:.2e}" for k, v in sorted(worst.items())))
     assert worst[("zl", "special")] <= 1e-13 and worst[("zt", "special")] <= 1e-13
     assert worst[("zl", "regular")] <= 1e-12 and worst[("zt", "regular")] <= 1e-12
+
+
+def bent_wire(pkg, m):
+    """m segments of uneven length from the surface down, turning at every joint: collinear, bent and image pairs that
+    touch, near pairs, and far ones."""
+    rng = np.random.default_rng(m)
+    steps = rng.uniform(0.3, 1.0, (m, 3)) * np.where((np.arange(m)[:, None] + 2) % 3 == np.arange(3), 1.0, 0.0)
+    steps[:, 2] *= -1.0
+    if m > 1:
+        steps[1] = 0.5 * steps[0]              # a collinear joint
+    pts = np.concatenate([[[0.0, 0.0, 0.0]], np.cumsum(steps, axis=0)])
+    return np.stack([pkg.populate_electrode(pts[i], pts[i + 1], 7e-3) for i in range(m)])
+
+
+@pytest.mark.parametrize("m", [1, 2, 5, 17])
+@pytest.mark.parametrize("x", [0.01, 0.7, 0.8, 3.4, 3.6, 6.0])
+def test_fill_series_and_its_limits_match_oracle(gpu_pkg, port, m, x):
+    """Moment series with 16 and 32 terms, and the direct rule past its reach
+    (x = |gamma| (Lmax + Lmax / 16), 3.5); oracle at 1e-10, entries at TOL."""
+    pkg = gpu_pkg
+    e = bent_wire(pkg, m)
+    img = pkg.images(e)
+    gamma = x / (e[:, 9].max() * 17 / 16) * np.exp(0.25j * np.pi)
+    s, kappa, ref_t = 1e5 + 1e6j, 0.01 + 1e-4j, 0.9 + 0.01j
+    got = [np.zeros(m * m, np.complex128) for _ in range(2)]
+    want = [np.zeros(m * m, np.complex128) for _ in range(2)]
+    assert pkg.calculate_impedances(*got, e, gamma, s, 1.0, kappa) == 0
+    assert pkg.impedances_images(*got, e, img, gamma, s, 1.0, kappa, 1.0, ref_t) == 0
+    assert port.calculate_impedances(*want, e, gamma, s, 1.0, kappa, req_abs=0.0, req_rel=1e-10) == 0
+    assert port.impedances_images(*want, e, img, gamma, s, 1.0, kappa, 1.0, ref_t, req_abs=0.0, req_rel=1e-10) == 0
+    for a, b in zip(got, want):
+        assert np.array_equal(a == 0, b == 0)
+        assert elementwise(a, b) < TOL
+
+
+def test_plan_fill_serves_samples_on_both_sides_of_the_series_limit(gpu_pkg):
+    """One pass with samples inside and beyond the series' reach equals passes of one sample each."""
+    pkg = gpu_pkg
+    e, nodes = pkg.electrode_grid(3, 3, 8.0, 8.0, 1, 2, 7e-3, -0.5)
+    s = 8e4 + 2j * np.pi * np.array([0.0, 1e5, 1e6, 8e6, 2e7])
+    kappa = 0.02 + s * 10 * pkg.EPS0
+    together, info, _ = pkg.hem_sweep(e, pkg.images(e), nodes, s, kappa, max_batch=5)
+    assert not info.any()
+    for k in range(len(s)):
+        alone, info, _ = pkg.hem_sweep(e, pkg.images(e), nodes, s[k:k + 1], kappa[k:k + 1])
+        assert not info.any()
+        assert rel_err(together[k], alone[0]) < 1e-10

@@ -145,7 +145,13 @@ static int fill_to_host(const Electrode* elec, const Electrode* img, size_t m, c
     out.ld = (long long)m;
     out.batch_stride = 0;
     out.sign = 1.0;
-    int err = tags_launch_fill_fp64(d_elec, img ? d_img : d_elec, (int)m, d_coef, 1, out, mode, itype, 1, c->status, st);
+    const SeriesGeo geo = itype == TAGS_INTG_DOUBLE
+                              ? tags_series_geometry(reinterpret_cast<const double*>(elec), (int)m,
+                                                     reinterpret_cast<const double*>(img), img ? (int)m : 0)
+                              : SeriesGeo{};
+    void* series = geo.nbk ? c->scratch(16, tags_series_workspace(geo, 1)) : nullptr;
+    int err = tags_launch_fill_fp64(d_elec, img ? d_img : d_elec, (int)m, d_coef, 1, out, mode, itype, 1, c->status, st,
+                                    &geo, series);
     if (err) return err;
     hl.resize(mm);
     ht.resize(mm);

@@ -730,6 +730,8 @@ extern "C" int tags_voltage_batch(const double* paths, size_t num_paths, const E
         g.len = sqrt(len2);
         g.radius = 0.0;
     }
+    const SeriesGeo geo = tags_series_geometry(segs[0].a, (int)(m + NL), nullptr, 0);
+    void* series = geo.nbk ? c->scratch(16, tags_series_workspace(geo, (int)cs)) : nullptr;
     TAGS_CUDA_OK(cudaMemcpyAsync(d_el, segs.data(), sizeof(Seg) * (m + NL), cudaMemcpyHostToDevice, st));
     TAGS_CUDA_OK(cudaMemcpyAsync(d_paths, paths, sizeof(double) * 6 * NL, cudaMemcpyHostToDevice, st));
     TAGS_CUDA_OK(cudaMemsetAsync(c->status, 0, sizeof(int), st));
@@ -752,7 +754,7 @@ extern "C" int tags_voltage_batch(const double* paths, size_t num_paths, const E
             }
             TAGS_CUDA_OK(cudaMemcpyAsync(d_coef, coef.data(), sizeof(SampleCoef) * ns, cudaMemcpyHostToDevice, st));
             if (int e = tags_launch_path_pairs((const double*)d_el, (int)m, (const double*)(d_el + m), (int)NL, d_coef,
-                                               (int)ns, jj, c->status, st))
+                                               (int)ns, jj, c->status, st, &geo, series))
                 return e;
         }
         TAGS_CUDA_OK(cudaMemcpyAsync(d_u, upts.data() + s0 * 2 * NL * R, sizeof(double2) * 2 * NL * R * ns,

@@ -640,6 +640,7 @@ static int fallback_plain(tags_plan_s* p, int q, cudaStream_t st) {
             return tags_fail(TAGS_E_NOMEM, "device allocation failed (FP64 fallback)");
         }
     }
+    if (int e = tags_plan_series_alloc(p, 1)) return e;
     double2* W = p->d_fbW;
     int* ipiv = p->d_fbpiv;
     TAGS_CUDA_OK(cudaMemsetAsync(W, 0, sizeof(double2) * NN, st));

@@ -171,6 +171,7 @@ static void plan_free(tags_plan_s* p) {
     if (p->d_fbpiv) cudaFree(p->d_fbpiv);
     if (p->d_pot) cudaFree(p->d_pot);
     if (p->d_coef1) cudaFree(p->d_coef1);
+    if (p->d_series) cudaFree(p->d_series);
     if (p->d_iein) cudaFree(p->d_iein);
     if (p->ev0) cudaEventDestroy(p->ev0);
     if (p->ev1) cudaEventDestroy(p->ev1);
@@ -252,6 +253,8 @@ extern "C" int tags_plan_create(tags_plan* out, const Electrode* electrodes, con
     PLAN_CHECK(cudaMalloc(&p->d_x, sizeof(double2) * N * b));
     PLAN_CHECK(cudaMalloc(&p->d_sin, sizeof(double2) * 2 * b));
     if (precision == TAGS_PLAIN_FP64) {
+        err = tags_plan_series_alloc(p, p->batch);
+        if (err) { plan_free(p); return err; }
         PLAN_CHECK(cudaMalloc(&p->d_ipiv, sizeof(int) * N * b));
         PLAN_CHECK(cudaMalloc(&p->d_W, sizeof(double2) * (size_t)NN * b));
         err = tags_lu_prepare();
@@ -270,12 +273,22 @@ extern "C" int tags_plan_destroy(tags_plan plan) {
     return 0;
 }
 
+int tags_plan_series_alloc(tags_plan_s* p, int ns) {
+    if (p->series_ns >= ns) return 0;
+    p->series = tags_series_geometry(p->h_elec.data(), p->m, p->h_img.data(), p->h_img.empty() ? 0 : p->m);
+    if (p->series.nbk == 0) return 0;            // no series for this geometry: the direct rule serves it
+    TAGS_CUDA_OK(cudaMalloc(&p->d_series, tags_series_workspace(p->series, ns)));
+    p->series_ns = ns;
+    return 0;
+}
+
 int tags_plan_fill_fp64(tags_plan_s* p, const SampleCoef* d_coef, int nb, const FillOut& out, cudaStream_t st) {
     if (p->fill_model == TAGS_INTG_MHEM)
         return tags_launch_mhem_fp64(p->d_elec, p->d_img, p->m, p->has_images, p->d_pot, d_coef, nb, out, p->d_status,
                                      st);
     return tags_launch_fill_fp64(p->d_elec, p->d_img, p->m, d_coef, nb, out,
-                                 p->has_images ? TAGS_FILL_BOTH : TAGS_FILL_DIRECT, TAGS_INTG_DOUBLE, 1, p->d_status, st);
+                                 p->has_images ? TAGS_FILL_BOTH : TAGS_FILL_DIRECT, TAGS_INTG_DOUBLE, 1, p->d_status, st,
+                                 &p->series, nb <= p->series_ns ? p->d_series : nullptr);
 }
 
 extern "C" int tags_plan_set_fill(tags_plan plan, int integration_type) {

@@ -13,8 +13,8 @@ struct DeviceCtx {
     int device = -1;
     cudaStream_t stream = nullptr;
     int* status = nullptr;             // device status word(s)
-    void* scratch_ptr[16] = {};
-    size_t scratch_bytes[16] = {};
+    void* scratch_ptr[20] = {};
+    size_t scratch_bytes[20] = {};
     void* scratch(int slot, size_t bytes);
 };
 
@@ -56,6 +56,9 @@ struct tags_plan_s {
     int* d_info = nullptr;          // batch
     int* d_ipiv = nullptr;          // batch x N
     double2* d_W = nullptr;         // plain: batch x N x N
+    SeriesGeo series;               // FP64 fill from per-pass moments (fill.cu) and its workspace,
+    void* d_series = nullptr;       // for series_ns samples (plain: the batch; mixed: 1, with the first FP64 re-solve)
+    int series_ns = 0;
     double2* d_x = nullptr;         // batch x N (solution, FP64)
     // mixed form
     float2* d_Z = nullptr;          // batch x 2 x m x m complex FP32 (ZL, ZT; full symmetric)
@@ -136,3 +139,5 @@ int tags_mixed_fallback_one(tags_plan_s* p, const double2* d_s, const double2* d
 // While-node after the work captured so far on `st` (condition 1 at launch);
 // its body graph is returned for a separate capture.
 int tags_plan_add_while_node(cudaStream_t st, cudaGraphConditionalHandle* cond, cudaGraph_t* body);
+// The FP64 moment series' geometry and workspace for up to ns samples (once per plan).
+int tags_plan_series_alloc(tags_plan_s* p, int ns);

@@ -105,15 +105,26 @@ int tags_launch_fill_mixed(const double* d_elec, const double* d_img, int m, voi
                            int nsamp, float2* d_zl, float2* d_zt, float2* d_zlo, float2* d_ztlo, long long bstride,
                            int has_img, const SpecialEntries& sp, const MomentFill& mf, int* d_status,
                            cudaStream_t st, float* rowpart = nullptr);
+// Geometry of the FP64 moment series over segment records (11 doubles each, on
+// the host): with it and a workspace for the samples of the launch, the
+// INTG_DOUBLE fill and the path integrals take their samples from per-launch
+// moments (fill.cu) instead of a quadrature per sample.
+struct SeriesGeo {
+    double h = 0.0, dmax = 0.0;      // spacing of the expansion centres, bound of |r - R| (m)
+    int nbk = 0;                     // expansion centres (0: no series)
+};
+SeriesGeo tags_series_geometry(const double* h_a, int na, const double* h_b, int nb);
+size_t tags_series_workspace(const SeriesGeo& g, int ns);
 int tags_launch_fill_fp64(const double* d_elec, const double* d_img, int m, const SampleCoef* d_coef,
                           int nsamp, const FillOut& out, int mode, int itype, int tight, int* d_status,
-                          cudaStream_t st);
+                          cudaStream_t st, const SeriesGeo* geo = nullptr, void* series_ws = nullptr);
 
 // Double integrals of e^{-gamma r}/r over [0,1]^2 between each path (a
 // segment record with radius 0) and each electrode, for every sample:
 // jj[(s * npaths + l) * m + e], unscaled (FP64, the plain fill's rule).
 int tags_launch_path_pairs(const double* d_elec, int m, const double* d_paths, int npaths, const SampleCoef* d_coef,
-                           int nsamp, double2* d_jj, int* d_status, cudaStream_t st);
+                           int nsamp, double2* d_jj, int* d_status, cudaStream_t st, const SeriesGeo* geo = nullptr,
+                           void* series_ws = nullptr);
 // Gauss-Legendre nodes (ascending) and weights on [0, 1] (host side).
 void tags_gauss_legendre(int q, double* x, double* w);
 
