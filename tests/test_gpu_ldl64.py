@@ -1,0 +1,87 @@
+"""The plain form's structured FP64 LDL^T (csrc/ldl64.cu) against dense numpy
+solves of the same system, at the edges of its panels (32 columns, the split at
+m and 2m), of its tiles and of its solve paths, and its hand-over to the
+pivoted LU. Tolerance: both sides solve in FP64 with backward errors of a few
+eps N; 1e-10 of the largest unknown covers systems of N = 400 by three orders."""
+import numpy as np
+import pytest
+
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-10
+
+
+def wire(pkg, m):
+    """A bent wire of m segments (m + 1 nodes) below the surface."""
+    rng = np.random.default_rng(m)
+    steps = rng.uniform(0.4, 1.0, (m, 3)) * np.where(np.arange(m)[:, None] % 2 == np.arange(3), 1.0, 0.0)
+    nodes = np.concatenate([[[0.0, 0.0, -0.6]], [0.0, 0.0, -0.6] + np.cumsum(steps, axis=0)])
+    return np.stack([pkg.populate_electrode(nodes[i], nodes[i + 1], 7e-3) for i in range(m)]), nodes
+
+
+def dense_solution(pkg, e, img, nodes, s, kappa, inj):
+    m, n = len(e), len(nodes)
+    N = n + 2 * m
+    zl, zt = np.zeros(m * m, np.complex128), np.zeros(m * m, np.complex128)
+    gamma, ref_t = pkg.medium(s, kappa)
+    assert pkg.calculate_impedances(zl, zt, e, gamma, s, 1.0, kappa) == 0
+    assert pkg.impedances_images(zl, zt, e, img, gamma, s, 1.0, kappa, 1.0, ref_t) == 0
+    wg = np.zeros(N * N, np.complex128)
+    assert pkg.fill_incidence_imm(wg, e, nodes) == 0
+    assert pkg.fill_impedance_imm(wg, zl, zt, m, n) == 0
+    w = np.tril(wg.reshape(N, N).T)
+    b = np.zeros(N, np.complex128)
+    b[inj] = 1.0
+    return np.linalg.solve(w + np.tril(w, -1).T, b)
+
+
+@pytest.mark.parametrize("m", [1, 2, 10, 11, 31, 32, 33, 64, 65, 106, 107, 129])
+@pytest.mark.parametrize("graphs", [True, False])
+def test_plain_plan_matches_dense_solve(gpu_pkg, m, graphs):
+    """One-CTA solves up to N = 320 (m = 106), panel launches above."""
+    pkg = gpu_pkg
+    e, nodes = wire(pkg, m)
+    img = pkg.images(e)
+    s = 8e4 + 2j * np.pi * np.array([1e3, 1e6])
+    kappa = 0.01 + s * 12 * pkg.EPS0
+    sol, info, _ = pkg.hem_sweep(e, img, nodes, s, kappa, inj_node=m // 2, graphs=graphs)
+    assert not info.any()
+    for k in range(2):
+        assert rel_err(sol[k], dense_solution(pkg, e, img, nodes, s[k], kappa[k], m // 2)) < TOL
+
+
+@pytest.mark.parametrize("ns", [1, 127, 128, 131])
+def test_plain_plan_batches_agree(gpu_pkg, ns):
+    """The panel launches' solve (up to 127 samples) and the one-CTA solve
+    (from 128) of N = 358, and both panel CTA sizes, against single samples."""
+    pkg = gpu_pkg
+    e, nodes = wire(pkg, 119)
+    img = pkg.images(e)
+    s = 8e4 + 2j * np.pi * np.linspace(1e4, 5e6, ns)
+    kappa = 0.002 + s * 8 * pkg.EPS0
+    sol, info, _ = pkg.hem_sweep(e, img, nodes, s, kappa, max_batch=ns)
+    assert not info.any()
+    for k in {0, ns // 2, ns - 1}:
+        alone, _, _ = pkg.hem_sweep(e, img, nodes, s[k:k + 1], kappa[k:k + 1])
+        assert rel_err(sol[k], alone[0]) < TOL
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_samples_without_static_pivots_go_to_the_pivoted_lu(gpu_pkg, graphs):
+    """s = 0 makes ZL zero: the static order meets zero pivots, the system of a
+    tree of segments is still regular."""
+    pkg = gpu_pkg
+    e, nodes = wire(pkg, 40)
+    img = pkg.images(e)
+    s = np.array([0.0, 8e4 + 1e6j, 0.0])
+    kappa = np.array([0.01 + 0j, 0.01 + 1e-4j, 0.02 + 0j])
+    sol, info, _ = pkg.hem_sweep(e, img, nodes, s, kappa, inj_node=3, graphs=graphs)
+    assert not info.any()
+    for k in range(3):
+        assert rel_err(sol[k], dense_solution(pkg, e, img, nodes, s[k], kappa[k], 3)) < TOL
+    jobs = [{"electrodes": e, "images": img, "nodes": nodes, "s": s, "kappa": kappa, "inj_node": 3}]
+    (got, binfo), = pkg.solve_batch(jobs, precision=pkg.PLAIN_FP64)
+    assert not binfo.any()
+    assert rel_err(got, sol) < TOL

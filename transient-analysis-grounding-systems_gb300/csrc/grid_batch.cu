@@ -86,7 +86,7 @@ static void batch_free(tags_batch_s* b) {
 // creation uses to size its batch).
 static double bytes_per_sample(int m, int n, int precision) {
     const double N = (double)n + 2.0 * m, NN = N * N;
-    return precision == TAGS_PLAIN_FP64 ? 16.0 * NN + 40.0 * N
+    return precision == TAGS_PLAIN_FP64 ? 16.0 * NN + 40.0 * N + (double)tags_ldl64_workspace((int)N, 1)
                                         : 8.0 * NN + 32.0 * (double)m * m + 80.0 * N +
                                               (double)tags_ldl_tc_workspace((int)N, 1);
 }
@@ -376,6 +376,21 @@ extern "C" int tags_batch_run(tags_batch batch, const tags_grid_job* jobs, size_
                                                     g.d_sol + (size_t)k * g.N, g.d_info + k, p->stream);
                     if (e) return e;
                 }
+            }
+            TAGS_CUDA_OK(cudaStreamSynchronize(p->stream));
+        } else if (!gst) {
+            // plain form: samples marked for the pivoted LU
+            std::vector<int> si(g.ns);
+            TAGS_CUDA_OK(cudaMemcpy(si.data(), g.d_info, sizeof(int) * g.ns, cudaMemcpyDeviceToHost));
+            for (int k = 0; k < g.ns; ++k) {
+                if (si[k] != TAGS_INFO_RESOLVE) continue;
+                int e = tags_plan_coef(p, g.d_s + k, g.d_k + k, b->mur, 1, p->stream);
+                if (!e) e = tags_plan_rhs(p, p->d_x, g.has_ie ? g.d_ie + (size_t)k * g.n : nullptr, (int)g.inj, 1, p->stream);
+                if (!e) e = tags_plan_lu_one(p, 0, p->d_W, p->d_ipiv, p->d_x, p->d_info, p->stream);
+                if (e) return e;
+                TAGS_CUDA_OK(cudaMemcpyAsync(g.d_sol + (size_t)k * g.N, p->d_x, sizeof(double2) * g.N,
+                                             cudaMemcpyDeviceToDevice, p->stream));
+                TAGS_CUDA_OK(cudaMemcpyAsync(g.d_info + k, p->d_info, sizeof(int), cudaMemcpyDeviceToDevice, p->stream));
             }
             TAGS_CUDA_OK(cudaStreamSynchronize(p->stream));
         }

@@ -1,0 +1,758 @@
+// FP64 solve of the immittance system in its structure (plain form).
+//
+// Same system as the reference's solve_immittance (src/linalg.c:112-139), in
+// the static order [I_L, I_T, U]:
+//     W = [ -ZL   0    A ]
+//         [  0   -ZT   B ]      b = [0; 0; I_E]
+//         [ A^T  B^T   0 ]
+// The elimination meets the impedance blocks first and the node block last,
+// so it needs no pivot search, and the coupling of ZL and ZT stays zero: an
+// LDL^T takes 2 (4/3 m^3 + 4 m^2 n + 4 m n^2) + 4/3 n^3 real flops where the
+// LU of the full matrix takes 8/3 N^3 (66.6 against 249 GFLOP at m = 1560,
+// n = 1417). FP64 runs at two fused multiply-adds per clock and SM here, so
+// the flops are the time. What the missing pivot search may cost in accuracy
+// is recovered by FP64 refinement against the untouched impedance blocks; a
+// sample whose corrections do not shrink to 1e-8 |x| (the next one would be
+// below FP64 rounding) is handed to the pivoted LU (lu.cu) by its caller.
+// Measured against that LU on GB300: 2 samples at m = 1560 714 -> 190 ms, 256
+// samples at m = 100 24.3 -> 8.4 ms, 100 samples at m = 10 0.66 -> 0.58 ms.
+//
+// Layout: column-major N x N per sample, leading dimension ld. Lower triangle:
+// the matrix, then L; the strict upper triangle keeps U = D L^T of the panels
+// (the update's right operand) and, in the ZL/ZT coupling blocks that the
+// elimination never touches, the full symmetric ZL (rows 0..m, columns m..2m)
+// and ZT (rows m..2m, columns 0..m) that the residual reads. Panels are 32
+// columns wide and never straddle m or 2m, so a ZL panel skips the ZT rows
+// exactly. The panels' factored diagonal blocks live in the workspace (every
+// CTA of a panel launch factors the block itself, which saves a launch per
+// panel), then their inverses, so that a solve's diagonal step is a product.
+#include <mutex>
+
+#include "tags_common.cuh"
+#include "tags_internal.h"
+#include "../../include/tags_gpu.h"
+#include "plan.h"
+
+namespace {
+
+constexpr int PB = 32;                    // panel width
+
+// Columns [j0, j0 + jb) of panel p; the rows below it are base + v, v < cnt,
+// plus `skip` from `lim` on (a ZL panel has no ZT rows).
+struct Panel {
+    int j0, jb, base, lim, skip, cnt;
+    TAGS_HD int row(int v) const {
+        const int r = base + v;
+        return r >= lim ? r + skip : r;
+    }
+};
+
+TAGS_HD int panel_count(int N, int m) {
+    return m == 0 ? (N + PB - 1) / PB : 2 * ((m + PB - 1) / PB) + (N - 2 * m + PB - 1) / PB;
+}
+
+TAGS_HD Panel panel_at(int p, int N, int m) {
+    Panel q;
+    const int pm = (m + PB - 1) / PB;
+    int end;
+    if (m == 0) {
+        q.j0 = PB * p;
+        end = N;
+    } else if (p < pm) {
+        q.j0 = PB * p;
+        end = m;
+    } else if (p < 2 * pm) {
+        q.j0 = m + PB * (p - pm);
+        end = 2 * m;
+    } else {
+        q.j0 = 2 * m + PB * (p - 2 * pm);
+        end = N;
+    }
+    q.jb = end - q.j0 < PB ? end - q.j0 : PB;
+    q.base = q.j0 + q.jb;
+    const bool zl = m > 0 && q.j0 < m;
+    q.lim = zl ? m : N;
+    q.skip = zl ? m : 0;
+    q.cnt = N - q.base - q.skip;
+    return q;
+}
+
+TAGS_D double2 crecip(double2 d) {
+    const double s = 1.0 / (d.x * d.x + d.y * d.y);      // out of range: not finite, the sample goes to the LU
+    return make_double2(d.x * s, -d.y * s);
+}
+
+// Diagonal block and rows of one panel: L21 = A21 L11^-T D^-1 (stored in
+// place) and U12 = D L21^T (stored in the upper triangle). One thread per row;
+// every CTA factors the 32 x 32 block in shared memory first, CTA 0 also
+// stores it (L11, 1/D on the diagonal) for the solves. Bound by the FP64 pipe:
+// 1984 multiply-adds per row and ~20,000 SM cycles per block; CTAs of 64 rows
+// while that leaves SMs idle, else of 128 (half the repeated block work).
+__global__ void __launch_bounds__(128) k_ldl64_panel(double2* __restrict__ A0, long long ld, long long stride,
+                                                     Panel q, int p, double2* __restrict__ ws0, long long wstride) {
+    double2* A = A0 + stride * blockIdx.y;
+    __shared__ double2 sL[PB][PB + 1];
+    __shared__ double2 sdi[PB], scol[PB];
+    const int tid = threadIdx.x;
+    for (int t = tid; t < PB * PB; t += blockDim.x) {
+        const int r = t % PB, c = t / PB;
+        double2 v = cz(r == c ? 1.0 : 0.0, 0.0);          // a short panel is padded with the identity
+        if (r < q.jb && c <= r) v = A[(q.j0 + r) + ld * (q.j0 + c)];
+        sL[r][c] = v;
+    }
+    __syncthreads();
+    for (int k = 0; k < q.jb; ++k) {
+        if (tid < 32) {
+            const double2 di = crecip(sL[k][k]);
+            if (tid == 0) sdi[k] = di;
+            scol[tid] = cmul(sL[tid][k], di);             // rows above k are not used
+        }
+        __syncthreads();
+        const int w = q.jb - k - 1;
+        for (int t = tid; t < w * w; t += blockDim.x) {
+            const int r = k + 1 + t % w, c = k + 1 + t / w;
+            if (c <= r) sL[r][c] = cfma(cneg(scol[r]), sL[c][k], sL[r][c]);
+        }
+        __syncthreads();
+    }
+    for (int k = q.jb + tid; k < PB; k += blockDim.x) sdi[k] = cz(1.0, 0.0);
+    __syncthreads();
+    for (int t = tid; t < PB * PB; t += blockDim.x) {     // unscaled columns -> L11
+        const int r = t % PB, c = t / PB;
+        if (r > c && r < q.jb) sL[r][c] = cmul(sL[r][c], sdi[c]);
+    }
+    __syncthreads();
+    if (blockIdx.x == 0) {
+        double2* ws = ws0 + wstride * blockIdx.y + (long long)p * PB * PB;
+        for (int t = tid; t < PB * PB; t += blockDim.x) {
+            const int r = t % PB, c = t / PB;
+            ws[c * PB + r] = r > c ? sL[r][c] : r == c ? sdi[c] : cz(0.0, 0.0);
+        }
+    }
+    const int v = blockIdx.x * blockDim.x + tid;
+    if (v >= q.cnt) return;
+    const int row = q.row(v);
+    double2 w[PB];
+#pragma unroll
+    for (int c = 0; c < PB; ++c) w[c] = c < q.jb ? A[row + ld * (q.j0 + c)] : cz(0.0, 0.0);
+#pragma unroll
+    for (int c = 1; c < PB; ++c)
+#pragma unroll
+        for (int k = 0; k < c; ++k) w[c] = cfma(cneg(w[k]), sL[c][k], w[c]);
+#pragma unroll
+    for (int c = 0; c < PB; ++c)
+        if (c < q.jb) {
+            A[row + ld * (q.j0 + c)] = cmul(w[c], sdi[c]);
+            A[(q.j0 + c) + ld * row] = w[c];
+        }
+}
+
+// Trailing update C -= L21 U12 over the lower triangle of the rows below the
+// panel, TL x TL tiles of 4 x 4 values per thread. FP64-bound: a tile of 64
+// takes 262,144 SM cycles of multiply-adds against 131 KB of C, so one panel
+// (K = 32) per update is enough, and the tile size only sets the work wasted
+// on the diagonal and the edge.
+template <int TL>
+__global__ void __launch_bounds__(TL * TL / 16) k_ldl64_update(double2* __restrict__ A0, long long ld,
+                                                               long long stride, Panel q) {
+    double2* A = A0 + stride * blockIdx.y;
+    constexpr int TH = TL / 4, NT = TH * TH;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2* sA = reinterpret_cast<double2*>(smem_raw);    // [PB][TL]
+    double2* sB = sA + PB * TL;                            // [PB][TL]
+    const int t = blockIdx.x;
+    int ty = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
+    while (ty > 0 && ty * (ty + 1) / 2 > t) --ty;
+    while ((ty + 1) * (ty + 2) / 2 <= t) ++ty;
+    const int r0 = ty * TL, c0 = (t - ty * (ty + 1) / 2) * TL;
+    for (int s = threadIdx.x; s < PB * TL; s += NT) {
+        const int r = s % TL, k = s / TL;
+        sA[k * TL + r] = (k < q.jb && r0 + r < q.cnt) ? A[q.row(r0 + r) + ld * (q.j0 + k)] : cz(0.0, 0.0);
+        const int kk = s % PB, c = s / PB;
+        sB[kk * TL + c] = (kk < q.jb && c0 + c < q.cnt) ? A[(q.j0 + kk) + ld * q.row(c0 + c)] : cz(0.0, 0.0);
+    }
+    __syncthreads();
+    const int tx = threadIdx.x % TH, tyy = threadIdx.x / TH;
+    double2 acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[a][b] = cz(0.0, 0.0);
+    for (int k = 0; k < q.jb; ++k) {
+        double2 av[4], bv[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) av[a] = sA[k * TL + tx + TH * a];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) bv[b] = sB[k * TL + tyy + TH * b];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) acc[a][b] = cfma(av[a], bv[b], acc[a][b]);
+    }
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        const int gc = c0 + tyy + TH * b;
+        if (gc >= q.cnt) continue;
+        const long long col = ld * q.row(gc);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const int gr = r0 + tx + TH * a;
+            if (gr < q.cnt && gr >= gc) {
+                const long long idx = q.row(gr) + col;
+                A[idx] = csub(A[idx], acc[a][b]);
+            }
+        }
+    }
+}
+
+// Inverses of the panels' unit lower blocks, in place (1/D stays on the
+// diagonal): a warp per panel and sample, lane = column of the inverse.
+__global__ void __launch_bounds__(32) k_ldl64_inv(double2* __restrict__ ws0, long long wstride) {
+    double2* ws = ws0 + wstride * blockIdx.y + (long long)blockIdx.x * PB * PB;
+    __shared__ double2 L[PB][PB + 1];
+    const int c = threadIdx.x;
+    for (int k = 0; k < PB; ++k) L[c][k] = ws[k * PB + c];
+    __syncwarp();
+    double2 x[PB];
+#pragma unroll
+    for (int r = 0; r < PB; ++r) {
+        double2 v = cz(r == c ? 1.0 : 0.0, 0.0);
+#pragma unroll
+        for (int k = 0; k < r; ++k) v = cfma(cneg(L[r][k]), x[k], v);   // x[k] = 0 for k < c
+        x[r] = v;
+    }
+#pragma unroll
+    for (int r = 0; r < PB; ++r)
+        if (r > c) ws[c * PB + r] = x[r];
+}
+
+// y = L11^-1 x (upper = 0) or L11^-T x (upper = 1) for a panel's 32 values by
+// the block's first 32 threads; raw and y in shared memory.
+TAGS_D void block_apply(const double2* __restrict__ ws, const double2* raw, double2* y, int upper) {
+    const int r = threadIdx.x;
+    if (r >= PB) return;
+    double2 a = raw[r];
+    if (!upper) {
+        for (int k = 0; k < r; ++k) a = cfma(ws[k * PB + r], raw[k], a);
+    } else {
+        for (int k = r + 1; k < PB; ++k) a = cfma(ws[r * PB + k], raw[k], a);
+    }
+    y[r] = a;
+}
+
+// One panel of the forward sweep: y = L11^-1 x_p (to Z), then x_r -= L_rp y
+// below it. 64 rows per CTA; x_p itself is left, so the CTAs agree on it.
+__global__ void __launch_bounds__(64) k_ldl64_fwd(const double2* __restrict__ A0, long long ld, long long stride,
+                                                  Panel q, int p, const double2* __restrict__ ws0, long long wstride,
+                                                  double2* __restrict__ X0, double2* __restrict__ Z0, int N,
+                                                  const int* __restrict__ active) {
+    const int b = blockIdx.y;
+    if (!active[b]) return;
+    const double2* A = A0 + stride * b;
+    double2* X = X0 + (long long)N * b;
+    __shared__ double2 raw[PB], y[PB];
+    if (threadIdx.x < PB) raw[threadIdx.x] = (int)threadIdx.x < q.jb ? X[q.j0 + threadIdx.x] : cz(0.0, 0.0);
+    __syncthreads();
+    block_apply(ws0 + wstride * b + (long long)p * PB * PB, raw, y, 0);
+    __syncthreads();
+    if (blockIdx.x == 0 && (int)threadIdx.x < q.jb) Z0[(long long)N * b + q.j0 + threadIdx.x] = y[threadIdx.x];
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= q.cnt) return;
+    const int row = q.row(v);
+    double2 acc = cz(0.0, 0.0);
+#pragma unroll 8
+    for (int c = 0; c < q.jb; ++c) acc = cfma(A[row + ld * (q.j0 + c)], y[c], acc);
+    X[row] = csub(X[row], acc);
+}
+
+// One panel of the backward sweep on T (which starts as D^-1 z): y = L11^-T
+// T_p (to S), then T_c -= L_pc^T y for the columns c0 .. j0 left of it.
+__global__ void __launch_bounds__(64) k_ldl64_bwd(const double2* __restrict__ A0, long long ld, long long stride,
+                                                  Panel q, int p, int c0, const double2* __restrict__ ws0,
+                                                  long long wstride, double2* __restrict__ T0,
+                                                  double2* __restrict__ S0, int N, const int* __restrict__ active) {
+    const int b = blockIdx.y;
+    if (!active[b]) return;
+    const double2* A = A0 + stride * b;
+    double2* T = T0 + (long long)N * b;
+    __shared__ double2 raw[PB], y[PB];
+    if (threadIdx.x < PB) raw[threadIdx.x] = (int)threadIdx.x < q.jb ? T[q.j0 + threadIdx.x] : cz(0.0, 0.0);
+    __syncthreads();
+    block_apply(ws0 + wstride * b + (long long)p * PB * PB, raw, y, 1);
+    __syncthreads();
+    if (blockIdx.x == 0 && (int)threadIdx.x < q.jb) S0[(long long)N * b + q.j0 + threadIdx.x] = y[threadIdx.x];
+    const int c = c0 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= q.j0) return;
+    double2 acc = cz(0.0, 0.0);
+#pragma unroll 8
+    for (int r = 0; r < q.jb; ++r) acc = cfma(A[(q.j0 + r) + ld * c], y[r], acc);
+    T[c] = csub(T[c], acc);
+}
+
+// T = D^-1 z (in place).
+__global__ void k_ldl64_dscale(double2* __restrict__ Z0, int N, int m, const double2* __restrict__ ws0,
+                               long long wstride, const int* __restrict__ active) {
+    const int b = blockIdx.y;
+    if (!active[b]) return;
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= N) return;
+    const int pm = (m + PB - 1) / PB;
+    const int blk = m == 0 || j < m ? 0 : j < 2 * m ? 1 : 2, o = j - blk * m;
+    const double2* ws = ws0 + wstride * b + (long long)(blk * pm + o / PB) * PB * PB;
+    double2* z = Z0 + (long long)N * b + j;
+    *z = cmul(*z, ws[(o % PB) * (PB + 1)]);
+}
+
+// Both sweeps of one sample by one CTA, the vector in shared memory: for
+// systems whose sweeps are shorter than the panel-by-panel launches (N up to
+// ~300: 81,000 SM cycles per sweep at N = 285), or batches that fill the SMs.
+constexpr int SOLVE_THREADS = 256;
+__global__ void __launch_bounds__(SOLVE_THREADS) k_ldl64_solve_cta(
+    const double2* __restrict__ A0, long long ld, long long stride, int N, int m, const double2* __restrict__ ws0,
+    long long wstride, const double2* __restrict__ X0, double2* __restrict__ S0, int p0,
+    const int* __restrict__ active) {
+    const int b = blockIdx.x;
+    if (!active[b]) return;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2* xs = reinterpret_cast<double2*>(smem_raw);     // N
+    __shared__ double2 raw[PB], y[PB];
+    const double2* A = A0 + stride * b;
+    const double2* ws = ws0 + wstride * b;
+    const int P = panel_count(N, m);
+    for (int j = threadIdx.x; j < N; j += blockDim.x) xs[j] = X0[(long long)N * b + j];
+    __syncthreads();
+    for (int p = p0; p < P; ++p) {                           // the right-hand side is zero above panel p0
+        const Panel q = panel_at(p, N, m);
+        if (threadIdx.x < PB) raw[threadIdx.x] = (int)threadIdx.x < q.jb ? xs[q.j0 + threadIdx.x] : cz(0.0, 0.0);
+        __syncthreads();
+        block_apply(ws + (long long)p * PB * PB, raw, y, 0);
+        __syncthreads();
+        if ((int)threadIdx.x < q.jb) xs[q.j0 + threadIdx.x] = cmul(y[threadIdx.x],
+                                                                   ws[(long long)p * PB * PB + threadIdx.x * (PB + 1)]);
+        for (int v = threadIdx.x; v < q.cnt; v += blockDim.x) {
+            const int row = q.row(v);
+            double2 acc = cz(0.0, 0.0);
+#pragma unroll 8
+            for (int c = 0; c < q.jb; ++c) acc = cfma(A[row + ld * (q.j0 + c)], y[c], acc);
+            xs[row] = csub(xs[row], acc);
+        }
+        __syncthreads();
+    }
+    for (int p = P - 1; p >= 0; --p) {
+        const Panel q = panel_at(p, N, m);
+        const int c0 = m > 0 && q.j0 >= m && q.j0 < 2 * m ? m : 0;
+        if (threadIdx.x < PB) raw[threadIdx.x] = (int)threadIdx.x < q.jb ? xs[q.j0 + threadIdx.x] : cz(0.0, 0.0);
+        __syncthreads();
+        block_apply(ws + (long long)p * PB * PB, raw, y, 1);
+        __syncthreads();
+        if ((int)threadIdx.x < q.jb) xs[q.j0 + threadIdx.x] = y[threadIdx.x];
+        for (int c = c0 + threadIdx.x; c < q.j0; c += blockDim.x) {
+            double2 acc = cz(0.0, 0.0);
+#pragma unroll 8
+            for (int r = 0; r < q.jb; ++r) acc = cfma(A[(q.j0 + r) + ld * c], y[r], acc);
+            xs[c] = csub(xs[c], acc);
+        }
+        __syncthreads();
+    }
+    for (int j = threadIdx.x; j < N; j += blockDim.x) S0[(long long)N * b + j] = xs[j];
+}
+
+// Reordered index -> index of the original order [U, I_L, I_T] (m = 0: equal).
+TAGS_D int orig_index(int ip, int m, int n) { return ip < 2 * m ? n + ip : ip - 2 * m; }
+
+// Start of a solve: b and r = b in the static order, x = 0, every sample active.
+__global__ void k_ldl64_start(const double2* __restrict__ rhs, long long rstride, int m, int n,
+                              double2* __restrict__ B0, double2* __restrict__ R0, double2* __restrict__ X0,
+                              int* __restrict__ active, int* __restrict__ conv) {
+    const int N = n + 2 * m, b = blockIdx.y;
+    const int ip = blockIdx.x * blockDim.x + threadIdx.x;
+    if (ip == 0) {
+        active[b] = 1;
+        conv[b] = 0;
+    }
+    if (ip >= N) return;
+    const double2 v = rhs[rstride * b + orig_index(ip, m, n)];
+    const long long o = (long long)N * b + ip;
+    B0[o] = v;
+    R0[o] = v;
+    X0[o] = cz(0.0, 0.0);
+}
+
+// x += dx and the stopping rule, one CTA per sample. Step 0's correction is x
+// itself. Later ones: dx <= 1e-8 |x| means a contraction below 1e-8, so the
+// next correction would be under FP64 rounding: done. A correction that did
+// not halve, or the last step's, leaves the sample to the pivoted LU.
+__global__ void __launch_bounds__(256) k_ldl64_apply(const double2* __restrict__ S0, double2* __restrict__ X0, int N,
+                                                     int step, int last, int* __restrict__ active,
+                                                     int* __restrict__ conv, double* __restrict__ prev) {
+    const int b = blockIdx.x;
+    if (!active[b]) return;
+    __shared__ double smx[2][8];
+    double dn = 0.0, xn = 0.0;
+    bool bad = false;
+    for (int j = threadIdx.x; j < N; j += blockDim.x) {
+        const long long o = (long long)N * b + j;
+        const double2 d = S0[o], x = cadd(X0[o], d);
+        X0[o] = x;
+        const double a = cabs1(d), c = cabs1(x);
+        bad = bad || !isfinite(a) || !isfinite(c);
+        dn = fmax(dn, a);
+        xn = fmax(xn, c);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        dn = fmax(dn, __shfl_xor_sync(0xffffffffu, dn, o));
+        xn = fmax(xn, __shfl_xor_sync(0xffffffffu, xn, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        smx[0][threadIdx.x >> 5] = dn;
+        smx[1][threadIdx.x >> 5] = xn;
+    }
+    const int anybad = __syncthreads_or(bad);
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < 8; ++w) {
+        dn = fmax(dn, smx[0][w]);
+        xn = fmax(xn, smx[1][w]);
+    }
+    if (anybad) {
+        active[b] = 0;
+        return;
+    }
+    if (step > 0) {
+        if (dn <= 1e-8 * xn) {
+            conv[b] = 1;
+            active[b] = 0;
+        } else if (last || dn > 0.5 * prev[b]) {
+            active[b] = 0;
+        }
+    }
+    prev[b] = dn;
+}
+
+// Solutions to the original order; info 0, or the marker of a sample that
+// needs the pivoted LU.
+__global__ void k_ldl64_out(const double2* __restrict__ X0, int m, int n, const int* __restrict__ conv,
+                            double2* __restrict__ out, long long ostride, int* __restrict__ info) {
+    const int N = n + 2 * m, b = blockIdx.y;
+    const int ip = blockIdx.x * blockDim.x + threadIdx.x;
+    if (ip == 0) info[b] = conv[b] ? 0 : TAGS_INFO_RESOLVE;
+    if (ip >= N) return;
+    out[ostride * b + orig_index(ip, m, n)] = X0[(long long)N * b + ip];
+}
+
+// The saved right-hand side of one sample back to the original order.
+__global__ void k_ldl64_rhs_back(const double2* __restrict__ B, int m, int n, double2* __restrict__ out) {
+    const int ip = blockIdx.x * blockDim.x + threadIdx.x;
+    if (ip < n + 2 * m) out[orig_index(ip, m, n)] = B[ip];
+}
+
+// ---- the plan's system: impedance blocks in the coupling blocks, sparse incidence
+
+// Lower triangle from the stored ZL, ZT (negated) and the incidence; a CTA
+// writes one column of one sample.
+__global__ void __launch_bounds__(128) k_ldl64_build(double2* __restrict__ W0, long long ld, long long stride,
+                                                     const Incidence inc, int m, int n) {
+    double2* W = W0 + stride * blockIdx.y;
+    const int N = n + 2 * m, j = blockIdx.x;
+    double2* col = W + ld * j;
+    const double2 zero = cz(0.0, 0.0);
+    if (j >= 2 * m) {
+        for (int i = j + (int)threadIdx.x; i < N; i += blockDim.x) col[i] = zero;
+        return;
+    }
+    const int bj = j < m ? 0 : 1, e = j - bj * m;
+    // the stored block's column e, indexed by the matrix row: ZL (i, m + e), ZT (i, e)
+    const double2* z = W + ld * (bj == 0 ? m + e : e);
+    for (int i = j + (int)threadIdx.x; i < (bj + 1) * m; i += blockDim.x) col[i] = cneg(z[i]);
+    for (int i = 2 * m + (int)threadIdx.x; i < N; i += blockDim.x) col[i] = zero;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int q = inc.seg_ptr[e]; q < inc.seg_ptr[e + 1]; ++q)
+            col[2 * m + inc.seg_node[q]] = cz(bj == 0 ? (double)inc.seg_a[q] : 0.5, 0.0);
+}
+
+// r = b - W x: impedance rows (blockIdx.y 0: I_L, 1: I_T), a thread per row
+// over the stored blocks' columns; FP64-bound (4 multiply-adds per 16 bytes).
+__global__ void __launch_bounds__(64) k_ldl64_resid_z(const double2* __restrict__ W0, long long ld, long long stride,
+                                                      const Incidence inc, int m, int n,
+                                                      const double2* __restrict__ B0, const double2* __restrict__ X0,
+                                                      double2* __restrict__ R0, const int* __restrict__ active) {
+    const int b = blockIdx.z, blk = blockIdx.y;
+    if (!active[b]) return;
+    __shared__ double2 xs[64];
+    const int N = n + 2 * m, k = blockIdx.x * blockDim.x + threadIdx.x;
+    const double2* X = X0 + (long long)N * b;
+    const double2* z = W0 + stride * b + (blk == 0 ? ld * m : (long long)m);
+    double2 acc = cz(0.0, 0.0);
+    for (int j0 = 0; j0 < m; j0 += 64) {
+        const int nj = min(64, m - j0);
+        __syncthreads();
+        if ((int)threadIdx.x < nj) xs[threadIdx.x] = X[blk * m + j0 + threadIdx.x];
+        __syncthreads();
+        if (k < m) {
+#pragma unroll 8
+            for (int j = 0; j < nj; ++j) acc = cfma(z[k + ld * (j0 + j)], xs[j], acc);
+        }
+    }
+    if (k >= m) return;
+    double2 u = cz(0.0, 0.0);
+    for (int q = inc.seg_ptr[k]; q < inc.seg_ptr[k + 1]; ++q)
+        u = cadd(u, cscale(X[2 * m + inc.seg_node[q]], blk == 0 ? (double)inc.seg_a[q] : 0.5));
+    const long long o = (long long)N * b + blk * m + k;
+    R0[o] = cadd(csub(B0[o], u), acc);
+}
+
+__global__ void k_ldl64_resid_nodes(const Incidence inc, int m, int n, const double2* __restrict__ B0,
+                                    const double2* __restrict__ X0, double2* __restrict__ R0,
+                                    const int* __restrict__ active) {
+    const int b = blockIdx.y;
+    if (!active[b]) return;
+    const int N = n + 2 * m, row = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row >= n) return;
+    const double2* X = X0 + (long long)N * b;
+    double2 acc = cz(0.0, 0.0);
+    for (int q = inc.node_ptr[row]; q < inc.node_ptr[row + 1]; ++q) {
+        const int e = inc.node_seg[q];
+        const double a = inc.node_a[q];
+        const double2 il = X[e], it = X[m + e];
+        acc.x += a * il.x + 0.5 * it.x;
+        acc.y += a * il.y + 0.5 * it.y;
+    }
+    const long long o = (long long)N * b + 2 * m + row;
+    R0[o] = csub(B0[o], acc);
+}
+
+// ---- a caller's symmetric matrix (full, original order)
+
+// Lower triangle in the static order; *coupled is raised by a nonzero entry
+// of the ZL/ZT coupling block.
+__global__ void k_ldl64_permute(const double2* __restrict__ W, double2* __restrict__ A, int m, int n,
+                                int* __restrict__ coupled) {
+    const int N = n + 2 * m, j = blockIdx.x;
+    const int i = blockIdx.y * blockDim.x + threadIdx.x;
+    if (i >= N || i < j) return;
+    const double2 v = W[orig_index(i, m, n) + (long long)N * orig_index(j, m, n)];
+    A[i + (long long)N * j] = v;
+    if (j < m && i >= m && i < 2 * m && (v.x != 0.0 || v.y != 0.0)) *coupled = 1;
+}
+
+// r = b - W x for the full symmetric W in the original order, x and r in the
+// static order; a thread per row.
+__global__ void __launch_bounds__(64) k_ldl64_resid_full(const double2* __restrict__ W, int m, int n,
+                                                         const double2* __restrict__ B,
+                                                         const double2* __restrict__ X, double2* __restrict__ R,
+                                                         const int* __restrict__ active) {
+    if (!active[0]) return;
+    __shared__ double2 xs[64];
+    const int N = n + 2 * m, ip = blockIdx.x * blockDim.x + threadIdx.x;
+    const int row = ip < N ? orig_index(ip, m, n) : 0;
+    double2 acc = cz(0.0, 0.0);
+    for (int j0 = 0; j0 < N; j0 += 64) {
+        const int nj = min(64, N - j0);
+        __syncthreads();
+        if ((int)threadIdx.x < nj) xs[threadIdx.x] = X[j0 + threadIdx.x];
+        __syncthreads();
+        if (ip < N) {
+#pragma unroll 8
+            for (int j = 0; j < nj; ++j)
+                acc = cfma(W[row + (long long)N * orig_index(j0 + j, m, n)], xs[j], acc);
+        }
+    }
+    if (ip < N) R[ip] = csub(B[ip], acc);
+}
+
+struct Ws {
+    double2 *linv, *b, *x, *r, *z;
+    double* prev;
+    int *active, *conv;
+    long long wstride;      // linv values per sample
+};
+
+Ws carve(void* p, int N, int batch) {
+    Ws w;
+    // the most panels any split of N into blocks can have
+    w.wstride = (long long)((N + PB - 1) / PB + 2) * PB * PB;
+    w.linv = reinterpret_cast<double2*>(p);
+    w.b = w.linv + w.wstride * batch;
+    w.x = w.b + (long long)N * batch;
+    w.r = w.x + (long long)N * batch;
+    w.z = w.r + (long long)N * batch;
+    w.prev = reinterpret_cast<double*>(w.z + (long long)N * batch);
+    w.active = reinterpret_cast<int*>(w.prev + batch);
+    w.conv = w.active + batch;
+    return w;
+}
+
+constexpr int SOLVE_N_MAX = 14000;        // 16 B per unknown in the one-CTA solve's shared memory
+
+int factor(double2* A, int N, long long ld, long long stride, int nb, int m, const Ws& w, cudaStream_t st) {
+    const int P = panel_count(N, m);
+    for (int p = 0; p < P; ++p) {
+        const Panel q = panel_at(p, N, m);
+        const int rows = (long long)nb * ((q.cnt + 63) / 64) > 608 ? 128 : 64;     // four CTAs of 64 per SM
+        const int ctas = q.cnt > 0 ? (q.cnt + rows - 1) / rows : 1;
+        int pf = tags_prof_begin(TAGS_PROF_LU64_OTHER, st);
+        k_ldl64_panel<<<dim3(ctas, nb), rows, 0, st>>>(A, ld, stride, q, p, w.linv, w.wstride);
+        tags_prof_end(TAGS_PROF_LU64_OTHER, pf, st, 0.0, 0.0);
+        tags_note_launch();
+        if (q.cnt <= 0) continue;
+        // tiles of 64, or of 32 where the larger ones waste more on the
+        // diagonal and the edge (under ten tile rows) or leave SMs idle
+        pf = tags_prof_begin(TAGS_PROF_LU64_GEMM, st);
+        const long long t64 = (q.cnt + 63) / 64, t32 = (q.cnt + 31) / 32;
+        if (t64 >= 10 && t64 * (t64 + 1) / 2 * nb >= 608)
+            k_ldl64_update<64><<<dim3((unsigned)(t64 * (t64 + 1) / 2), nb), 256, 2 * PB * 64 * sizeof(double2), st>>>(
+                A, ld, stride, q);
+        else
+            k_ldl64_update<32><<<dim3((unsigned)(t32 * (t32 + 1) / 2), nb), 64, 2 * PB * 32 * sizeof(double2), st>>>(
+                A, ld, stride, q);
+        tags_prof_end(TAGS_PROF_LU64_GEMM, pf, st, 4.0 * q.cnt * (q.cnt + 1.0) * q.jb * nb,
+                      (16.0 * q.cnt * (q.cnt + 1.0) + 32.0 * q.cnt * q.jb) * nb);
+        tags_note_launch();
+    }
+    k_ldl64_inv<<<dim3(P, nb), 32, 0, st>>>(w.linv, w.wstride);
+    tags_note_launch();
+    TAGS_CUDA_OK(cudaGetLastError());
+    return 0;
+}
+
+// w.z = W^-1 w.r for the active samples (w.r is used up); the right-hand side
+// is zero above row `lead`.
+int solve(const double2* A, int N, long long ld, long long stride, int nb, int m, const Ws& w, int lead,
+          cudaStream_t st) {
+    const int P = panel_count(N, m);
+    int p0 = 0;
+    while (p0 + 1 < P && panel_at(p0, N, m).base <= lead) ++p0;
+    int pf = tags_prof_begin(TAGS_PROF_LU64_OTHER, st);
+    if (N <= 320 || (nb >= 128 && N <= SOLVE_N_MAX)) {
+        k_ldl64_solve_cta<<<nb, SOLVE_THREADS, sizeof(double2) * N, st>>>(A, ld, stride, N, m, w.linv, w.wstride, w.r,
+                                                                          w.z, p0, w.active);
+        tags_prof_end(TAGS_PROF_LU64_OTHER, pf, st, 0.0, 0.0);
+        tags_note_launch();
+        TAGS_CUDA_OK(cudaGetLastError());
+        return 0;
+    }
+    TAGS_CUDA_OK(cudaMemsetAsync(w.z, 0, sizeof(double2) * N * nb, st));
+    for (int p = p0; p < P; ++p) {
+        const Panel q = panel_at(p, N, m);
+        k_ldl64_fwd<<<dim3(q.cnt > 0 ? (q.cnt + 63) / 64 : 1, nb), 64, 0, st>>>(A, ld, stride, q, p, w.linv,
+                                                                                w.wstride, w.r, w.z, N, w.active);
+    }
+    k_ldl64_dscale<<<dim3((N + 127) / 128, nb), 128, 0, st>>>(w.z, N, m, w.linv, w.wstride, w.active);
+    // the backward sweep runs on z and leaves the solution in r; then r -> z
+    for (int p = P - 1; p >= 0; --p) {
+        const Panel q = panel_at(p, N, m);
+        const int c0 = m > 0 && q.j0 >= m && q.j0 < 2 * m ? m : 0, left = q.j0 - c0;
+        k_ldl64_bwd<<<dim3(left > 0 ? (left + 63) / 64 : 1, nb), 64, 0, st>>>(A, ld, stride, q, p, c0, w.linv,
+                                                                              w.wstride, w.z, w.r, N, w.active);
+    }
+    TAGS_CUDA_OK(cudaMemcpyAsync(w.z, w.r, sizeof(double2) * N * nb, cudaMemcpyDeviceToDevice, st));
+    tags_prof_end(TAGS_PROF_LU64_OTHER, pf, st, 0.0, 0.0);
+    tags_note_launch(2 * P - p0 + 1);
+    TAGS_CUDA_OK(cudaGetLastError());
+    return 0;
+}
+
+constexpr int MAX_CORRECTIONS = 4;         // x itself and up to three refinements
+
+}  // namespace
+
+int tags_ldl64_prepare() {
+    static std::once_flag once;
+    static int rc = 0;
+    std::call_once(once, [] {
+        if (cudaFuncSetAttribute(k_ldl64_update<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(2 * PB * 64 * sizeof(double2))) != cudaSuccess ||
+            cudaFuncSetAttribute(k_ldl64_solve_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(SOLVE_N_MAX * sizeof(double2))) != cudaSuccess)
+            rc = tags_fail(TAGS_E_CUDA, "cudaFuncSetAttribute(k_ldl64) failed");
+    });
+    return rc;
+}
+
+size_t tags_ldl64_workspace(int N, int batch) {
+    const size_t per = sizeof(double2) * (((size_t)(N + PB - 1) / PB + 2) * PB * PB + 4 * (size_t)N) + sizeof(double) +
+                       2 * sizeof(int);
+    return per * batch + 64;
+}
+
+FillOut tags_ldl64_fill_out(double2* W, int m, int n) {
+    const long long N = n + 2LL * m;
+    FillOut out{};
+    out.zl = W;
+    out.zt = W;
+    out.ld = N;
+    out.batch_stride = N * N;
+    out.col0_l = m;
+    out.row0_t = m;
+    out.sign = 1.0;
+    out.mirror = 1;
+    return out;
+}
+
+int tags_ldl64_plan_solve(double2* W, const Incidence& inc, int m, int n, int nb, int batch, void* ws,
+                          const double2* rhs, double2* x, int* info, cudaStream_t st) {
+    if (int e = tags_ldl64_prepare()) return e;
+    const int N = n + 2 * m;
+    const long long NN = (long long)N * N;
+    const Ws w = carve(ws, N, batch);
+    k_ldl64_start<<<dim3((N + 127) / 128, nb), 128, 0, st>>>(rhs, N, m, n, w.b, w.r, w.x, w.active, w.conv);
+    k_ldl64_build<<<dim3(N, nb), 128, 0, st>>>(W, N, NN, inc, m, n);
+    tags_note_launch(2);
+    int err = factor(W, N, N, NN, nb, m, w, st);
+    for (int step = 0; step < MAX_CORRECTIONS && !err; ++step) {
+        if (step > 0) {
+            k_ldl64_resid_z<<<dim3((m + 63) / 64, 2, nb), 64, 0, st>>>(W, N, NN, inc, m, n, w.b, w.x, w.r, w.active);
+            k_ldl64_resid_nodes<<<dim3((n + 127) / 128, nb), 128, 0, st>>>(inc, m, n, w.b, w.x, w.r, w.active);
+            tags_note_launch(2);
+        }
+        err = solve(W, N, N, NN, nb, m, w, step == 0 ? 2 * m : 0, st);
+        if (err) break;
+        k_ldl64_apply<<<nb, 256, 0, st>>>(w.z, w.x, N, step, step + 1 == MAX_CORRECTIONS, w.active, w.conv, w.prev);
+        tags_note_launch();
+    }
+    if (err) return err;
+    k_ldl64_out<<<dim3((N + 127) / 128, nb), 128, 0, st>>>(w.x, m, n, w.conv, x, N, info);
+    tags_note_launch();
+    TAGS_CUDA_OK(cudaGetLastError());
+    return 0;
+}
+
+int tags_ldl64_saved_rhs(void* ws, int m, int n, int batch, int q, double2* out, cudaStream_t st) {
+    const int N = n + 2 * m;
+    const Ws w = carve(ws, N, batch);
+    k_ldl64_rhs_back<<<(N + 127) / 128, 128, 0, st>>>(w.b + (long long)N * q, m, n, out);
+    tags_note_launch();
+    TAGS_CUDA_OK(cudaGetLastError());
+    return 0;
+}
+
+int tags_ldl64_sym_solve(const double2* W, double2* A, int m, int n, void* ws, int* d_flag, double2* x, int* info,
+                         cudaStream_t st) {
+    if (int e = tags_ldl64_prepare()) return e;
+    const int N = n + 2 * m;
+    const Ws w = carve(ws, N, 1);
+    TAGS_CUDA_OK(cudaMemsetAsync(d_flag, 0, sizeof(int), st));
+    k_ldl64_start<<<dim3((N + 127) / 128, 1), 128, 0, st>>>(x, N, m, n, w.b, w.r, w.x, w.active, w.conv);
+    k_ldl64_permute<<<dim3(N, (N + 127) / 128), 128, 0, st>>>(W, A, m, n, d_flag);
+    tags_note_launch(2);
+    int coupled = 0;
+    TAGS_CUDA_OK(cudaMemcpyAsync(&coupled, d_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    TAGS_CUDA_OK(cudaStreamSynchronize(st));
+    const int zm = coupled ? 0 : m;          // the structure skipped by the elimination, if it is there
+    int err = factor(A, N, N, 0, 1, zm, w, st);
+    for (int step = 0; step < 3 && !err; ++step) {
+        if (step > 0) {
+            k_ldl64_resid_full<<<(N + 63) / 64, 64, 0, st>>>(W, m, n, w.b, w.x, w.r, w.active);
+            tags_note_launch();
+        }
+        err = solve(A, N, N, 0, 1, zm, w, 0, st);
+        if (err) break;
+        k_ldl64_apply<<<1, 256, 0, st>>>(w.z, w.x, N, step, step == 2, w.active, w.conv, w.prev);
+        tags_note_launch();
+    }
+    if (err) return err;
+    k_ldl64_out<<<dim3((N + 127) / 128, 1), 128, 0, st>>>(w.x, m, n, w.conv, x, N, info);
+    tags_note_launch();
+    TAGS_CUDA_OK(cudaGetLastError());
+    return 0;
+}

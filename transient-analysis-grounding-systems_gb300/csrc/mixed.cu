@@ -27,8 +27,7 @@
 //      under a conditional while-node. The first step's right-hand side is b,
 //      zero in the impedance rows, and its forward sweep starts at the node
 //      rows;
-//   5. samples that do not converge are re-solved by the plain FP64 path
-//      (LU with partial pivoting).
+//   5. samples that do not converge are re-solved by the plain FP64 path.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -627,41 +626,37 @@ int tags_mixed_free(tags_plan_s* p) {
     return 0;
 }
 
-// Re-solve sample `q` of the current pass in plain FP64 (partial pivoting).
+// Re-solve sample `q` of the current pass in plain FP64: the structured LDL^T
+// with refinement (ldl64.cu), and where that does not converge the LU with
+// partial pivoting.
 static int fallback_plain(tags_plan_s* p, int q, cudaStream_t st) {
     TagsRange range("tags FP64 re-solve");
     const long long N = p->N, NN = N * N;
     if (!p->d_fbW) {
         if (cudaMalloc(&p->d_fbW, sizeof(double2) * NN) != cudaSuccess ||
-            cudaMalloc(&p->d_fbpiv, sizeof(int) * (N + 1)) != cudaSuccess) {
+            cudaMalloc(&p->d_fbpiv, sizeof(int) * (N + 1)) != cudaSuccess ||
+            cudaMalloc(&p->d_ldl64, tags_ldl64_workspace((int)N, 1)) != cudaSuccess) {
             cudaGetLastError();
             if (p->d_fbW) cudaFree(p->d_fbW);
+            if (p->d_fbpiv) cudaFree(p->d_fbpiv);
             p->d_fbW = nullptr;
+            p->d_fbpiv = nullptr;
             return tags_fail(TAGS_E_NOMEM, "device allocation failed (FP64 fallback)");
         }
     }
     if (int e = tags_plan_series_alloc(p, 1)) return e;
     double2* W = p->d_fbW;
-    int* ipiv = p->d_fbpiv;
-    TAGS_CUDA_OK(cudaMemsetAsync(W, 0, sizeof(double2) * NN, st));
-    int err = tags_wg_incidence(W, N, NN, 1, p->d_cond, p->n, p->m, st);
-    if (err) return err;
-    FillOut out{};
-    out.zl = W;
-    out.zt = W;
-    out.ld = N;
-    out.row0_l = out.col0_l = p->n;
-    out.row0_t = out.col0_t = p->n + p->m;
-    out.sign = -1.0;
-    out.mirror = 1;
-    err = tags_plan_fill_fp64(p, p->d_coef + q, 1, out, st);
-    if (err) return err;
-    err = tags_lu_z(W, (int)N, N, NN, 1, 1, ipiv, p->d_info + q, st);
-    if (err) return err;
     double2* x = p->d_x + (size_t)q * N;
     const double2* bvec = p->d_r + (size_t)p->batch * N + (size_t)q * N;
+    int err = tags_plan_fill_fp64(p, p->d_coef + q, 1, tags_ldl64_fill_out(W, p->m, p->n), st);
+    if (!err) err = tags_ldl64_plan_solve(W, p->inc, p->m, p->n, 1, 1, p->d_ldl64, bvec, x, p->d_info + q, st);
+    if (err) return err;
+    int info = 0;
+    TAGS_CUDA_OK(cudaMemcpyAsync(&info, p->d_info + q, sizeof(int), cudaMemcpyDeviceToHost, st));
+    TAGS_CUDA_OK(cudaStreamSynchronize(st));
+    if (info != TAGS_INFO_RESOLVE) return 0;
     TAGS_CUDA_OK(cudaMemcpyAsync(x, bvec, sizeof(double2) * N, cudaMemcpyDeviceToDevice, st));
-    return tags_lu_solve_z(W, (int)N, N, NN, 1, ipiv, x, 1, N, N, st);
+    return tags_plan_lu_one(p, q, W, p->d_fbpiv, x, p->d_info + q, st);
 }
 
 int tags_plan_rhs(tags_plan_s* p, double2* d_X, const double2* d_ie, int inj_node, int nb, cudaStream_t st);

@@ -1,7 +1,8 @@
 // Batched plan API (include/tags_gpu.h, part 2): geometry, incidence and
 // workspaces stay on the device; every pass handles `batch` Laplace samples:
-//   plain FP64: W_G assembled in place (incidence + fused direct/image fill,
-//               both triangles), LU with partial pivoting, triangular solves;
+//   plain FP64: the impedance blocks (fused direct/image fill), LDL^T in the
+//               static order with FP64 refinement (ldl64.cu), LU with partial
+//               pivoting (lu.cu) for samples that it does not serve;
 //   mixed:      see mixed.cu.
 // The per-sample medium terms follow examples/three_grids.c:326-333
 // (gamma = sqrt(s mur mu0 kappa), ref_t = (kappa - s eps0)/(kappa + s eps0),
@@ -172,6 +173,7 @@ static void plan_free(tags_plan_s* p) {
     if (p->d_pot) cudaFree(p->d_pot);
     if (p->d_coef1) cudaFree(p->d_coef1);
     if (p->d_series) cudaFree(p->d_series);
+    if (p->d_ldl64) cudaFree(p->d_ldl64);
     if (p->d_iein) cudaFree(p->d_iein);
     if (p->ev0) cudaEventDestroy(p->ev0);
     if (p->ev1) cudaEventDestroy(p->ev1);
@@ -241,7 +243,7 @@ extern "C" int tags_plan_create(tags_plan* out, const Electrode* electrodes, con
     PLAN_CHECK(tags_free_memory(&freeb));
     const double NN = (double)N * (double)N;
     double per = precision == TAGS_PLAIN_FP64
-                     ? 16.0 * NN + 40.0 * N
+                     ? 16.0 * NN + 40.0 * N + (double)tags_ldl64_workspace((int)N, 1)
                      : 8.0 * NN + 32.0 * (double)p->m * p->m + 80.0 * N + (double)tags_ldl_tc_workspace((int)N, 1);
     long long cap = (long long)(0.45 * (double)freeb / per);
     long long b = max_batch ? (long long)max_batch : std::min<long long>(cap, 64);
@@ -255,9 +257,11 @@ extern "C" int tags_plan_create(tags_plan* out, const Electrode* electrodes, con
     if (precision == TAGS_PLAIN_FP64) {
         err = tags_plan_series_alloc(p, p->batch);
         if (err) { plan_free(p); return err; }
-        PLAN_CHECK(cudaMalloc(&p->d_ipiv, sizeof(int) * N * b));
+        PLAN_CHECK(cudaMalloc(&p->d_ipiv, sizeof(int) * (N + 1)));
+        PLAN_CHECK(cudaMalloc(&p->d_ldl64, tags_ldl64_workspace(p->N, p->batch)));
         PLAN_CHECK(cudaMalloc(&p->d_W, sizeof(double2) * (size_t)NN * b));
         err = tags_lu_prepare();
+        if (!err) err = tags_ldl64_prepare();
         if (err) { plan_free(p); return err; }
     } else {
         err = tags_mixed_alloc(p);
@@ -313,31 +317,56 @@ extern "C" int tags_plan_set_fill(tags_plan plan, int integration_type) {
 }
 
 // Plain FP64 pass over nb samples whose coefficients and right-hand sides are
-// already in p->d_coef and p->d_x.
+// already in p->d_coef and p->d_x: fill, LDL^T in the static order, refinement.
+// info of a sample that needs the pivoted LU is TAGS_INFO_RESOLVE
+// (tags_plan_finish_plain).
 int tags_plan_run_plain(tags_plan_s* p, const double2*, int nb, cudaStream_t st) {
+    TagsRange range("tags fill");
+    int err = tags_plan_fill_fp64(p, p->d_coef, nb, tags_ldl64_fill_out(p->d_W, p->m, p->n), st);
+    if (err) return err;
+    range.next("tags factor");
+    return tags_ldl64_plan_solve(p->d_W, p->inc, p->m, p->n, nb, p->batch, p->d_ldl64, p->d_x, p->d_x, p->d_info, st);
+}
+
+// W_G of sample q's coefficients, its LU with partial pivoting and the solve.
+int tags_plan_lu_one(tags_plan_s* p, int q, double2* W, int* ipiv, double2* x, int* info, cudaStream_t st) {
     const long long N = p->N, NN = N * N;
-    TagsRange range("tags assemble");
-    TAGS_CUDA_OK(cudaMemsetAsync(p->d_W, 0, sizeof(double2) * NN * nb, st));
-    int err = tags_wg_incidence(p->d_W, N, NN, nb, p->d_cond, p->n, p->m, st);
+    TagsRange range("tags FP64 re-solve");
+    TAGS_CUDA_OK(cudaMemsetAsync(W, 0, sizeof(double2) * NN, st));
+    int err = tags_wg_incidence(W, N, NN, 1, p->d_cond, p->n, p->m, st);
     if (err) return err;
     FillOut out{};
-    out.zl = p->d_W;
-    out.zt = p->d_W;
+    out.zl = W;
+    out.zt = W;
     out.ld = N;
     out.batch_stride = NN;
     out.row0_l = out.col0_l = p->n;
     out.row0_t = out.col0_t = p->n + p->m;
     out.sign = -1.0;
     out.mirror = 1;
-    out.accumulate = 0;
-    range.next("tags fill");
-    err = tags_plan_fill_fp64(p, p->d_coef, nb, out, st);
-    if (err) return err;
-    range.next("tags factor");
-    err = tags_lu_z(p->d_W, (int)N, N, NN, nb, 1, p->d_ipiv, p->d_info, st);
-    if (err) return err;
-    range.next("tags solve");
-    return tags_lu_solve_z(p->d_W, (int)N, N, NN, nb, p->d_ipiv, p->d_x, 1, N, N, st);
+    err = tags_plan_fill_fp64(p, p->d_coef + q, 1, out, st);
+    if (!err) err = tags_lu_z(W, (int)N, N, NN, 1, 1, ipiv, info, st);
+    return err ? err : tags_lu_solve_z(W, (int)N, N, NN, 1, ipiv, x, 1, N, N, st);
+}
+
+// After a plain pass: samples marked for the pivoted LU are solved by it, one
+// by one in the first sample's matrix. A pass whose fill failed is left as it
+// is (the run reports the status).
+static int finish_plain(tags_plan_s* p, int nb, cudaStream_t st) {
+    std::vector<int> info(nb);
+    int status = 0;
+    TAGS_CUDA_OK(cudaMemcpyAsync(info.data(), p->d_info, sizeof(int) * nb, cudaMemcpyDeviceToHost, st));
+    TAGS_CUDA_OK(cudaMemcpyAsync(&status, p->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
+    TAGS_CUDA_OK(cudaStreamSynchronize(st));
+    if (status) return 0;
+    for (int q = 0; q < nb; ++q) {
+        if (info[q] != TAGS_INFO_RESOLVE) continue;
+        double2* x = p->d_x + (size_t)q * p->N;
+        int err = tags_ldl64_saved_rhs(p->d_ldl64, p->m, p->n, p->batch, q, x, st);
+        if (!err) err = tags_plan_lu_one(p, q, p->d_W, p->d_ipiv, x, p->d_info + q, st);
+        if (err) return err;
+    }
+    return 0;
 }
 
 // ---- graph passes ------------------------------------------------------------------
@@ -744,14 +773,18 @@ static int run_passes(tags_plan_s* p, const tags_cdouble* s, const tags_cdouble*
                 err = tags_mixed_finish(p, nb, st, iters.data(), berr.data(), conv.data(), &steps);
                 if (err) return err;
                 launched += (long long)steps * gp->launches_step;
+            } else if (int e = finish_plain(p, nb, st)) {
+                return e;
             }
             tags_note_launch(launched);
         } else {
             err = tags_plan_coef(p, ds, dk, mur, nb, st);
             if (!err) err = tags_plan_rhs(p, p->d_x, die, (int)inj_node, nb, st);
             if (err) return err;
-            if (p->precision == TAGS_PLAIN_FP64) err = tags_plan_run_plain(p, ds, nb, st);
-            else err = tags_mixed_solve_batch(p, nb, nullptr, iters.data(), berr.data(), conv.data(), st);
+            if (p->precision == TAGS_PLAIN_FP64) {
+                err = tags_plan_run_plain(p, ds, nb, st);
+                if (!err) err = finish_plain(p, nb, st);
+            } else err = tags_mixed_solve_batch(p, nb, nullptr, iters.data(), berr.data(), conv.data(), st);
             if (err) return err;
         }
         if (p->precision != TAGS_PLAIN_FP64) {

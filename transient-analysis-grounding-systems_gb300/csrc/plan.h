@@ -54,8 +54,9 @@ struct tags_plan_s {
     SampleCoef* d_coef = nullptr;   // batch
     int* d_status = nullptr;        // 4 words
     int* d_info = nullptr;          // batch
-    int* d_ipiv = nullptr;          // batch x N
+    int* d_ipiv = nullptr;          // N + 1 (pivoted LU of one sample)
     double2* d_W = nullptr;         // plain: batch x N x N
+    void* d_ldl64 = nullptr;        // plain: workspace of the FP64 LDL^T
     SeriesGeo series;               // FP64 fill from per-pass moments (fill.cu) and its workspace,
     void* d_series = nullptr;       // for series_ns samples (plain: the batch; mixed: 1, with the first FP64 re-solve)
     int series_ns = 0;
@@ -141,3 +142,24 @@ int tags_mixed_fallback_one(tags_plan_s* p, const double2* d_s, const double2* d
 int tags_plan_add_while_node(cudaStream_t st, cudaGraphConditionalHandle* cond, cudaGraph_t* body);
 // The FP64 moment series' geometry and workspace for up to ns samples (once per plan).
 int tags_plan_series_alloc(tags_plan_s* p, int ns);
+
+// ldl64.cu: FP64 LDL^T in the static order with refinement (plain form). A
+// sample whose corrections do not shrink gets info = TAGS_INFO_RESOLVE: its
+// caller solves it by the pivoted LU.
+constexpr int TAGS_INFO_RESOLVE = -1000000;
+int tags_ldl64_prepare();
+size_t tags_ldl64_workspace(int N, int batch);
+// where the fill of a pass writes ZL and ZT inside W (n + 2m square per sample)
+FillOut tags_ldl64_fill_out(double2* W, int m, int n);
+// after that fill: x (original order, may be rhs) = W^-1 rhs for nb samples
+int tags_ldl64_plan_solve(double2* W, const Incidence& inc, int m, int n, int nb, int batch, void* ws,
+                          const double2* rhs, double2* x, int* info, cudaStream_t st);
+// the right-hand side of sample q of the last solve, in the original order
+int tags_ldl64_saved_rhs(void* ws, int m, int n, int batch, int q, double2* out, cudaStream_t st);
+// one full symmetric matrix W (original order, kept), A of the same size for
+// the factors, x the right-hand side and the solution; *d_flag is scratch
+int tags_ldl64_sym_solve(const double2* W, double2* A, int m, int n, void* ws, int* d_flag, double2* x, int* info,
+                         cudaStream_t st);
+// the pivoted LU of one sample from the plan's coefficients slot q into W
+// (N x N), right-hand side and solution in x, info on the device
+int tags_plan_lu_one(tags_plan_s* p, int q, double2* W, int* ipiv, double2* x, int* info, cudaStream_t st);
