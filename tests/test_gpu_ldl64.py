@@ -85,3 +85,51 @@ def test_samples_without_static_pivots_go_to_the_pivoted_lu(gpu_pkg, graphs):
     (got, binfo), = pkg.solve_batch(jobs, precision=pkg.PLAIN_FP64)
     assert not binfo.any()
     assert rel_err(got, sol) < TOL
+
+
+def symmetric(rng, N):
+    a = rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N))
+    return a + a.T + 2 * N * np.eye(N)
+
+
+@pytest.mark.parametrize("m,n", [(1, 1), (15, 2), (16, 1), (40, 33), (110, 101)])
+@pytest.mark.parametrize("kind", ["structured", "coupled", "zero pivots"])
+def test_solve_immittance_of_any_symmetric_matrix(gpu_pkg, m, n, kind):
+    """The structured elimination, a caller's matrix with a ZL/ZT coupling, and
+    one whose impedance blocks have a zero diagonal (pivoted LU)."""
+    pkg = gpu_pkg
+    rng = np.random.default_rng(m + n)
+    N = n + 2 * m
+    w = symmetric(rng, N)
+    if kind != "coupled":
+        w[n:n + m, n + m:] = 0
+        w[n + m:, n:n + m] = 0
+    if kind == "zero pivots":
+        w -= np.diag(np.diag(w))
+        if m == 1:
+            w[n, 0] = w[0, n] = 3.0
+            w[n + 1, n + 1] = 2.0
+    x = rng.standard_normal(N) + 1j * rng.standard_normal(N)
+    b = w @ x
+    lower = np.tril(w).T.ravel().copy()             # column-major, upper triangle unread
+    got = b.copy()
+    assert pkg.solve_immittance(lower, got, m, n) == 0
+    assert rel_err(got, np.linalg.solve(w, b)) < 1e-9
+
+
+@pytest.mark.parametrize("m,n", [(1, 1), (31, 3), (32, 33), (65, 40), (130, 7)])
+@pytest.mark.parametrize("zero_diagonal", [False, True])
+def test_yla_ytb_of_any_symmetric_blocks(gpu_pkg, m, n, zero_diagonal):
+    pkg = gpu_pkg
+    rng = np.random.default_rng(m * n)
+    z = [symmetric(rng, m) for _ in range(2)]
+    if zero_diagonal and m > 1:
+        z[1] -= np.diag(np.diag(z[1]))
+    rhs = [(rng.standard_normal((m, n)) + 0j) for _ in range(2)]
+    zl, zt = (np.tril(v).T.ravel().copy() for v in z)
+    a, b = (v.T.ravel().copy() for v in rhs)
+    yla, ytb = np.zeros(m * n, np.complex128), np.zeros(m * n, np.complex128)
+    assert pkg.calculate_yla_ytb(yla, ytb, zl, zt, a, b, m, n) == 0
+    for got, inv, v, r in ((yla, zl, z[0], rhs[0]), (ytb, zt, z[1], rhs[1])):
+        assert rel_err(got.reshape(n, m).T, np.linalg.solve(v, r)) < 1e-9
+        assert rel_err(np.tril(inv.reshape(m, m).T), np.tril(np.linalg.inv(v))) < 1e-9

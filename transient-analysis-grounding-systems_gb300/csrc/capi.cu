@@ -341,12 +341,46 @@ extern "C" int fill_impedance_imm(tags_cdouble* wg, const tags_cdouble* zl, cons
 
 // ---- drop-in: solve -------------------------------------------------------------
 
+int tags_sym_solve_host(const tags_cdouble* w, tags_cdouble* x, size_t m, size_t n, int* done) {
+    *done = 0;
+    DeviceCtx* c = tags_ctx();
+    if (!c) return tags_fail(TAGS_E_CUDA, "no usable CUDA device");
+    cudaStream_t st = c->stream;
+    const size_t N = 2 * m + n;
+    // the second matrix stays with the context: up to 8 GB (N = 23,170)
+    if (sizeof(double2) * N * N > ((size_t)8 << 30)) return 0;
+    double2* d_W = (double2*)c->scratch(3, sizeof(double2) * N * N);
+    double2* d_A = (double2*)c->scratch(17, sizeof(double2) * N * N);
+    double2* d_x = (double2*)c->scratch(4, sizeof(double2) * N);
+    void* ws = c->scratch(18, tags_ldl64_workspace((int)N, 1));
+    if (!d_W || !d_A || !d_x || !ws) {
+        cudaGetLastError();                              // no room for two matrices: the LU needs one
+        return 0;
+    }
+    TAGS_CUDA_OK(cudaMemcpyAsync(d_W, w, sizeof(double2) * N * N, cudaMemcpyHostToDevice, st));
+    TAGS_CUDA_OK(cudaMemcpyAsync(d_x, x, sizeof(double2) * N, cudaMemcpyHostToDevice, st));
+    int err = tags_symmetrize_lower(d_W, (int)N, (long long)N, 0, 1, st);
+    if (!err) err = tags_ldl64_sym_solve(d_W, d_A, (int)m, (int)n, ws, c->status, d_x, c->status + 1, st);
+    if (err) return err;
+    int info = 0;
+    TAGS_CUDA_OK(cudaMemcpyAsync(&info, c->status + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+    TAGS_CUDA_OK(cudaStreamSynchronize(st));
+    if (info != 0) return 0;
+    TAGS_CUDA_OK(cudaMemcpyAsync(x, d_x, sizeof(double2) * N, cudaMemcpyDeviceToHost, st));
+    TAGS_CUDA_OK(cudaStreamSynchronize(st));
+    *done = 1;
+    return 0;
+}
+
 extern "C" int solve_immittance(tags_cdouble* wg, tags_cdouble* ie, size_t num_electrodes, size_t num_nodes) {
     std::lock_guard<std::mutex> lk(g_mutex);
     const size_t N = 2 * num_electrodes + num_nodes;
     if (N == 0) return 0;
     if (!wg || !ie) return tags_fail(TAGS_E_ARG, "null pointer argument");
     if (N > 200000) return tags_fail(TAGS_E_ARG, "system too large");
+    int done = 0;
+    if (int e = tags_sym_solve_host(wg, ie, num_electrodes, num_nodes, &done)) return e;
+    if (done) return 0;
     DeviceCtx* c = tags_ctx();
     if (!c) return tags_fail(TAGS_E_CUDA, "no usable CUDA device");
     cudaStream_t st = c->stream;

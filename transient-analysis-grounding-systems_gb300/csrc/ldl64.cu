@@ -148,15 +148,17 @@ __global__ void __launch_bounds__(128) k_ldl64_panel(double2* __restrict__ A0, l
 }
 
 // Trailing update C -= L21 U12 over the lower triangle of the rows below the
-// panel, TL x TL tiles of 4 x 4 values per thread. FP64-bound: a tile of 64
-// takes 262,144 SM cycles of multiply-adds against 131 KB of C, so one panel
-// (K = 32) per update is enough, and the tile size only sets the work wasted
-// on the diagonal and the edge.
-template <int TL>
-__global__ void __launch_bounds__(TL * TL / 16) k_ldl64_update(double2* __restrict__ A0, long long ld,
+// panel, TL x TL tiles of TT x TT values per thread. FP64-bound (a warp's FP64
+// instruction holds its quarter of the SM for 64 cycles): a tile of 64 takes
+// 262,144 SM cycles of multiply-adds against 131 KB of C, so one panel (K = 32)
+// per update is enough. The tile size sets the work wasted on the diagonal and
+// the edge, and with four or more warps per tile how long a launch of few
+// tiles takes at least: 131, 33 and 8 us for 64, 32 and 16.
+template <int TL, int TT>
+__global__ void __launch_bounds__(TL * TL / (TT * TT)) k_ldl64_update(double2* __restrict__ A0, long long ld,
                                                                long long stride, Panel q) {
     double2* A = A0 + stride * blockIdx.y;
-    constexpr int TH = TL / 4, NT = TH * TH;
+    constexpr int TH = TL / TT, NT = TH * TH;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* sA = reinterpret_cast<double2*>(smem_raw);    // [PB][TL]
     double2* sB = sA + PB * TL;                            // [PB][TL]
@@ -173,29 +175,29 @@ __global__ void __launch_bounds__(TL * TL / 16) k_ldl64_update(double2* __restri
     }
     __syncthreads();
     const int tx = threadIdx.x % TH, tyy = threadIdx.x / TH;
-    double2 acc[4][4];
+    double2 acc[TT][TT];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < TT; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = cz(0.0, 0.0);
+        for (int b = 0; b < TT; ++b) acc[a][b] = cz(0.0, 0.0);
     for (int k = 0; k < q.jb; ++k) {
-        double2 av[4], bv[4];
+        double2 av[TT], bv[TT];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) av[a] = sA[k * TL + tx + TH * a];
+        for (int a = 0; a < TT; ++a) av[a] = sA[k * TL + tx + TH * a];
 #pragma unroll
-        for (int b = 0; b < 4; ++b) bv[b] = sB[k * TL + tyy + TH * b];
+        for (int b = 0; b < TT; ++b) bv[b] = sB[k * TL + tyy + TH * b];
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+        for (int a = 0; a < TT; ++a)
 #pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b] = cfma(av[a], bv[b], acc[a][b]);
+            for (int b = 0; b < TT; ++b) acc[a][b] = cfma(av[a], bv[b], acc[a][b]);
     }
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
+    for (int b = 0; b < TT; ++b) {
         const int gc = c0 + tyy + TH * b;
         if (gc >= q.cnt) continue;
         const long long col = ld * q.row(gc);
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
+        for (int a = 0; a < TT; ++a) {
             const int gr = r0 + tx + TH * a;
             if (gr < q.cnt && gr >= gc) {
                 const long long idx = q.row(gr) + col;
@@ -560,6 +562,227 @@ __global__ void __launch_bounds__(64) k_ldl64_resid_full(const double2* __restri
     if (ip < N) R[ip] = csub(B[ip], acc);
 }
 
+// ---- many right-hand sides (the nodal admittance drop-ins)
+
+// One panel of a sweep over R right-hand sides (columns of X, leading
+// dimension ldx): y = L11^-1 X_p (BWD: L11^-T X_p), to Y as D^-1 y (BWD: y),
+// then X_c -= L_cp y for the rows c below the panel (BWD: X_c -= L_pc^T y for
+// those above). 64 x 32 tiles; every tile forms its 32 columns of y itself, X_p
+// is left as it is. FP64-bound like the factorisation's updates.
+template <bool BWD>
+__global__ void __launch_bounds__(128) k_ldl64_msolve(const double2* __restrict__ A0, long long ld, long long stride,
+                                                      Panel q, int p, const double2* __restrict__ ws0,
+                                                      long long wstride, double2* __restrict__ X0,
+                                                      double2* __restrict__ Y0, long long ldx, long long xstride,
+                                                      int R) {
+    const int b = blockIdx.z;
+    const double2* A = A0 + stride * b;
+    const double2* ws = ws0 + wstride * b + (long long)p * PB * PB;
+    double2* X = X0 + xstride * b;
+    double2* Y = Y0 + xstride * b;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2* sL = reinterpret_cast<double2*>(smem_raw);    // [PB][64]: L of the tile, k-major; first L11^-1
+    double2* raw = sL + PB * 64;                            // [PB][PB + 1]: X_p, k-major
+    double2* y = raw + PB * (PB + 1);                       // [PB][PB + 1]
+    const int r0 = blockIdx.y * PB, c0 = blockIdx.x * 64, ncols = BWD ? q.j0 : q.cnt;
+    for (int t = threadIdx.x; t < PB * PB; t += 128) {
+        const int k = t % PB, r = t / PB;
+        raw[k * (PB + 1) + r] = (k < q.jb && r0 + r < R) ? X[q.j0 + k + ldx * (r0 + r)] : cz(0.0, 0.0);
+        sL[t] = ws[t];                                      // (row, column) at column * PB + row
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < PB * PB; t += 128) {
+        const int k = t / PB, r = t % PB;
+        double2 a = raw[k * (PB + 1) + r];
+        if (!BWD) {
+            for (int j = 0; j < k; ++j) a = cfma(sL[j * PB + k], raw[j * (PB + 1) + r], a);
+        } else {
+            for (int j = k + 1; j < PB; ++j) a = cfma(sL[k * PB + j], raw[j * (PB + 1) + r], a);
+        }
+        y[k * (PB + 1) + r] = a;
+        if (blockIdx.x == 0 && k < q.jb && r0 + r < R)
+            Y[q.j0 + k + ldx * (r0 + r)] = BWD ? a : cmul(a, sL[k * (PB + 1)]);
+    }
+    __syncthreads();
+    if (c0 >= ncols) return;
+    for (int t = threadIdx.x; t < PB * 64; t += 128) {
+        const int c = BWD ? t / PB : t % 64, k = BWD ? t % PB : t / 64;
+        double2 v = cz(0.0, 0.0);
+        if (k < q.jb && c0 + c < ncols)
+            v = BWD ? A[(q.j0 + k) + ld * (c0 + c)] : A[q.base + c0 + c + ld * (q.j0 + k)];
+        sL[k * 64 + c] = v;
+    }
+    __syncthreads();
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    double2 acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[a][e] = cz(0.0, 0.0);
+    for (int k = 0; k < q.jb; ++k) {
+        double2 av[4], bv[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) av[a] = sL[k * 64 + tx + 16 * a];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) bv[e] = y[k * (PB + 1) + ty + 8 * e];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[a][e] = cfma(av[a], bv[e], acc[a][e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const int r = r0 + ty + 8 * e;
+        if (r >= R) continue;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const int c = c0 + tx + 16 * a;
+            if (c >= ncols) continue;
+            double2* x = X + (BWD ? c : q.base + c) + ldx * r;
+            *x = csub(*x, acc[a][e]);
+        }
+    }
+}
+
+constexpr size_t MSOLVE_SMEM = sizeof(double2) * (PB * 64 + 2 * PB * (PB + 1));
+
+// Identity columns [n, n + M) of X (M x (n + M)).
+__global__ void k_ldl64_identity(double2* __restrict__ X0, int M, int n, long long xstride) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)M * M) return;
+    X0[xstride * blockIdx.y + (long long)M * n + t] = cz(t % M == t / M ? 1.0 : 0.0, 0.0);
+}
+
+// E = [rhs, I] - Z X for the refinement of all right-hand sides (M x R, R = n +
+// M); 64 x 32 tiles, FP64-bound.
+__global__ void __launch_bounds__(128) k_ldl64_mresid(const double2* __restrict__ Z0, int M, long long zstride,
+                                                      const double2* __restrict__ B0, int n, long long bstride,
+                                                      const double2* __restrict__ X0, double2* __restrict__ E0,
+                                                      long long xstride, int R) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2* sZ = reinterpret_cast<double2*>(smem_raw);    // [PB][64], k-major
+    double2* sX = sZ + PB * 64;                             // [PB][PB + 1], k-major
+    const double2* Z = Z0 + zstride * blockIdx.z;
+    const double2* X = X0 + xstride * blockIdx.z;
+    const int i0 = blockIdx.x * 64, r0 = blockIdx.y * PB;
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    double2 tot[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) tot[a][e] = cz(0.0, 0.0);
+    for (int k0 = 0; k0 < M; k0 += PB) {
+        const int nk = min(PB, M - k0);
+        __syncthreads();
+        for (int t = threadIdx.x; t < PB * 64; t += 128) {
+            const int i = t % 64, k = t / 64;
+            sZ[t] = (k < nk && i0 + i < M) ? Z[i0 + i + (long long)M * (k0 + k)] : cz(0.0, 0.0);
+        }
+        for (int t = threadIdx.x; t < PB * PB; t += 128) {
+            const int k = t % PB, r = t / PB;
+            sX[k * (PB + 1) + r] = (k < nk && r0 + r < R) ? X[k0 + k + (long long)M * (r0 + r)] : cz(0.0, 0.0);
+        }
+        __syncthreads();
+        double2 acc[4][4];                                  // sums of 32 terms, then of those: less rounding than one chain
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[a][e] = cz(0.0, 0.0);
+        for (int k = 0; k < nk; ++k) {
+            double2 av[4], bv[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) av[a] = sZ[k * 64 + tx + 16 * a];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) bv[e] = sX[k * (PB + 1) + ty + 8 * e];
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[a][e] = cfma(av[a], bv[e], acc[a][e]);
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) tot[a][e] = cadd(tot[a][e], acc[a][e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const int r = r0 + ty + 8 * e;
+        if (r >= R) continue;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const int i = i0 + tx + 16 * a;
+            if (i >= M) continue;
+            const double2 b = r < n ? B0[bstride * blockIdx.z + i + (long long)M * r] : cz(r - n == i ? 1.0 : 0.0, 0.0);
+            E0[xstride * blockIdx.z + i + (long long)M * r] = csub(b, tot[a][e]);
+        }
+    }
+}
+
+__global__ void k_ldl64_add(double2* __restrict__ X, const double2* __restrict__ E, long long n) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n) X[t] = cadd(X[t], E[t]);
+}
+
+// Signs of the check's combination of right-hand sides.
+TAGS_D double check_sign(int r) { return (((unsigned)r * 2654435761u) >> 15) & 1u ? 1.0 : -1.0; }
+
+// Check of the whole solve on one random combination of its right-hand sides:
+// v = sum_r sign_r X_r, u = sum_r sign_r B_r (B = [rhs, I]). Warp per row.
+__global__ void __launch_bounds__(128) k_ldl64_check_sum(const double2* __restrict__ X0, const double2* __restrict__ B0,
+                                                         int M, int n, long long xstride, long long bstride,
+                                                         double2* __restrict__ vu0) {
+    const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, b = blockIdx.y;
+    if (row >= M) return;
+    double2 v = cz(0.0, 0.0), u = cz(0.0, 0.0);
+    for (int r = lane; r < n + M; r += 32) {
+        const double sg = check_sign(r);
+        const double2 x = X0[xstride * b + row + (long long)M * r];
+        v.x += sg * x.x;
+        v.y += sg * x.y;
+        if (r < n) {
+            const double2 w = B0[bstride * b + row + (long long)M * r];
+            u.x += sg * w.x;
+            u.y += sg * w.y;
+        } else if (r - n == row) {
+            u.x += sg;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+        v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+        u.x += __shfl_xor_sync(0xffffffffu, u.x, o);
+        u.y += __shfl_xor_sync(0xffffffffu, u.y, o);
+    }
+    if (lane == 0) {
+        vu0[(2LL * b) * M + row] = v;
+        vu0[(2LL * b + 1) * M + row] = u;
+    }
+}
+
+// Row by row |Z v - u| against 1e-14 (sum |Z| |v| + |u|), the backward error
+// of a stable solve with room for M ~ 50 eps; *bad is raised above it (or by a
+// value that is not finite). Z: full symmetric. Warp per row.
+__global__ void __launch_bounds__(128) k_ldl64_check(const double2* __restrict__ Z0, int M, long long zstride,
+                                                     const double2* __restrict__ vu0, int* __restrict__ bad) {
+    const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, b = blockIdx.y;
+    if (row >= M) return;
+    const double2* v = vu0 + 2LL * b * M;
+    const double2 u = v[M + row];
+    double2 acc = cz(0.0, 0.0);
+    double mag = 0.0;
+    for (int j = lane; j < M; j += 32) {
+        const double2 z = Z0[zstride * b + j + (long long)M * row], x = v[j];
+        acc = cfma(z, x, acc);
+        mag = fma(cabs1(z), cabs1(x), mag);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+        acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+        mag += __shfl_xor_sync(0xffffffffu, mag, o);
+    }
+    if (lane == 0 && !(cabs1(csub(acc, u)) <= 1e-14 * (mag + cabs1(u)))) *bad = 1;
+}
+
 struct Ws {
     double2 *linv, *b, *x, *r, *z;
     double* prev;
@@ -595,15 +818,18 @@ int factor(double2* A, int N, long long ld, long long stride, int nb, int m, con
         tags_prof_end(TAGS_PROF_LU64_OTHER, pf, st, 0.0, 0.0);
         tags_note_launch();
         if (q.cnt <= 0) continue;
-        // tiles of 64, or of 32 where the larger ones waste more on the
-        // diagonal and the edge (under ten tile rows) or leave SMs idle
+        // the largest tile that wastes little on the diagonal and the edge (ten
+        // tile rows) and fills the SMs
         pf = tags_prof_begin(TAGS_PROF_LU64_GEMM, st);
-        const long long t64 = (q.cnt + 63) / 64, t32 = (q.cnt + 31) / 32;
+        const long long t64 = (q.cnt + 63) / 64, t32 = (q.cnt + 31) / 32, t16 = (q.cnt + 15) / 16;
         if (t64 >= 10 && t64 * (t64 + 1) / 2 * nb >= 608)
-            k_ldl64_update<64><<<dim3((unsigned)(t64 * (t64 + 1) / 2), nb), 256, 2 * PB * 64 * sizeof(double2), st>>>(
+            k_ldl64_update<64, 4><<<dim3((unsigned)(t64 * (t64 + 1) / 2), nb), 256, 2 * PB * 64 * sizeof(double2), st>>>(
+                A, ld, stride, q);
+        else if (t32 >= 10 && t32 * (t32 + 1) / 2 * nb >= 304)
+            k_ldl64_update<32, 2><<<dim3((unsigned)(t32 * (t32 + 1) / 2), nb), 256, 2 * PB * 32 * sizeof(double2), st>>>(
                 A, ld, stride, q);
         else
-            k_ldl64_update<32><<<dim3((unsigned)(t32 * (t32 + 1) / 2), nb), 64, 2 * PB * 32 * sizeof(double2), st>>>(
+            k_ldl64_update<16, 1><<<dim3((unsigned)(t16 * (t16 + 1) / 2), nb), 256, 2 * PB * 16 * sizeof(double2), st>>>(
                 A, ld, stride, q);
         tags_prof_end(TAGS_PROF_LU64_GEMM, pf, st, 4.0 * q.cnt * (q.cnt + 1.0) * q.jb * nb,
                       (16.0 * q.cnt * (q.cnt + 1.0) + 32.0 * q.cnt * q.jb) * nb);
@@ -660,7 +886,13 @@ int tags_ldl64_prepare() {
     static std::once_flag once;
     static int rc = 0;
     std::call_once(once, [] {
-        if (cudaFuncSetAttribute(k_ldl64_update<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (cudaFuncSetAttribute(k_ldl64_msolve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)MSOLVE_SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_ldl64_mresid, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)MSOLVE_SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_ldl64_msolve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)MSOLVE_SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_ldl64_update<64, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(2 * PB * 64 * sizeof(double2))) != cudaSuccess ||
             cudaFuncSetAttribute(k_ldl64_solve_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(SOLVE_N_MAX * sizeof(double2))) != cudaSuccess)
@@ -753,6 +985,56 @@ int tags_ldl64_sym_solve(const double2* W, double2* A, int m, int n, void* ws, i
     if (err) return err;
     k_ldl64_out<<<dim3((N + 127) / 128, 1), 128, 0, st>>>(w.x, m, n, w.conv, x, N, info);
     tags_note_launch();
+    TAGS_CUDA_OK(cudaGetLastError());
+    return 0;
+}
+
+size_t tags_ldl64_multi_workspace(int M, int R) {
+    return 2 * sizeof(double2) * (((size_t)(M + PB - 1) / PB + 2) * PB * PB + 2 * (size_t)M + 2 * (size_t)M * R +
+                                  (size_t)M * M) + 64;
+}
+
+int tags_ldl64_multi_solve(const double2* Z, const double2* rhs, int M, int n, int nb, double2* X, void* wsp,
+                           int* d_bad, cudaStream_t st) {
+    if (int e = tags_ldl64_prepare()) return e;
+    const int R = n + M, P = panel_count(M, 0);
+    const long long MM = (long long)M * M, MR = (long long)M * R, MN = (long long)M * n;
+    Ws w{};
+    w.wstride = (long long)((M + PB - 1) / PB + 2) * PB * PB;
+    w.linv = reinterpret_cast<double2*>(wsp);
+    double2* vu = w.linv + w.wstride * nb;           // nb x 2 x M
+    double2* A = vu + 2LL * M * nb;                  // nb x M x M, the factors
+    double2* Y = A + MM * nb;                        // nb x M x R
+    double2* E = Y + MR * nb;                        // nb x M x R
+    TAGS_CUDA_OK(cudaMemsetAsync(d_bad, 0, sizeof(int), st));
+    TAGS_CUDA_OK(cudaMemcpyAsync(A, Z, sizeof(double2) * MM * nb, cudaMemcpyDeviceToDevice, st));
+    for (int b = 0; b < nb && n > 0; ++b)
+        TAGS_CUDA_OK(cudaMemcpyAsync(X + MR * b, rhs + MN * b, sizeof(double2) * MN, cudaMemcpyDeviceToDevice, st));
+    k_ldl64_identity<<<dim3((unsigned)((MM + 255) / 256), nb), 256, 0, st>>>(X, M, n, MR);
+    tags_note_launch();
+    if (int e = factor(A, M, M, MM, nb, 0, w, st)) return e;
+    auto sweeps = [&](double2* x) {
+        for (int p = 0; p < P; ++p) {
+            const Panel q = panel_at(p, M, 0);
+            k_ldl64_msolve<false><<<dim3(q.cnt > 0 ? (q.cnt + 63) / 64 : 1, (R + PB - 1) / PB, nb), 128, MSOLVE_SMEM,
+                                    st>>>(A, M, MM, q, p, w.linv, w.wstride, x, Y, M, MR, R);
+        }
+        for (int p = P - 1; p >= 0; --p) {
+            const Panel q = panel_at(p, M, 0);
+            k_ldl64_msolve<true><<<dim3(q.j0 > 0 ? (q.j0 + 63) / 64 : 1, (R + PB - 1) / PB, nb), 128, MSOLVE_SMEM,
+                                   st>>>(A, M, MM, q, p, w.linv, w.wstride, Y, x, M, MR, R);
+        }
+    };
+    sweeps(X);
+    // one refinement of every column: the factors were taken without pivoting
+    // and the diagonal steps use inverses, so X alone is some times eps off
+    k_ldl64_mresid<<<dim3((M + 63) / 64, (R + PB - 1) / PB, nb), 128, MSOLVE_SMEM, st>>>(Z, M, MM, rhs, n, MN, X, E, MR,
+                                                                                      R);
+    sweeps(E);
+    k_ldl64_add<<<(unsigned)((MR * nb + 255) / 256), 256, 0, st>>>(X, E, MR * nb);
+    k_ldl64_check_sum<<<dim3((M + 3) / 4, nb), 128, 0, st>>>(X, rhs, M, n, MR, MN, vu);
+    k_ldl64_check<<<dim3((M + 3) / 4, nb), 128, 0, st>>>(Z, M, MM, vu, d_bad);
+    tags_note_launch(4 * P + 4);
     TAGS_CUDA_OK(cudaGetLastError());
     return 0;
 }

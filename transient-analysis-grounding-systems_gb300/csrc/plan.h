@@ -160,6 +160,16 @@ int tags_ldl64_saved_rhs(void* ws, int m, int n, int batch, int q, double2* out,
 // the factors, x the right-hand side and the solution; *d_flag is scratch
 int tags_ldl64_sym_solve(const double2* W, double2* A, int m, int n, void* ws, int* d_flag, double2* x, int* info,
                          cudaStream_t st);
+// nb full symmetric matrices Z (M x M): X = Z^-1 [rhs, I] (M x (n + M) each;
+// rhs M x n). *d_bad is raised when a check of the result finds it less
+// accurate than a pivoted solve would be.
+size_t tags_ldl64_multi_workspace(int M, int R);     // two matrices
+int tags_ldl64_multi_solve(const double2* Z, const double2* rhs, int M, int n, int nb, double2* X, void* ws,
+                           int* d_bad, cudaStream_t st);
+// capi.cu: x = W^-1 x for a caller's W (lower triangle read, original order) by
+// tags_ldl64_sym_solve; *done = 0 (x as it was) where the pivoted LU is wanted.
+// The caller holds the drop-in lock.
+int tags_sym_solve_host(const tags_cdouble* w, tags_cdouble* x, size_t m, size_t n, int* done);
 // the pivoted LU of one sample from the plan's coefficients slot q into W
 // (N x N), right-hand side and solution in x, info on the device
 int tags_plan_lu_one(tags_plan_s* p, int q, double2* W, int* ipiv, double2* x, int* info, cudaStream_t st);
