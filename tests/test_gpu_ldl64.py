@@ -37,10 +37,11 @@ def dense_solution(pkg, e, img, nodes, s, kappa, inj):
     return np.linalg.solve(w + np.tril(w, -1).T, b)
 
 
-@pytest.mark.parametrize("m", [1, 2, 10, 11, 31, 32, 33, 64, 65, 106, 107, 129])
+@pytest.mark.parametrize("m", [1, 2, 10, 11, 20, 21, 22, 31, 32, 33, 64, 65, 106, 107, 129])
 @pytest.mark.parametrize("graphs", [True, False])
 def test_plain_plan_matches_dense_solve(gpu_pkg, m, graphs):
-    """One-CTA solves up to N = 320 (m = 106), panel launches above."""
+    """One CTA per sample up to N = 64 (m = 21), one-CTA solves up to N = 320
+    (m = 106), panel launches above."""
     pkg = gpu_pkg
     e, nodes = wire(pkg, m)
     img = pkg.images(e)

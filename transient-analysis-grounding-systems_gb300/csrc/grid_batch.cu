@@ -384,6 +384,7 @@ extern "C" int tags_batch_run(tags_batch batch, const tags_grid_job* jobs, size_
             TAGS_CUDA_OK(cudaMemcpy(si.data(), g.d_info, sizeof(int) * g.ns, cudaMemcpyDeviceToHost));
             for (int k = 0; k < g.ns; ++k) {
                 if (si[k] != TAGS_INFO_RESOLVE) continue;
+                if (!p->d_ipiv) TAGS_CUDA_OK(cudaMalloc(&p->d_ipiv, sizeof(int) * (p->N + 1)));
                 int e = tags_plan_coef(p, g.d_s + k, g.d_k + k, b->mur, 1, p->stream);
                 if (!e) e = tags_plan_rhs(p, p->d_x, g.has_ie ? g.d_ie + (size_t)k * g.n : nullptr, (int)g.inj, 1, p->stream);
                 if (!e) e = tags_plan_lu_one(p, 0, p->d_W, p->d_ipiv, p->d_x, p->d_info, p->stream);

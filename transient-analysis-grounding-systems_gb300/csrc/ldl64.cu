@@ -14,8 +14,8 @@
 // is recovered by FP64 refinement against the untouched impedance blocks; a
 // sample whose corrections do not shrink to 1e-8 |x| (the next one would be
 // below FP64 rounding) is handed to the pivoted LU (lu.cu) by its caller.
-// Measured against that LU on GB300: 2 samples at m = 1560 714 -> 190 ms, 256
-// samples at m = 100 24.3 -> 8.4 ms, 100 samples at m = 10 0.66 -> 0.58 ms.
+// Measured against that LU on GB300: 2 samples at m = 1560 714 -> 162 ms, 256
+// samples at m = 100 24.3 -> 7.2 ms, 100 samples at m = 10 0.66 -> 0.29 ms.
 //
 // Layout: column-major N x N per sample, leading dimension ld. Lower triangle:
 // the matrix, then L; the strict upper triangle keeps U = D L^T of the panels
@@ -26,6 +26,7 @@
 // exactly. The panels' factored diagonal blocks live in the workspace (every
 // CTA of a panel launch factors the block itself, which saves a launch per
 // panel), then their inverses, so that a solve's diagonal step is a product.
+#include <algorithm>
 #include <mutex>
 
 #include "tags_common.cuh"
@@ -83,68 +84,86 @@ TAGS_D double2 crecip(double2 d) {
 }
 
 // Diagonal block and rows of one panel: L21 = A21 L11^-T D^-1 (stored in
-// place) and U12 = D L21^T (stored in the upper triangle). One thread per row;
-// every CTA factors the 32 x 32 block in shared memory first, CTA 0 also
-// stores it (L11, 1/D on the diagonal) for the solves. Bound by the FP64 pipe:
-// 1984 multiply-adds per row and ~20,000 SM cycles per block; CTAs of 64 rows
-// while that leaves SMs idle, else of 128 (half the repeated block work).
+// place) and U12 = D L21^T (stored in the upper triangle). Every CTA factors
+// the 32 x 32 block in shared memory first, CTA 0 also stores it (L11, 1/D on
+// the diagonal) for the solves. A warp's FP64 instruction holds its quarter of
+// the SM for 64 cycles, so time is the FP64 instructions of the busiest warp:
+// the block's columns go round the four warps, each forming the pivot's
+// reciprocal itself (one barrier per step), and four lanes share a row of L21,
+// eight columns each (576 instructions instead of a whole row's 1984 in one
+// thread: panels of m = 1560, 2 samples, 142 -> 70 us). `passes` groups of 32
+// rows per CTA: as few as fill the SMs, since the block's work is repeated.
 __global__ void __launch_bounds__(128) k_ldl64_panel(double2* __restrict__ A0, long long ld, long long stride,
-                                                     Panel q, int p, double2* __restrict__ ws0, long long wstride) {
+                                                     Panel q, int p, double2* __restrict__ ws0, long long wstride,
+                                                     int passes) {
     double2* A = A0 + stride * blockIdx.y;
     __shared__ double2 sL[PB][PB + 1];
-    __shared__ double2 sdi[PB], scol[PB];
-    const int tid = threadIdx.x;
-    for (int t = tid; t < PB * PB; t += blockDim.x) {
+    __shared__ double2 sdi[PB];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int t = tid; t < PB * PB; t += 128) {
         const int r = t % PB, c = t / PB;
         double2 v = cz(r == c ? 1.0 : 0.0, 0.0);          // a short panel is padded with the identity
         if (r < q.jb && c <= r) v = A[(q.j0 + r) + ld * (q.j0 + c)];
         sL[r][c] = v;
     }
+    if (tid < PB) sdi[tid] = cz(1.0, 0.0);
     __syncthreads();
     for (int k = 0; k < q.jb; ++k) {
-        if (tid < 32) {
-            const double2 di = crecip(sL[k][k]);
-            if (tid == 0) sdi[k] = di;
-            scol[tid] = cmul(sL[tid][k], di);             // rows above k are not used
-        }
-        __syncthreads();
-        const int w = q.jb - k - 1;
-        for (int t = tid; t < w * w; t += blockDim.x) {
-            const int r = k + 1 + t % w, c = k + 1 + t / w;
-            if (c <= r) sL[r][c] = cfma(cneg(scol[r]), sL[c][k], sL[r][c]);
-        }
+        const double2 di = crecip(sL[k][k]);
+        if (tid == 0) sdi[k] = di;
+        const double2 l = cneg(cmul(sL[lane][k], di));     // rows up to k are not used
+        for (int c = k + 1 + warp; c < q.jb; c += 4)
+            if (lane >= c) sL[lane][c] = cfma(l, sL[c][k], sL[lane][c]);
         __syncthreads();
     }
-    for (int k = q.jb + tid; k < PB; k += blockDim.x) sdi[k] = cz(1.0, 0.0);
-    __syncthreads();
-    for (int t = tid; t < PB * PB; t += blockDim.x) {     // unscaled columns -> L11
+    for (int t = tid; t < PB * PB; t += 128) {            // unscaled columns -> L11
         const int r = t % PB, c = t / PB;
         if (r > c && r < q.jb) sL[r][c] = cmul(sL[r][c], sdi[c]);
     }
     __syncthreads();
     if (blockIdx.x == 0) {
         double2* ws = ws0 + wstride * blockIdx.y + (long long)p * PB * PB;
-        for (int t = tid; t < PB * PB; t += blockDim.x) {
+        for (int t = tid; t < PB * PB; t += 128) {
             const int r = t % PB, c = t / PB;
             ws[c * PB + r] = r > c ? sL[r][c] : r == c ? sdi[c] : cz(0.0, 0.0);
         }
     }
-    const int v = blockIdx.x * blockDim.x + tid;
-    if (v >= q.cnt) return;
-    const int row = q.row(v);
-    double2 w[PB];
+    const int g = tid & 3;                                  // lane of the row's four: columns g, g + 4, ..
+    for (int pass = 0; pass < passes; ++pass) {
+        const int v0 = (blockIdx.x * passes + pass) * 32;
+        if (v0 >= q.cnt) return;                            // the whole CTA
+        const int v = v0 + (tid >> 2);
+        const bool on = v < q.cnt;
+        const int row = on ? q.row(v) : 0;
+        double2 w[PB / 4];
 #pragma unroll
-    for (int c = 0; c < PB; ++c) w[c] = c < q.jb ? A[row + ld * (q.j0 + c)] : cz(0.0, 0.0);
-#pragma unroll
-    for (int c = 1; c < PB; ++c)
-#pragma unroll
-        for (int k = 0; k < c; ++k) w[c] = cfma(cneg(w[k]), sL[c][k], w[c]);
-#pragma unroll
-    for (int c = 0; c < PB; ++c)
-        if (c < q.jb) {
-            A[row + ld * (q.j0 + c)] = cmul(w[c], sdi[c]);
-            A[(q.j0 + c) + ld * row] = w[c];
+        for (int i = 0; i < PB / 4; ++i) {
+            const int c = 4 * i + g;
+            w[i] = on && c < q.jb ? A[row + ld * (q.j0 + c)] : cz(0.0, 0.0);
         }
+#pragma unroll
+        for (int k = 0; k < PB - 1; ++k) {
+            if (k + 1 < q.jb) {                             // the same in every thread
+                const double2 wk = cz(-__shfl_sync(0xffffffffu, w[k / 4].x, k % 4, 4),
+                                      -__shfl_sync(0xffffffffu, w[k / 4].y, k % 4, 4));
+#pragma unroll
+                for (int i = k / 4; i < PB / 4; ++i) {
+                    const int c = 4 * i + g;
+                    if (c > k) w[i] = cfma(wk, sL[c][k], w[i]);
+                }
+            }
+        }
+        if (on) {
+#pragma unroll
+            for (int i = 0; i < PB / 4; ++i) {
+                const int c = 4 * i + g;
+                if (c < q.jb) {
+                    A[row + ld * (q.j0 + c)] = cmul(w[i], sdi[c]);
+                    A[(q.j0 + c) + ld * row] = w[i];
+                }
+            }
+        }
+    }
 }
 
 // Trailing update C -= L21 U12 over the lower triangle of the rows below the
@@ -208,87 +227,118 @@ __global__ void __launch_bounds__(TL * TL / (TT * TT)) k_ldl64_update(double2* _
 }
 
 // Inverses of the panels' unit lower blocks, in place (1/D stays on the
-// diagonal): a warp per panel and sample, lane = column of the inverse.
-__global__ void __launch_bounds__(32) k_ldl64_inv(double2* __restrict__ ws0, long long wstride) {
+// diagonal): a CTA per panel and sample, a lane per column of the inverse,
+// eight rows at a time: the four warps form the products with the rows above
+// (two rows each), then one warp's lanes finish the eight rows.
+__global__ void __launch_bounds__(128) k_ldl64_inv(double2* __restrict__ ws0, long long wstride) {
     double2* ws = ws0 + wstride * blockIdx.y + (long long)blockIdx.x * PB * PB;
-    __shared__ double2 L[PB][PB + 1];
-    const int c = threadIdx.x;
-    for (int k = 0; k < PB; ++k) L[c][k] = ws[k * PB + c];
-    __syncwarp();
-    double2 x[PB];
+    __shared__ double2 L[PB][PB + 1], X[PB][PB + 1];
+    const int c = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int t = threadIdx.x; t < PB * PB; t += 128) L[t % PB][t / PB] = ws[t];
+    __syncthreads();
+#pragma unroll 1
+    for (int r0 = 0; r0 < PB; r0 += 8) {
+        for (int r = r0 + 2 * warp; r < r0 + 2 * warp + 2; ++r) {
+            double2 v = cz(r == c ? 1.0 : 0.0, 0.0);
+            for (int k = 0; k < r0; ++k) v = cfma(cneg(L[r][k]), X[k][c], v);
+            X[r][c] = v;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            double2 x[8];
 #pragma unroll
-    for (int r = 0; r < PB; ++r) {
-        double2 v = cz(r == c ? 1.0 : 0.0, 0.0);
+            for (int i = 0; i < 8; ++i) {
+                double2 v = X[r0 + i][c];
 #pragma unroll
-        for (int k = 0; k < r; ++k) v = cfma(cneg(L[r][k]), x[k], v);   // x[k] = 0 for k < c
-        x[r] = v;
+                for (int k = 0; k < i; ++k) v = cfma(cneg(L[r0 + i][r0 + k]), x[k], v);
+                x[i] = v;
+                X[r0 + i][c] = v;
+            }
+        }
+        __syncthreads();
     }
-#pragma unroll
-    for (int r = 0; r < PB; ++r)
-        if (r > c) ws[c * PB + r] = x[r];
+    for (int t = threadIdx.x; t < PB * PB; t += 128) {
+        const int r = t % PB, k = t / PB;
+        if (r > k) ws[t] = X[r][k];
+    }
 }
 
-// y = L11^-1 x (upper = 0) or L11^-T x (upper = 1) for a panel's 32 values by
-// the block's first 32 threads; raw and y in shared memory.
-TAGS_D void block_apply(const double2* __restrict__ ws, const double2* raw, double2* y, int upper) {
-    const int r = threadIdx.x;
-    if (r >= PB) return;
-    double2 a = raw[r];
-    if (!upper) {
-        for (int k = 0; k < r; ++k) a = cfma(ws[k * PB + r], raw[k], a);
-    } else {
-        for (int k = r + 1; k < PB; ++k) a = cfma(ws[r * PB + k], raw[k], a);
+// y = L11^-1 x (upper = 0) or L11^-T x (upper = 1) for a panel's 32 values,
+// eight terms per thread in the CTA's first four warps; raw, y and part in
+// shared memory. Ends with a barrier.
+TAGS_D void block_apply(const double2* __restrict__ ws, const double2* raw, double2* y, double2 (*part)[PB], int upper) {
+    const int r = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (w < 4) {
+        double2 a = w == 0 ? raw[r] : cz(0.0, 0.0);
+        for (int k = 8 * w; k < 8 * w + 8; ++k)
+            if (upper ? k > r : k < r) a = cfma(ws[upper ? r * PB + k : k * PB + r], raw[k], a);
+        part[w][r] = a;
     }
-    y[r] = a;
+    __syncthreads();
+    if (threadIdx.x < PB) y[r] = cadd(cadd(part[0][r], part[1][r]), cadd(part[2][r], part[3][r]));
+    __syncthreads();
 }
 
 // One panel of the forward sweep: y = L11^-1 x_p (to Z), then x_r -= L_rp y
-// below it. 64 rows per CTA; x_p itself is left, so the CTAs agree on it.
-__global__ void __launch_bounds__(64) k_ldl64_fwd(const double2* __restrict__ A0, long long ld, long long stride,
-                                                  Panel q, int p, const double2* __restrict__ ws0, long long wstride,
-                                                  double2* __restrict__ X0, double2* __restrict__ Z0, int N,
-                                                  const int* __restrict__ active) {
+// below it. 32 rows per CTA, eight columns per warp; x_p itself is left, so the
+// CTAs agree on it.
+__global__ void __launch_bounds__(128) k_ldl64_fwd(const double2* __restrict__ A0, long long ld, long long stride,
+                                                   Panel q, int p, const double2* __restrict__ ws0, long long wstride,
+                                                   double2* __restrict__ X0, double2* __restrict__ Z0, int N,
+                                                   const int* __restrict__ active) {
     const int b = blockIdx.y;
     if (!active[b]) return;
     const double2* A = A0 + stride * b;
     double2* X = X0 + (long long)N * b;
-    __shared__ double2 raw[PB], y[PB];
-    if (threadIdx.x < PB) raw[threadIdx.x] = (int)threadIdx.x < q.jb ? X[q.j0 + threadIdx.x] : cz(0.0, 0.0);
+    __shared__ double2 raw[PB], y[PB], part[4][PB];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (threadIdx.x < PB) raw[lane] = lane < q.jb ? X[q.j0 + lane] : cz(0.0, 0.0);
     __syncthreads();
-    block_apply(ws0 + wstride * b + (long long)p * PB * PB, raw, y, 0);
-    __syncthreads();
+    block_apply(ws0 + wstride * b + (long long)p * PB * PB, raw, y, part, 0);
     if (blockIdx.x == 0 && (int)threadIdx.x < q.jb) Z0[(long long)N * b + q.j0 + threadIdx.x] = y[threadIdx.x];
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= q.cnt) return;
-    const int row = q.row(v);
+    const int v = blockIdx.x * 32 + lane;
+    const int row = v < q.cnt ? q.row(v) : 0;
     double2 acc = cz(0.0, 0.0);
-#pragma unroll 8
-    for (int c = 0; c < q.jb; ++c) acc = cfma(A[row + ld * (q.j0 + c)], y[c], acc);
-    X[row] = csub(X[row], acc);
+    if (v < q.cnt)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int c = 8 * w + i;
+            if (c < q.jb) acc = cfma(A[row + ld * (q.j0 + c)], y[c], acc);
+        }
+    part[w][lane] = acc;
+    __syncthreads();
+    if (w == 0 && v < q.cnt)
+        X[row] = csub(X[row], cadd(cadd(part[0][lane], part[1][lane]), cadd(part[2][lane], part[3][lane])));
 }
 
 // One panel of the backward sweep on T (which starts as D^-1 z): y = L11^-T
 // T_p (to S), then T_c -= L_pc^T y for the columns c0 .. j0 left of it.
-__global__ void __launch_bounds__(64) k_ldl64_bwd(const double2* __restrict__ A0, long long ld, long long stride,
-                                                  Panel q, int p, int c0, const double2* __restrict__ ws0,
-                                                  long long wstride, double2* __restrict__ T0,
-                                                  double2* __restrict__ S0, int N, const int* __restrict__ active) {
+__global__ void __launch_bounds__(128) k_ldl64_bwd(const double2* __restrict__ A0, long long ld, long long stride,
+                                                   Panel q, int p, int c0, const double2* __restrict__ ws0,
+                                                   long long wstride, double2* __restrict__ T0,
+                                                   double2* __restrict__ S0, int N, const int* __restrict__ active) {
     const int b = blockIdx.y;
     if (!active[b]) return;
     const double2* A = A0 + stride * b;
     double2* T = T0 + (long long)N * b;
-    __shared__ double2 raw[PB], y[PB];
-    if (threadIdx.x < PB) raw[threadIdx.x] = (int)threadIdx.x < q.jb ? T[q.j0 + threadIdx.x] : cz(0.0, 0.0);
+    __shared__ double2 raw[PB], y[PB], part[4][PB];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (threadIdx.x < PB) raw[lane] = lane < q.jb ? T[q.j0 + lane] : cz(0.0, 0.0);
     __syncthreads();
-    block_apply(ws0 + wstride * b + (long long)p * PB * PB, raw, y, 1);
-    __syncthreads();
+    block_apply(ws0 + wstride * b + (long long)p * PB * PB, raw, y, part, 1);
     if (blockIdx.x == 0 && (int)threadIdx.x < q.jb) S0[(long long)N * b + q.j0 + threadIdx.x] = y[threadIdx.x];
-    const int c = c0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= q.j0) return;
+    const int c = c0 + blockIdx.x * 32 + lane;
     double2 acc = cz(0.0, 0.0);
-#pragma unroll 8
-    for (int r = 0; r < q.jb; ++r) acc = cfma(A[(q.j0 + r) + ld * c], y[r], acc);
-    T[c] = csub(T[c], acc);
+    if (c < q.j0)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int r = 8 * w + i;
+            if (r < q.jb) acc = cfma(A[(q.j0 + r) + ld * c], y[r], acc);
+        }
+    part[w][lane] = acc;
+    __syncthreads();
+    if (w == 0 && c < q.j0)
+        T[c] = csub(T[c], cadd(cadd(part[0][lane], part[1][lane]), cadd(part[2][lane], part[3][lane])));
 }
 
 // T = D^-1 z (in place).
@@ -317,7 +367,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_ldl64_solve_cta(
     if (!active[b]) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* xs = reinterpret_cast<double2*>(smem_raw);     // N
-    __shared__ double2 raw[PB], y[PB];
+    __shared__ double2 raw[PB], y[PB], part[4][PB];
     const double2* A = A0 + stride * b;
     const double2* ws = ws0 + wstride * b;
     const int P = panel_count(N, m);
@@ -327,8 +377,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_ldl64_solve_cta(
         const Panel q = panel_at(p, N, m);
         if (threadIdx.x < PB) raw[threadIdx.x] = (int)threadIdx.x < q.jb ? xs[q.j0 + threadIdx.x] : cz(0.0, 0.0);
         __syncthreads();
-        block_apply(ws + (long long)p * PB * PB, raw, y, 0);
-        __syncthreads();
+        block_apply(ws + (long long)p * PB * PB, raw, y, part, 0);
         if ((int)threadIdx.x < q.jb) xs[q.j0 + threadIdx.x] = cmul(y[threadIdx.x],
                                                                    ws[(long long)p * PB * PB + threadIdx.x * (PB + 1)]);
         for (int v = threadIdx.x; v < q.cnt; v += blockDim.x) {
@@ -345,8 +394,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_ldl64_solve_cta(
         const int c0 = m > 0 && q.j0 >= m && q.j0 < 2 * m ? m : 0;
         if (threadIdx.x < PB) raw[threadIdx.x] = (int)threadIdx.x < q.jb ? xs[q.j0 + threadIdx.x] : cz(0.0, 0.0);
         __syncthreads();
-        block_apply(ws + (long long)p * PB * PB, raw, y, 1);
-        __syncthreads();
+        block_apply(ws + (long long)p * PB * PB, raw, y, part, 1);
         if ((int)threadIdx.x < q.jb) xs[q.j0 + threadIdx.x] = y[threadIdx.x];
         for (int c = c0 + threadIdx.x; c < q.j0; c += blockDim.x) {
             double2 acc = cz(0.0, 0.0);
@@ -523,6 +571,140 @@ __global__ void k_ldl64_resid_nodes(const Incidence inc, int m, int n, const dou
     R0[o] = csub(B0[o], acc);
 }
 
+// ---- small systems: one CTA per sample does it all
+
+constexpr int SMALL_N = 64;
+constexpr size_t small_smem(int N) { return sizeof(double2) * ((size_t)N * (N | 1) + 5 * (size_t)N); }
+
+// The whole solve of a sample with N <= 64 unknowns in shared memory: build,
+// LDL^T column by column (the columns of a step go round the four warps),
+// solves by one warp (a lane per row), refinement as in the launches above.
+// Bound by the FP64 instructions of a step's pivot and columns, ~2000 SM
+// cycles; 100 rods of 10 segments take 60 us where the panel launches took
+// ~450.
+__global__ void __launch_bounds__(128) k_ldl64_small(const double2* __restrict__ W0, long long ld, long long stride,
+                                                     const Incidence inc, int m, int n,
+                                                     const double2* rhs, double2* out,   // may be the same
+                                                     double2* __restrict__ saved, int* __restrict__ info) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int N = n + 2 * m, P = N | 1, b = blockIdx.x;
+    double2* A = reinterpret_cast<double2*>(smem_raw);     // (r, c) at c P + r
+    double2* bv = A + (size_t)N * P;
+    double2 *x = bv + N, *r = x + N, *dinv = r + N, *z = dinv + N;
+    __shared__ double smx[2][4];
+    __shared__ int sstate;                                  // 0: go on, 1: done, 2: to the pivoted LU
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const double2* W = W0 + stride * b;
+    for (int t = tid; t < N * P; t += 128) A[t] = cz(0.0, 0.0);
+    for (int i = tid; i < N; i += 128) {
+        const double2 v = rhs[(long long)N * b + orig_index(i, m, n)];
+        bv[i] = r[i] = v;
+        x[i] = cz(0.0, 0.0);
+        saved[(long long)N * b + i] = v;
+    }
+    __syncthreads();
+    for (int t = tid; t < 2 * m * m; t += 128) {
+        const int blk = t / (m * m), u = t - blk * m * m, c = u / m, i = u - c * m;
+        if (i >= c) A[(blk * m + c) * P + blk * m + i] = cneg(blk == 0 ? W[i + ld * (m + c)] : W[m + i + ld * c]);
+    }
+    for (int e = tid; e < m; e += 128)
+        for (int q = inc.seg_ptr[e]; q < inc.seg_ptr[e + 1]; ++q) {
+            A[e * P + 2 * m + inc.seg_node[q]] = cz((double)inc.seg_a[q], 0.0);
+            A[(m + e) * P + 2 * m + inc.seg_node[q]] = cz(0.5, 0.0);
+        }
+    __syncthreads();
+    for (int k = 0; k < N; ++k) {
+        const double2 di = crecip(A[k * P + k]);
+        if (tid == 0) dinv[k] = di;
+        // rows lane and lane + 32 of this warp's columns
+        const int r1 = lane + 32;
+        const double2 l0 = lane < N ? cneg(cmul(A[k * P + lane], di)) : cz(0.0, 0.0);
+        const double2 l1 = r1 < N ? cneg(cmul(A[k * P + r1], di)) : cz(0.0, 0.0);
+        for (int c = k + 1 + warp; c < N; c += 4) {
+            if (k < m && c >= m && c < 2 * m) continue;     // the ZL/ZT coupling stays zero
+            const double2 w = A[k * P + c];
+            if (c < 32 && lane >= c && lane < N) A[c * P + lane] = cfma(l0, w, A[c * P + lane]);
+            if (r1 >= c && r1 < N) A[c * P + r1] = cfma(l1, w, A[c * P + r1]);
+        }
+        __syncthreads();
+    }
+    for (int t = tid; t < N * N; t += 128) {
+        const int c = t / N, i = t - c * N;
+        if (i > c) A[c * P + i] = cmul(A[c * P + i], dinv[c]);
+    }
+    __syncthreads();
+    double prev = 0.0;
+    for (int step = 0; step < 4; ++step) {
+        if (step > 0) {
+            for (int i = tid; i < N; i += 128) {
+                double2 a = cz(0.0, 0.0), u = cz(0.0, 0.0);
+                if (i < 2 * m) {
+                    const int blk = i < m ? 0 : 1, k = i - blk * m;
+                    const double2* zc = W + (blk == 0 ? ld * m : (long long)m) + k;
+                    for (int j = 0; j < m; ++j) a = cfma(zc[ld * j], x[blk * m + j], a);
+                    for (int q = inc.seg_ptr[k]; q < inc.seg_ptr[k + 1]; ++q)
+                        u = cadd(u, cscale(x[2 * m + inc.seg_node[q]], blk == 0 ? (double)inc.seg_a[q] : 0.5));
+                } else {
+                    const int k = i - 2 * m;
+                    for (int q = inc.node_ptr[k]; q < inc.node_ptr[k + 1]; ++q)
+                        u = cadd(u, cadd(cscale(x[inc.node_seg[q]], (double)inc.node_a[q]),
+                                         cscale(x[m + inc.node_seg[q]], 0.5)));
+                }
+                r[i] = cadd(csub(bv[i], u), a);
+            }
+            __syncthreads();
+        }
+        if (warp == 0) {
+            for (int k = 0; k < N; ++k) {
+                const double2 rk = cneg(r[k]);
+                if (lane > k && lane < N) r[lane] = cfma(A[k * P + lane], rk, r[lane]);
+                if (lane + 32 > k && lane + 32 < N) r[lane + 32] = cfma(A[k * P + lane + 32], rk, r[lane + 32]);
+                __syncwarp();
+            }
+            for (int i = lane; i < N; i += 32) z[i] = cmul(r[i], dinv[i]);
+            __syncwarp();
+            for (int k = N - 1; k > 0; --k) {
+                const double2 zk = cneg(z[k]);
+                if (lane < k) z[lane] = cfma(A[lane * P + k], zk, z[lane]);
+                if (lane + 32 < k) z[lane + 32] = cfma(A[(lane + 32) * P + k], zk, z[lane + 32]);
+                __syncwarp();
+            }
+        }
+        __syncthreads();
+        double dn = 0.0, xn = 0.0;
+        bool bad = false;
+        for (int i = tid; i < N; i += 128) {
+            const double2 d = z[i], v = cadd(x[i], d);
+            x[i] = v;
+            bad = bad || !isfinite(cabs1(d)) || !isfinite(cabs1(v));
+            dn = fmax(dn, cabs1(d));
+            xn = fmax(xn, cabs1(v));
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            dn = fmax(dn, __shfl_xor_sync(0xffffffffu, dn, o));
+            xn = fmax(xn, __shfl_xor_sync(0xffffffffu, xn, o));
+        }
+        if (lane == 0) {
+            smx[0][warp] = dn;
+            smx[1][warp] = xn;
+        }
+        const int anybad = __syncthreads_or(bad);
+        if (tid == 0) {
+            dn = fmax(fmax(smx[0][0], smx[0][1]), fmax(smx[0][2], smx[0][3]));
+            xn = fmax(fmax(smx[1][0], smx[1][1]), fmax(smx[1][2], smx[1][3]));
+            sstate = 0;
+            if (anybad) sstate = 2;
+            else if (step > 0 && dn <= 1e-8 * xn) sstate = 1;
+            else if (step == 3 || (step > 0 && dn > 0.5 * prev)) sstate = 2;
+            prev = dn;
+        }
+        __syncthreads();
+        if (sstate) break;
+    }
+    for (int i = tid; i < N; i += 128) out[(long long)N * b + orig_index(i, m, n)] = x[i];
+    if (tid == 0) info[b] = sstate == 1 ? 0 : TAGS_INFO_RESOLVE;
+}
+
 // ---- a caller's symmetric matrix (full, original order)
 
 // Lower triangle in the static order; *coupled is raised by a nonzero entry
@@ -567,10 +749,11 @@ __global__ void __launch_bounds__(64) k_ldl64_resid_full(const double2* __restri
 // One panel of a sweep over R right-hand sides (columns of X, leading
 // dimension ldx): y = L11^-1 X_p (BWD: L11^-T X_p), to Y as D^-1 y (BWD: y),
 // then X_c -= L_cp y for the rows c below the panel (BWD: X_c -= L_pc^T y for
-// those above). 64 x 32 tiles; every tile forms its 32 columns of y itself, X_p
-// is left as it is. FP64-bound like the factorisation's updates.
-template <bool BWD>
-__global__ void __launch_bounds__(128) k_ldl64_msolve(const double2* __restrict__ A0, long long ld, long long stride,
+// those above). Tiles of 16 TA rows and 32 right-hand sides; every tile forms
+// its 32 columns of y itself (16 us of one SM's FP64 pipe, TA * 16 us for the
+// rest), X_p is left as it is. TA = 4 where that still fills the SMs, else 2.
+template <bool BWD, int TA>
+__global__ void __launch_bounds__(256) k_ldl64_msolve(const double2* __restrict__ A0, long long ld, long long stride,
                                                       Panel q, int p, const double2* __restrict__ ws0,
                                                       long long wstride, double2* __restrict__ X0,
                                                       double2* __restrict__ Y0, long long ldx, long long xstride,
@@ -581,17 +764,18 @@ __global__ void __launch_bounds__(128) k_ldl64_msolve(const double2* __restrict_
     double2* X = X0 + xstride * b;
     double2* Y = Y0 + xstride * b;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double2* sL = reinterpret_cast<double2*>(smem_raw);    // [PB][64]: L of the tile, k-major; first L11^-1
-    double2* raw = sL + PB * 64;                            // [PB][PB + 1]: X_p, k-major
+    constexpr int TC = 16 * TA;
+    double2* sL = reinterpret_cast<double2*>(smem_raw);    // [PB][TC]: L of the tile, k-major; first L11^-1
+    double2* raw = sL + PB * TC;                            // [PB][PB + 1]: X_p, k-major
     double2* y = raw + PB * (PB + 1);                       // [PB][PB + 1]
-    const int r0 = blockIdx.y * PB, c0 = blockIdx.x * 64, ncols = BWD ? q.j0 : q.cnt;
-    for (int t = threadIdx.x; t < PB * PB; t += 128) {
+    const int r0 = blockIdx.y * PB, c0 = blockIdx.x * TC, ncols = BWD ? q.j0 : q.cnt;
+    for (int t = threadIdx.x; t < PB * PB; t += 256) {
         const int k = t % PB, r = t / PB;
         raw[k * (PB + 1) + r] = (k < q.jb && r0 + r < R) ? X[q.j0 + k + ldx * (r0 + r)] : cz(0.0, 0.0);
         sL[t] = ws[t];                                      // (row, column) at column * PB + row
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < PB * PB; t += 128) {
+    for (int t = threadIdx.x; t < PB * PB; t += 256) {
         const int k = t / PB, r = t % PB;
         double2 a = raw[k * (PB + 1) + r];
         if (!BWD) {
@@ -605,37 +789,37 @@ __global__ void __launch_bounds__(128) k_ldl64_msolve(const double2* __restrict_
     }
     __syncthreads();
     if (c0 >= ncols) return;
-    for (int t = threadIdx.x; t < PB * 64; t += 128) {
-        const int c = BWD ? t / PB : t % 64, k = BWD ? t % PB : t / 64;
+    for (int t = threadIdx.x; t < PB * TC; t += 256) {
+        const int c = BWD ? t / PB : t % TC, k = BWD ? t % PB : t / TC;
         double2 v = cz(0.0, 0.0);
         if (k < q.jb && c0 + c < ncols)
             v = BWD ? A[(q.j0 + k) + ld * (c0 + c)] : A[q.base + c0 + c + ld * (q.j0 + k)];
-        sL[k * 64 + c] = v;
+        sL[k * TC + c] = v;
     }
     __syncthreads();
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    double2 acc[4][4];
+    double2 acc[TA][2];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < TA; ++a)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[a][e] = cz(0.0, 0.0);
+        for (int e = 0; e < 2; ++e) acc[a][e] = cz(0.0, 0.0);
     for (int k = 0; k < q.jb; ++k) {
-        double2 av[4], bv[4];
+        double2 av[TA], bv[2];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) av[a] = sL[k * 64 + tx + 16 * a];
+        for (int a = 0; a < TA; ++a) av[a] = sL[k * TC + tx + 16 * a];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) bv[e] = y[k * (PB + 1) + ty + 8 * e];
+        for (int e = 0; e < 2; ++e) bv[e] = y[k * (PB + 1) + ty + 16 * e];
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+        for (int a = 0; a < TA; ++a)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) acc[a][e] = cfma(av[a], bv[e], acc[a][e]);
+            for (int e = 0; e < 2; ++e) acc[a][e] = cfma(av[a], bv[e], acc[a][e]);
     }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const int r = r0 + ty + 8 * e;
+    for (int e = 0; e < 2; ++e) {
+        const int r = r0 + ty + 16 * e;
         if (r >= R) continue;
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
+        for (int a = 0; a < TA; ++a) {
             const int c = c0 + tx + 16 * a;
             if (c >= ncols) continue;
             double2* x = X + (BWD ? c : q.base + c) + ldx * r;
@@ -811,10 +995,12 @@ int factor(double2* A, int N, long long ld, long long stride, int nb, int m, con
     const int P = panel_count(N, m);
     for (int p = 0; p < P; ++p) {
         const Panel q = panel_at(p, N, m);
-        const int rows = (long long)nb * ((q.cnt + 63) / 64) > 608 ? 128 : 64;     // four CTAs of 64 per SM
-        const int ctas = q.cnt > 0 ? (q.cnt + rows - 1) / rows : 1;
+        // 32 rows per pass; up to four passes per CTA once the grid has one CTA per SM
+        const int groups = q.cnt > 0 ? (q.cnt + 31) / 32 : 1;
+        const int passes = (int)std::min<long long>(4, std::max<long long>(1, (long long)nb * groups / 152));
+        const int ctas = (groups + passes - 1) / passes;
         int pf = tags_prof_begin(TAGS_PROF_LU64_OTHER, st);
-        k_ldl64_panel<<<dim3(ctas, nb), rows, 0, st>>>(A, ld, stride, q, p, w.linv, w.wstride);
+        k_ldl64_panel<<<dim3(ctas, nb), 128, 0, st>>>(A, ld, stride, q, p, w.linv, w.wstride, passes);
         tags_prof_end(TAGS_PROF_LU64_OTHER, pf, st, 0.0, 0.0);
         tags_note_launch();
         if (q.cnt <= 0) continue;
@@ -835,7 +1021,7 @@ int factor(double2* A, int N, long long ld, long long stride, int nb, int m, con
                       (16.0 * q.cnt * (q.cnt + 1.0) + 32.0 * q.cnt * q.jb) * nb);
         tags_note_launch();
     }
-    k_ldl64_inv<<<dim3(P, nb), 32, 0, st>>>(w.linv, w.wstride);
+    k_ldl64_inv<<<dim3(P, nb), 128, 0, st>>>(w.linv, w.wstride);
     tags_note_launch();
     TAGS_CUDA_OK(cudaGetLastError());
     return 0;
@@ -860,7 +1046,7 @@ int solve(const double2* A, int N, long long ld, long long stride, int nb, int m
     TAGS_CUDA_OK(cudaMemsetAsync(w.z, 0, sizeof(double2) * N * nb, st));
     for (int p = p0; p < P; ++p) {
         const Panel q = panel_at(p, N, m);
-        k_ldl64_fwd<<<dim3(q.cnt > 0 ? (q.cnt + 63) / 64 : 1, nb), 64, 0, st>>>(A, ld, stride, q, p, w.linv,
+        k_ldl64_fwd<<<dim3(q.cnt > 0 ? (q.cnt + 31) / 32 : 1, nb), 128, 0, st>>>(A, ld, stride, q, p, w.linv,
                                                                                 w.wstride, w.r, w.z, N, w.active);
     }
     k_ldl64_dscale<<<dim3((N + 127) / 128, nb), 128, 0, st>>>(w.z, N, m, w.linv, w.wstride, w.active);
@@ -868,7 +1054,7 @@ int solve(const double2* A, int N, long long ld, long long stride, int nb, int m
     for (int p = P - 1; p >= 0; --p) {
         const Panel q = panel_at(p, N, m);
         const int c0 = m > 0 && q.j0 >= m && q.j0 < 2 * m ? m : 0, left = q.j0 - c0;
-        k_ldl64_bwd<<<dim3(left > 0 ? (left + 63) / 64 : 1, nb), 64, 0, st>>>(A, ld, stride, q, p, c0, w.linv,
+        k_ldl64_bwd<<<dim3(left > 0 ? (left + 31) / 32 : 1, nb), 128, 0, st>>>(A, ld, stride, q, p, c0, w.linv,
                                                                               w.wstride, w.z, w.r, N, w.active);
     }
     TAGS_CUDA_OK(cudaMemcpyAsync(w.z, w.r, sizeof(double2) * N * nb, cudaMemcpyDeviceToDevice, st));
@@ -886,12 +1072,14 @@ int tags_ldl64_prepare() {
     static std::once_flag once;
     static int rc = 0;
     std::call_once(once, [] {
-        if (cudaFuncSetAttribute(k_ldl64_msolve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)MSOLVE_SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(k_ldl64_mresid, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)MSOLVE_SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(k_ldl64_msolve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)MSOLVE_SMEM) != cudaSuccess ||
+        auto msolve_fits = [](const void* f) {
+            return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MSOLVE_SMEM) == cudaSuccess;
+        };
+        if (!msolve_fits((const void*)k_ldl64_msolve<false, 2>) || !msolve_fits((const void*)k_ldl64_msolve<false, 4>) ||
+            !msolve_fits((const void*)k_ldl64_msolve<true, 2>) || !msolve_fits((const void*)k_ldl64_msolve<true, 4>) ||
+            !msolve_fits((const void*)k_ldl64_mresid) ||
+            cudaFuncSetAttribute(k_ldl64_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)small_smem(SMALL_N)) != cudaSuccess ||
             cudaFuncSetAttribute(k_ldl64_update<64, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(2 * PB * 64 * sizeof(double2))) != cudaSuccess ||
             cudaFuncSetAttribute(k_ldl64_solve_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -927,6 +1115,12 @@ int tags_ldl64_plan_solve(double2* W, const Incidence& inc, int m, int n, int nb
     const int N = n + 2 * m;
     const long long NN = (long long)N * N;
     const Ws w = carve(ws, N, batch);
+    if (N <= SMALL_N) {
+        k_ldl64_small<<<nb, 128, small_smem(N), st>>>(W, N, NN, inc, m, n, rhs, x, w.b, info);
+        tags_note_launch();
+        TAGS_CUDA_OK(cudaGetLastError());
+        return 0;
+    }
     k_ldl64_start<<<dim3((N + 127) / 128, nb), 128, 0, st>>>(rhs, N, m, n, w.b, w.r, w.x, w.active, w.conv);
     k_ldl64_build<<<dim3(N, nb), 128, 0, st>>>(W, N, NN, inc, m, n);
     tags_note_launch(2);
@@ -1013,17 +1207,19 @@ int tags_ldl64_multi_solve(const double2* Z, const double2* rhs, int M, int n, i
     k_ldl64_identity<<<dim3((unsigned)((MM + 255) / 256), nb), 256, 0, st>>>(X, M, n, MR);
     tags_note_launch();
     if (int e = factor(A, M, M, MM, nb, 0, w, st)) return e;
+    const int rt = (R + PB - 1) / PB;
+    auto sweep = [&](bool bwd, const Panel& q, int p, double2* x, double2* y) {
+        const int cols = bwd ? q.j0 : q.cnt;
+        const bool wide = (long long)((cols + 63) / 64) * rt * nb >= 304;
+        const int tc = wide ? 64 : 32;
+        const dim3 g(cols > 0 ? (cols + tc - 1) / tc : 1, rt, nb);
+        auto kern = bwd ? (wide ? k_ldl64_msolve<true, 4> : k_ldl64_msolve<true, 2>)
+                        : (wide ? k_ldl64_msolve<false, 4> : k_ldl64_msolve<false, 2>);
+        kern<<<g, 256, MSOLVE_SMEM, st>>>(A, M, MM, q, p, w.linv, w.wstride, x, y, M, MR, R);
+    };
     auto sweeps = [&](double2* x) {
-        for (int p = 0; p < P; ++p) {
-            const Panel q = panel_at(p, M, 0);
-            k_ldl64_msolve<false><<<dim3(q.cnt > 0 ? (q.cnt + 63) / 64 : 1, (R + PB - 1) / PB, nb), 128, MSOLVE_SMEM,
-                                    st>>>(A, M, MM, q, p, w.linv, w.wstride, x, Y, M, MR, R);
-        }
-        for (int p = P - 1; p >= 0; --p) {
-            const Panel q = panel_at(p, M, 0);
-            k_ldl64_msolve<true><<<dim3(q.j0 > 0 ? (q.j0 + 63) / 64 : 1, (R + PB - 1) / PB, nb), 128, MSOLVE_SMEM,
-                                   st>>>(A, M, MM, q, p, w.linv, w.wstride, Y, x, M, MR, R);
-        }
+        for (int p = 0; p < P; ++p) sweep(false, panel_at(p, M, 0), p, x, Y);
+        for (int p = P - 1; p >= 0; --p) sweep(true, panel_at(p, M, 0), p, Y, x);
     };
     sweeps(X);
     // one refinement of every column: the factors were taken without pivoting

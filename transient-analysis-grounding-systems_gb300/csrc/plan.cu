@@ -172,8 +172,10 @@ static void plan_free(tags_plan_s* p) {
     if (p->d_fbpiv) cudaFree(p->d_fbpiv);
     if (p->d_pot) cudaFree(p->d_pot);
     if (p->d_coef1) cudaFree(p->d_coef1);
-    if (p->d_series) cudaFree(p->d_series);
-    if (p->d_ldl64) cudaFree(p->d_ldl64);
+    if (p->precision != TAGS_PLAIN_FP64) {       // parts of d_W in a plain plan
+        if (p->d_series) cudaFree(p->d_series);
+        if (p->d_ldl64) cudaFree(p->d_ldl64);
+    }
     if (p->d_iein) cudaFree(p->d_iein);
     if (p->ev0) cudaEventDestroy(p->ev0);
     if (p->ev1) cudaEventDestroy(p->ev1);
@@ -255,11 +257,15 @@ extern "C" int tags_plan_create(tags_plan* out, const Electrode* electrodes, con
     PLAN_CHECK(cudaMalloc(&p->d_x, sizeof(double2) * N * b));
     PLAN_CHECK(cudaMalloc(&p->d_sin, sizeof(double2) * 2 * b));
     if (precision == TAGS_PLAIN_FP64) {
-        err = tags_plan_series_alloc(p, p->batch);
-        if (err) { plan_free(p); return err; }
-        PLAN_CHECK(cudaMalloc(&p->d_ipiv, sizeof(int) * (N + 1)));
-        PLAN_CHECK(cudaMalloc(&p->d_ldl64, tags_ldl64_workspace(p->N, p->batch)));
-        PLAN_CHECK(cudaMalloc(&p->d_W, sizeof(double2) * (size_t)NN * b));
+        // one allocation: matrices, LDL^T workspace, the fill series' tables
+        const size_t wb = sizeof(double2) * (size_t)NN * b, lb = (tags_ldl64_workspace(p->N, p->batch) + 255) / 256 * 256;
+        p->series = tags_series_geometry(p->h_elec.data(), p->m, p->h_img.data(), p->h_img.empty() ? 0 : p->m);
+        PLAN_CHECK(cudaMalloc(&p->d_W, wb + lb + tags_series_workspace(p->series, p->batch)));
+        p->d_ldl64 = reinterpret_cast<char*>(p->d_W) + wb;
+        if (p->series.nbk) {
+            p->d_series = static_cast<char*>(p->d_ldl64) + lb;
+            p->series_ns = p->batch;
+        }
         err = tags_lu_prepare();
         if (!err) err = tags_ldl64_prepare();
         if (err) { plan_free(p); return err; }
@@ -362,6 +368,7 @@ static int finish_plain(tags_plan_s* p, int nb, cudaStream_t st) {
     for (int q = 0; q < nb; ++q) {
         if (info[q] != TAGS_INFO_RESOLVE) continue;
         double2* x = p->d_x + (size_t)q * p->N;
+        if (!p->d_ipiv) TAGS_CUDA_OK(cudaMalloc(&p->d_ipiv, sizeof(int) * (p->N + 1)));
         int err = tags_ldl64_saved_rhs(p->d_ldl64, p->m, p->n, p->batch, q, x, st);
         if (!err) err = tags_plan_lu_one(p, q, p->d_W, p->d_ipiv, x, p->d_info + q, st);
         if (err) return err;

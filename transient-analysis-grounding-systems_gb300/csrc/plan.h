@@ -54,11 +54,11 @@ struct tags_plan_s {
     SampleCoef* d_coef = nullptr;   // batch
     int* d_status = nullptr;        // 4 words
     int* d_info = nullptr;          // batch
-    int* d_ipiv = nullptr;          // N + 1 (pivoted LU of one sample)
+    int* d_ipiv = nullptr;          // N + 1 (pivoted LU of one sample, allocated with the first)
     double2* d_W = nullptr;         // plain: batch x N x N
-    void* d_ldl64 = nullptr;        // plain: workspace of the FP64 LDL^T
+    void* d_ldl64 = nullptr;        // workspace of the FP64 LDL^T (plain: part of d_W; mixed: with the first re-solve)
     SeriesGeo series;               // FP64 fill from per-pass moments (fill.cu) and its workspace,
-    void* d_series = nullptr;       // for series_ns samples (plain: the batch; mixed: 1, with the first FP64 re-solve)
+    void* d_series = nullptr;       // for series_ns samples (plain: the batch, part of d_W; mixed: 1, with the first re-solve)
     int series_ns = 0;
     double2* d_x = nullptr;         // batch x N (solution, FP64)
     // mixed form
