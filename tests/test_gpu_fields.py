@@ -161,3 +161,36 @@ def test_more_injections_than_one_pass(gpu_pkg, port):
             va = port.magnetic_potential(pts[p], d["elec"], il[0, r], d["gamma"][1], 1.0, 0, 1e-14, 1e-12)
             assert abs(out["pot"][0, p, r] - u) <= TOL * abs(u)
             assert _close(out["vecpot"][0, p, r], va) <= TOL
+
+
+@pytest.mark.parametrize("x", [0.05, 0.3, 0.6, 1.9, 2.1, 5.0])
+@pytest.mark.parametrize("ns,nrhs,m,P", [(1, 1, 1, 3), (3, 5, 7, 4), (33, 2, 40, 2), (130, 1, 3, 1)])
+def test_field_series_and_its_limits_match_oracle(gpu_pkg, port, x, ns, nrhs, m, P):
+    """Moment series with 12, 16 and 24 terms and the rule per sample past
+    their reach (x = |gamma| (L + L/8) / 2, 2.0), mixed in one call: the last
+    sample is ten times higher. Points near (within 2 L of) and far from the
+    electrodes; oracle at 1e-11, TOL of the largest magnitude."""
+    pkg = gpu_pkg
+    rng = np.random.default_rng(m)
+    e, _ = pkg.segment_electrode([0.0, 0.0, -0.5], [1.0 * m, 0.0, -0.5], m, 7e-3)
+    pts = np.stack([np.linspace(-0.3, 1.1 * m, P), np.full(P, 0.2), np.linspace(0.0, 30.0, P) - 0.4], axis=1)
+    gamma = x / 0.5625 * np.exp(0.25j * np.pi) * np.linspace(0.5, 1.0, ns)
+    if ns > 1:
+        gamma[-1] *= 10
+    kappa = np.full(ns, 0.01 + 1e-3j)
+    il, it = (rng.standard_normal((ns, nrhs, m)) + 1j * rng.standard_normal((ns, nrhs, m)) for _ in range(2))
+    il[0, 0, 0] = 1e-17                     # below DBL_EPSILON: skipped in the vector potential and the field
+    it[0, 0, 0] = 1e-17
+    out = pkg.fields_batch(pts, e, il, it, gamma, kappa)
+    assert out["status"] == 0
+    for k in sorted({0, ns // 2, ns - 1}):
+        for r in range(nrhs):
+            for p in range(P):
+                u = port.electric_potential(pts[p], e, it[k, r], gamma[k], kappa[k], req_abs=0.0, req_rel=1e-11)
+                va = port.magnetic_potential(pts[p], e, il[k, r], gamma[k], req_abs=0.0, req_rel=1e-11)
+                ve, _ = port.electric_field(pts[p], e, il[k, r], it[k, r], gamma[k], 0.0, kappa[k], req_abs=0.0,
+                                            req_rel=1e-11)
+                # e^{-gamma r} underflows at the far points of the high samples: what is below the
+                # smallest normal number carries fewer than 53 bits on either side
+                for got, want in ((out["pot"][k, p, r], u), (out["vecpot"][k, p, r], va), (out["efield"][k, p, r], ve)):
+                    assert np.max(np.abs(got - want)) <= TOL * np.max(np.abs(want)) + np.finfo(float).tiny

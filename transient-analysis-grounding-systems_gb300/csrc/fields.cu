@@ -31,6 +31,7 @@
 // [sample][point][injection]; vecpot and efield [sample][point][injection][3];
 // path voltages [sample][path][injection].
 #include <algorithm>
+#include <cmath>
 #include <complex>
 #include <cstring>
 #include <mutex>
@@ -85,6 +86,9 @@ struct FieldArgs {
     unsigned long long* evals;  // node x sample evaluations (work counter)
     int nchunk;             // electrode chunks (warps per point and sample group)
     double2* part;          // [nchunk][S][P][R][7] raw sums: pot, vec xyz, ef xyz
+    const int* nt;          // S: terms of the moment series (0: the rule per sample serves this one)
+    int schunk;             // the series' partial sums: [schunk][S][P][R][7]
+    double2* spart;
 };
 
 TAGS_D double warp_max(double v) {
@@ -118,7 +122,8 @@ __global__ void __launch_bounds__(FW * 32) k_fields(FieldArgs a, int r0) {
     const int e_end = (int)((long long)(chunk + 1) * a.m / a.nchunk);
     const int si = lane % G, sub = lane / G;
     const int smp = grp * G + si;
-    const bool valid = smp < a.S;
+    const bool valid = smp < a.S && a.nt[smp] == 0;   // the others take the moment series
+    if (!__any_sync(0xffffffffu, valid)) return;
     const int nr = min(RMAX, a.R - r0);
     const double2 gam = valid ? a.gamma[smp] : cz(0.0, 0.0);
     const double gmax = warp_max(valid ? sqrt(cabs2(gam)) : 0.0);
@@ -292,6 +297,268 @@ __global__ void __launch_bounds__(FW * 32) k_fields(FieldArgs a, int r0) {
     }
 }
 
+// ---- moment series over the samples ------------------------------------------------
+//
+// With r = R + d about R = b h, the multiple of h nearest the distance to the
+// electrode's midpoint, the three integrals of a (point, electrode) pair are
+//   e^{-gamma R} sum_n p_n M_n,   p_n = (-gamma)^n / n!,
+// for 1/r:                    N_n = \int d^n / r dt,
+// for (1 + gamma r) / r^3:    A_n = \int (d^n - n d^(n-1) r) / r^3 dt
+// (gamma r e^{-gamma d} contributes -n p_n d^(n-1) r), and B_n with the axial
+// offset as a further factor. The moments are geometry only: one rule per pair
+// serves all samples, a sample then costs 6 FP64 multiply-adds per term instead
+// of a complex exponential and ~30 operations per node. |d| <= Lmax / 2 + h / 2 =
+// dmax; terms up to x^n / n! <= 1e-17 at x = |gamma| dmax, at most FS_NT (x <= 2);
+// samples beyond keep the rule of k_fields.
+constexpr int FS_NT = 24;
+constexpr double FS_XMAX = 2.0;
+constexpr int FS_THREADS = 128;
+// |c| >= DBL_EPSILON = 2^-52 (the square's rounded root), without FP64 work for
+// the usual currents: a part of 2^-52 or more is seen in its exponent.
+TAGS_D bool cur_big(double2 c) {
+    const int hx = __double2hiint(c.x) & 0x7fffffff, hy = __double2hiint(c.y) & 0x7fffffff;
+    const int lim = (1023 - 52) << 20;
+    if (hx >= lim && hx < 0x7ff00000) return true;
+    if (hy >= lim && hy < 0x7ff00000 && hx < 0x7ff00000) return true;
+    return cabs2(c) >= 0x1.fffffffffffffp-105;      // the squares whose root rounds to 2^-52 or more
+}
+constexpr int FS_ORDERS[5] = {6, 7, 8, 9, 12};
+constexpr int FS_GL = 6 + 7 + 8 + 9 + 12;
+
+__constant__ double c_fsx[FS_GL], c_fsw[FS_GL];   // nodes and weights on [0, 1], order by order
+
+struct SerArgs {
+    FieldArgs f;
+    const double2* pw;      // [FS_NT][S]
+    const double2* tab;     // [bucket][S]: e^{-gamma b h}
+    double h;
+    int nbk, ngc, echunk;   // buckets; sample groups per CTA (1, 2, 4); electrodes per CTA
+};
+
+__global__ void k_fser_tables(const double2* __restrict__ gamma, const int* __restrict__ nt, int S, int nbk, double h,
+                              double2* __restrict__ pw, double2* __restrict__ tab) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
+    if (s >= S) return;
+    const double2 g = nt[s] > 0 ? gamma[s] : cz(0.0, 0.0);
+    if (b < nbk) {
+        tab[(long long)b * S + s] = cexp_d(cz(-g.x * (b * h), -g.y * (b * h)));
+        return;
+    }
+    double2 p = cz(1.0, 0.0);
+    for (int n = 0; n < FS_NT; ++n) {
+        pw[(long long)n * S + s] = n < nt[s] ? p : cz(0.0, 0.0);
+        p = cscale(cmul(p, cneg(g)), 1.0 / (double)(n + 1));
+    }
+}
+
+// What the samples need of a pair besides its moments.
+struct SerPair {
+    double D[3], wp[3], iL;     // electrode vector, offset of the point from its line, 1 / length
+    int b, bad;
+};
+
+// Moments of one (point, electrode) pair by one thread: Gauss-Legendre in t
+// where the point is at least two lengths away (6 to 12 nodes by the distance),
+// else the sinh rule above in panels of at most 0.75.
+template <int NT>
+TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, double h, int nbk, const double* gx,
+                         const double* gw, SerPair& q, double* mom) {
+    const double D[3] = {S.b[0] - S.a[0], S.b[1] - S.a[1], S.b[2] - S.a[2]};
+    const double L2 = D[0] * D[0] + D[1] * D[1] + D[2] * D[2], Lg = sqrt(L2);
+    const double w0[3] = {P0 - S.a[0], P1 - S.a[1], P2 - S.a[2]};
+    const double u0 = (w0[0] * D[0] + w0[1] * D[1] + w0[2] * D[2]) / L2;
+    double d2 = 0.0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        q.D[c] = D[c];
+        q.wp[c] = w0[c] - u0 * D[c];
+        d2 += q.wp[c] * q.wp[c];
+    }
+    q.iL = 1.0 / Lg;
+    const double uc = fmin(fmax(u0, 0.0), 1.0), du = (u0 - uc) * Lg;
+    const double dist = sqrt(d2 + du * du);
+    const double dm = (u0 - 0.5) * Lg, rc = sqrt(d2 + dm * dm);
+    q.b = min(nbk - 1, max(0, (int)rint(rc / h)));
+    const double R = q.b * h;
+    double aN[NT], aA[NT], aB[NT];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) aN[n] = aA[n] = aB[n] = 0.0;
+    auto node = [&](double s, double r2, double w) {       // axial offset from the foot, r^2, weight
+        const double ir = rsqrt(r2), r = r2 * ir, d = r - R, ir2 = ir * ir, ir3 = ir2 * ir;
+        double pn = w, pm = 0.0, c = 0.0;                  // w d^n, w d^(n-1), n / r^2
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            const double t = fma(-c, pm, pn * ir3);
+            aN[n] = fma(pn, ir, aN[n]);
+            aA[n] += t;
+            aB[n] = fma(t, s, aB[n]);
+            pm = pn;
+            pn *= d;
+            c += ir2;
+        }
+    };
+    q.bad = !(dist > 1e-12 * Lg) || !isfinite(rc);
+    if (!q.bad && dist >= 2.0 * Lg) {
+        const double ratio = dist * q.iL;
+        const int o = ratio >= 16.0 ? 0 : ratio >= 8.0 ? 1 : ratio >= 4.0 ? 3 : 4;
+        const int nq = o == 0 ? 6 : o == 1 ? 7 : o == 3 ? 9 : 12, off = o == 0 ? 0 : o == 1 ? 6 : o == 3 ? 21 : 30;
+        for (int i = 0; i < nq; ++i) {
+            const double s = (gx[off + i] - u0) * Lg;
+            node(s, fma(s, s, d2), gw[off + i]);
+        }
+    } else if (!q.bad) {
+        const double d = sqrt(d2), dp = fmax(d, 1e-6 * Lg);
+        const double va = asinh(-u0 * Lg / dp), vb = asinh((1.0 - u0) * Lg / dp);
+        // panels on either side of the foot, or one range
+        const bool split = va < 0.0 && vb > 0.0;
+        for (int side = 0; side < (split ? 2 : 1); ++side) {
+            const double lo = split && side == 1 ? 0.0 : va, hi = split && side == 0 ? 0.0 : vb;
+            const int np = max(1, (int)ceil(fmin((hi - lo) / 0.75, 64.0)));
+            const double ph = (hi - lo) / np;
+            for (int p = 0; p < np; ++p)
+                for (int i = 0; i < 8; ++i) {
+                    const double v = lo + (p + gx[13 + i]) * ph, s = dp * sinh(v);
+                    node(s, fma(s, s, d2), gw[13 + i] * ph * (dp * q.iL) * cosh(v));
+                }
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+        mom[n] = aN[n];
+        mom[NT + n] = aA[n];
+        mom[2 * NT + n] = aB[n];
+    }
+}
+
+// A CTA per (point, electrode chunk, four sample groups at most): FS_E electrodes
+// at a time, a thread forms a pair's moments, then the warps (sample group x
+// share of the electrodes; lanes: G samples x 32 / G electrodes) sum the series
+// and accumulate the currents' terms. FP64-bound: 6 nt + 24 multiply-adds per
+// (pair, sample) and 26 per injection. The 1560-segment grid, 251 points, 64
+// samples, 4 injections: 58.8 ms by the rule per sample, 14.2 ms so (error of the
+// field against 64-bit quadrature 1.6e-13 -> 2.2e-15).
+constexpr int FS_E = 128;                 // pairs per tile, a thread each
+template <int NT>
+__global__ void __launch_bounds__(FS_THREADS) k_fields_series(SerArgs sa, int r0) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double* mom = reinterpret_cast<double*>(smem_raw);              // [FS_E][3 NT]
+    __shared__ SerPair pr[FS_E];
+    __shared__ double gx[FS_GL], gw[FS_GL];
+    const FieldArgs& a = sa.f;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int p = blockIdx.x;
+    if (tid < FS_GL) {
+        gx[tid] = c_fsx[tid];
+        gw[tid] = c_fsw[tid];
+    }
+    const int G = a.G, NS = 32 / G, ngroups = (a.S + G - 1) / G;
+    const int nshare = (FS_THREADS / 32) / sa.ngc;
+    const int grp = blockIdx.z * sa.ngc + warp % sa.ngc, share = warp / sa.ngc;
+    const int si = lane % G, sub = lane / G, smp = grp * G + si;
+    const bool valid = grp < ngroups && smp < a.S && a.nt[smp] > 0;
+    const int nt = __reduce_max_sync(0xffffffffu, valid ? a.nt[smp] : 0);
+    const int nr = min(RMAX, a.R - r0);
+    const double P0 = a.pts[3 * p], P1 = a.pts[3 * p + 1], P2 = a.pts[3 * p + 2];
+    const bool wv = (a.want & (WANT_VEC | WANT_EF)) != 0;
+    const int e_begin = blockIdx.y * sa.echunk, e_end = min(a.m, e_begin + sa.echunk);
+
+    double2 pot[RMAX], vec[RMAX][3], ef[RMAX][3];
+#pragma unroll
+    for (int r = 0; r < RMAX; ++r) {
+        pot[r] = cz(0.0, 0.0);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) { vec[r][c] = cz(0.0, 0.0); ef[r][c] = cz(0.0, 0.0); }
+    }
+    for (int e0 = e_begin; e0 < e_end; e0 += FS_E) {
+        const int ne = min(FS_E, e_end - e0);
+        __syncthreads();
+        if (tid < ne) {
+            fser_moments<NT>(a.elec[e0 + tid], P0, P1, P2, sa.h, sa.nbk, gx, gw, pr[tid], mom + (size_t)tid * 3 * NT);
+            if (pr[tid].bad) raise_status(a.status, TAGS_ST_DEGENERATE_PAIR);
+        }
+        __syncthreads();
+        if (!valid) continue;
+        for (int el = share * NS + sub; el < ne; el += nshare * NS) {
+            const SerPair& q = pr[el];
+            const double* mo = mom + (size_t)el * 3 * NT;
+            double2 J1 = cz(0.0, 0.0), Ap = cz(0.0, 0.0), Bp = cz(0.0, 0.0);
+            for (int n = 0; n < nt; ++n) {
+                const double2 pn = sa.pw[(long long)n * a.S + smp];
+                J1.x = fma(pn.x, mo[n], J1.x);
+                J1.y = fma(pn.y, mo[n], J1.y);
+                if (wv) {
+                    Ap.x = fma(pn.x, mo[NT + n], Ap.x);
+                    Ap.y = fma(pn.y, mo[NT + n], Ap.y);
+                    Bp.x = fma(pn.x, mo[2 * NT + n], Bp.x);
+                    Bp.y = fma(pn.y, mo[2 * NT + n], Bp.y);
+                }
+            }
+            const double2 ex = sa.tab[(long long)q.b * a.S + smp];
+            J1 = cmul(J1, ex);
+            if (wv) {
+                Ap = cmul(Ap, ex);
+                Bp = cscale(cmul(Bp, ex), q.iL);
+            }
+            if (q.bad) J1 = Ap = Bp = cz(nan(""), nan(""));
+            double2 F[3];                                   // the field of a unit current
+            if (a.want & WANT_EF)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) F[c] = cz(Ap.x * q.wp[c] - Bp.x * q.D[c], Ap.y * q.wp[c] - Bp.y * q.D[c]);
+#pragma unroll
+            for (int r = 0; r < RMAX; ++r) {
+                if (r >= nr) break;
+                const long long ci = ((long long)(e0 + el) * a.R + r0 + r) * a.S + smp;
+                if (a.want & (WANT_POT | WANT_EF)) {
+                    const double2 ct = a.cur_t[ci];
+                    const bool big = cur_big(ct);
+                    if (!a.skip_pot || big) pot[r] = cfma(ct, J1, pot[r]);
+                    if ((a.want & WANT_EF) && big) {
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) ef[r][c] = cfma(ct, F[c], ef[r][c]);
+                    }
+                }
+                if (a.want & WANT_VEC) {
+                    const double2 cl = a.cur_l[ci];
+                    if (cur_big(cl)) {
+                        const double2 cj = cmul(cl, J1);
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            vec[r][c].x = fma(cj.x, q.D[c], vec[r][c].x);
+                            vec[r][c].y = fma(cj.y, q.D[c], vec[r][c].y);
+                        }
+                    }
+                }
+            }
+        }
+    }
+    // the electrode shares of a warp's lanes
+    for (int o = G; o < 32; o <<= 1) {
+#pragma unroll
+        for (int r = 0; r < RMAX; ++r) {
+            if (r >= nr) break;
+            pot[r] = cadd(pot[r], shfl_xor2(pot[r], o));
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                vec[r][c] = cadd(vec[r][c], shfl_xor2(vec[r][c], o));
+                ef[r][c] = cadd(ef[r][c], shfl_xor2(ef[r][c], o));
+            }
+        }
+    }
+    if (!valid || sub != 0) return;
+    const long long chunk = (long long)blockIdx.y * nshare + share;
+#pragma unroll
+    for (int r = 0; r < RMAX; ++r) {
+        if (r >= nr) break;
+        double2* o = a.spart + (((chunk * a.S + smp) * a.P + p) * a.R + r0 + r) * 7;
+        o[0] = pot[r];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            o[1 + c] = vec[r][c];
+            o[4 + c] = ef[r][c];
+        }
+    }
+}
+
 // Sum of the electrode chunks and the scale factors: 1 / (4 pi kappa) for the
 // potential and field, mur mu0 / (4 pi) for the vector potential.
 __global__ void k_fields_reduce(FieldArgs a) {
@@ -302,8 +569,11 @@ __global__ void k_fields_reduce(FieldArgs a) {
     double2 v[7];
 #pragma unroll
     for (int c = 0; c < 7; ++c) v[c] = cz(0.0, 0.0);
-    for (int ch = 0; ch < a.nchunk; ++ch) {
-        const double2* q = a.part + ((long long)ch * n + i) * 7;
+    const bool ser = a.nt[smp] > 0;
+    const double2* part = ser ? a.spart : a.part;
+    const int nchunk = ser ? a.schunk : a.nchunk;
+    for (int ch = 0; ch < nchunk; ++ch) {
+        const double2* q = part + ((long long)ch * n + i) * 7;
 #pragma unroll
         for (int c = 0; c < 7; ++c) v[c] = cadd(v[c], q[c]);
     }
@@ -446,6 +716,20 @@ int fields_tables(int dev) {
     tags_gauss_legendre(FQ, x, w);
     TAGS_CUDA_OK(cudaMemcpyToSymbol(c_fx, x, sizeof(x)));
     TAGS_CUDA_OK(cudaMemcpyToSymbol(c_fw, w, sizeof(w)));
+    double sx[FS_GL], sw[FS_GL];
+    int off = 0;
+    for (int q : FS_ORDERS) {
+        tags_gauss_legendre(q, sx + off, sw + off);
+        off += q;
+    }
+    TAGS_CUDA_OK(cudaMemcpyToSymbol(c_fsx, sx, sizeof(sx)));
+    TAGS_CUDA_OK(cudaMemcpyToSymbol(c_fsw, sw, sizeof(sw)));
+    const int smem = FS_E * 3 * (int)sizeof(double);            // per term
+    if (cudaFuncSetAttribute(k_fields_series<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem * 12) != cudaSuccess ||
+        cudaFuncSetAttribute(k_fields_series<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem * 16) != cudaSuccess ||
+        cudaFuncSetAttribute(k_fields_series<FS_NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem * FS_NT) !=
+            cudaSuccess)
+        return tags_fail(TAGS_E_CUDA, "cudaFuncSetAttribute(k_fields_series) failed");
     TAGS_CUDA_OK(cudaMalloc(&g_evals[dev], sizeof(unsigned long long)));
     TAGS_CUDA_OK(cudaMemset(g_evals[dev], 0, sizeof(unsigned long long)));
     g_tables_ready[dev] = true;
@@ -481,14 +765,92 @@ int field_chunks(size_t P, size_t ns, size_t R, size_t m, size_t part_cap) {
     return (int)std::max<size_t>(1, c);
 }
 
-int launch_fields(const FieldArgs& base, cudaStream_t st) {
+// Geometry of the moment series over a call's points and electrodes.
+struct SerGeo {
+    double h = 0.0, dmax = 0.0;
+    int nbk = 0;                  // 0: geometry that is not finite, no series
+};
+
+SerGeo series_geo(const double* pts, size_t P, const Seg* el, size_t m) {
+    SerGeo g;
+    double lo[3], hi[3], lmax = 0.0;
+    bool fine = true;
+    for (int c = 0; c < 3; ++c) {
+        lo[c] = INFINITY;
+        hi[c] = -INFINITY;
+    }
+    auto take = [&](const double* p) {
+        for (int c = 0; c < 3; ++c) {
+            fine = fine && std::isfinite(p[c]);
+            lo[c] = std::min(lo[c], p[c]);
+            hi[c] = std::max(hi[c], p[c]);
+        }
+    };
+    for (size_t p = 0; p < P; ++p) take(pts + 3 * p);
+    for (size_t e = 0; e < m; ++e) {
+        take(el[e].a);
+        take(el[e].b);
+        double l2 = 0.0;
+        for (int c = 0; c < 3; ++c) l2 += (el[e].b[c] - el[e].a[c]) * (el[e].b[c] - el[e].a[c]);
+        lmax = std::max(lmax, sqrt(l2));
+    }
+    double d2 = 0.0;
+    for (int c = 0; c < 3; ++c) d2 += (hi[c] - lo[c]) * (hi[c] - lo[c]);
+    if (!fine || !std::isfinite(d2) || !(lmax > 0.0)) return g;
+    g.h = std::max(lmax / 8.0, sqrt(d2) / 4000.0);
+    g.dmax = 0.5 * (lmax + g.h);
+    g.nbk = (int)(sqrt(d2) / g.h) + 2;
+    return g;
+}
+
+// Terms of the series at |gamma|, 0 past its reach: x^(n-1) / (n-1)! <= 1e-17
+// (one more than N_n alone needs, for the d^(n-1) of A_n).
+int series_terms(const SerGeo& g, zd gamma) {
+    const double x = std::abs(gamma) * g.dmax;
+    if (g.nbk == 0 || !(x <= FS_XMAX)) return 0;
+    double t = 1.0;
+    int n = 1;
+    while (n < FS_NT && t > 1e-17) t *= x / n++;
+    return std::min(n + 1, FS_NT);
+}
+
+// Electrode chunks of the series: CTAs for four per SM, at least 32
+// electrodes each, partial sums of at most part_cap bytes.
+void series_chunks(SerArgs* s, size_t part_cap) {
+    FieldArgs& a = s->f;
+    const int ngroups = (a.S + a.G - 1) / a.G;
+    s->ngc = ngroups >= 3 ? 4 : ngroups;
+    const long long ctas = (long long)a.P * ((ngroups + s->ngc - 1) / s->ngc);
+    const size_t per = 7 * sizeof(double2) * a.P * a.R * (size_t)a.S * (4 / s->ngc);
+    long long c = (152 * 4 + ctas - 1) / ctas;
+    c = std::min<long long>(c, std::max<long long>(1, (long long)(part_cap / std::max<size_t>(per, 1))));
+    c = std::min<long long>(c, (a.m + 31) / 32);
+    s->echunk = (int)((a.m + c - 1) / c);
+    a.schunk = (int)((a.m + s->echunk - 1) / s->echunk) * (4 / s->ngc);
+}
+
+// `direct`: samples past the series' reach are among these; `most`: the
+// series' largest number of terms (0: none of these samples takes it).
+int launch_fields(const SerArgs& sa, int most, bool direct, cudaStream_t st) {
+    const FieldArgs& base = sa.f;
     const int ngroups = (base.S + base.G - 1) / base.G;
     const long long items = (long long)base.P * ngroups * base.nchunk;
     if (items == 0 || base.m == 0) return 0;
     const long long blocks = (items + FW - 1) / FW;
     if (blocks > 0x7fffffffLL) return tags_fail(TAGS_E_ARG, "too many points x samples for one launch");
     const int pf = tags_prof_begin(TAGS_PROF_FIELDS, st);
-    for (int r0 = 0; r0 < base.R; r0 += RMAX) {
+    if (most > 0) {
+        const dim3 g((unsigned)base.P, (unsigned)(base.schunk / (4 / sa.ngc)), (unsigned)((ngroups + sa.ngc - 1) / sa.ngc));
+        for (int r0 = 0; r0 < base.R; r0 += RMAX) {
+            const size_t smem = FS_E * 3 * sizeof(double);
+            if (most <= 12) k_fields_series<12><<<g, FS_THREADS, smem * 12, st>>>(sa, r0);
+            else if (most <= 16) k_fields_series<16><<<g, FS_THREADS, smem * 16, st>>>(sa, r0);
+            else k_fields_series<FS_NT><<<g, FS_THREADS, smem * FS_NT, st>>>(sa, r0);
+            tags_note_launch();
+            TAGS_CUDA_OK(cudaGetLastError());
+        }
+    }
+    for (int r0 = 0; direct && r0 < base.R; r0 += RMAX) {
         k_fields<<<(unsigned)blocks, FW * 32, 0, st>>>(base, r0);
         tags_note_launch();
         TAGS_CUDA_OK(cudaGetLastError());
@@ -526,12 +888,38 @@ int fields_run(const FieldsIn& in) {
     const size_t P = in.P, m = in.m, R = in.R, S = in.S;
     const size_t per_sample = sizeof(double2) * (4 * R * m + P * R * 7 + 2);
     const size_t cs = chunk_samples(S, per_sample);
-    const int nchunk = field_chunks(P, cs, R, m, (size_t)1e9);
+    // samples of the moment series, and those past its reach
+    const SerGeo geo = series_geo(in.points, P, reinterpret_cast<const Seg*>(in.elec), m);
+    std::vector<int> nt(S);
+    bool any_direct = false, any_series = false;
+    for (size_t k = 0; k < S; ++k) {
+        nt[k] = series_terms(geo, zd(in.gamma[k].re, in.gamma[k].im));
+        any_direct = any_direct || nt[k] == 0;
+        any_series = any_series || nt[k] > 0;
+    }
+    const int nchunk = any_direct ? field_chunks(P, cs, R, m, (size_t)1e9) : 1;
+    auto series_args = [&](size_t ns) {
+        SerArgs s{};
+        s.f.P = (int)P;
+        s.f.m = (int)m;
+        s.f.R = (int)R;
+        s.f.S = (int)ns;
+        s.f.G = samples_per_warp(ns);
+        s.h = geo.h;
+        s.nbk = geo.nbk;
+        series_chunks(&s, (size_t)1e9);
+        return s;
+    };
+    // partial sums of either kernel, for the largest pass
+    size_t parts = any_direct ? (size_t)nchunk : 0;
+    if (any_series)
+        for (size_t s0 = 0; s0 < S; s0 += cs)
+            parts = std::max(parts, (any_direct ? (size_t)nchunk : 0) + (size_t)series_args(std::min(cs, S - s0)).f.schunk);
     double* d_pts = (double*)c->scratch(10, sizeof(double) * 3 * P + 16);
     Seg* d_el = (Seg*)c->scratch(11, sizeof(Seg) * m + 16);
     double2* d_cur = (double2*)c->scratch(12, sizeof(double2) * 4 * R * m * cs + 16);
-    double2* d_out = (double2*)c->scratch(13, sizeof(double2) * 7 * P * R * cs * (1 + (size_t)nchunk) + 16);
-    double2* d_gk = (double2*)c->scratch(14, sizeof(double2) * 2 * cs + 16);
+    double2* d_out = (double2*)c->scratch(13, sizeof(double2) * 7 * P * R * cs * (1 + parts) + 16);
+    double2* d_gk = (double2*)c->scratch(14, sizeof(double2) * ((2 + FS_NT + (size_t)geo.nbk) * cs) + sizeof(int) * cs + 16);
     if (!d_pts || !d_el || !d_cur || !d_out || !d_gk) return tags_fail(TAGS_E_NOMEM, "device allocation failed");
     TAGS_CUDA_OK(cudaMemcpyAsync(d_pts, in.points, sizeof(double) * 3 * P, cudaMemcpyHostToDevice, st));
     TAGS_CUDA_OK(cudaMemcpyAsync(d_el, in.elec, sizeof(Seg) * m, cudaMemcpyHostToDevice, st));
@@ -559,7 +947,21 @@ int fields_run(const FieldsIn& in) {
         }
         TAGS_CUDA_OK(cudaMemcpyAsync(d_gk, in.gamma + s0, sizeof(double2) * ns, cudaMemcpyHostToDevice, st));
         TAGS_CUDA_OK(cudaMemcpyAsync(d_gk + ns, in.kappa + s0, sizeof(double2) * ns, cudaMemcpyHostToDevice, st));
-        FieldArgs a{};
+        SerArgs sa = series_args(ns);
+        FieldArgs& a = sa.f;
+        double2* pw = d_gk + 2 * ns;
+        double2* tab = pw + (size_t)FS_NT * ns;
+        int* d_nt = reinterpret_cast<int*>(tab + (size_t)geo.nbk * ns);
+        TAGS_CUDA_OK(cudaMemcpyAsync(d_nt, nt.data() + s0, sizeof(int) * ns, cudaMemcpyHostToDevice, st));
+        const int most = *std::max_element(nt.begin() + s0, nt.begin() + s0 + ns);
+        if (most > 0) {
+            k_fser_tables<<<dim3((unsigned)((ns + 31) / 32), geo.nbk + 1), 32, 0, st>>>(d_gk, d_nt, (int)ns, geo.nbk,
+                                                                                    geo.h, pw, tab);
+            tags_note_launch();
+            TAGS_CUDA_OK(cudaGetLastError());
+        }
+        sa.pw = pw;
+        sa.tab = tab;
         a.pts = d_pts;
         a.elec = d_el;
         a.cur_t = cur_t;
@@ -567,11 +969,6 @@ int fields_run(const FieldsIn& in) {
         a.gamma = d_gk;
         a.kappa = d_gk + ns;
         a.mur = in.mur;
-        a.P = (int)P;
-        a.m = (int)m;
-        a.R = (int)R;
-        a.S = (int)ns;
-        a.G = samples_per_warp(ns);
         a.want = in.want;
         a.skip_pot = in.skip_pot;
         a.pot = d_out;
@@ -581,7 +978,9 @@ int fields_run(const FieldsIn& in) {
         a.evals = g_evals[c->device];
         a.nchunk = nchunk;
         a.part = d_out + 7 * P * R * ns;
-        if (int e = launch_fields(a, st)) return e;
+        a.nt = d_nt;
+        a.spart = a.part + 7 * P * R * ns * (any_direct ? (size_t)nchunk : 0);
+        if (int e = launch_fields(sa, most, any_direct, st)) return e;
         if (in.pot && (in.want & WANT_POT))
             TAGS_CUDA_OK(cudaMemcpyAsync(in.pot + s0 * P * R, a.pot, sizeof(double2) * P * R * ns,
                                          cudaMemcpyDeviceToHost, st));
