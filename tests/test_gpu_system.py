@@ -439,3 +439,37 @@ def test_solve_paths_match_in_plans(gpu_pkg, count, per_pass):
     for sol, it in out[1:]:
         assert np.array_equal(sol, out[0][0]) and it == out[0][1]
     assert np.max(np.abs(out[0][0][:, 0] - gd["u0"][idx]) / np.abs(gd["u0"][idx])) < 1e-6
+
+
+@pytest.mark.parametrize("nt", [3, 4, 5, 17, 96, 128, 255, 338, 1009, 2046, 4094, 6561, 7001])
+def test_many_series_inverse_laplace_matches_numpy(gpu_pkg, nt):
+    """Enough series for the mixed-radix transform (odd counts leave a single
+    series in the last pair; 1009 is prime and keeps the direct sums, 7001 is
+    past the shared-memory buffers), sizes 1e12 apart side by side, and a series
+    with an infinity and one with a NaN beside finite ones. Bound: 4e-16 nt of
+    each series' undamped transform."""
+    pkg = gpu_pkg
+    nser = 333
+    rng = np.random.default_rng(nt)
+    ns, tmax = nt // 2 + 1, 1e-4
+    s = np.log(float(nt) ** 2) / tmax + 2j * np.pi / tmax * np.arange(ns)
+    g = (rng.standard_normal((ns, nser)) + 1j * rng.standard_normal((ns, nser))) * 10.0 ** rng.uniform(-6, 6, nser)
+    for filt in (0, 2):
+        sigma = (1 + np.cos(np.pi * s.imag / s.imag[-1])) / 2 if filt else np.ones(ns)
+        x = sigma[:, None] * g
+        x[0].imag = 0
+        if nt % 2 == 0:
+            x[-1].imag = 0
+        dt = tmax / (nt - 1)
+        damp = np.exp(s[0].real * dt * np.arange(nt))[:, None] / dt
+        got = pkg.inv_laplace_batch(g, s, tmax, nt, filt) / damp
+        want = np.fft.irfft(x, n=nt, axis=0)
+        assert np.all(np.abs(got - want).max(axis=0) <= 4e-16 * nt * np.abs(want).max(axis=0) + 1e-300)
+    bad = g.copy()
+    bad[1, 4], bad[ns - 1, 7] = np.inf, np.nan
+    f = pkg.inv_laplace_batch(bad, s, tmax, nt, 0)
+    clean = pkg.inv_laplace_batch(g, s, tmax, nt, 0)
+    fine = np.ones(nser, bool)
+    fine[[4, 7]] = False
+    assert not np.isfinite(f[:, 4]).any() and np.isnan(f[:, 7]).all()
+    assert np.allclose(f[:, fine], clean[:, fine], rtol=0, atol=4e-16 * nt * np.abs(clean[:, fine]).max())

@@ -422,7 +422,7 @@ extern "C" int laplace_trans(double* f, tags_cdouble* g, tags_cdouble* s, double
     if (!c) return tags_fail(TAGS_E_CUDA, "no usable CUDA device");
     cudaStream_t st = c->stream;
     const size_t ns = nt / 2 + 1;
-    double2* d_tw = (double2*)c->scratch(6, sizeof(double2) * nt);
+    void* d_tw = c->scratch(6, tags_inlt_workspace((long long)nt));
     double* d_f = (double*)c->scratch(7, sizeof(double) * nt);
     double2* d_g = (double2*)c->scratch(8, sizeof(double2) * ns);
     if (!d_tw || !d_f || !d_g) return tags_fail(TAGS_E_NOMEM, "device allocation failed");
@@ -430,8 +430,7 @@ extern "C" int laplace_trans(double* f, tags_cdouble* g, tags_cdouble* s, double
     double cc = log(pow((double)nt, 2.0)) / tmax, dw = TAGS_TWO_PI / tmax;
     for (size_t k = 0; k < ns; ++k) s[k] = {cc, dw * (double)k};
     TAGS_CUDA_OK(cudaMemcpyAsync(d_f, f, sizeof(double) * nt, cudaMemcpyHostToDevice, st));
-    int err = tags_twiddles(d_tw, (long long)nt, st);
-    if (!err) err = tags_launch_nlt(d_f, 0, (long long)nt, d_tw, tmax, d_g, 0, 1, st);
+    int err = tags_launch_nlt(d_f, (long long)nt, d_tw, tmax, d_g, st);
     if (err) return err;
     TAGS_CUDA_OK(cudaMemcpyAsync(g, d_g, sizeof(double2) * ns, cudaMemcpyDeviceToHost, st));
     TAGS_CUDA_OK(cudaStreamSynchronize(st));
@@ -445,16 +444,14 @@ extern "C" int inv_laplace_trans(double* f, tags_cdouble* g, tags_cdouble* s, do
     if (!c) return tags_fail(TAGS_E_CUDA, "no usable CUDA device");
     cudaStream_t st = c->stream;
     const size_t ns = nt / 2 + 1;
-    double2* d_tw = (double2*)c->scratch(6, sizeof(double2) * nt);
+    void* d_tw = c->scratch(6, tags_inlt_workspace((long long)nt));
     double* d_f = (double*)c->scratch(7, sizeof(double) * nt);
     double2* d_g = (double2*)c->scratch(8, sizeof(double2) * ns * 2);
     if (!d_tw || !d_f || !d_g) return tags_fail(TAGS_E_NOMEM, "device allocation failed");
     TAGS_CUDA_OK(cudaMemcpyAsync(d_g, g, sizeof(double2) * ns, cudaMemcpyHostToDevice, st));
     TAGS_CUDA_OK(cudaMemcpyAsync(d_g + ns, s, sizeof(double2) * ns, cudaMemcpyHostToDevice, st));
-    int err = tags_twiddles(d_tw, (long long)nt, st);
-    if (!err)
-        err = tags_launch_inlt(d_g, 0, (long long)ns, d_g + ns, d_tw, (long long)nt, tmax,
-                               (filter >= 1 && filter <= 4) ? filter : 0, d_f, 0, 1, st);
+    int err = tags_launch_inlt(d_g, 0, 1, d_g + ns, d_tw, (long long)nt, tmax, (filter >= 1 && filter <= 4) ? filter : 0,
+                               d_f, 0, 1, 1, st);
     if (err) return err;
     TAGS_CUDA_OK(cudaMemcpyAsync(f, d_f, sizeof(double) * nt, cudaMemcpyDeviceToHost, st));
     TAGS_CUDA_OK(cudaStreamSynchronize(st));
@@ -475,9 +472,9 @@ extern "C" int tags_inv_laplace_batch(double* f, const tags_cdouble* g, const ta
     cudaStream_t st = c->stream;
     const bool dev = (flags & TAGS_RUN_DEVICE_PTRS) != 0;
     const size_t ns = nt / 2 + 1;
-    double2* d_tw = (double2*)c->scratch(6, sizeof(double2) * (nt + ns));
-    if (!d_tw) return tags_fail(TAGS_E_NOMEM, "device allocation failed");
-    double2* d_s = d_tw + nt;
+    double2* d_s = (double2*)c->scratch(6, sizeof(double2) * ns + tags_inlt_workspace((long long)nt));
+    if (!d_s) return tags_fail(TAGS_E_NOMEM, "device allocation failed");
+    void* d_tw = d_s + ns;
     const double2* d_g = reinterpret_cast<const double2*>(g);
     double* d_f = f;
     if (!dev) {
@@ -489,10 +486,9 @@ extern "C" int tags_inv_laplace_batch(double* f, const tags_cdouble* g, const ta
     }
     TAGS_CUDA_OK(cudaMemcpyAsync(d_s, s, sizeof(double2) * ns, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                                  st));
-    int err = tags_twiddles(d_tw, (long long)nt, st);
-    if (!err)
-        err = tags_launch_inlt_rows(d_g, (long long)ns, d_s, d_tw, (long long)nt, tmax,
-                                    (filter >= 1 && filter <= 4) ? filter : 0, d_f, (long long)nseries, st);
+    int err = tags_launch_inlt(d_g, 1, (long long)nseries, d_s, d_tw, (long long)nt, tmax,
+                               (filter >= 1 && filter <= 4) ? filter : 0, d_f, 1, (long long)nseries, (long long)nseries,
+                               st);
     if (err) return err;
     if (!dev) TAGS_CUDA_OK(cudaMemcpyAsync(f, d_f, sizeof(double) * nt * nseries, cudaMemcpyDeviceToHost, st));
     TAGS_CUDA_OK(cudaStreamSynchronize(st));

@@ -159,14 +159,13 @@ int tags_lu_solve_c(const float2* A, int n, long long ld, long long stride, int 
                     int nrhs, long long ldx, long long xstride, cudaStream_t st);
 
 // inlt.cu
-int tags_twiddles(double2* d_tw, long long nt, cudaStream_t st);
-int tags_launch_inlt(const double2* d_g, long long gstride, long long ns, const double2* d_s, const double2* d_tw,
-                     long long nt, double tmax, int filter, double* d_f, long long fstride, int nseries,
+// Inverse of nser series (samples at stride gk, series at gseries; outputs at
+// fj, fseries) and forward transform of one; ws: tables, tags_inlt_workspace(nt).
+size_t tags_inlt_workspace(long long nt);
+int tags_launch_inlt(const double2* d_g, long long gseries, long long gk, const double2* d_s, void* ws, long long nt,
+                     double tmax, int filter, double* d_f, long long fseries, long long fj, long long nser,
                      cudaStream_t st);
-int tags_launch_inlt_rows(const double2* d_g, long long ns, const double2* d_s, const double2* d_tw, long long nt,
-                          double tmax, int filter, double* d_f, long long nser, cudaStream_t st);
-int tags_launch_nlt(const double* d_f, long long fstride, long long nt, const double2* d_tw, double tmax,
-                    double2* d_g, long long gstride, int nseries, cudaStream_t st);
+int tags_launch_nlt(const double* d_f, long long nt, void* ws, double tmax, double2* d_g, cudaStream_t st);
 
 // ldl_tc.cu: tensor-core LDL^T of complex FP32 symmetric matrices (no pivoting)
 // Split forms of the tensor-core LDL^T (`pieces` argument of tags_ldl_tc):
