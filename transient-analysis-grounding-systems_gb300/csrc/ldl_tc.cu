@@ -1546,8 +1546,8 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_ldl_solve_cta(
 // 32 g .. 32 g + 31 of every 128-row block, and keeps them in its shared
 // memory. Per block and sweep: every CTA gathers the block's 128 values from
 // their owners (distributed shared memory), applies the block inverse to its
-// own rows, and after a cluster barrier gathers the new values and updates its
-// own rows outside the block. Each row's sums are formed in the order of the
+// own rows (kept apart until the barrier), and after a cluster barrier gathers
+// the new values and updates its own rows outside the block. Each row's sums are formed in the order of the
 // per-block kernels (identical results); the tail steps of a refinement, with
 // few samples still active, get G SMs per sample instead of one. Shared
 // memory: v (TB), part (4 TB), x (N) complex values; the cluster barriers are
@@ -1560,6 +1560,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_ldl_solve_cl(
     static_assert(G == 2 || G == 4 || G == 8, "cluster of 2, 4 or 8 CTAs");
     extern __shared__ float2 solve_sm[];
     __shared__ int s_smp;
+    __shared__ float2 zs[TB];                       // own rows of the block's solved values
     float2* v = solve_sm;
     float2* part = solve_sm + TB;
     float2* xs = solve_sm + 5 * TB;
@@ -1601,21 +1602,25 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_ldl_solve_cl(
     for (int i = tid; i < N; i += SOLVE_THREADS)
         if (own(i)) xs[i] = x[i];
     __syncthreads();
-    // v = the block's values x[j0 ..), zero beyond jb, read from their owners
-    auto gather = [&](int j0, int jb) {
+    // v = the block's values, zero beyond jb, read from their owners: x[j0 ..),
+    // or, solved, their zs. The solved values are kept apart until the barrier
+    // after inv_apply, so an owner never overwrites x values that another CTA
+    // has still to gather.
+    auto gather = [&](int j0, int jb, bool solved) {
         if (tid < TB) {
             float2 val = make_float2(0.f, 0.f);
             if (tid < jb) {
                 const int i = j0 + tid;
-                const uint32_t a = mapa_cta(smem_u32(xs + i), (uint32_t)((i >> 5) & (G - 1)));
+                const uint32_t a = mapa_cta(smem_u32(solved ? zs + tid : xs + i), (uint32_t)((i >> 5) & (G - 1)));
                 asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(val.x), "=f"(val.y) : "r"(a) : "memory");
             }
             v[tid] = val;
+            if (solved && tid < jb && own(j0 + tid)) xs[j0 + tid] = val;
         }
         __syncthreads();
     };
-    // own rows of z_b = M v (M[r][k] at Mt[k TB + r]), as k_blk_inv_apply:
-    // four quarter sums of 32 k each per row
+    // own rows of z_b = M v (M[r][k] at Mt[k TB + r]) to zs, as
+    // k_blk_inv_apply: four quarter sums of 32 k each per row
     auto inv_apply = [&](const float2* Mt, int j0, int jb) {
         for (int t = tid; t < 4 * TB; t += SOLVE_THREADS) {
             const int r = t & (TB - 1), qt = t >> 7, k0 = 32 * qt;
@@ -1634,7 +1639,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_ldl_solve_cl(
         __syncthreads();
         if (tid < jb && own(j0 + tid)) {
             const float2 a = part[tid], b = part[TB + tid], c = part[2 * TB + tid], d = part[3 * TB + tid];
-            xs[j0 + tid] = make_float2((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y));
+            zs[tid] = make_float2((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y));
         }
         __syncthreads();
     };
@@ -1642,10 +1647,10 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_ldl_solve_cl(
     for (int b = b0; b < nblk; ++b) {
         const int j0 = b * TB, jb = N - j0 < TB ? N - j0 : TB;
         cluster_sync_all();                        // the block's rows are updated by all earlier blocks
-        gather(j0, jb);
+        gather(j0, jb, false);
         inv_apply(Lv + (long long)b * 2 * TB * TB + TB * TB, j0, jb);
         cluster_sync_all();                        // every owner has applied the block inverse
-        gather(j0, jb);
+        gather(j0, jb, true);
         // own rows below the block, as k_blk_fwd_update (ZT rows skipped while
         // the block lies in the ZL columns)
         const int i_lo = j0 + jb;
@@ -1678,11 +1683,11 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_ldl_solve_cl(
     for (int b = nblk - 1; b >= 0; --b) {
         const int j0 = b * TB, jb = N - j0 < TB ? N - j0 : TB;
         cluster_sync_all();                        // the block's rows are updated by all later blocks
-        gather(j0, jb);
+        gather(j0, jb, false);
         inv_apply(Lv + (long long)b * 2 * TB * TB, j0, jb);
         cluster_sync_all();
+        gather(j0, jb, true);
         if (j0 == 0) break;
-        gather(j0, jb);
         // own rows above the block, as k_blk_bwd_update: a warp per 4
         // consecutive rows, 8 groups per own chunk
         const bool zero_cols = j0 >= zl_m && j0 + jb <= 2 * zl_m;   // L[ZT rows, ZL cols] = 0
@@ -1722,7 +1727,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_ldl_solve_cl(
             }
         }
     }
-    // the last cluster barrier followed every read of another CTA's x
+    cluster_sync_all();                            // no CTA leaves while another reads its zs
     for (int i = tid; i < N; i += SOLVE_THREADS)
         if (own(i)) x[i] = xs[i];
 }
