@@ -14,8 +14,8 @@
 // is recovered by FP64 refinement against the untouched impedance blocks; a
 // sample whose corrections do not shrink to 1e-8 |x| (the next one would be
 // below FP64 rounding) is handed to the pivoted LU (lu.cu) by its caller.
-// Measured against that LU on GB300: 2 samples at m = 1560 714 -> 162 ms, 256
-// samples at m = 100 24.3 -> 7.2 ms, 100 samples at m = 10 0.66 -> 0.29 ms.
+// Measured against that LU on GB300: 2 samples at m = 1560 714 -> 149 ms, 256
+// samples at m = 100 24.3 -> 6.7 ms, 100 samples at m = 10 0.66 -> 0.29 ms.
 //
 // Layout: column-major N x N per sample, leading dimension ld. Lower triangle:
 // the matrix, then L; the strict upper triangle keeps U = D L^T of the panels
@@ -173,14 +173,19 @@ __global__ void __launch_bounds__(128) k_ldl64_panel(double2* __restrict__ A0, l
 // per update is enough. The tile size sets the work wasted on the diagonal and
 // the edge, and with four or more warps per tile how long a launch of few
 // tiles takes at least: 131, 33 and 8 us for 64, 32 and 16.
+// The complex products as three real ones: with s = re + im of each operand,
+//   re = sum ar br - sum ai bi,  im = sum as bs - sum ar br - sum ai bi,
+// a quarter fewer FP64 instructions; the sums s are formed once per tile, in
+// shared memory. The imaginary part's rounding is then that of the larger part:
+// the refinement's residual takes the products in full.
 template <int TL, int TT>
 __global__ void __launch_bounds__(TL * TL / (TT * TT)) k_ldl64_update(double2* __restrict__ A0, long long ld,
-                                                               long long stride, Panel q) {
+                                                                   long long stride, Panel q) {
     double2* A = A0 + stride * blockIdx.y;
     constexpr int TH = TL / TT, NT = TH * TH;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double2* sA = reinterpret_cast<double2*>(smem_raw);    // [PB][TL]
-    double2* sB = sA + PB * TL;                            // [PB][TL]
+    double* sA = reinterpret_cast<double*>(smem_raw);      // [3][PB][TL]: re, im, re + im
+    double* sB = sA + 3 * PB * TL;                         // [3][PB][TL]
     const int t = blockIdx.x;
     int ty = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
     while (ty > 0 && ty * (ty + 1) / 2 > t) --ty;
@@ -188,27 +193,38 @@ __global__ void __launch_bounds__(TL * TL / (TT * TT)) k_ldl64_update(double2* _
     const int r0 = ty * TL, c0 = (t - ty * (ty + 1) / 2) * TL;
     for (int s = threadIdx.x; s < PB * TL; s += NT) {
         const int r = s % TL, k = s / TL;
-        sA[k * TL + r] = (k < q.jb && r0 + r < q.cnt) ? A[q.row(r0 + r) + ld * (q.j0 + k)] : cz(0.0, 0.0);
-        const int kk = s % PB, c = s / PB;
-        sB[kk * TL + c] = (kk < q.jb && c0 + c < q.cnt) ? A[(q.j0 + kk) + ld * q.row(c0 + c)] : cz(0.0, 0.0);
+        const double2 a = (k < q.jb && r0 + r < q.cnt) ? A[q.row(r0 + r) + ld * (q.j0 + k)] : cz(0.0, 0.0);
+        sA[s] = a.x;
+        sA[PB * TL + s] = a.y;
+        sA[2 * PB * TL + s] = a.x + a.y;
+        const int kk = s % PB, c = s / PB, o = kk * TL + c;
+        const double2 b = (kk < q.jb && c0 + c < q.cnt) ? A[(q.j0 + kk) + ld * q.row(c0 + c)] : cz(0.0, 0.0);
+        sB[o] = b.x;
+        sB[PB * TL + o] = b.y;
+        sB[2 * PB * TL + o] = b.x + b.y;
     }
     __syncthreads();
     const int tx = threadIdx.x % TH, tyy = threadIdx.x / TH;
-    double2 acc[TT][TT];
+    double acc[3][TT][TT];
 #pragma unroll
-    for (int a = 0; a < TT; ++a)
-#pragma unroll
-        for (int b = 0; b < TT; ++b) acc[a][b] = cz(0.0, 0.0);
-    for (int k = 0; k < q.jb; ++k) {
-        double2 av[TT], bv[TT];
-#pragma unroll
-        for (int a = 0; a < TT; ++a) av[a] = sA[k * TL + tx + TH * a];
-#pragma unroll
-        for (int b = 0; b < TT; ++b) bv[b] = sB[k * TL + tyy + TH * b];
+    for (int p = 0; p < 3; ++p)
 #pragma unroll
         for (int a = 0; a < TT; ++a)
 #pragma unroll
-            for (int b = 0; b < TT; ++b) acc[a][b] = cfma(av[a], bv[b], acc[a][b]);
+            for (int b = 0; b < TT; ++b) acc[p][a][b] = 0.0;
+    for (int k = 0; k < q.jb; ++k) {
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            double av[TT], bv[TT];
+#pragma unroll
+            for (int a = 0; a < TT; ++a) av[a] = sA[(p * PB + k) * TL + tx + TH * a];
+#pragma unroll
+            for (int b = 0; b < TT; ++b) bv[b] = sB[(p * PB + k) * TL + tyy + TH * b];
+#pragma unroll
+            for (int a = 0; a < TT; ++a)
+#pragma unroll
+                for (int b = 0; b < TT; ++b) acc[p][a][b] = fma(av[a], bv[b], acc[p][a][b]);
+        }
     }
 #pragma unroll
     for (int b = 0; b < TT; ++b) {
@@ -220,7 +236,8 @@ __global__ void __launch_bounds__(TL * TL / (TT * TT)) k_ldl64_update(double2* _
             const int gr = r0 + tx + TH * a;
             if (gr < q.cnt && gr >= gc) {
                 const long long idx = q.row(gr) + col;
-                A[idx] = csub(A[idx], acc[a][b]);
+                const double rr = acc[0][a][b], ii = acc[1][a][b];
+                A[idx] = csub(A[idx], cz(rr - ii, acc[2][a][b] - rr - ii));
             }
         }
     }
@@ -1009,13 +1026,13 @@ int factor(double2* A, int N, long long ld, long long stride, int nb, int m, con
         pf = tags_prof_begin(TAGS_PROF_LU64_GEMM, st);
         const long long t64 = (q.cnt + 63) / 64, t32 = (q.cnt + 31) / 32, t16 = (q.cnt + 15) / 16;
         if (t64 >= 10 && t64 * (t64 + 1) / 2 * nb >= 608)
-            k_ldl64_update<64, 4><<<dim3((unsigned)(t64 * (t64 + 1) / 2), nb), 256, 2 * PB * 64 * sizeof(double2), st>>>(
+            k_ldl64_update<64, 4><<<dim3((unsigned)(t64 * (t64 + 1) / 2), nb), 256, 6 * PB * 64 * sizeof(double), st>>>(
                 A, ld, stride, q);
         else if (t32 >= 10 && t32 * (t32 + 1) / 2 * nb >= 304)
-            k_ldl64_update<32, 2><<<dim3((unsigned)(t32 * (t32 + 1) / 2), nb), 256, 2 * PB * 32 * sizeof(double2), st>>>(
+            k_ldl64_update<32, 2><<<dim3((unsigned)(t32 * (t32 + 1) / 2), nb), 256, 6 * PB * 32 * sizeof(double), st>>>(
                 A, ld, stride, q);
         else
-            k_ldl64_update<16, 1><<<dim3((unsigned)(t16 * (t16 + 1) / 2), nb), 256, 2 * PB * 16 * sizeof(double2), st>>>(
+            k_ldl64_update<16, 1><<<dim3((unsigned)(t16 * (t16 + 1) / 2), nb), 256, 6 * PB * 16 * sizeof(double), st>>>(
                 A, ld, stride, q);
         tags_prof_end(TAGS_PROF_LU64_GEMM, pf, st, 4.0 * q.cnt * (q.cnt + 1.0) * q.jb * nb,
                       (16.0 * q.cnt * (q.cnt + 1.0) + 32.0 * q.cnt * q.jb) * nb);
@@ -1081,7 +1098,9 @@ int tags_ldl64_prepare() {
             cudaFuncSetAttribute(k_ldl64_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)small_smem(SMALL_N)) != cudaSuccess ||
             cudaFuncSetAttribute(k_ldl64_update<64, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(2 * PB * 64 * sizeof(double2))) != cudaSuccess ||
+                                 (int)(6 * PB * 64 * sizeof(double))) != cudaSuccess ||
+            cudaFuncSetAttribute(k_ldl64_update<32, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(6 * PB * 32 * sizeof(double))) != cudaSuccess ||
             cudaFuncSetAttribute(k_ldl64_solve_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(SOLVE_N_MAX * sizeof(double2))) != cudaSuccess)
             rc = tags_fail(TAGS_E_CUDA, "cudaFuncSetAttribute(k_ldl64) failed");
