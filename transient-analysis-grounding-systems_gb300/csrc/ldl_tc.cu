@@ -1401,14 +1401,18 @@ __global__ void k_diag_scale(const float2* __restrict__ A0, long long ld, long l
 
 // How the triangular solves run (tags_debug_solve_path): 0 the per-block
 // kernels; 1 k_ldl_solve_cta (one CTA per sample); 2, 4, 8 k_ldl_solve_cl
-// (a cluster of that many CTAs per sample); -1 (default) the larger of the
-// cluster sizes 4 and 2 with G x samples <= SMs, else one CTA per sample: with
+// (a cluster of that many CTAs per sample); -1 (default) the largest of the
+// cluster sizes 16 and 8 with G x samples <= SMs / 2 and all clusters resident,
+// else of 4 and 2 with G x samples <= SMs, else one CTA per sample: with
 // the SMs full, one CTA per sample already saturates HBM and clusters only add
 // barriers and waves (measured on the 1560-segment grid, 2048 samples in
 // passes of 128: solves 104 ms against 113, 134 and 209 ms for G = 2, 4, 8),
 // while a pass of few samples gets G SMs per sample (passes of 16: 51 ms with
 // one CTA, 35, 24 and 34 ms for G = 2, 4, 8; passes of 32: 39 ms, then 27, 20
-// and 41 ms). Paths 1.. need x in shared memory and fall back to the
+// and 41 ms). Half the SMs are where the larger clusters still gain, since a
+// few CTAs leave the memory idle: passes of 1, 4 and 8 samples of N = 17425 take
+// 62, 93 and 134 ms against 84, 114 and 148 ms with G = 4, those of N = 4537
+// 10.6, 11.5 and 13.0 ms against 11.7, 12.7 and 13.7 ms. Paths 1.. need x in shared memory and fall back to the
 // per-block kernels where it does not fit.
 static int g_solve_path = -1;
 
@@ -1541,7 +1545,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_ldl_solve_cta(
     for (int i = tid; i < N; i += SOLVE_THREADS) x[i] = xs[i];
 }
 
-// The solve of one sample on a cluster of G CTAs (G = 2, 4 or 8): CTA g owns
+// The solve of one sample on a cluster of G CTAs (G = 2, 4, 8 or 16): CTA g owns
 // the rows whose 32-row chunk index is g mod G, so for G = 4 it owns rows
 // 32 g .. 32 g + 31 of every 128-row block, and keeps them in its shared
 // memory. Per block and sweep: every CTA gathers the block's 128 values from
@@ -1557,7 +1561,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_ldl_solve_cl(
     const float2* __restrict__ A0, long long ld, long long mstride, int N, const float2* __restrict__ linv32,
     long long lstride, float2* __restrict__ x0, long long xstride, int zl_m, const int* __restrict__ active,
     const int* __restrict__ lead_step, int lead_zero, const int* __restrict__ nact, int few, int nb) {
-    static_assert(G == 2 || G == 4 || G == 8, "cluster of 2, 4 or 8 CTAs");
+    static_assert(G == 2 || G == 4 || G == 8 || G == 16, "cluster of 2, 4, 8 or 16 CTAs");
     extern __shared__ float2 solve_sm[];
     __shared__ int s_smp;
     __shared__ float2 zs[TB];                       // own rows of the block's solved values
@@ -1851,11 +1855,16 @@ static int set_gemm2_attr() {
 
 // Cluster solves: shared-memory size and whether a cluster of G CTAs with the
 // largest shared memory fits at all (else the one-CTA solve runs).
-static bool g_solve_cl_ok[9] = {};
+static int g_solve_cl_ok[17] = {};          // clusters of that size resident at once
 
 template <int G>
 static int set_solve_cl_attr() {
     TAGS_CUDA_OK(cudaFuncSetAttribute(k_ldl_solve_cl<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, SOLVE_SMEM_MAX));
+    if (G > 8 && cudaFuncSetAttribute(k_ldl_solve_cl<G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+                     cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(G);
     cfg.blockDim = dim3(SOLVE_THREADS);
@@ -1872,7 +1881,7 @@ static int set_solve_cl_attr() {
         cudaGetLastError();
         n = 0;
     }
-    g_solve_cl_ok[G] = n > 0;
+    g_solve_cl_ok[G] = n;
     return 0;
 }
 
@@ -1923,6 +1932,7 @@ int tags_ldl_tc_prepare() {
         if (!rc) rc = set_solve_cl_attr<2>();
         if (!rc) rc = set_solve_cl_attr<4>();
         if (!rc) rc = set_solve_cl_attr<8>();
+        if (!rc) rc = set_solve_cl_attr<16>();
         if (!rc && !encode_fn()) rc = tags_fail(TAGS_E_CUDA, "cuTensorMapEncodeTiled is not available");
     });
     return rc;
@@ -1991,8 +2001,8 @@ int tags_ldl_solve_c(const float2* A, int N, long long ld, long long mstride, in
     bool split = false;
     if (path < 0) {
         path = 1;
-        for (int G = 4; G >= 2; G /= 2)
-            if ((long long)nb * G <= num_sms() && g_solve_cl_ok[G]) {
+        for (int G = 16; G >= 2; G /= 2)
+            if ((long long)nb * G <= (G > 4 ? num_sms() / 2 : num_sms()) && g_solve_cl_ok[G] >= (G > 4 ? nb : 1)) {
                 path = G;
                 break;
             }
@@ -2007,8 +2017,10 @@ int tags_ldl_solve_c(const float2* A, int N, long long ld, long long mstride, in
                                                  lead_zero, nb, smem, st)
                 : path == 4 ? launch_solve_cl<4>(A, ld, mstride, N, L32, ls, x, xstride, zl_m, active, lead_step,
                                                  lead_zero, nb, smem, st)
-                            : launch_solve_cl<8>(A, ld, mstride, N, L32, ls, x, xstride, zl_m, active, lead_step,
-                                                 lead_zero, nb, smem, st);
+                : path == 8 ? launch_solve_cl<8>(A, ld, mstride, N, L32, ls, x, xstride, zl_m, active, lead_step,
+                                                 lead_zero, nb, smem, st)
+                            : launch_solve_cl<16>(A, ld, mstride, N, L32, ls, x, xstride, zl_m, active, lead_step,
+                                                  lead_zero, nb, smem, st);
         } else {
             const int few = split ? num_sms() / 4 : 0;
             k_ldl_solve_cta<<<nb, SOLVE_THREADS, smem, st>>>(A, ld, mstride, N, L32, ls, x, xstride, zl_m, active,
