@@ -263,3 +263,24 @@ def test_plan_fill_serves_samples_on_both_sides_of_the_series_limit(gpu_pkg):
         alone, info, _ = pkg.hem_sweep(e, pkg.images(e), nodes, s[k:k + 1], kappa[k:k + 1])
         assert not info.any()
         assert rel_err(together[k], alone[0]) < 1e-10
+
+
+@pytest.mark.parametrize("m", [1, 31, 33, 70])
+def test_mixed_fill_of_few_samples_matches_many(gpu_pkg, m):
+    """Passes of up to 16 samples put 2, 4 or 8 rows side by side in a warp:
+    every count against the same samples among 33 (entries are good to ~1e-13
+    either way, warps differ only in the terms past each sample's need)."""
+    pkg = gpu_pkg
+    e = bent_wire(pkg, m)
+    nodes = np.concatenate([e[:1, :3], e[:, 3:6]])
+    s = 8e4 + 2j * np.pi * np.linspace(1e4, 2e7, 33)
+    kappa = 0.005 + s * 12 * pkg.EPS0
+    plan = pkg.Plan(e, pkg.images(e), nodes, pkg.MIXED, 33)
+    try:
+        all_l, all_t = plan.mixed_fill(s, kappa)
+        for ns in (1, 2, 4, 5, 8, 9, 16, 17, 32):
+            zl, zt = plan.mixed_fill(s[:ns], kappa[:ns])
+            assert rel_err(zl, all_l[:ns]) < 1e-12
+            assert rel_err(zt, all_t[:ns]) < 1e-12
+    finally:
+        plan.close()

@@ -1683,6 +1683,81 @@ __global__ void __launch_bounds__(MOM_WARPS * 32) k_fill_moment(
     }
 }
 
+// The same for passes of at most 16 samples: a warp takes 32 / SW rows at a time,
+// its lanes SW samples of each, where the kernel above would leave lanes
+// without a sample idle (75 % of them for eight: 22.7 ms at m = 6150; passes of
+// 1, 4 and 8 samples at m = 6000 62, 93 and 134 -> 50, 75 and 119 ms in all).
+template <int SW>
+__global__ void __launch_bounds__(MOM_WARPS * 32) k_fill_moment_rows(
+    int m, const float* __restrict__ mom, const MomRec* __restrict__ rec, const MomCoef* __restrict__ coef,
+    const float4* __restrict__ tab, int tstride, int tnb, int nsamp, float2* zl0, float2* zt0, float2* zlo0,
+    float2* ztlo0, long long bstride, long long ntiles, int* status) {
+    constexpr int R = 32 / SW;                      // rows at a time
+    __shared__ float mv_all[MOM_WARPS][R][2][MOM_FLOATS + 1];
+    __shared__ MomRec rc_all[MOM_WARPS][R][2];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long tile = (long long)blockIdx.x * MOM_WARPS + warp;
+    if (tile >= ntiles) return;                      // whole warp leaves together
+    auto mv = mv_all[warp];
+    auto rcs = rc_all[warp];
+    int kb, i;
+    fill_tile(tile, m, kb, i);
+    const int r = lane / SW, smp = blockIdx.y * SW + lane % SW;
+    bool valid = smp < nsamp;
+    MomCoef c{};
+    if (valid) c = coef[smp];
+    valid = valid && c.ok;
+    if (!__any_sync(0xffffffffu, valid)) return;
+    const int ntw = __reduce_max_sync(0xffffffffu, valid ? c.nt : 0);
+    const long long pstart = (long long)i * (2LL * m - i + 1) / 2;
+    const int k_lo = max(i, 32 * kb), k_hi = min(m, 32 * kb + 32);
+    // the next rows' moments and records, read while these rows' series run
+    float nm[2 * R];
+    MomRec nrc{0, 0, 0.f, 0.f};
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int q = 0; q < 2 * R; ++q)
+            if (k0 + (q >> 1) < k_hi) nm[q] = mom[(2 * (pstart + k0 - i) + q) * MOM_FLOATS + lane];
+        if (lane < 2 * R && k0 + (lane >> 1) < k_hi) nrc = rec[2 * (pstart + k0 - i) + lane];
+    };
+#pragma unroll
+    for (int q = 0; q < 2 * R; ++q) nm[q] = 0.f;
+    fetch(k_lo);
+    for (int k0 = k_lo; k0 < k_hi; k0 += R) {
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 2 * R; ++q) mv[q >> 1][q & 1][lane] = nm[q];
+        if (lane < 2 * R) rcs[lane >> 1][lane & 1] = nrc;
+        __syncwarp();
+        fetch(k0 + R);
+        const int k = k0 + r;
+        if (k >= k_hi || !valid) continue;
+        CDF zt{DF{0.f, 0.f}, DF{0.f, 0.f}}, zl = zt;
+#pragma unroll
+        for (int kind = 0; kind < 2; ++kind) {
+            const MomRec rc = rcs[r][kind];
+            if (!rc.regular) continue;
+            const CDF S = mom_series(mv[r][kind], ntw, c);
+            const float4 tt = tab[((long long)kind * tnb + rc.b) * tstride + smp];
+            zt = cdf_add(zt, cdf_mul(CDF{DF{tt.x, tt.y}, DF{tt.z, tt.w}}, S));
+            const DF fl{rc.fl_hi, rc.fl_lo};
+            if (fl.h != 0.f) {
+                const float4 tl = tab[((long long)2 * tnb + rc.b) * tstride + smp];
+                const CDF lj = cdf_mul(CDF{DF{tl.x, tl.y}, DF{tl.z, tl.w}}, S);
+                zl = cdf_add(zl, CDF{df_mul(lj.re, fl), df_mul(lj.im, fl)});
+            }
+        }
+        zl = CDF{df_norm(zl.re), df_norm(zl.im)};
+        zt = CDF{df_norm(zt.re), df_norm(zt.im)};
+        const long long off = bstride * smp + k + (long long)m * i;
+        if (!isfinite(zl.re.h + zl.im.h + zt.re.h + zt.im.h)) raise_status(status, TAGS_ST_NONFINITE);
+        zl0[off] = make_float2(zl.re.h, zl.im.h);
+        zt0[off] = make_float2(zt.re.h, zt.im.h);
+        zlo0[off] = make_float2(zl.re.l, zl.im.l);
+        ztlo0[off] = make_float2(zt.re.l, zt.im.l);
+    }
+}
+
 __global__ void k_seg_dirs(const double* __restrict__ elec, const double* __restrict__ img, int m, int has_img,
                            float4* __restrict__ sdir, float4* __restrict__ idir) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1811,10 +1886,12 @@ int tags_launch_fill_mixed(const double* d_elec, const double* d_img, int m, voi
     k_coef32<<<(nsamp + 127) / 128, 128, 0, st>>>(d_coef, nsamp, w.c32);
     const int KB = (m + 31) / 32;
     const long long ntiles = 16LL * (KB - 1) * KB + m;
-    dim3 grid((unsigned)((ntiles + MOM_WARPS - 1) / MOM_WARPS), (unsigned)((nsamp + 31) / 32));
-    k_fill_moment<<<grid, MOM_WARPS * 32, 0, st>>>(m, mf.mom, reinterpret_cast<const MomRec*>(mf.rec), mc, mf.tab,
-                                                   mf.batch, mf.nb, nsamp, d_zl, d_zt, d_zlo, d_ztlo, bstride, ntiles,
-                                                   d_status);
+    const int sw = nsamp > 16 ? 32 : nsamp > 8 ? 16 : nsamp > 4 ? 8 : 4;     // samples side by side in a warp
+    auto moment = sw == 32 ? k_fill_moment : sw == 16 ? k_fill_moment_rows<16> : sw == 8 ? k_fill_moment_rows<8>
+                                                                                         : k_fill_moment_rows<4>;
+    dim3 grid((unsigned)((ntiles + MOM_WARPS - 1) / MOM_WARPS), (unsigned)((nsamp + sw - 1) / sw));
+    moment<<<grid, MOM_WARPS * 32, 0, st>>>(m, mf.mom, reinterpret_cast<const MomRec*>(mf.rec), mc, mf.tab, mf.batch,
+                                            mf.nb, nsamp, d_zl, d_zt, d_zlo, d_ztlo, bstride, ntiles, d_status);
     // samples the series does not reach: FP32 quadrature (warps with none leave at once)
     dim3 gq((unsigned)((ntiles + FILL_WARPS - 1) / FILL_WARPS), (unsigned)((nsamp + 31) / 32));
     k_fill_mixed<<<gq, FILL_WARPS * 32, 0, st>>>(d_elec, d_img, w.sdir, w.idir, m, w.codes, w.recs, w.c32, nsamp,
