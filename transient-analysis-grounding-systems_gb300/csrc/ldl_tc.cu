@@ -1129,6 +1129,7 @@ __global__ void __launch_bounds__(512, 1) k_ldl_diag(float2* __restrict__ A0, lo
     // A[j][k] for j > k.
 #pragma unroll
     for (int kq = 0; kq < 8; ++kq) {
+        if (16 * kq >= jb) break;                // the identity's steps change nothing
         for (int kw = 0; kw < 16; ++kw) {
             const int k = 16 * kq + kw, buf = k & 1;
             if (tx == (k & 31)) {                // row k of X, final since step k - 1
