@@ -817,6 +817,8 @@ int tags_mixed_finish(tags_plan_s* p, int nb, cudaStream_t st, int* h_iters, dou
         TAGS_CUDA_OK(cudaMemsetAsync(p->d_ldlerr, 0, 2 * sizeof(int), st));
     }
     if (h_steps) *h_steps = iri[3 * b];
+    // converged samples report success; fallbacks write their own info after
+    TAGS_CUDA_OK(cudaMemsetAsync(p->d_info, 0, sizeof(int) * nb, st));
     for (int q = 0; q < nb; ++q) {
         h_iters[q] = iri[2 * b + q];
         h_conv[q] = iri[b + q];
@@ -826,9 +828,6 @@ int tags_mixed_finish(tags_plan_s* p, int nb, cudaStream_t st, int* h_iters, dou
             if (err) return err;
         }
     }
-    // converged samples report success; fallbacks keep their own LU info
-    for (int q = 0; q < nb; ++q)
-        if (h_conv[q]) TAGS_CUDA_OK(cudaMemsetAsync(p->d_info + q, 0, sizeof(int), st));
     return 0;
 }
 
