@@ -139,3 +139,29 @@ def test_memory_budget_below_one_sample_reports_nomem(gpu_pkg):
         assert rel_err(sol[:, :n], plain[:, :n]) < 1e-6
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("m,ns", [(7, 1), (7, 70), (21, 65), (40, 33), (107, 3)])
+def test_resolves_side_by_side_match_plain(gpu_pkg, m, ns):
+    """Every sample re-solved in FP64 (one refinement step allowed), several at
+    a time (at most 64) and over both forms of the structured solve, with one
+    sample (s = 0) that needs the pivoted LU: equal to the plain form."""
+    pkg = gpu_pkg
+    z = -0.6 - 0.7 * np.arange(m + 1)
+    nodes = np.stack([0.5 * (np.arange(m + 1) % 2), np.zeros(m + 1), z], axis=1)
+    e = np.stack([pkg.populate_electrode(nodes[i], nodes[i + 1], 7e-3) for i in range(m)])
+    img = pkg.images(e)
+    s = 8e4 + 2j * np.pi * np.linspace(1e4, 5e6, ns)
+    kappa = 0.004 + s * 10 * pkg.EPS0
+    if ns > 2:
+        s[1], kappa[1] = 0.0, 0.004
+    ref, info, _ = pkg.hem_sweep(e, img, nodes, s, kappa, inj_node=1)
+    assert not info.any()
+    plan = pkg.Plan(e, img, nodes, pkg.MIXED, ns)
+    try:
+        plan.set_max_steps(1)
+        sol, info, st = plan.run(s, kappa, inj_node=1)
+        assert st.fallbacks == ns and not info.any()
+        assert np.max(np.abs(sol - ref)) < 1e-10 * np.max(np.abs(ref))
+    finally:
+        plan.close()

@@ -327,6 +327,8 @@ extern "C" int tags_batch_run(tags_batch batch, const tags_grid_job* jobs, size_
     acc.split = b->precision == TAGS_PLAIN_FP64 ? 0 : TAGS_SPLIT_F16;
     long long launched = b->launches_fixed;
     int first_err = 0, all_status = 0;
+    std::vector<std::vector<int>> failed(njobs);          // per grid: samples for the FP64 re-solve
+    std::vector<int> grid_status(njobs, 0);
     for (size_t q = 0; q < njobs; ++q) {
         const tags_grid_job& j = jobs[q];
         GridSlot& g = b->grids[q];
@@ -336,6 +338,7 @@ extern "C" int tags_batch_run(tags_batch batch, const tags_grid_job* jobs, size_
         int gst = 0;
         TAGS_CUDA_OK(cudaMemcpy(&gst, p->d_status, sizeof(int), cudaMemcpyDeviceToHost));
         all_status |= gst;
+        grid_status[q] = gst;
         if (b->precision != TAGS_PLAIN_FP64 && !gst) {
             const int bc = p->batch;
             std::vector<int> si((size_t)g.passes * (3 * bc + 2)), se(2 * (size_t)g.passes);
@@ -370,15 +373,34 @@ extern "C" int tags_batch_run(tags_batch batch, const tags_grid_job* jobs, size_
                     // not converged, or the pass's tensor-core factorisation
                     // reported an error: plain FP64 re-solve of this sample
                     acc.fallbacks++;
-                    const int k = k0 + s;
-                    int e = tags_mixed_fallback_one(p, g.d_s + k, g.d_k + k, b->mur,
-                                                    g.has_ie ? g.d_ie + (size_t)k * g.n : nullptr, (int)g.inj,
-                                                    g.d_sol + (size_t)k * g.N, g.d_info + k, p->stream);
-                    if (e) return e;
+                    failed[q].push_back(k0 + s);
                 }
             }
+            // queued on the grid's own stream: the grids' re-solves, chains of
+            // small launches, run side by side
+            if (!failed[q].empty())
+                if (int e = tags_mixed_fallback_start(p, failed[q], g.d_s, g.d_k, b->mur, g.has_ie ? g.d_ie : nullptr,
+                                                      (int)g.inj, g.d_sol, g.d_info, p->stream))
+                    return e;
+        }
+    }
+    for (size_t q = 0; q < njobs; ++q) {
+        const tags_grid_job& j = jobs[q];
+        GridSlot& g = b->grids[q];
+        tags_plan_s* p = g.plan;
+        if (!failed[q].empty()) {
             TAGS_CUDA_OK(cudaStreamSynchronize(p->stream));
-        } else if (!gst) {
+            std::vector<int> si(g.ns);
+            TAGS_CUDA_OK(cudaMemcpy(si.data(), g.d_info, sizeof(int) * g.ns, cudaMemcpyDeviceToHost));
+            for (int k : failed[q]) {
+                if (si[k] != TAGS_INFO_RESOLVE) continue;
+                int e = tags_mixed_fallback_lu(p, g.d_s + k, g.d_k + k, b->mur,
+                                               g.has_ie ? g.d_ie + (size_t)k * g.n : nullptr, (int)g.inj,
+                                               g.d_sol + (size_t)k * g.N, g.d_info + k, p->stream);
+                if (e) return e;
+            }
+            TAGS_CUDA_OK(cudaStreamSynchronize(p->stream));
+        } else if (b->precision == TAGS_PLAIN_FP64 && !grid_status[q]) {
             // plain form: samples marked for the pivoted LU
             std::vector<int> si(g.ns);
             TAGS_CUDA_OK(cudaMemcpy(si.data(), g.d_info, sizeof(int) * g.ns, cudaMemcpyDeviceToHost));

@@ -168,14 +168,9 @@ static void plan_free(tags_plan_s* p) {
     tags_plan_drop_graphs(p);
     if (p->d_sin) cudaFree(p->d_sin);
     if (p->d_stage) cudaFree(p->d_stage);
-    if (p->d_fbW) cudaFree(p->d_fbW);
-    if (p->d_fbpiv) cudaFree(p->d_fbpiv);
+    if (p->d_fb) cudaFree(p->d_fb);
     if (p->d_pot) cudaFree(p->d_pot);
     if (p->d_coef1) cudaFree(p->d_coef1);
-    if (p->precision != TAGS_PLAIN_FP64) {       // parts of d_W in a plain plan
-        if (p->d_series) cudaFree(p->d_series);
-        if (p->d_ldl64) cudaFree(p->d_ldl64);
-    }
     if (p->d_iein) cudaFree(p->d_iein);
     if (p->ev0) cudaEventDestroy(p->ev0);
     if (p->ev1) cudaEventDestroy(p->ev1);
@@ -280,15 +275,6 @@ extern "C" int tags_plan_create(tags_plan* out, const Electrode* electrodes, con
 
 extern "C" int tags_plan_destroy(tags_plan plan) {
     plan_free(plan);
-    return 0;
-}
-
-int tags_plan_series_alloc(tags_plan_s* p, int ns) {
-    if (p->series_ns >= ns) return 0;
-    p->series = tags_series_geometry(p->h_elec.data(), p->m, p->h_img.data(), p->h_img.empty() ? 0 : p->m);
-    if (p->series.nbk == 0) return 0;            // no series for this geometry: the direct rule serves it
-    TAGS_CUDA_OK(cudaMalloc(&p->d_series, tags_series_workspace(p->series, ns)));
-    p->series_ns = ns;
     return 0;
 }
 

@@ -56,9 +56,9 @@ struct tags_plan_s {
     int* d_info = nullptr;          // batch
     int* d_ipiv = nullptr;          // N + 1 (pivoted LU of one sample, allocated with the first)
     double2* d_W = nullptr;         // plain: batch x N x N
-    void* d_ldl64 = nullptr;        // workspace of the FP64 LDL^T (plain: part of d_W; mixed: with the first re-solve)
+    void* d_ldl64 = nullptr;        // plain: workspace of the FP64 LDL^T (part of d_W)
     SeriesGeo series;               // FP64 fill from per-pass moments (fill.cu) and its workspace,
-    void* d_series = nullptr;       // for series_ns samples (plain: the batch, part of d_W; mixed: 1, with the first re-solve)
+    void* d_series = nullptr;       // for series_ns samples (plain: the batch, part of d_W; mixed: part of d_fb)
     int series_ns = 0;
     double2* d_x = nullptr;         // batch x N (solution, FP64)
     // mixed form
@@ -109,8 +109,8 @@ struct tags_plan_s {
     // threads): host-input staging of kernel-by-kernel passes, FP64 fallback
     double2* d_stage = nullptr;
     size_t stage_bytes = 0;
-    double2* d_fbW = nullptr;       // N x N (allocated on the first fallback)
-    int* d_fbpiv = nullptr;         // N + 1
+    void* d_fb = nullptr;           // FP64 re-solves of fb_cap samples at a time (allocated with the first)
+    int fb_cap = 0, fb_full = 0;    // fb_full: no room for more
     // host copy of the geometry (11 doubles per segment; nodes 3 per node), so
     // a twin plan can be built from it
     std::vector<double> h_elec, h_img, h_nodes;
@@ -134,15 +134,16 @@ int tags_mixed_ir_setup(tags_plan_s* p, int nb, cudaStream_t st);
 int tags_mixed_ir_step(tags_plan_s* p, int nb, cudaStream_t st, cudaGraphConditionalHandle cond, int set_cond);
 int tags_mixed_finish(tags_plan_s* p, int nb, cudaStream_t st, int* h_iters, double* h_berr, int* h_conv,
                       int* h_steps);
-// Plain FP64 re-solve of one sample (inputs on the device) into x_out / info_out.
-int tags_mixed_fallback_one(tags_plan_s* p, const double2* d_s, const double2* d_kappa, double mur,
-                            const double2* d_ie, int inj_node, double2* x_out, int* info_out, cudaStream_t st);
+// Plain FP64 re-solves of samples idx of a sweep (inputs and outputs on the
+// device, sample by sample), queued on st; info TAGS_INFO_RESOLVE asks for
+// tags_mixed_fallback_lu of that sample (its own inputs and outputs).
+int tags_mixed_fallback_start(tags_plan_s* p, const std::vector<int>& idx, const double2* d_s, const double2* d_kappa,
+                              double mur, const double2* d_ie, int inj_node, double2* x, int* info, cudaStream_t st);
+int tags_mixed_fallback_lu(tags_plan_s* p, const double2* d_s, const double2* d_kappa, double mur, const double2* d_ie,
+                           int inj_node, double2* x_out, int* info_out, cudaStream_t st);
 // While-node after the work captured so far on `st` (condition 1 at launch);
 // its body graph is returned for a separate capture.
 int tags_plan_add_while_node(cudaStream_t st, cudaGraphConditionalHandle* cond, cudaGraph_t* body);
-// The FP64 moment series' geometry and workspace for up to ns samples (once per plan).
-int tags_plan_series_alloc(tags_plan_s* p, int ns);
-
 // ldl64.cu: FP64 LDL^T in the static order with refinement (plain form). A
 // sample whose corrections do not shrink gets info = TAGS_INFO_RESOLVE: its
 // caller solves it by the pivoted LU.
