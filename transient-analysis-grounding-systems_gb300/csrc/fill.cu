@@ -310,8 +310,7 @@ __global__ void __launch_bounds__(128) k_fill_fp64(const double* __restrict__ el
                                                    const double* __restrict__ img, int m,
                                                    const SampleCoef* __restrict__ coef, int nsamp,
                                                    FillOut out, int mode, int itype, int tight,
-                                                   int* status, const int* __restrict__ done) {
-    if (done && done[blockIdx.y]) return;          // the moment series served this sample
+                                                   int* status) {
     __shared__ double sx[GL_TOTAL], sw[GL_TOTAL];
     for (int t = threadIdx.x; t < GL_TOTAL; t += blockDim.x) { sx[t] = g_glx[t]; sw[t] = g_glw[t]; }
     __syncthreads();
@@ -379,8 +378,7 @@ __global__ void __launch_bounds__(128) k_fill_fp64(const double* __restrict__ el
 __global__ void __launch_bounds__(128) k_path_pairs(const double* __restrict__ elec, int m,
                                                     const double* __restrict__ paths, int npaths,
                                                     const SampleCoef* __restrict__ coef, double2* __restrict__ jj,
-                                                    int* status, const int* __restrict__ done) {
-    if (done && done[blockIdx.y]) return;          // the moment series served this sample
+                                                    int* status) {
     __shared__ double sx[GL_TOTAL], sw[GL_TOTAL];
     for (int t = threadIdx.x; t < GL_TOTAL; t += blockDim.x) { sx[t] = g_glx[t]; sw[t] = g_glw[t]; }
     __syncthreads();
@@ -412,7 +410,8 @@ __global__ void __launch_bounds__(128) k_path_pairs(const double* __restrict__ e
 // \int_0^1 (t rho - R)^n dt = g_n / (n + 1), g_n = sum_i (rho - R)^i (-R)^(n-i).
 // Terms: x^nt / nt! <= 1e-17 at x = max |gamma| dmax (16 up to x ~ 0.75, else
 // 32, which reach x = 3.5, where the sum's largest term is e^3.5 of N_0 and
-// the rounding ~1e-14 of the entry). Samples beyond that keep the direct rule.
+// the rounding ~1e-14 of the entry). Samples beyond that keep an exponential per
+// point (k_fill_far).
 // Measured on GB300 against the direct rule for every sample: the plain form's
 // pass of 256 samples at m = 100 217 -> 24.3 ms, 100 samples at m = 10 3.50 ->
 // 0.66 ms, one sample at m = 100 through the drop-ins 11.9 -> 6.7 ms (the fill
@@ -428,6 +427,7 @@ struct SeriesView {
     double2* tab;                // [bucket][sample]: e^{-gamma b h}
     unsigned long long* gmax;    // largest |gamma| among the samples of the series (double bits)
     int* ok;                     // per sample: 1 = the series serves it
+    int *nfar, *far;             // the samples past its reach: their number and a list
     int nbk, ns;
     double h, dmax;
 };
@@ -439,6 +439,7 @@ __global__ void k_series_coef(const SampleCoef* __restrict__ coef, SeriesView v)
     const double ga = sqrt(cabs2(g));
     const bool ok = ga * v.dmax <= SER_XMAX;
     v.ok[q] = ok;
+    if (!ok) v.far[atomicAdd(v.nfar, 1)] = q;
     if (ok) atomicMax(v.gmax, (unsigned long long)__double_as_longlong(ga));
     double2 p = cz(1.0, 0.0);
     for (int n = 0; n < SER_NT; ++n) {
@@ -460,7 +461,8 @@ enum : int { SK_NONE = 0, SK_TENSOR = 1, SK_TOUCH = 2, SK_BAD = 3 };
 struct SeriesPk {
     double o[3], dr[3], ds[3];   // tensor: r = |o + t0 dr - t1 ds|; touch: dr, ds = the corner vectors
     double R, fl;                // expansion centre; ZL factor |d_i . d_k| (0 where the reference drops ZL)
-    int kind, P, q, b;
+    double gl;                   // |gamma| times the longer panel
+    int kind, Pr, Ps, q, b;      // panels of receiver and sender, order of the closest panel pair
 };
 
 // One (pair, kind) classified as pair_integral does; ga: the pass's largest |gamma|.
@@ -484,7 +486,8 @@ TAGS_D void series_classify(const Seg& S, const Seg& R, bool direct, double ga, 
         const double* so = ib == 0 ? S.b : S.a;
         const double od = fmax(fabs(ro[0] - so[0]), fmax(fabs(ro[1] - so[1]), fabs(ro[2] - so[2])));
         k.kind = od <= 1e-9 * lmax ? SK_BAD : SK_TOUCH;
-        k.P = 1;
+        k.Pr = k.Ps = 1;
+        k.gl = 0.0;
         k.q = min(QMAX, 16 + 2 * (int)ceil(fmin(ga * lmax, (double)QMAX)));
         rc = 0.5 * (sqrt(dot3(k.dr, k.dr)) + sqrt(dot3(k.ds, k.ds)));
         for (int c = 0; c < 3; ++c) {
@@ -493,10 +496,15 @@ TAGS_D void series_classify(const Seg& S, const Seg& R, bool direct, double ga, 
         }
     } else {
         const double dmin = seg_seg_dist(R.a, R.b, S.a, S.b);
-        const double ratio = dmin / lmax;
         k.kind = dmin <= 1e-12 * lmax ? SK_BAD : SK_TENSOR;
-        k.P = ratio < 2.0 ? (int)fmin(32.0, ceil(2.0 / fmax(ratio, 1e-12))) : 1;
-        k.q = order_for(ratio * k.P, ga * lmax / k.P, true);
+        // panels no longer than half the distance, each segment by its own
+        // length (the direct rule of k_fill_fp64 splits both by the longer)
+        const double d = fmax(dmin, 1e-12 * lmax);
+        k.Pr = (int)fmin(32.0, fmax(1.0, ceil(2.0 * R.len / d)));
+        k.Ps = (int)fmin(32.0, fmax(1.0, ceil(2.0 * S.len / d)));
+        const double lp = fmax(R.len / k.Pr, S.len / k.Ps);
+        k.gl = ga * lp;
+        k.q = order_for(dmin / lp, k.gl, true);
     }
     k.b = min(v.nbk - 1, max(0, (int)rint(rc / v.h)));
     k.R = k.b * v.h;
@@ -520,44 +528,84 @@ TAGS_D double warp_transpose_sum(double (&acc)[NT], int lane) {
     return r;
 }
 
+// The tensor rule of one record by a warp: f(r, weight) per point. The lanes
+// share the points, or, with 32 panel pairs and more, the panel pairs, each at
+// the order its own distance needs (order_for's rule; only the closest need
+// k.q), which is where nearly all points of a finely split pair lie.
+template <class F>
+TAGS_D void tensor_points(const SeriesPk& k, int lane, F f) {
+    const double hr = 1.0 / k.Pr, hs = 1.0 / k.Ps;
+    auto point = [&](double t0, double t1, double w) {
+        double d2 = 0.0;
+        for (int c = 0; c < 3; ++c) {
+            const double d = fma(t0, k.dr[c], fma(-t1, k.ds[c], k.o[c]));
+            d2 = fma(d, d, d2);
+        }
+        f(sqrt(d2), w * (hr * hs));
+    };
+    if (k.Pr * k.Ps >= 32) {
+        const double lr = sqrt(dot3(k.dr, k.dr)) * hr, ls = sqrt(dot3(k.ds, k.ds)) * hs, lp = fmax(lr, ls);
+        for (int pp = lane; pp < k.Pr * k.Ps; pp += 32) {
+            const int pi = pp / k.Ps, pj = pp - pi * k.Ps;
+            const double m0 = (pi + 0.5) * hr, m1 = (pj + 0.5) * hs;
+            double d2 = 0.0;
+            for (int c = 0; c < 3; ++c) {
+                const double d = k.o[c] + m0 * k.dr[c] - m1 * k.ds[c];
+                d2 += d * d;
+            }
+            const double ratio = (sqrt(d2) - 0.5 * (lr + ls)) / lp;     // at least that far apart
+            const int q = ratio >= 2.0 ? min(k.q, order_for(ratio, k.gl, true)) : k.q;
+            const double* x = g_glx + gl_off(q);
+            const double* w = g_glw + gl_off(q);
+            for (int qi = 0; qi < q; ++qi)
+                for (int qj = 0; qj < q; ++qj) point((pi + x[qi]) * hr, (pj + x[qj]) * hs, w[qi] * w[qj]);
+        }
+        return;
+    }
+    const double* x = g_glx + gl_off(k.q);
+    const double* w = g_glw + gl_off(k.q);
+    const int qq = k.q * k.q, npts = k.Pr * k.Ps * qq;
+    for (int t = lane; t < npts; t += 32) {
+        const int pp = t / qq, u = t - pp * qq;
+        const int pi = pp / k.Ps, pj = pp - pi * k.Ps, qi = u / k.q, qj = u - qi * k.q;
+        point((pi + x[qi]) * hr, (pj + x[qj]) * hs, w[qi] * w[qj]);
+    }
+}
+
+// Node t of 2 q of the touching pair's Duffy rule: rho and w / rho.
+TAGS_D void touch_node(const SeriesPk& k, int t, double& rho, double& v) {
+    const int half = t >= k.q, i = half ? t - k.q : t;
+    const double s = g_glx[gl_off(k.q) + i];
+    double d2 = 0.0;
+    for (int c = 0; c < 3; ++c) {
+        const double d = half ? fma(s, k.dr[c], -k.ds[c]) : fma(-s, k.ds[c], k.dr[c]);
+        d2 = fma(d, d, d2);
+    }
+    rho = sqrt(d2);
+    v = g_glw[gl_off(k.q) + i] / rho;
+}
+
 // Moments of one record by a warp, lanes over the rule's points -> mom[0..NT).
 template <int NT>
 TAGS_D void series_moments(const SeriesPk& k, int lane, double* mom) {
     double acc[NT];
 #pragma unroll
     for (int n = 0; n < NT; ++n) acc[n] = 0.0;
-    const double* x = g_glx + gl_off(k.q);
-    const double* w = g_glw + gl_off(k.q);
     if (k.kind == SK_TENSOR) {
-        const double h = 1.0 / k.P;
-        const int qq = k.q * k.q, npts = k.P * k.P * qq;
-        for (int t = lane; t < npts; t += 32) {
-            const int pp = t / qq, u = t - pp * qq;
-            const int pi = pp / k.P, pj = pp - pi * k.P, qi = u / k.q, qj = u - qi * k.q;
-            const double t0 = (pi + x[qi]) * h, t1 = (pj + x[qj]) * h;
-            double d2 = 0.0;
-            for (int c = 0; c < 3; ++c) {
-                const double d = fma(t0, k.dr[c], fma(-t1, k.ds[c], k.o[c]));
-                d2 = fma(d, d, d2);
-            }
-            const double r = sqrt(d2), d = r - k.R;
-            double v = w[qi] * w[qj] * (h * h) / r;
+        tensor_points(k, lane, [&](double r, double w) {
+            const double d = r - k.R;
+            double v = w / r;
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
                 acc[n] += v;
                 v *= d;
             }
-        }
+        });
     } else {
         for (int t = lane; t < 2 * k.q; t += 32) {
-            const int half = t >= k.q, i = half ? t - k.q : t;
-            const double s = x[i];
-            double d2 = 0.0;
-            for (int c = 0; c < 3; ++c) {
-                const double d = half ? fma(s, k.dr[c], -k.ds[c]) : fma(-s, k.ds[c], k.dr[c]);
-                d2 = fma(d, d, d2);
-            }
-            const double rho = sqrt(d2), a = rho - k.R, v = w[i] / rho;
+            double rho, v;
+            touch_node(k, t, rho, v);
+            const double a = rho - k.R;
             double g = v, bp = v;                       // v g_n, v (-R)^n
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
@@ -592,6 +640,112 @@ TAGS_D double2 series_sum(const SeriesView& v, const double* mom, int nt, int s)
         a.y = fma(p.y, mom[n], a.y);
     }
     return a;
+}
+
+// J of one (pair, kind) at one sample by a warp (all lanes get it).
+TAGS_D double2 direct_integral(const SeriesPk& k, double2 g, int lane) {
+    double2 a = cz(0.0, 0.0);
+    if (k.kind == SK_TENSOR) {
+        tensor_points(k, lane, [&](double r, double w) {
+            const double2 e = cexp_d(cz(-g.x * r, -g.y * r));
+            const double v = w / r;
+            a.x = fma(e.x, v, a.x);
+            a.y = fma(e.y, v, a.y);
+        });
+    } else {
+        for (int t = lane; t < 2 * k.q; t += 32) {
+            double rho, v;
+            touch_node(k, t, rho, v);
+            a = cadd(a, cscale(phi_c(cz(g.x * rho, g.y * rho)), v));
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
+        a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
+    }
+    return a;
+}
+
+// The entry (k, i) of sample s to its places.
+TAGS_D void store_entry(const FillOut& out, int s, int i, int k, double2 zl, double2 zt, int* status) {
+    if (!isfinite(zl.x + zl.y + zt.x + zt.y)) raise_status(status, TAGS_ST_NONFINITE);
+    const bool accum = out.accumulate != 0;
+    zl = cscale(zl, out.sign);
+    zt = cscale(zt, out.sign);
+    const long long bs = out.batch_stride * s;
+    if (out.zl) {
+        store(out.zl + bs, (long long)(out.row0_l + k) + out.ld * (out.col0_l + i), zl, accum);
+        if (out.mirror && k != i) store(out.zl + bs, (long long)(out.row0_l + i) + out.ld * (out.col0_l + k), zl, accum);
+    }
+    if (out.zt) {
+        store(out.zt + bs, (long long)(out.row0_t + k) + out.ld * (out.col0_t + i), zt, accum);
+        if (out.mirror && k != i) store(out.zt + bs, (long long)(out.row0_t + i) + out.ld * (out.col0_t + k), zt, accum);
+    }
+}
+
+// The entries of the samples past the series' reach (long segments at high
+// frequency): the quadrature with an exponential per point, a warp per (pair,
+// sample), so that a finely split pair's thousands of points are shared by the
+// lanes. A grid of a few warps per SM strides over the items, or leaves at once.
+// Path voltages over a grid of 5 and 10 m segments, all four samples past the
+// reach in part: 67.3 (a thread per pair and sample) -> 1.8 ms.
+__global__ void __launch_bounds__(SER_THREADS) k_fill_far(const double* __restrict__ elec,
+                                                          const double* __restrict__ img, int m,
+                                                          const SampleCoef* __restrict__ coef, SeriesView v,
+                                                          FillOut out, int mode, int* status) {
+    const int nfar = *v.nfar, lane = threadIdx.x & 31;
+    const long long items = (long long)m * (m + 1) / 2 * nfar;
+    for (long long t = (long long)blockIdx.x * (SER_THREADS / 32) + (threadIdx.x >> 5); t < items;
+         t += (long long)gridDim.x * (SER_THREADS / 32)) {
+        const int s = v.far[t % nfar];
+        int i, k;
+        pair_index(t / nfar, m, i, k);
+        const SampleCoef c = coef[s];
+        const double ga = sqrt(cabs2(c.gamma));
+        Seg S, R;
+        ld_seg(elec + 11LL * i, S);
+        double2 zl = cz(0.0, 0.0), zt = cz(0.0, 0.0);
+        if ((mode & TAGS_FILL_DIRECT) && i == k) {
+            const double intg = self_integral_d(S);
+            zl = cscale(c.cL, intg);
+            zt = cscale(c.cT, intg / (S.len * S.len));
+        }
+        for (int kind = 0; kind < 2; ++kind) {
+            if (!(kind == 0 ? (mode & TAGS_FILL_DIRECT) && i != k : (mode & TAGS_FILL_IMAGE) != 0)) continue;
+            ld_seg((kind == 0 ? elec : img) + 11LL * k, R);
+            SeriesPk r;
+            series_classify(S, R, kind == 0, ga, v, r);
+            double2 J = cz(nan(""), nan(""));
+            if (r.kind == SK_BAD) raise_status(status, TAGS_ST_DEGENERATE_PAIR);
+            else J = direct_integral(r, c.gamma, lane);
+            zt = cfma(kind == 0 ? c.cT : c.cTi, J, zt);
+            if (r.fl != 0.0) zl = cfma(kind == 0 ? c.cL : c.cLi, cscale(J, r.fl), zl);
+        }
+        if (lane == 0) store_entry(out, s, i, k, zl, zt, status);
+    }
+}
+
+__global__ void __launch_bounds__(SER_THREADS) k_path_far(const double* __restrict__ elec, int m,
+                                                          const double* __restrict__ paths, int npaths,
+                                                          const SampleCoef* __restrict__ coef, SeriesView v,
+                                                          double2* __restrict__ jj, int* status) {
+    const int nfar = *v.nfar, lane = threadIdx.x & 31;
+    const long long n = (long long)m * npaths, items = n * nfar;
+    for (long long t = (long long)blockIdx.x * (SER_THREADS / 32) + (threadIdx.x >> 5); t < items;
+         t += (long long)gridDim.x * (SER_THREADS / 32)) {
+        const int s = v.far[t % nfar];
+        const long long p = t / nfar;
+        Seg S, R;
+        ld_seg(paths + 11LL * (p / m), S);
+        ld_seg(elec + 11LL * (p % m), R);
+        const double2 g = coef[s].gamma;
+        SeriesPk r;
+        series_classify(S, R, true, sqrt(cabs2(g)), v, r);
+        double2 J = cz(nan(""), nan(""));
+        if (r.kind == SK_BAD) raise_status(status, TAGS_ST_DEGENERATE_PAIR);
+        else J = direct_integral(r, g, lane);
+        if (lane == 0) jj[(long long)s * n + p] = J;
+    }
 }
 
 // A CTA takes `npt` consecutive pairs (column by column): one warp classifies
@@ -630,7 +784,6 @@ __global__ void __launch_bounds__(SER_THREADS) k_fill_series(const double* __res
         else series_moments<32>(pk[q], lane, mom[q]);
     }
     __syncthreads();
-    const bool accum = out.accumulate != 0;
     for (long long t = tid; t < (long long)np * v.ns; t += SER_THREADS) {
         const int lp = (int)(t / v.ns), s = (int)(t - (long long)lp * v.ns);
         if (!v.ok[s]) continue;
@@ -654,18 +807,7 @@ __global__ void __launch_bounds__(SER_THREADS) k_fill_series(const double* __res
             zt = cfma(kind == 0 ? c.cT : c.cTi, J, zt);
             if (r.fl != 0.0) zl = cfma(kind == 0 ? c.cL : c.cLi, cscale(J, r.fl), zl);
         }
-        if (!isfinite(zl.x + zl.y + zt.x + zt.y)) raise_status(status, TAGS_ST_NONFINITE);
-        zl = cscale(zl, out.sign);
-        zt = cscale(zt, out.sign);
-        const long long bs = out.batch_stride * s;
-        if (out.zl) {
-            store(out.zl + bs, (long long)(out.row0_l + k) + out.ld * (out.col0_l + i), zl, accum);
-            if (out.mirror && k != i) store(out.zl + bs, (long long)(out.row0_l + i) + out.ld * (out.col0_l + k), zl, accum);
-        }
-        if (out.zt) {
-            store(out.zt + bs, (long long)(out.row0_t + k) + out.ld * (out.col0_t + i), zt, accum);
-            if (out.mirror && k != i) store(out.zt + bs, (long long)(out.row0_t + i) + out.ld * (out.col0_t + k), zt, accum);
-        }
+        store_entry(out, s, i, k, zl, zt, status);
     }
 }
 
@@ -2188,7 +2330,7 @@ SeriesGeo tags_series_geometry(const double* h_a, int na, const double* h_b, int
 }
 
 size_t tags_series_workspace(const SeriesGeo& g, int ns) {
-    return sizeof(double2) * (size_t)ns * (SER_NT + g.nbk) + 16 + sizeof(int) * (size_t)ns;
+    return sizeof(double2) * (size_t)ns * (SER_NT + g.nbk) + 16 + 2 * sizeof(int) * (size_t)ns;
 }
 
 static SeriesView series_view(const SeriesGeo& g, void* ws, int ns) {
@@ -2196,7 +2338,9 @@ static SeriesView series_view(const SeriesGeo& g, void* ws, int ns) {
     v.pw = reinterpret_cast<double2*>(ws);
     v.tab = v.pw + (size_t)SER_NT * ns;
     v.gmax = reinterpret_cast<unsigned long long*>(v.tab + (size_t)g.nbk * ns);
+    v.nfar = reinterpret_cast<int*>(v.gmax + 1);
     v.ok = reinterpret_cast<int*>(v.gmax + 2);
+    v.far = v.ok + ns;
     v.nbk = g.nbk;
     v.ns = ns;
     v.h = g.h;
@@ -2205,12 +2349,17 @@ static SeriesView series_view(const SeriesGeo& g, void* ws, int ns) {
 }
 
 static int series_tables(const SampleCoef* d_coef, const SeriesView& v, cudaStream_t st) {
-    TAGS_CUDA_OK(cudaMemsetAsync(v.gmax, 0, sizeof(unsigned long long), st));
+    TAGS_CUDA_OK(cudaMemsetAsync(v.gmax, 0, 2 * sizeof(unsigned long long), st));     // and nfar
     k_series_coef<<<(v.ns + 127) / 128, 128, 0, st>>>(d_coef, v);
     k_series_tab<<<dim3((v.ns + 31) / 32, v.nbk), 32, 0, st>>>(d_coef, v);
     tags_note_launch(2);
     TAGS_CUDA_OK(cudaGetLastError());
     return 0;
+}
+
+// CTAs of the kernels for the samples past the reach: four per SM at most.
+static unsigned far_ctas(long long pairs, int ns) {
+    return (unsigned)std::min<long long>(608, (pairs * ns + SER_THREADS / 32 - 1) / (SER_THREADS / 32));
 }
 
 // Records per CTA: up to `most`, fewer while the grid would leave SMs idle.
@@ -2225,7 +2374,6 @@ int tags_launch_fill_fp64(const double* d_elec, const double* d_img, int m, cons
                           cudaStream_t st, const SeriesGeo* geo, void* series_ws) {
     if (m <= 0 || nsamp <= 0) return 0;
     const long long npairs = (long long)m * (m + 1) / 2;
-    const int* done = nullptr;
     int pf = tags_prof_begin(TAGS_PROF_FILL_FP64, st);
     if (itype == TAGS_INTG_DOUBLE && tight && geo && geo->nbk > 0 && series_ws) {
         const SeriesView v = series_view(*geo, series_ws, nsamp);
@@ -2233,13 +2381,14 @@ int tags_launch_fill_fp64(const double* d_elec, const double* d_img, int m, cons
         const int npt = series_tile(npairs, SER_PK / 2);
         k_fill_series<<<(unsigned)((npairs + npt - 1) / npt), SER_THREADS, 0, st>>>(d_elec, d_img, m, d_coef, v, out,
                                                                                    mode, npt, d_status);
+        k_fill_far<<<far_ctas(npairs, nsamp), SER_THREADS, 0, st>>>(d_elec, d_img, m, d_coef, v, out, mode, d_status);
+        tags_note_launch(2);
+    } else {
+        dim3 grid((unsigned)((npairs + 127) / 128), (unsigned)nsamp);
+        k_fill_fp64<<<grid, 128, 0, st>>>(d_elec, d_img, m, d_coef, nsamp, out, mode, itype, tight, d_status);
         tags_note_launch();
-        done = v.ok;
     }
-    dim3 grid((unsigned)((npairs + 127) / 128), (unsigned)nsamp);
-    k_fill_fp64<<<grid, 128, 0, st>>>(d_elec, d_img, m, d_coef, nsamp, out, mode, itype, tight, d_status, done);
     tags_prof_end(TAGS_PROF_FILL_FP64, pf, st, 0.0, 0.0);
-    tags_note_launch();
     TAGS_CUDA_OK(cudaGetLastError());
     return 0;
 }
@@ -2251,19 +2400,19 @@ int tags_launch_path_pairs(const double* d_elec, int m, const double* d_paths, i
     if (nsamp > 65535) return tags_fail_cuda(cudaErrorInvalidValue, "path_pairs: more than 65535 samples", __FILE__,
                                              __LINE__);
     const long long n = (long long)m * npaths;
-    const int* done = nullptr;
     if (geo && geo->nbk > 0 && series_ws) {
         const SeriesView v = series_view(*geo, series_ws, nsamp);
         if (int e = series_tables(d_coef, v, st)) return e;
         const int npt = series_tile(n, SER_PK);
         k_path_series<<<(unsigned)((n + npt - 1) / npt), SER_THREADS, 0, st>>>(d_elec, m, d_paths, npaths, v, d_jj, npt,
                                                                               d_status);
+        k_path_far<<<far_ctas(n, nsamp), SER_THREADS, 0, st>>>(d_elec, m, d_paths, npaths, d_coef, v, d_jj, d_status);
+        tags_note_launch(2);
+    } else {
+        k_path_pairs<<<dim3((unsigned)((n + 127) / 128), (unsigned)nsamp), 128, 0, st>>>(d_elec, m, d_paths, npaths,
+                                                                                           d_coef, d_jj, d_status);
         tags_note_launch();
-        done = v.ok;
     }
-    k_path_pairs<<<dim3((unsigned)((n + 127) / 128), (unsigned)nsamp), 128, 0, st>>>(d_elec, m, d_paths, npaths,
-                                                                                       d_coef, d_jj, d_status, done);
-    tags_note_launch();
     TAGS_CUDA_OK(cudaGetLastError());
     return 0;
 }
