@@ -23,9 +23,9 @@
 // elimination never touches, the full symmetric ZL (rows 0..m, columns m..2m)
 // and ZT (rows m..2m, columns 0..m) that the residual reads. Panels are 32
 // columns wide and never straddle m or 2m, so a ZL panel skips the ZT rows
-// exactly. The panels' factored diagonal blocks live in the workspace (every
-// CTA of a panel launch factors the block itself, which saves a launch per
-// panel), then their inverses, so that a solve's diagonal step is a product.
+// exactly. The inverses of the panels' factored diagonal blocks live in the
+// workspace, so that a solve's diagonal step is a product (every CTA of a panel
+// launch factors the block itself, which saves a launch per panel).
 #include <algorithm>
 #include <mutex>
 
@@ -85,21 +85,29 @@ TAGS_D double2 crecip(double2 d) {
 
 // Diagonal block and rows of one panel: L21 = A21 L11^-T D^-1 (stored in
 // place) and U12 = D L21^T (stored in the upper triangle). Every CTA factors
-// the 32 x 32 block in shared memory first, CTA 0 also stores it (L11, 1/D on
-// the diagonal) for the solves. A warp's FP64 instruction holds its quarter of
-// the SM for 64 cycles, so time is the FP64 instructions of the busiest warp:
-// the block's columns go round the four warps, each forming the pivot's
-// reciprocal itself (one barrier per step), and four lanes share a row of L21,
-// eight columns each (576 instructions instead of a whole row's 1984 in one
-// thread: panels of m = 1560, 2 samples, 142 -> 70 us). `passes` groups of 32
-// rows per CTA: as few as fill the SMs, since the block's work is repeated.
+// the 32 x 32 block first; the 32 rows after the last one are the identity's,
+// whose result L11^-T goes to the workspace for the solves, with 1/D on the
+// diagonal. A warp's FP64 instruction holds its quarter of the SM for 64
+// cycles, so time is the FP64 instructions of the busiest warp. The block: its
+// 496 elements right of column 0 are dealt to the threads column by column, four
+// each in registers, so that a step's live ones fill whole warps (252
+// instructions for the products instead of 544 with a lane per row and a warp
+// per column), every warp forms the pivot's reciprocal and the scaled column
+// itself (14 a step), one barrier per step. The rows: LPR lanes share a row,
+// 32 / LPR columns each: 576 instructions with 4 lanes, 320 with 8, 192 with 16,
+// which take more CTAs for the same rows (panel_split). The 11 panels of one
+// system at m = 100, n = 85 608 -> 400 us (the drop-in chain 1.80 -> 1.60 ms), the
+// plain form's 256 samples 6.65 -> 6.19 ms.
+template <int LPR>
 __global__ void __launch_bounds__(128) k_ldl64_panel(double2* __restrict__ A0, long long ld, long long stride,
                                                      Panel q, int p, double2* __restrict__ ws0, long long wstride,
                                                      int passes) {
+    constexpr int ROWS = 128 / LPR, NC = PB / LPR;
     double2* A = A0 + stride * blockIdx.y;
+    double2* ws = ws0 + wstride * blockIdx.y + (long long)p * PB * PB;
     __shared__ double2 sL[PB][PB + 1];
     __shared__ double2 sdi[PB];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31;
     for (int t = tid; t < PB * PB; t += 128) {
         const int r = t % PB, c = t / PB;
         double2 v = cz(r == c ? 1.0 : 0.0, 0.0);          // a short panel is padded with the identity
@@ -108,59 +116,69 @@ __global__ void __launch_bounds__(128) k_ldl64_panel(double2* __restrict__ A0, l
     }
     if (tid < PB) sdi[tid] = cz(1.0, 0.0);
     __syncthreads();
+    int er[4], ec[4];
+    double2 ev[4];
+    for (int i = 0, c = 1, first = 0; i < 4; ++i) {        // element tid + 128 i: column c starts at `first`
+        const int e = tid + 128 * i;
+        while (c < PB && e - first >= PB - c) first += PB - c++;
+        ec[i] = c < PB ? c : 0;                             // 0: none
+        er[i] = c < PB ? c + e - first : 0;
+        ev[i] = sL[er[i]][ec[i]];
+    }
     for (int k = 0; k < q.jb; ++k) {
         const double2 di = crecip(sL[k][k]);
         if (tid == 0) sdi[k] = di;
         const double2 l = cneg(cmul(sL[lane][k], di));     // rows up to k are not used
-        for (int c = k + 1 + warp; c < q.jb; c += 4)
-            if (lane >= c) sL[lane][c] = cfma(l, sL[c][k], sL[lane][c]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (!__any_sync(0xffffffffu, ec[i] > k)) continue;
+            const double2 lr = cz(__shfl_sync(0xffffffffu, l.x, er[i]), __shfl_sync(0xffffffffu, l.y, er[i]));
+            if (ec[i] > k) {
+                ev[i] = cfma(lr, sL[ec[i]][k], ev[i]);
+                if (ec[i] == k + 1) sL[er[i]][ec[i]] = ev[i];     // the next step's column
+            }
+        }
         __syncthreads();
     }
     for (int t = tid; t < PB * PB; t += 128) {            // unscaled columns -> L11
         const int r = t % PB, c = t / PB;
         if (r > c && r < q.jb) sL[r][c] = cmul(sL[r][c], sdi[c]);
+        if (blockIdx.x == 0 && r <= c) ws[c * PB + r] = r == c ? sdi[c] : cz(0.0, 0.0);
     }
     __syncthreads();
-    if (blockIdx.x == 0) {
-        double2* ws = ws0 + wstride * blockIdx.y + (long long)p * PB * PB;
-        for (int t = tid; t < PB * PB; t += 128) {
-            const int r = t % PB, c = t / PB;
-            ws[c * PB + r] = r > c ? sL[r][c] : r == c ? sdi[c] : cz(0.0, 0.0);
-        }
-    }
-    const int g = tid & 3;                                  // lane of the row's four: columns g, g + 4, ..
+    const int g = tid % LPR;                                // lane of the row's LPR: columns g, g + LPR, ..
     for (int pass = 0; pass < passes; ++pass) {
-        const int v0 = (blockIdx.x * passes + pass) * 32;
-        if (v0 >= q.cnt) return;                            // the whole CTA
-        const int v = v0 + (tid >> 2);
+        const int v0 = (blockIdx.x * passes + pass) * ROWS;
+        if (v0 >= q.cnt + PB) return;                       // the whole CTA
+        const int v = v0 + tid / LPR, unit = v - q.cnt;     // unit >= 0: row of the identity
         const bool on = v < q.cnt;
         const int row = on ? q.row(v) : 0;
-        double2 w[PB / 4];
+        double2 w[NC];
 #pragma unroll
-        for (int i = 0; i < PB / 4; ++i) {
-            const int c = 4 * i + g;
-            w[i] = on && c < q.jb ? A[row + ld * (q.j0 + c)] : cz(0.0, 0.0);
+        for (int i = 0; i < NC; ++i) {
+            const int c = LPR * i + g;
+            w[i] = on && c < q.jb ? A[row + ld * (q.j0 + c)] : cz(c == unit ? 1.0 : 0.0, 0.0);
         }
 #pragma unroll
         for (int k = 0; k < PB - 1; ++k) {
             if (k + 1 < q.jb) {                             // the same in every thread
-                const double2 wk = cz(-__shfl_sync(0xffffffffu, w[k / 4].x, k % 4, 4),
-                                      -__shfl_sync(0xffffffffu, w[k / 4].y, k % 4, 4));
+                const double2 wk = cz(-__shfl_sync(0xffffffffu, w[k / LPR].x, k % LPR, LPR),
+                                      -__shfl_sync(0xffffffffu, w[k / LPR].y, k % LPR, LPR));
 #pragma unroll
-                for (int i = k / 4; i < PB / 4; ++i) {
-                    const int c = 4 * i + g;
+                for (int i = k / LPR; i < NC; ++i) {
+                    const int c = LPR * i + g;
                     if (c > k) w[i] = cfma(wk, sL[c][k], w[i]);
                 }
             }
         }
-        if (on) {
 #pragma unroll
-            for (int i = 0; i < PB / 4; ++i) {
-                const int c = 4 * i + g;
-                if (c < q.jb) {
-                    A[row + ld * (q.j0 + c)] = cmul(w[i], sdi[c]);
-                    A[(q.j0 + c) + ld * row] = w[i];
-                }
+        for (int i = 0; i < NC; ++i) {
+            const int c = LPR * i + g;
+            if (on && c < q.jb) {
+                A[row + ld * (q.j0 + c)] = cmul(w[i], sdi[c]);
+                A[(q.j0 + c) + ld * row] = w[i];
+            } else if (unit >= 0 && unit < c) {
+                ws[unit * PB + c] = w[i];
             }
         }
     }
@@ -240,43 +258,6 @@ __global__ void __launch_bounds__(TL * TL / (TT * TT)) k_ldl64_update(double2* _
                 A[idx] = csub(A[idx], cz(rr - ii, acc[2][a][b] - rr - ii));
             }
         }
-    }
-}
-
-// Inverses of the panels' unit lower blocks, in place (1/D stays on the
-// diagonal): a CTA per panel and sample, a lane per column of the inverse,
-// eight rows at a time: the four warps form the products with the rows above
-// (two rows each), then one warp's lanes finish the eight rows.
-__global__ void __launch_bounds__(128) k_ldl64_inv(double2* __restrict__ ws0, long long wstride) {
-    double2* ws = ws0 + wstride * blockIdx.y + (long long)blockIdx.x * PB * PB;
-    __shared__ double2 L[PB][PB + 1], X[PB][PB + 1];
-    const int c = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int t = threadIdx.x; t < PB * PB; t += 128) L[t % PB][t / PB] = ws[t];
-    __syncthreads();
-#pragma unroll 1
-    for (int r0 = 0; r0 < PB; r0 += 8) {
-        for (int r = r0 + 2 * warp; r < r0 + 2 * warp + 2; ++r) {
-            double2 v = cz(r == c ? 1.0 : 0.0, 0.0);
-            for (int k = 0; k < r0; ++k) v = cfma(cneg(L[r][k]), X[k][c], v);
-            X[r][c] = v;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            double2 x[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                double2 v = X[r0 + i][c];
-#pragma unroll
-                for (int k = 0; k < i; ++k) v = cfma(cneg(L[r0 + i][r0 + k]), x[k], v);
-                x[i] = v;
-                X[r0 + i][c] = v;
-            }
-        }
-        __syncthreads();
-    }
-    for (int t = threadIdx.x; t < PB * PB; t += 128) {
-        const int r = t % PB, k = t / PB;
-        if (r > k) ws[t] = X[r][k];
     }
 }
 
@@ -1008,16 +989,38 @@ Ws carve(void* p, int N, int batch) {
 
 constexpr int SOLVE_N_MAX = 14000;        // 16 B per unknown in the one-CTA solve's shared memory
 
+// Split of a panel's rows (the identity's 32 included): lanes per row, groups
+// of rows per CTA, CTAs per sample. Taken is what leaves the busiest SM the
+// least FP64 instructions per warp: 690 for a CTA's block and 576, 320 or 192
+// per group of 32, 16 or 8 rows.
+int panel_split(int rows, int nb, int& lpr, int& passes) {
+    long long best = -1;
+    int ctas = 1;
+    for (int l = 4, ins = 576; l <= 16; l *= 2, ins = l == 8 ? 320 : 192)
+        for (int ps = 1, last = 0; ps <= 16; ++ps) {
+            const int groups = (rows * l + 127) / 128, c = (groups + ps - 1) / ps;
+            if (c == last) continue;                       // as many CTAs with fewer passes
+            last = c;
+            const long long cost = ((long long)nb * c + 151) / 152 * (690 + ins * ps);
+            if (best < 0 || cost < best) {
+                best = cost;
+                lpr = l;
+                passes = ps;
+                ctas = c;
+            }
+        }
+    return ctas;
+}
+
 int factor(double2* A, int N, long long ld, long long stride, int nb, int m, const Ws& w, cudaStream_t st) {
     const int P = panel_count(N, m);
     for (int p = 0; p < P; ++p) {
         const Panel q = panel_at(p, N, m);
-        // 32 rows per pass; up to four passes per CTA once the grid has one CTA per SM
-        const int groups = q.cnt > 0 ? (q.cnt + 31) / 32 : 1;
-        const int passes = (int)std::min<long long>(4, std::max<long long>(1, (long long)nb * groups / 152));
-        const int ctas = (groups + passes - 1) / passes;
+        int lpr, passes;
+        const int ctas = panel_split(q.cnt + PB, nb, lpr, passes);
         int pf = tags_prof_begin(TAGS_PROF_LU64_OTHER, st);
-        k_ldl64_panel<<<dim3(ctas, nb), 128, 0, st>>>(A, ld, stride, q, p, w.linv, w.wstride, passes);
+        auto panel = lpr == 16 ? k_ldl64_panel<16> : lpr == 8 ? k_ldl64_panel<8> : k_ldl64_panel<4>;
+        panel<<<dim3(ctas, nb), 128, 0, st>>>(A, ld, stride, q, p, w.linv, w.wstride, passes);
         tags_prof_end(TAGS_PROF_LU64_OTHER, pf, st, 0.0, 0.0);
         tags_note_launch();
         if (q.cnt <= 0) continue;
@@ -1038,8 +1041,6 @@ int factor(double2* A, int N, long long ld, long long stride, int nb, int m, con
                       (16.0 * q.cnt * (q.cnt + 1.0) + 32.0 * q.cnt * q.jb) * nb);
         tags_note_launch();
     }
-    k_ldl64_inv<<<dim3(P, nb), 128, 0, st>>>(w.linv, w.wstride);
-    tags_note_launch();
     TAGS_CUDA_OK(cudaGetLastError());
     return 0;
 }
