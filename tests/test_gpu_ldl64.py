@@ -134,3 +134,9 @@ def test_yla_ytb_of_any_symmetric_blocks(gpu_pkg, m, n, zero_diagonal):
     for got, inv, v, r in ((yla, zl, z[0], rhs[0]), (ytb, zt, z[1], rhs[1])):
         assert rel_err(got.reshape(n, m).T, np.linalg.solve(v, r)) < 1e-9
         assert rel_err(np.tril(inv.reshape(m, m).T), np.tril(np.linalg.inv(v))) < 1e-9
+
+
+@pytest.mark.parametrize("m,n", [(1, 700), (32, 1100), (33, 290), (97, 80), (257, 40)])
+def test_yla_ytb_of_one_to_eight_columns_per_cta(gpu_pkg, m, n):
+    """Widths of the column tiles of the nodal solve, with a ragged last one."""
+    test_yla_ytb_of_any_symmetric_blocks(gpu_pkg, m, n, False)

@@ -107,7 +107,7 @@ int sym_solve(const tags_cdouble* z, const tags_cdouble* rhs, size_t m, size_t n
 // without pivoting (ldl64.cu), both blocks side by side; *done = 0 where its
 // check asks for the pivoted LU (nothing of the caller's is written then). One
 // pass of FP64 tiles instead of a CTA per 32 x 32 step for all right-hand
-// sides: 46.8 -> 3.5 ms for the examples' loop body at m = 220, n = 121 (FP64,
+// sides: 46.8 -> 2.3 ms for the examples' loop body at m = 220, n = 121 (FP64,
 // one refinement of every column; errors against 128-bit solves 2-4e-16, as the LU).
 int yla_ytb_ldl(tags_cdouble* yla, tags_cdouble* ytb, tags_cdouble* zl, tags_cdouble* zt, const tags_cdouble* a,
                 const tags_cdouble* b, size_t m, size_t n, cudaStream_t st, int* done) {
@@ -115,11 +115,14 @@ int yla_ytb_ldl(tags_cdouble* yla, tags_cdouble* ytb, tags_cdouble* zl, tags_cdo
     DeviceCtx* c = tags_ctx();
     const size_t mm = m * m, mn = m * n;
     // the scratch stays with the context: no more than 8 GB (the LU's is smaller);
-    // the solve's grid takes two million right-hand sides
-    if (n + m > 2000000 || sizeof(double2) * 2 * (5 * mm + 4 * mn) > ((size_t)8 << 30)) return 0;
+    // two columns of m values in a CTA's shared memory; the solve's grid takes
+    // two million right-hand sides
+    if (!tags_ldl64_multi_fits((int)m) || n + m > 2000000 ||
+        sizeof(double2) * 2 * (3 * mm + 2 * mn) > ((size_t)8 << 30))
+        return 0;
     double2* d_Z = (double2*)c->scratch(6, sizeof(double2) * (2 * mm + 2 * mn + 1));
     double2* d_X = (double2*)c->scratch(7, sizeof(double2) * 2 * m * (n + m));
-    void* ws = c->scratch(18, tags_ldl64_multi_workspace((int)m, (int)(n + m)));
+    void* ws = c->scratch(18, tags_ldl64_multi_workspace((int)m));
     if (!d_Z || !d_X || !ws) {
         cudaGetLastError();                                // no room: the LU needs less
         return 0;

@@ -744,165 +744,113 @@ __global__ void __launch_bounds__(64) k_ldl64_resid_full(const double2* __restri
 
 // ---- many right-hand sides (the nodal admittance drop-ins)
 
-// One panel of a sweep over R right-hand sides (columns of X, leading
-// dimension ldx): y = L11^-1 X_p (BWD: L11^-T X_p), to Y as D^-1 y (BWD: y),
-// then X_c -= L_cp y for the rows c below the panel (BWD: X_c -= L_pc^T y for
-// those above). Tiles of 16 TA rows and 32 right-hand sides; every tile forms
-// its 32 columns of y itself (16 us of one SM's FP64 pipe, TA * 16 us for the
-// rest), X_p is left as it is. TA = 4 where that still fills the SMs, else 2.
-template <bool BWD, int TA>
-__global__ void __launch_bounds__(256) k_ldl64_msolve(const double2* __restrict__ A0, long long ld, long long stride,
-                                                      Panel q, int p, const double2* __restrict__ ws0,
-                                                      long long wstride, double2* __restrict__ X0,
-                                                      double2* __restrict__ Y0, long long ldx, long long xstride,
-                                                      int R) {
-    const int b = blockIdx.z;
-    const double2* A = A0 + stride * b;
-    const double2* ws = ws0 + wstride * b + (long long)p * PB * PB;
-    double2* X = X0 + xstride * b;
-    double2* Y = Y0 + xstride * b;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int TC = 16 * TA;
-    double2* sL = reinterpret_cast<double2*>(smem_raw);    // [PB][TC]: L of the tile, k-major; first L11^-1
-    double2* raw = sL + PB * TC;                            // [PB][PB + 1]: X_p, k-major
-    double2* y = raw + PB * (PB + 1);                       // [PB][PB + 1]
-    const int r0 = blockIdx.y * PB, c0 = blockIdx.x * TC, ncols = BWD ? q.j0 : q.cnt;
-    for (int t = threadIdx.x; t < PB * PB; t += 256) {
-        const int k = t % PB, r = t / PB;
-        raw[k * (PB + 1) + r] = (k < q.jb && r0 + r < R) ? X[q.j0 + k + ldx * (r0 + r)] : cz(0.0, 0.0);
-        sL[t] = ws[t];                                      // (row, column) at column * PB + row
+// X = Z^-1 [rhs, I] for R = n + M right-hand sides, one refinement of each
+// included. Columns do not depend on one another, so a CTA takes ct of them
+// through everything in shared memory: both sweeps, the residual against Z,
+// both sweeps again. A warp's unit of work is 32 rows of one column, a lane per
+// row: one load of 16 bytes per four FP64 instructions, which hold the SM's
+// quarter for 256 cycles, so L2 and the loads' latency are far from the bound;
+// the CTAs take as many columns as give every SM the same number. The backward
+// sweep reads U = D L^T from the upper triangle, whose rows lie side by side,
+// and so needs 1/D only at the diagonal step. Sums over a panel first, then of
+// those: less rounding than one chain. 16 warps, since 8 (two per quarter) leave
+// the pipe waiting for L2 at M = 1560 (422 against 317 ms). calculate_yla_ytb
+// against launches per panel over 32-column tiles: M = 4, n = 4 0.23 -> 0.11 ms,
+// 220 and 121 2.74 -> 1.53, 600 and 400 24.2 -> 18.5, 1560 and 1417 362 -> 317.
+constexpr int MCOLS_THREADS = 512;
+constexpr int MCOLS_MAX = 8;              // columns of a CTA, at most
+constexpr size_t MCOLS_SMEM = 227 * 1024 - 64;
+
+// part -> X_p of the diagonal step: y = L11^-1 X_p (upper = 0), L11^-T (D^-1 X_p) (upper = 1).
+// A unit is one column's sum over eight terms.
+TAGS_D void mcols_block(const double2* __restrict__ ws, double2* x, int M, int ct, const Panel& q, int upper,
+                        double2* raw, double2* part, double2* y) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int t = threadIdx.x; t < PB * ct; t += MCOLS_THREADS) {
+        const int k = t % PB, c = t / PB;
+        double2 v = k < q.jb ? x[c * M + q.j0 + k] : cz(0.0, 0.0);
+        if (upper) v = cmul(v, ws[k * (PB + 1)]);
+        raw[t] = v;
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < PB * PB; t += 256) {
-        const int k = t / PB, r = t % PB;
-        double2 a = raw[k * (PB + 1) + r];
-        if (!BWD) {
-            for (int j = 0; j < k; ++j) a = cfma(sL[j * PB + k], raw[j * (PB + 1) + r], a);
-        } else {
-            for (int j = k + 1; j < PB; ++j) a = cfma(sL[k * PB + j], raw[j * (PB + 1) + r], a);
-        }
-        y[k * (PB + 1) + r] = a;
-        if (blockIdx.x == 0 && k < q.jb && r0 + r < R)
-            Y[q.j0 + k + ldx * (r0 + r)] = BWD ? a : cmul(a, sL[k * (PB + 1)]);
+    for (int u = warp; u < 4 * ct; u += MCOLS_THREADS / 32) {
+        const int c = u >> 2, k0 = 8 * (u & 3);
+        double2 a = (u & 3) == 0 ? raw[c * PB + lane] : cz(0.0, 0.0);
+        for (int k = k0; k < k0 + 8; ++k)
+            if (upper ? k > lane : k < lane)
+                a = cfma(ws[upper ? lane * PB + k : k * PB + lane], raw[c * PB + k], a);
+        part[u * PB + lane] = a;
     }
     __syncthreads();
-    if (c0 >= ncols) return;
-    for (int t = threadIdx.x; t < PB * TC; t += 256) {
-        const int c = BWD ? t / PB : t % TC, k = BWD ? t % PB : t / TC;
-        double2 v = cz(0.0, 0.0);
-        if (k < q.jb && c0 + c < ncols)
-            v = BWD ? A[(q.j0 + k) + ld * (c0 + c)] : A[q.base + c0 + c + ld * (q.j0 + k)];
-        sL[k * TC + c] = v;
+    for (int t = threadIdx.x; t < PB * ct; t += MCOLS_THREADS) {
+        const int k = t % PB, c = t / PB;
+        const double2* pc = part + 4 * c * PB + k;
+        const double2 a = cadd(cadd(pc[0], pc[PB]), cadd(pc[2 * PB], pc[3 * PB]));
+        y[t] = a;
+        if (k < q.jb) x[c * M + q.j0 + k] = a;
     }
     __syncthreads();
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    double2 acc[TA][2];
-#pragma unroll
-    for (int a = 0; a < TA; ++a)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) acc[a][e] = cz(0.0, 0.0);
-    for (int k = 0; k < q.jb; ++k) {
-        double2 av[TA], bv[2];
-#pragma unroll
-        for (int a = 0; a < TA; ++a) av[a] = sL[k * TC + tx + 16 * a];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) bv[e] = y[k * (PB + 1) + ty + 16 * e];
-#pragma unroll
-        for (int a = 0; a < TA; ++a)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) acc[a][e] = cfma(av[a], bv[e], acc[a][e]);
-    }
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-        const int r = r0 + ty + 16 * e;
-        if (r >= R) continue;
-#pragma unroll
-        for (int a = 0; a < TA; ++a) {
-            const int c = c0 + tx + 16 * a;
-            if (c >= ncols) continue;
-            double2* x = X + (BWD ? c : q.base + c) + ldx * r;
-            *x = csub(*x, acc[a][e]);
-        }
-    }
 }
 
-constexpr size_t MSOLVE_SMEM = sizeof(double2) * (PB * 64 + 2 * PB * (PB + 1));
-
-// Identity columns [n, n + M) of X (M x (n + M)).
-__global__ void k_ldl64_identity(double2* __restrict__ X0, int M, int n, long long xstride) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)M * M) return;
-    X0[xstride * blockIdx.y + (long long)M * n + t] = cz(t % M == t / M ? 1.0 : 0.0, 0.0);
-}
-
-// E = [rhs, I] - Z X for the refinement of all right-hand sides (M x R, R = n +
-// M); 64 x 32 tiles, FP64-bound.
-__global__ void __launch_bounds__(128) k_ldl64_mresid(const double2* __restrict__ Z0, int M, long long zstride,
-                                                      const double2* __restrict__ B0, int n, long long bstride,
-                                                      const double2* __restrict__ X0, double2* __restrict__ E0,
-                                                      long long xstride, int R) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    double2* sZ = reinterpret_cast<double2*>(smem_raw);    // [PB][64], k-major
-    double2* sX = sZ + PB * 64;                             // [PB][PB + 1], k-major
-    const double2* Z = Z0 + zstride * blockIdx.z;
-    const double2* X = X0 + xstride * blockIdx.z;
-    const int i0 = blockIdx.x * 64, r0 = blockIdx.y * PB;
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    double2 tot[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) tot[a][e] = cz(0.0, 0.0);
-    for (int k0 = 0; k0 < M; k0 += PB) {
-        const int nk = min(PB, M - k0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < PB * 64; t += 128) {
-            const int i = t % 64, k = t / 64;
-            sZ[t] = (k < nk && i0 + i < M) ? Z[i0 + i + (long long)M * (k0 + k)] : cz(0.0, 0.0);
-        }
-        for (int t = threadIdx.x; t < PB * PB; t += 128) {
-            const int k = t % PB, r = t / PB;
-            sX[k * (PB + 1) + r] = (k < nk && r0 + r < R) ? X[k0 + k + (long long)M * (r0 + r)] : cz(0.0, 0.0);
+// x (M x ct in shared memory) <- Z^-1 x.
+TAGS_D void mcols_sweeps(const double2* __restrict__ A, const double2* __restrict__ ws, double2* x, int M, int ct,
+                         double2* raw, double2* part, double2* y) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, P = panel_count(M, 0);
+    for (int s = 0; s < 2 * P; ++s) {
+        const int bwd = s >= P, p = bwd ? 2 * P - 1 - s : s;
+        const Panel q = panel_at(p, M, 0);
+        mcols_block(ws + (long long)p * PB * PB, x, M, ct, q, bwd, raw, part, y);
+        const int r0 = bwd ? 0 : q.base, nr = bwd ? q.j0 : q.cnt, groups = (nr + 31) / 32;
+        const double2* L = A + r0 + (long long)M * q.j0;           // L21, or the rows of U above the block
+        for (int u = warp; u < groups * ct; u += MCOLS_THREADS / 32) {
+            const int c = u % ct, v = 32 * (u / ct) + lane;
+            if (v >= nr) continue;
+            double2 acc = cz(0.0, 0.0);
+#pragma unroll 8
+            for (int k = 0; k < q.jb; ++k) acc = cfma(L[v + (long long)M * k], y[c * PB + k], acc);
+            x[c * M + r0 + v] = csub(x[c * M + r0 + v], acc);
         }
         __syncthreads();
-        double2 acc[4][4];                                  // sums of 32 terms, then of those: less rounding than one chain
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[a][e] = cz(0.0, 0.0);
-        for (int k = 0; k < nk; ++k) {
-            double2 av[4], bv[4];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) av[a] = sZ[k * 64 + tx + 16 * a];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) bv[e] = sX[k * (PB + 1) + ty + 8 * e];
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) acc[a][e] = cfma(av[a], bv[e], acc[a][e]);
-        }
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) tot[a][e] = cadd(tot[a][e], acc[a][e]);
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const int r = r0 + ty + 8 * e;
-        if (r >= R) continue;
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const int i = i0 + tx + 16 * a;
-            if (i >= M) continue;
-            const double2 b = r < n ? B0[bstride * blockIdx.z + i + (long long)M * r] : cz(r - n == i ? 1.0 : 0.0, 0.0);
-            E0[xstride * blockIdx.z + i + (long long)M * r] = csub(b, tot[a][e]);
-        }
     }
 }
 
-__global__ void k_ldl64_add(double2* __restrict__ X, const double2* __restrict__ E, long long n) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n) X[t] = cadd(X[t], E[t]);
+constexpr size_t mcols_smem(int M, int ct) { return sizeof(double2) * ((2 * (size_t)M + 6 * PB) * ct); }
+
+__global__ void __launch_bounds__(MCOLS_THREADS) k_ldl64_mcols(const double2* __restrict__ Z0,
+                                                               const double2* __restrict__ A0, int M,
+                                                               const double2* __restrict__ ws0, long long wstride,
+                                                               const double2* __restrict__ B0, int n, int R, int ct,
+                                                               double2* __restrict__ X0) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int b = blockIdx.y, c0 = blockIdx.x * ct, nc = min(ct, R - c0);
+    const long long MM = (long long)M * M;
+    const double2 *Z = Z0 + MM * b, *A = A0 + MM * b, *ws = ws0 + wstride * b, *B = B0 + (long long)M * n * b;
+    double2* x = reinterpret_cast<double2*>(smem_raw);
+    double2* e = x + (long long)M * ct;
+    double2 *raw = e + (long long)M * ct, *y = raw + PB * ct, *part = y + PB * ct;
+    auto rhs = [&](int i, int c) {
+        return c0 + c < n ? B[i + (long long)M * (c0 + c)] : cz(c0 + c - n == i ? 1.0 : 0.0, 0.0);
+    };
+    for (int t = threadIdx.x; t < M * nc; t += MCOLS_THREADS) x[t] = rhs(t % M, t / M);
+    __syncthreads();
+    mcols_sweeps(A, ws, x, M, nc, raw, part, y);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int u = warp; u < (M + 31) / 32 * nc; u += MCOLS_THREADS / 32) {
+        const int c = u % nc, i = 32 * (u / nc) + lane;
+        if (i >= M) continue;
+        double2 tot = cz(0.0, 0.0);
+        for (int k0 = 0; k0 < M; k0 += PB) {
+            double2 acc = cz(0.0, 0.0);
+#pragma unroll 8
+            for (int k = k0; k < min(k0 + PB, M); ++k) acc = cfma(Z[i + (long long)M * k], x[c * M + k], acc);
+            tot = cadd(tot, acc);
+        }
+        e[c * M + i] = csub(rhs(i, c), tot);
+    }
+    __syncthreads();
+    mcols_sweeps(A, ws, e, M, nc, raw, part, y);
+    double2* X = X0 + (long long)M * R * b + (long long)M * c0;
+    for (int t = threadIdx.x; t < M * nc; t += MCOLS_THREADS) X[t] = cadd(x[t], e[t]);
 }
 
 // Signs of the check's combination of right-hand sides.
@@ -1090,12 +1038,8 @@ int tags_ldl64_prepare() {
     static std::once_flag once;
     static int rc = 0;
     std::call_once(once, [] {
-        auto msolve_fits = [](const void* f) {
-            return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MSOLVE_SMEM) == cudaSuccess;
-        };
-        if (!msolve_fits((const void*)k_ldl64_msolve<false, 2>) || !msolve_fits((const void*)k_ldl64_msolve<false, 4>) ||
-            !msolve_fits((const void*)k_ldl64_msolve<true, 2>) || !msolve_fits((const void*)k_ldl64_msolve<true, 4>) ||
-            !msolve_fits((const void*)k_ldl64_mresid) ||
+        if (cudaFuncSetAttribute(k_ldl64_mcols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MCOLS_SMEM) !=
+                cudaSuccess ||
             cudaFuncSetAttribute(k_ldl64_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)small_smem(SMALL_N)) != cudaSuccess ||
             cudaFuncSetAttribute(k_ldl64_update<64, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1203,54 +1147,43 @@ int tags_ldl64_sym_solve(const double2* W, double2* A, int m, int n, void* ws, i
     return 0;
 }
 
-size_t tags_ldl64_multi_workspace(int M, int R) {
-    return 2 * sizeof(double2) * (((size_t)(M + PB - 1) / PB + 2) * PB * PB + 2 * (size_t)M + 2 * (size_t)M * R +
-                                  (size_t)M * M) + 64;
+bool tags_ldl64_multi_fits(int M) { return mcols_smem(M, 1) <= MCOLS_SMEM; }
+
+size_t tags_ldl64_multi_workspace(int M) {
+    return 2 * sizeof(double2) * (((size_t)(M + PB - 1) / PB + 2) * PB * PB + 2 * (size_t)M + (size_t)M * M) +
+           64;
 }
 
 int tags_ldl64_multi_solve(const double2* Z, const double2* rhs, int M, int n, int nb, double2* X, void* wsp,
                            int* d_bad, cudaStream_t st) {
     if (int e = tags_ldl64_prepare()) return e;
-    const int R = n + M, P = panel_count(M, 0);
+    const int R = n + M;
     const long long MM = (long long)M * M, MR = (long long)M * R, MN = (long long)M * n;
     Ws w{};
     w.wstride = (long long)((M + PB - 1) / PB + 2) * PB * PB;
     w.linv = reinterpret_cast<double2*>(wsp);
     double2* vu = w.linv + w.wstride * nb;           // nb x 2 x M
     double2* A = vu + 2LL * M * nb;                  // nb x M x M, the factors
-    double2* Y = A + MM * nb;                        // nb x M x R
-    double2* E = Y + MR * nb;                        // nb x M x R
     TAGS_CUDA_OK(cudaMemsetAsync(d_bad, 0, sizeof(int), st));
     TAGS_CUDA_OK(cudaMemcpyAsync(A, Z, sizeof(double2) * MM * nb, cudaMemcpyDeviceToDevice, st));
-    for (int b = 0; b < nb && n > 0; ++b)
-        TAGS_CUDA_OK(cudaMemcpyAsync(X + MR * b, rhs + MN * b, sizeof(double2) * MN, cudaMemcpyDeviceToDevice, st));
-    k_ldl64_identity<<<dim3((unsigned)((MM + 255) / 256), nb), 256, 0, st>>>(X, M, n, MR);
-    tags_note_launch();
     if (int e = factor(A, M, M, MM, nb, 0, w, st)) return e;
-    const int rt = (R + PB - 1) / PB;
-    auto sweep = [&](bool bwd, const Panel& q, int p, double2* x, double2* y) {
-        const int cols = bwd ? q.j0 : q.cnt;
-        const bool wide = (long long)((cols + 63) / 64) * rt * nb >= 304;
-        const int tc = wide ? 64 : 32;
-        const dim3 g(cols > 0 ? (cols + tc - 1) / tc : 1, rt, nb);
-        auto kern = bwd ? (wide ? k_ldl64_msolve<true, 4> : k_ldl64_msolve<true, 2>)
-                        : (wide ? k_ldl64_msolve<false, 4> : k_ldl64_msolve<false, 2>);
-        kern<<<g, 256, MSOLVE_SMEM, st>>>(A, M, MM, q, p, w.linv, w.wstride, x, y, M, MR, R);
-    };
-    auto sweeps = [&](double2* x) {
-        for (int p = 0; p < P; ++p) sweep(false, panel_at(p, M, 0), p, x, Y);
-        for (int p = P - 1; p >= 0; --p) sweep(true, panel_at(p, M, 0), p, Y, x);
-    };
-    sweeps(X);
+    // as many columns per CTA as leave the busiest SM the least to do
+    int ct = 1;
+    long long best = 0;
+    for (int t = 1; t <= MCOLS_MAX && mcols_smem(M, t) <= MCOLS_SMEM; ++t) {
+        const long long ctas = (long long)((R + t - 1) / t) * nb, cost = (ctas + 151) / 152 * t;
+        if (t == 1 || cost <= best) {
+            best = cost;
+            ct = t;
+        }
+    }
     // one refinement of every column: the factors were taken without pivoting
     // and the diagonal steps use inverses, so X alone is some times eps off
-    k_ldl64_mresid<<<dim3((M + 63) / 64, (R + PB - 1) / PB, nb), 128, MSOLVE_SMEM, st>>>(Z, M, MM, rhs, n, MN, X, E, MR,
-                                                                                      R);
-    sweeps(E);
-    k_ldl64_add<<<(unsigned)((MR * nb + 255) / 256), 256, 0, st>>>(X, E, MR * nb);
+    k_ldl64_mcols<<<dim3((R + ct - 1) / ct, nb), MCOLS_THREADS, mcols_smem(M, ct), st>>>(Z, A, M, w.linv, w.wstride, rhs,
+                                                                                    n, R, ct, X);
     k_ldl64_check_sum<<<dim3((M + 3) / 4, nb), 128, 0, st>>>(X, rhs, M, n, MR, MN, vu);
     k_ldl64_check<<<dim3((M + 3) / 4, nb), 128, 0, st>>>(Z, M, MM, vu, d_bad);
-    tags_note_launch(4 * P + 4);
+    tags_note_launch(3);
     TAGS_CUDA_OK(cudaGetLastError());
     return 0;
 }

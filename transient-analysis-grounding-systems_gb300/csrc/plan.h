@@ -164,7 +164,8 @@ int tags_ldl64_sym_solve(const double2* W, double2* A, int m, int n, void* ws, i
 // nb full symmetric matrices Z (M x M): X = Z^-1 [rhs, I] (M x (n + M) each;
 // rhs M x n). *d_bad is raised when a check of the result finds it less
 // accurate than a pivoted solve would be.
-size_t tags_ldl64_multi_workspace(int M, int R);     // two matrices
+bool tags_ldl64_multi_fits(int M);            // columns of M values fit a CTA's shared memory
+size_t tags_ldl64_multi_workspace(int M);     // two matrices
 int tags_ldl64_multi_solve(const double2* Z, const double2* rhs, int M, int n, int nb, double2* X, void* ws,
                            int* d_bad, cudaStream_t st);
 // capi.cu: x = W^-1 x for a caller's W (lower triangle read, original order) by
