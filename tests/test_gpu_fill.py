@@ -284,3 +284,47 @@ def test_mixed_fill_of_few_samples_matches_many(gpu_pkg, m):
             assert rel_err(zt, all_t[:ns]) < 1e-12
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("length,offset,shift", [(1.0, 0.1, 0.0), (1.0, 0.06, 0.4), (0.3, 0.2, -0.9), (1.0000001, 5.0, 2.0),
+                                                 (2.5, 0.0, 1.05), (0.7, 30.0, -0.2)])
+@pytest.mark.parametrize("turn", [0.0, 1e-9, 1e-3])
+@pytest.mark.parametrize("x", [0.05, 3.0, 6.0])
+def test_parallel_segments_match_oracle(gpu_pkg, port, length, offset, shift, turn, x):
+    """The single integral of parallel segments (equal, longer, shorter, opposed, in line, far) and the tensor rule just
+    off it, along an axis and askew, within the series' reach and past it; oracle at 1e-10, entries at TOL."""
+    pkg = gpu_pkg
+    askew = np.linalg.qr(np.array([[1.0, 2.0, 0.5], [0.3, 1.0, 1.7], [2.0, 0.1, 1.0]]))[0]
+    a = np.array([0.0, 0.0, -2.0])
+    b, c = a + [1.0, 0.0, 0.0], a + [shift, offset, 0.0]
+    for basis in (np.eye(3), askew):
+        for sign in (1.0, -1.0):
+            d = c + length * np.array([np.cos(turn), 0.0, np.sin(turn)])
+            ends = ((a, b), (c, d) if sign > 0 else (d, c))
+            e = np.stack([pkg.populate_electrode(p @ basis, q @ basis, 7e-3) for p, q in ends])
+            gamma = x / (e[:, 9].max() * 17 / 16) * np.exp(0.25j * np.pi)
+            s, kappa = 1e5 + 1e6j, 0.01 + 1e-4j
+            got = [np.zeros(4, np.complex128) for _ in range(2)]
+            want = [np.zeros(4, np.complex128) for _ in range(2)]
+            assert pkg.calculate_impedances(*got, e, gamma, s, 1.0, kappa) == 0
+            assert port.calculate_impedances(*want, e, gamma, s, 1.0, kappa, req_abs=0.0, req_rel=1e-10) == 0
+            for g, w in zip(got, want):
+                assert elementwise(g, w) < TOL
+
+
+@pytest.mark.parametrize("m", [70, 100, 140])
+def test_fill_of_many_segments_matches_few(gpu_pkg, m):
+    """4, 8 and 16 lanes per moment record against a whole warp (the first 20 segments alone), the same rule's points in
+    another order: sums of up to 64 terms of one sign, 1e-13."""
+    pkg = gpu_pkg
+    e = bent_wire(pkg, m)
+    for x in (0.1, 2.5):
+        gamma = x / (e[:, 9].max() * 17 / 16) * np.exp(0.25j * np.pi)
+        s, kappa = 1e5 + 1e6j, 0.01 + 1e-4j
+        out = {}
+        for k in (m, 20):
+            z = [np.zeros(k * k, np.complex128) for _ in range(2)]
+            assert pkg.calculate_impedances(*z, e[:k], gamma, s, 1.0, kappa) == 0
+            out[k] = [np.tril(v.reshape(k, k).T)[:20, :20] for v in z]
+        for a, b in zip(out[m], out[20]):
+            assert rel_err(a, b) < 1e-13

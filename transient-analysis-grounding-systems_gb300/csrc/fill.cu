@@ -456,14 +456,61 @@ __global__ void k_series_tab(const SampleCoef* __restrict__ coef, SeriesView v) 
     v.tab[(long long)b * v.ns + q] = cexp_d(cz(-g.x * R, -g.y * R));
 }
 
-enum : int { SK_NONE = 0, SK_TENSOR = 1, SK_TOUCH = 2, SK_BAD = 3 };
+enum : int { SK_NONE = 0, SK_TENSOR = 1, SK_TOUCH = 2, SK_BAD = 3, SK_PAR = 4 };
 
 struct SeriesPk {
     double o[3], dr[3], ds[3];   // tensor: r = |o + t0 dr - t1 ds|; touch: dr, ds = the corner vectors
     double R, fl;                // expansion centre; ZL factor |d_i . d_k| (0 where the reference drops ZL)
     double gl;                   // |gamma| times the longer panel
     int kind, Pr, Ps, q, b;      // panels of receiver and sender, order of the closest panel pair
+    double h2, z0, s, l;         // parallel: squared offset, coordinate at u = 0, shorter and longer length
+    int qm, npts;                // parallel: order on the middle piece (its panels are Ps); points in all
 };
+
+// Parallel segments: the distance depends on u = t0 |dr| -+ t1 |ds| alone, and
+// the pairs of points at one u make up a trapezoid, rising over [0, s], level
+// over [s, l], falling over [l, s + l]. So the double integral is a single one
+// over three pieces, in panels no longer than half the distance, one order more
+// than the tensor rule's for the weight's slope: 13 points instead of 25 for a
+// far pair of equal lengths, hundreds instead of tens of thousands for a wire
+// and its image. A level piece shorter than 1e-5 of the distance takes its
+// midpoint. Taken where the sender's deviation from the receiver's direction is
+// below 1e-15 of the distance (exactly zero along the axes) and no piece needs
+// more than 32 panels, the tensor rule's limit. With cta_moments' short rules, m
+// = 1560, 2 samples 135.4 -> 121.2 ms, 20 samples of a grid of 8 m segments in
+// four passes 33.5 -> 23.4, 12 segments of 11 m past the reach 23.1 -> 5.9.
+TAGS_D void series_parallel(const Seg& S, const Seg& R, double d, double ga, SeriesPk& k) {
+    double c2 = 0.0, par = 0.0, dot = 0.0;
+    for (int c = 0; c < 3; ++c) {
+        const int c1 = (c + 1) % 3, c3 = (c + 2) % 3;
+        const double x = k.dr[c1] * k.ds[c3] - k.dr[c3] * k.ds[c1];
+        c2 += x * x;
+        dot += k.dr[c] * k.ds[c];
+        par += k.dr[c] * k.o[c];
+    }
+    const double a2 = dot3(k.dr, k.dr);
+    if (!(c2 <= 1e-30 * d * d * a2)) return;
+    const double a = sqrt(a2), b = sqrt(dot3(k.ds, k.ds)), s = fmin(a, b), l = fmax(a, b);
+    const double p1 = ceil(2.0 * s / d), p2 = ceil(2.0 * (l - s) / d);
+    if (!(p1 <= 32.0 && p2 <= 32.0)) return;
+    par /= a;
+    k.h2 = 0.0;
+    for (int c = 0; c < 3; ++c) {
+        const double v = k.o[c] - par / a * k.dr[c];
+        k.h2 += v * v;
+    }
+    k.z0 = par - (dot > 0.0 ? b : 0.0);
+    k.s = s;
+    k.l = l;
+    k.Pr = max(1, (int)p1);
+    k.Ps = max(1, (int)p2);
+    const double lp = fmax(s / k.Pr, (l - s) / k.Ps);
+    k.gl = ga * lp;
+    k.q = min(QMAX, order_for(d / lp, k.gl, true) + 1);
+    k.qm = l == s ? 0 : l - s <= 1e-5 * d && ga * (l - s) <= 1e-6 ? 1 : k.q;
+    k.npts = 2 * k.Pr * k.q + k.Ps * k.qm;
+    k.kind = SK_PAR;
+}
 
 // One (pair, kind) classified as pair_integral does; ga: the pass's largest |gamma|.
 TAGS_D void series_classify(const Seg& S, const Seg& R, bool direct, double ga, const SeriesView& v, SeriesPk& k) {
@@ -488,6 +535,7 @@ TAGS_D void series_classify(const Seg& S, const Seg& R, bool direct, double ga, 
         k.kind = od <= 1e-9 * lmax ? SK_BAD : SK_TOUCH;
         k.Pr = k.Ps = 1;
         k.gl = 0.0;
+        k.npts = QMAX * QMAX;                              // by a whole warp
         k.q = min(QMAX, 16 + 2 * (int)ceil(fmin(ga * lmax, (double)QMAX)));
         rc = 0.5 * (sqrt(dot3(k.dr, k.dr)) + sqrt(dot3(k.ds, k.ds)));
         for (int c = 0; c < 3; ++c) {
@@ -505,35 +553,56 @@ TAGS_D void series_classify(const Seg& S, const Seg& R, bool direct, double ga, 
         const double lp = fmax(R.len / k.Pr, S.len / k.Ps);
         k.gl = ga * lp;
         k.q = order_for(dmin / lp, k.gl, true);
+        k.npts = k.Pr * k.Ps * k.q * k.q;
+        if (k.kind == SK_TENSOR) series_parallel(S, R, d, ga, k);
     }
     k.b = min(v.nbk - 1, max(0, (int)rint(rc / v.h)));
     k.R = k.b * v.h;
 }
 
-// Sum over the warp of acc[0..NT): lane l gets moment l (NT = 32) or l / 2
-// (NT = 16), each halving step keeping the half that the lane's bit names.
-template <int NT>
-TAGS_D double warp_transpose_sum(double (&acc)[NT], int lane) {
+// Sums over groups of L lanes of acc[0..NT), every lane of the warp taking part:
+// lane g of a group gets moments g NT / L onwards into acc[0..NT / L) (NT < L:
+// moment g NT / L), each halving step keeping the half that the lane's bit names.
+template <int NT, int L>
+TAGS_D void group_transpose_sum(double (&acc)[NT], int g) {
 #pragma unroll
-    for (int o = 16, w = NT / 2; w >= 1; o >>= 1, w >>= 1) {
-        const bool up = (lane & o) != 0;
+    for (int o = L / 2, w = NT / 2; o >= 1; o >>= 1, w >>= 1) {
+        const bool up = (g & o) != 0;
+        if (w == 0) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
 #pragma unroll
         for (int i = 0; i < w; ++i) {
             const double send = up ? acc[i] : acc[i + w], keep = up ? acc[i + w] : acc[i];
             acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
         }
     }
-    double r = acc[0];
-    if (NT == 16) r += __shfl_xor_sync(0xffffffffu, r, 1);
-    return r;
 }
 
-// The tensor rule of one record by a warp: f(r, weight) per point. The lanes
-// share the points, or, with 32 panel pairs and more, the panel pairs, each at
-// the order its own distance needs (order_for's rule; only the closest need
-// k.q), which is where nearly all points of a finely split pair lie.
+// The rule of one untouched record by nl lanes: f(r, weight / r) per point.
+// Parallel segments: the points of the rising and falling pieces, then the
+// level one's. Others: the tensor rule; the lanes share the points, or, a whole
+// warp with 32 panel pairs and more, the panel pairs, each at the order its own
+// distance needs (order_for's rule; only the closest need k.q), which is where
+// nearly all points of a finely split pair lie. The distance by rsqrt, 1 ulp,
+// which saves a root or a division of the point's ~20 instructions.
 template <class F>
-TAGS_D void tensor_points(const SeriesPk& k, int lane, F f) {
+TAGS_D void rule_points(const SeriesPk& k, int lane, int nl, F f) {
+    auto at = [&](double d2, double w) {
+        const double ri = rsqrt(d2);
+        f(d2 * ri, w * ri);
+    };
+    if (k.kind == SK_PAR) {
+        const int n1 = k.Pr * k.q;
+        const double hs = k.s / k.Pr, hl = (k.l - k.s) / k.Ps, il = 1.0 / k.l;
+        for (int t = lane; t < k.npts; t += nl) {
+            const bool level = t >= 2 * n1;
+            const int u = level ? t - 2 * n1 : t >= n1 ? t - n1 : t, q = level ? k.qm : k.q, pp = u / q;
+            const double x = (pp + g_glx[gl_off(q) + u - pp * q]) * (level ? hl : hs);
+            const double w = g_glw[gl_off(q) + u - pp * q] * (level ? hl : x / k.Pr) * il;
+            const double z = k.z0 + (level ? k.s + x : t >= n1 ? k.s + k.l - x : x);
+            at(fma(z, z, k.h2), w);
+        }
+        return;
+    }
     const double hr = 1.0 / k.Pr, hs = 1.0 / k.Ps;
     auto point = [&](double t0, double t1, double w) {
         double d2 = 0.0;
@@ -541,9 +610,9 @@ TAGS_D void tensor_points(const SeriesPk& k, int lane, F f) {
             const double d = fma(t0, k.dr[c], fma(-t1, k.ds[c], k.o[c]));
             d2 = fma(d, d, d2);
         }
-        f(sqrt(d2), w * (hr * hs));
+        at(d2, w * (hr * hs));
     };
-    if (k.Pr * k.Ps >= 32) {
+    if (nl == 32 && k.Pr * k.Ps >= 32) {
         const double lr = sqrt(dot3(k.dr, k.dr)) * hr, ls = sqrt(dot3(k.ds, k.ds)) * hs, lp = fmax(lr, ls);
         for (int pp = lane; pp < k.Pr * k.Ps; pp += 32) {
             const int pi = pp / k.Ps, pj = pp - pi * k.Ps;
@@ -565,7 +634,7 @@ TAGS_D void tensor_points(const SeriesPk& k, int lane, F f) {
     const double* x = g_glx + gl_off(k.q);
     const double* w = g_glw + gl_off(k.q);
     const int qq = k.q * k.q, npts = k.Pr * k.Ps * qq;
-    for (int t = lane; t < npts; t += 32) {
+    for (int t = lane; t < npts; t += nl) {
         const int pp = t / qq, u = t - pp * qq;
         const int pi = pp / k.Ps, pj = pp - pi * k.Ps, qi = u / k.q, qj = u - qi * k.q;
         point((pi + x[qi]) * hr, (pj + x[qj]) * hs, w[qi] * w[qj]);
@@ -585,24 +654,24 @@ TAGS_D void touch_node(const SeriesPk& k, int t, double& rho, double& v) {
     v = g_glw[gl_off(k.q) + i] / rho;
 }
 
-// Moments of one record by a warp, lanes over the rule's points -> mom[0..NT).
-template <int NT>
-TAGS_D void series_moments(const SeriesPk& k, int lane, double* mom) {
+// Moments of one record by a group of L lanes (all of the warp's groups take
+// part, `on` or not), lanes over the rule's points -> mom[0..NT).
+template <int NT, int L>
+TAGS_D void series_moments(const SeriesPk& k, bool on, int lane, double* mom) {
     double acc[NT];
 #pragma unroll
     for (int n = 0; n < NT; ++n) acc[n] = 0.0;
-    if (k.kind == SK_TENSOR) {
-        tensor_points(k, lane, [&](double r, double w) {
+    if (on && k.kind != SK_TOUCH) {
+        rule_points(k, lane, L, [&](double r, double v) {
             const double d = r - k.R;
-            double v = w / r;
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
                 acc[n] += v;
                 v *= d;
             }
         });
-    } else {
-        for (int t = lane; t < 2 * k.q; t += 32) {
+    } else if (on) {
+        for (int t = lane; t < 2 * k.q; t += L) {
             double rho, v;
             touch_node(k, t, rho, v);
             const double a = rho - k.R;
@@ -615,10 +684,38 @@ TAGS_D void series_moments(const SeriesPk& k, int lane, double* mom) {
             }
         }
     }
-    double r = warp_transpose_sum<NT>(acc, lane);
-    const int n = NT == 32 ? lane : lane >> 1;
-    if (k.kind == SK_TOUCH) r /= (double)(n + 1);
-    if (NT == 32 || (lane & 1) == 0) mom[n] = r;
+    group_transpose_sum<NT, L>(acc, lane);
+    constexpr int W = NT > L ? NT / L : 1;
+    const int n0 = NT > L ? lane * W : lane * NT / L;
+    if (!on || (NT < L && lane % (L / NT) != 0)) return;
+#pragma unroll
+    for (int i = 0; i < W; ++i) mom[n0 + i] = k.kind == SK_TOUCH ? acc[i] / (double)(n0 + i + 1) : acc[i];
+}
+
+// Moments of a CTA's nrec records (128 / L at most): the short rules by L lanes
+// each, all at once, then the touching and the finely split ones warp by warp.
+// A far pair takes 13 or 25 points, so a warp per record leaves lanes idle and
+// adds up 32 lanes' moments; with 4 lanes 8 records share those instructions.
+constexpr int SER_SHORT = 64;            // points of a short rule, at most
+template <int NT, int L>
+TAGS_D void cta_moments(const SeriesPk* pk, int nrec, double (*mom)[SER_NT], int tid) {
+    if (L < 32) {
+        const int r = tid / L;
+        const bool on = r < nrec && (pk[r].kind == SK_TENSOR || pk[r].kind == SK_PAR) && pk[r].npts <= SER_SHORT;
+        series_moments<NT, L>(pk[on ? r : 0], on, tid % L, mom[r]);
+    }
+    constexpr int NW = NT == 12 ? 16 : NT;
+    for (int r = tid >> 5; r < nrec; r += SER_THREADS / 32)
+        if (pk[r].kind == SK_TOUCH ||
+            ((pk[r].kind == SK_TENSOR || pk[r].kind == SK_PAR) && (L == 32 || pk[r].npts > SER_SHORT)))
+            series_moments<NW, 32>(pk[r], true, tid & 31, mom[r]);
+}
+
+template <int L>
+TAGS_D void cta_moments_of(int nt, const SeriesPk* pk, int nrec, double (*mom)[SER_NT], int tid) {
+    if (L == 4 && nt <= 12) cta_moments<12, 4>(pk, nrec, mom, tid);
+    else if (nt <= 16) cta_moments<16, L>(pk, nrec, mom, tid);
+    else cta_moments<32, L>(pk, nrec, mom, tid);
 }
 
 // Terms needed at x = max |gamma| dmax.
@@ -645,10 +742,9 @@ TAGS_D double2 series_sum(const SeriesView& v, const double* mom, int nt, int s)
 // J of one (pair, kind) at one sample by a warp (all lanes get it).
 TAGS_D double2 direct_integral(const SeriesPk& k, double2 g, int lane) {
     double2 a = cz(0.0, 0.0);
-    if (k.kind == SK_TENSOR) {
-        tensor_points(k, lane, [&](double r, double w) {
+    if (k.kind != SK_TOUCH) {
+        rule_points(k, lane, 32, [&](double r, double v) {
             const double2 e = cexp_d(cz(-g.x * r, -g.y * r));
-            const double v = w / r;
             a.x = fma(e.x, v, a.x);
             a.y = fma(e.y, v, a.y);
         });
@@ -749,15 +845,18 @@ __global__ void __launch_bounds__(SER_THREADS) k_path_far(const double* __restri
 }
 
 // A CTA takes `npt` consecutive pairs (column by column): one warp classifies
-// their kinds, the warps form the moments record by record, then the threads
-// run over (pair, sample). Bound by the FP64 pipe in both parts.
+// their kinds, L lanes form each record's moments, then the threads run over
+// (pair, sample). Bound by the FP64 pipe in all parts; the classifying warp and
+// the samples' first go round the four SM quarters with the CTA's number, since
+// a warp's FP64 instructions hold its quarter only.
+template <int L>
 __global__ void __launch_bounds__(SER_THREADS) k_fill_series(const double* __restrict__ elec,
                                                              const double* __restrict__ img, int m,
                                                              const SampleCoef* __restrict__ coef, SeriesView v,
                                                              FillOut out, int mode, int npt, int* status) {
     __shared__ SeriesPk pk[SER_PK];
     __shared__ double mom[SER_PK][SER_NT];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = (threadIdx.x + 32 * (blockIdx.x & 3)) & (SER_THREADS - 1);
     const long long npairs = (long long)m * (m + 1) / 2;
     const long long p0 = (long long)blockIdx.x * npt;
     const int np = (int)min((long long)npt, npairs - p0);
@@ -778,11 +877,7 @@ __global__ void __launch_bounds__(SER_THREADS) k_fill_series(const double* __res
         }
     }
     __syncthreads();
-    for (int q = warp; q < 2 * np; q += SER_THREADS / 32) {
-        if (pk[q].kind != SK_TENSOR && pk[q].kind != SK_TOUCH) continue;
-        if (nt <= 16) series_moments<16>(pk[q], lane, mom[q]);
-        else series_moments<32>(pk[q], lane, mom[q]);
-    }
+    cta_moments_of<L>(nt, pk, 2 * np, mom, tid);
     __syncthreads();
     for (long long t = tid; t < (long long)np * v.ns; t += SER_THREADS) {
         const int lp = (int)(t / v.ns), s = (int)(t - (long long)lp * v.ns);
@@ -813,13 +908,14 @@ __global__ void __launch_bounds__(SER_THREADS) k_fill_series(const double* __res
 
 // The path/electrode integrals of k_path_pairs from moments: a CTA takes npt
 // consecutive (electrode, path) records.
+template <int L>
 __global__ void __launch_bounds__(SER_THREADS) k_path_series(const double* __restrict__ elec, int m,
                                                              const double* __restrict__ paths, int npaths,
                                                              SeriesView v, double2* __restrict__ jj, int npt,
                                                              int* status) {
     __shared__ SeriesPk pk[SER_PK];
     __shared__ double mom[SER_PK][SER_NT];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = (threadIdx.x + 32 * (blockIdx.x & 3)) & (SER_THREADS - 1);
     const long long n = (long long)m * npaths, p0 = (long long)blockIdx.x * npt;
     const int np = (int)min((long long)npt, n - p0);
     const double ga = __longlong_as_double((long long)*v.gmax);
@@ -833,11 +929,7 @@ __global__ void __launch_bounds__(SER_THREADS) k_path_series(const double* __res
         if (pk[tid].kind == SK_BAD) raise_status(status, TAGS_ST_DEGENERATE_PAIR);
     }
     __syncthreads();
-    for (int q = warp; q < np; q += SER_THREADS / 32) {
-        if (pk[q].kind == SK_BAD) continue;
-        if (nt <= 16) series_moments<16>(pk[q], lane, mom[q]);
-        else series_moments<32>(pk[q], lane, mom[q]);
-    }
+    cta_moments_of<L>(nt, pk, np, mom, tid);
     __syncthreads();
     // records fastest: a sample's values are written side by side
     for (long long t = tid; t < (long long)np * v.ns; t += SER_THREADS) {
@@ -2379,8 +2471,10 @@ int tags_launch_fill_fp64(const double* d_elec, const double* d_img, int m, cons
         const SeriesView v = series_view(*geo, series_ws, nsamp);
         if (int e = series_tables(d_coef, v, st)) return e;
         const int npt = series_tile(npairs, SER_PK / 2);
-        k_fill_series<<<(unsigned)((npairs + npt - 1) / npt), SER_THREADS, 0, st>>>(d_elec, d_img, m, d_coef, v, out,
-                                                                                   mode, npt, d_status);
+        auto fill = npt == 16 ? k_fill_series<4> : npt == 8 ? k_fill_series<8> : npt == 4 ? k_fill_series<16>
+                                                                                          : k_fill_series<32>;
+        fill<<<(unsigned)((npairs + npt - 1) / npt), SER_THREADS, 0, st>>>(d_elec, d_img, m, d_coef, v, out, mode, npt,
+                                                                          d_status);
         k_fill_far<<<far_ctas(npairs, nsamp), SER_THREADS, 0, st>>>(d_elec, d_img, m, d_coef, v, out, mode, d_status);
         tags_note_launch(2);
     } else {
@@ -2404,8 +2498,9 @@ int tags_launch_path_pairs(const double* d_elec, int m, const double* d_paths, i
         const SeriesView v = series_view(*geo, series_ws, nsamp);
         if (int e = series_tables(d_coef, v, st)) return e;
         const int npt = series_tile(n, SER_PK);
-        k_path_series<<<(unsigned)((n + npt - 1) / npt), SER_THREADS, 0, st>>>(d_elec, m, d_paths, npaths, v, d_jj, npt,
-                                                                              d_status);
+        auto path = npt == 32 ? k_path_series<4> : npt == 16 ? k_path_series<8> : npt == 8 ? k_path_series<16>
+                                                                                           : k_path_series<32>;
+        path<<<(unsigned)((n + npt - 1) / npt), SER_THREADS, 0, st>>>(d_elec, m, d_paths, npaths, v, d_jj, npt, d_status);
         k_path_far<<<far_ctas(n, nsamp), SER_THREADS, 0, st>>>(d_elec, m, d_paths, npaths, d_coef, v, d_jj, d_status);
         tags_note_launch(2);
     } else {
