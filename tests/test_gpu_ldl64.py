@@ -140,3 +140,17 @@ def test_yla_ytb_of_any_symmetric_blocks(gpu_pkg, m, n, zero_diagonal):
 def test_yla_ytb_of_one_to_eight_columns_per_cta(gpu_pkg, m, n):
     """Widths of the column tiles of the nodal solve, with a ragged last one."""
     test_yla_ytb_of_any_symmetric_blocks(gpu_pkg, m, n, False)
+
+
+@pytest.mark.parametrize("m,ns", [(22, 1), (106, 38), (106, 39), (107, 19), (107, 20), (171, 3), (341, 2), (342, 2)])
+def test_plain_plan_solves_on_clusters(gpu_pkg, m, ns):
+    """The cluster solve and its limits: N = 1024 (m = 341), two waves of clusters up to N = 320, one above."""
+    pkg = gpu_pkg
+    e, nodes = wire(pkg, m)
+    img = pkg.images(e)
+    s = 8e4 + 2j * np.pi * np.linspace(1e3, 1e6, ns)
+    kappa = 0.01 + s * 12 * pkg.EPS0
+    sol, info, _ = pkg.hem_sweep(e, img, nodes, s, kappa, inj_node=m // 2, max_batch=ns)
+    assert not info.any()
+    for k in {0, ns - 1}:
+        assert rel_err(sol[k], dense_solution(pkg, e, img, nodes, s[k], kappa[k], m // 2)) < TOL

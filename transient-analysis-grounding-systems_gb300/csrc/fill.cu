@@ -442,7 +442,8 @@ __global__ void k_series_coef(const SampleCoef* __restrict__ coef, SeriesView v)
     if (!ok) v.far[atomicAdd(v.nfar, 1)] = q;
     if (ok) atomicMax(v.gmax, (unsigned long long)__double_as_longlong(ga));
     double2 p = cz(1.0, 0.0);
-    for (int n = 0; n < SER_NT; ++n) {
+#pragma unroll
+    for (int n = 0; n < SER_NT; ++n) {                     // constant reciprocals
         v.pw[(long long)n * v.ns + q] = ok ? p : cz(0.0, 0.0);
         p = cscale(cmul(p, cneg(g)), 1.0 / (double)(n + 1));
     }

@@ -78,6 +78,23 @@ TAGS_HD Panel panel_at(int p, int N, int m) {
     return q;
 }
 
+// All CTAs of the cluster; their shared memory's writes before it are seen after.
+TAGS_D void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// *p of the cluster's CTA `rank`, p in shared memory.
+TAGS_D double2 ld_cluster(const double2* p, int rank) {
+    uint32_t a;
+    double2 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(a)
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"((uint32_t)rank));
+    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a) : "memory");
+    return v;
+}
+
 TAGS_D double2 crecip(double2 d) {
     const double s = 1.0 / (d.x * d.x + d.y * d.y);      // out of range: not finite, the sample goes to the LU
     return make_double2(d.x * s, -d.y * s);
@@ -405,6 +422,97 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_ldl64_solve_cta(
     for (int j = threadIdx.x; j < N; j += blockDim.x) S0[(long long)N * b + j] = xs[j];
 }
 
+// The same of one sample by a cluster of 8 CTAs, for a few samples of up to 1024
+// unknowns, whose sweeps leave the SMs idle in the kernels above: CTA g owns the
+// rows whose 32-row chunk is g mod 8. Per panel every CTA gathers the panel's 32
+// values from their owners' shared memory, forms the diagonal step itself and
+// updates its own rows, eight columns per warp; one cluster barrier. The matrix's
+// values do not wait for the vector, so a step's first two chunks are on their
+// way before the barrier. The forward sweep works in xs and leaves its values in
+// zs, the backward sweep the other way round, so nothing is overwritten that
+// another CTA has still to gather. The backward sweep reads U = D L^T, whose rows
+// lie side by side, with 1/D at the diagonal step. One sample at N = 285 195 ->
+// 118 us; at N = 801 six samples' solves 0.31 -> 0.22 ms each. Where the line lies:
+// N <= 64 gains nothing from eight CTAs (280 against 267 us for a whole nodal
+// chain of 4 segments); up to N = 320 two waves of clusters still beat a CTA per
+// sample, above that one wave beats the launches per panel.
+constexpr int SCL_G = 8, SCL_N = 1024, SCL_UNITS = (SCL_N / 32 + SCL_G - 1) / SCL_G + 1;
+constexpr size_t scl_smem(int N) { return sizeof(double2) * 2 * (size_t)N; }
+
+__global__ void __cluster_dims__(SCL_G, 1, 1) __launch_bounds__(128) k_ldl64_solve_cl(
+    const double2* __restrict__ A0, long long ld, long long stride, int N, int m, const double2* __restrict__ ws0,
+    long long wstride, const double2* __restrict__ X0, double2* __restrict__ S0, int p0,
+    const int* __restrict__ active) {
+    const int b = blockIdx.y, g = blockIdx.x;
+    if (!active[b]) return;                                  // the whole cluster
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2* xs = reinterpret_cast<double2*>(smem_raw);      // N, own rows
+    double2* zs = xs + N;                                    // N, own rows
+    __shared__ double2 raw[PB], y[PB], part[4][PB], sum[SCL_UNITS][4][PB];
+    const double2* A = A0 + stride * b;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, P = panel_count(N, m);
+    auto own = [&](int i) { return ((i >> 5) & (SCL_G - 1)) == g; };
+    for (int i = tid; i < N; i += 128)
+        if (own(i)) {
+            xs[i] = X0[(long long)N * b + i];
+            zs[i] = cz(0.0, 0.0);                            // the sweep is zero above panel p0
+        }
+    for (int s = p0; s < 2 * P; ++s) {
+        const int bwd = s >= P, p = bwd ? 2 * P - 1 - s : s;
+        const Panel q = panel_at(p, N, m);
+        const double2* ws = ws0 + wstride * b + (long long)p * PB * PB;
+        double2 *work = bwd ? zs : xs, *fin = bwd ? xs : zs;
+        // the rows to update: [lo, hi) without [q.lim, q.lim + q.skip) below a ZL panel
+        const int lo = bwd ? (m > 0 && q.j0 >= m && q.j0 < 2 * m ? m : 0) : q.base, hi = bwd ? q.j0 : N;
+        const int b0 = bwd ? N : q.lim, b1 = bwd ? N : q.lim + q.skip;
+        auto live = [&](int i) { return i >= lo && i < hi && !(i >= b0 && i < b1); };
+        const int c0 = (lo >> 5) + ((g - (lo >> 5)) & (SCL_G - 1));     // first own chunk
+        const double2* col = A + ld * (q.j0 + 8 * warp);
+        double2 pre[2][8];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int i = 32 * (c0 + SCL_G * u) + lane;
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                pre[u][k] = live(i) && 8 * warp + k < q.jb ? col[i + ld * k] : cz(0.0, 0.0);
+        }
+        cluster_barrier();                                   // the panel's values are updated by all panels before
+        if (tid < PB) {
+            double2 v = cz(0.0, 0.0);
+            if (tid < q.jb) {
+                const int i = q.j0 + tid;
+                v = ld_cluster(work + i, (i >> 5) & (SCL_G - 1));
+                if (bwd) v = cmul(v, ws[tid * (PB + 1)]);
+            }
+            raw[tid] = v;
+        }
+        __syncthreads();
+        block_apply(ws, raw, y, part, bwd);
+        if (tid < q.jb && own(q.j0 + tid)) fin[q.j0 + tid] = y[tid];
+        int nu = 0;
+        for (int c = c0; 32 * c < hi; c += SCL_G, ++nu) {
+            const int i = 32 * c + lane;
+            double2 acc = cz(0.0, 0.0);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const double2 l = nu == 0 ? pre[0][k] : nu == 1 ? pre[1][k]
+                                : live(i) && 8 * warp + k < q.jb ? col[i + ld * k] : cz(0.0, 0.0);
+                acc = cfma(l, y[8 * warp + k], acc);
+            }
+            sum[nu][warp][lane] = acc;
+        }
+        __syncthreads();
+        for (int u = warp; u < nu; u += 4) {
+            const int i = 32 * (c0 + SCL_G * u) + lane;
+            if (live(i))
+                work[i] = csub(work[i], cadd(cadd(sum[u][0][lane], sum[u][1][lane]), cadd(sum[u][2][lane], sum[u][3][lane])));
+        }
+    }
+    cluster_barrier();                                       // no CTA leaves while another gathers from it
+    for (int i = tid; i < N; i += 128)
+        if (own(i)) S0[(long long)N * b + i] = xs[i];
+}
+
 // Reordered index -> index of the original order [U, I_L, I_T] (m = 0: equal).
 TAGS_D int orig_index(int ip, int m, int n) { return ip < 2 * m ? n + ip : ip - 2 * m; }
 
@@ -718,28 +826,23 @@ __global__ void k_ldl64_permute(const double2* __restrict__ W, double2* __restri
 }
 
 // r = b - W x for the full symmetric W in the original order, x and r in the
-// static order; a thread per row.
-__global__ void __launch_bounds__(64) k_ldl64_resid_full(const double2* __restrict__ W, int m, int n,
-                                                         const double2* __restrict__ B,
-                                                         const double2* __restrict__ X, double2* __restrict__ R,
-                                                         const int* __restrict__ active) {
+// static order; a warp per row, read as the column (95 us with a thread per row
+// at N = 285).
+__global__ void __launch_bounds__(128) k_ldl64_resid_full(const double2* __restrict__ W, int m, int n,
+                                                          const double2* __restrict__ B,
+                                                          const double2* __restrict__ X, double2* __restrict__ R,
+                                                          const int* __restrict__ active) {
     if (!active[0]) return;
-    __shared__ double2 xs[64];
-    const int N = n + 2 * m, ip = blockIdx.x * blockDim.x + threadIdx.x;
-    const int row = ip < N ? orig_index(ip, m, n) : 0;
+    const int N = n + 2 * m, ip = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (ip >= N) return;
+    const double2* row = W + (long long)N * orig_index(ip, m, n);
     double2 acc = cz(0.0, 0.0);
-    for (int j0 = 0; j0 < N; j0 += 64) {
-        const int nj = min(64, N - j0);
-        __syncthreads();
-        if ((int)threadIdx.x < nj) xs[threadIdx.x] = X[j0 + threadIdx.x];
-        __syncthreads();
-        if (ip < N) {
-#pragma unroll 8
-            for (int j = 0; j < nj; ++j)
-                acc = cfma(W[row + (long long)N * orig_index(j0 + j, m, n)], xs[j], acc);
-        }
+    for (int j = lane; j < N; j += 32) acc = cfma(row[orig_index(j, m, n)], X[j], acc);
+    for (int o = 16; o > 0; o >>= 1) {
+        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+        acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
     }
-    if (ip < N) R[ip] = csub(B[ip], acc);
+    if (lane == 0) R[ip] = csub(B[ip], acc);
 }
 
 // ---- many right-hand sides (the nodal admittance drop-ins)
@@ -1001,6 +1104,14 @@ int solve(const double2* A, int N, long long ld, long long stride, int nb, int m
     int p0 = 0;
     while (p0 + 1 < P && panel_at(p0, N, m).base <= lead) ++p0;
     int pf = tags_prof_begin(TAGS_PROF_LU64_OTHER, st);
+    if (N > 64 && N <= SCL_N && nb <= (N <= 320 ? 38 : 19)) {
+        k_ldl64_solve_cl<<<dim3(SCL_G, nb), 128, scl_smem(N), st>>>(A, ld, stride, N, m, w.linv, w.wstride, w.r, w.z, p0,
+                                                                    w.active);
+        tags_prof_end(TAGS_PROF_LU64_OTHER, pf, st, 0.0, 0.0);
+        tags_note_launch();
+        TAGS_CUDA_OK(cudaGetLastError());
+        return 0;
+    }
     if (N <= 320 || (nb >= 128 && N <= SOLVE_N_MAX)) {
         k_ldl64_solve_cta<<<nb, SOLVE_THREADS, sizeof(double2) * N, st>>>(A, ld, stride, N, m, w.linv, w.wstride, w.r,
                                                                           w.z, p0, w.active);
@@ -1132,7 +1243,7 @@ int tags_ldl64_sym_solve(const double2* W, double2* A, int m, int n, void* ws, i
     int err = factor(A, N, N, 0, 1, zm, w, st);
     for (int step = 0; step < 3 && !err; ++step) {
         if (step > 0) {
-            k_ldl64_resid_full<<<(N + 63) / 64, 64, 0, st>>>(W, m, n, w.b, w.x, w.r, w.active);
+            k_ldl64_resid_full<<<(N + 3) / 4, 128, 0, st>>>(W, m, n, w.b, w.x, w.r, w.active);
             tags_note_launch();
         }
         err = solve(A, N, N, 0, 1, zm, w, 0, st);
