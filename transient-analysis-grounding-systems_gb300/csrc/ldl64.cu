@@ -109,12 +109,12 @@ TAGS_D double2 crecip(double2 d) {
 // 496 elements right of column 0 are dealt to the threads column by column, four
 // each in registers, so that a step's live ones fill whole warps (252
 // instructions for the products instead of 544 with a lane per row and a warp
-// per column), every warp forms the pivot's reciprocal and the scaled column
-// itself (14 a step), one barrier per step. The rows: LPR lanes share a row,
-// 32 / LPR columns each: 576 instructions with 4 lanes, 320 with 8, 192 with 16,
-// which take more CTAs for the same rows (panel_split). The 11 panels of one
-// system at m = 100, n = 85 608 -> 400 us (the drop-in chain 1.80 -> 1.60 ms), the
-// plain form's 256 samples 6.65 -> 6.19 ms.
+// per column); every warp forms the scaled column itself (15 a step); one
+// barrier per step. The rows: LPR lanes share a row, 32 / LPR columns each: 576
+// instructions with 4 lanes, 320 with 8, 192 with 16, which take more CTAs for
+// the same rows (panel_split). The 11 panels and block inverses of one system at m
+// = 100, n = 85 644 -> 400 us, the panels of the plain form's 256 samples 2.3 ->
+// 1.9 ms.
 template <int LPR>
 __global__ void __launch_bounds__(128) k_ldl64_panel(double2* __restrict__ A0, long long ld, long long stride,
                                                      Panel q, int p, double2* __restrict__ ws0, long long wstride,
@@ -131,7 +131,6 @@ __global__ void __launch_bounds__(128) k_ldl64_panel(double2* __restrict__ A0, l
         if (r < q.jb && c <= r) v = A[(q.j0 + r) + ld * (q.j0 + c)];
         sL[r][c] = v;
     }
-    if (tid < PB) sdi[tid] = cz(1.0, 0.0);
     __syncthreads();
     int er[4], ec[4];
     double2 ev[4];
@@ -143,9 +142,9 @@ __global__ void __launch_bounds__(128) k_ldl64_panel(double2* __restrict__ A0, l
         ev[i] = sL[er[i]][ec[i]];
     }
     for (int k = 0; k < q.jb; ++k) {
-        const double2 di = crecip(sL[k][k]);
-        if (tid == 0) sdi[k] = di;
-        const double2 l = cneg(cmul(sL[lane][k], di));     // rows up to k are not used
+        // -W / d as (-W conj(d)) / |d|^2: the product is formed while the reciprocal is
+        const double2 d = sL[k][k], w = cmul(sL[lane][k], cz(-d.x, d.y));
+        const double2 l = cscale(w, 1.0 / (d.x * d.x + d.y * d.y));     // rows up to k are not used
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             if (!__any_sync(0xffffffffu, ec[i] > k)) continue;
@@ -157,6 +156,8 @@ __global__ void __launch_bounds__(128) k_ldl64_panel(double2* __restrict__ A0, l
         }
         __syncthreads();
     }
+    if (tid < PB) sdi[tid] = crecip(sL[tid][tid]);         // 1 past jb
+    __syncthreads();
     for (int t = tid; t < PB * PB; t += 128) {            // unscaled columns -> L11
         const int r = t % PB, c = t / PB;
         if (r > c && r < q.jb) sL[r][c] = cmul(sL[r][c], sdi[c]);
