@@ -328,3 +328,29 @@ def test_fill_of_many_segments_matches_few(gpu_pkg, m):
             out[k] = [np.tril(v.reshape(k, k).T)[:20, :20] for v in z]
         for a, b in zip(out[m], out[20]):
             assert rel_err(a, b) < 1e-13
+
+
+@pytest.mark.parametrize("m", [2, 9])
+def test_mixed_fill_touching_pairs_on_both_sides_of_their_series_limit(gpu_pkg, m):
+    """The series of the touching pairs about half the largest distance (R, the longest segment; 24 terms to |gamma| R =
+    1.75) and the Duffy rule past it, in one pass of 32 samples per warp and one sample alone; 1e-13 as above."""
+    pkg = gpu_pkg
+    e = bent_wire(pkg, m)
+    nodes = np.concatenate([e[:1, :3], e[:, 3:6]])
+    x = np.concatenate([np.geomspace(1e-3, 1.7, 32), np.linspace(1.5, 2.5, 32)])
+    s = 1e5 + 1e6j
+    kappa = (x / e[:, 9].max() * np.exp(0.25j * np.pi)) ** 2 / (s * 4e-7 * np.pi)
+    spec = np.zeros((m, m), bool)
+    spec[tuple(np.array(sorted(_touching_pairs(e))).T)] = True
+    spec[np.diag_indices(m)] = True
+    spec &= np.tril(np.ones((m, m), bool))
+    for take in (slice(None), slice(63, 64), slice(0, 1)):
+        plan = pkg.Plan(e, None, nodes, pkg.MIXED, max_batch=64)
+        try:
+            got = plan.mixed_fill(np.full(64, s)[take], kappa[take])
+        finally:
+            plan.close()
+        for b, k in enumerate(np.arange(64)[take]):
+            for z, want in zip(got, gpu_fill(pkg, e, None, s, kappa[k])):
+                nz = spec & (np.abs(want) > 0)
+                assert elementwise(z[b][nz], want[nz]) < 1e-13

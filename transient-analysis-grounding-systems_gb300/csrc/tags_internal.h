@@ -74,7 +74,7 @@ struct SpecialEntries {
     int n = 0;                   // entries
     int2* ent = nullptr;         // (pair index p of (k, i), k >= i; kinds mask: bit 0 direct, 1 image, 2 self)
     double* tm = nullptr;        // FP64 Duffy moments of the touching kinds: [entry][kind][24]
-    double tdmax = 0.0;          // bound of the Duffy distances (2 x the longest segment)
+    double rc = 0.0;             // centre of their expansion: half the bound of the Duffy distances
 };
 int tags_mixed_special_build(void* ws, int m, int batch, SpecialEntries* sp, cudaStream_t st);
 // the Duffy moments of the special entries' touching kinds (once per plan)
