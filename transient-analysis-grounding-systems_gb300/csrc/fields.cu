@@ -434,9 +434,10 @@ TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, double h
 // at a time, a thread forms a pair's moments, then the warps (sample group x
 // share of the electrodes; lanes: G samples x 32 / G electrodes) sum the series
 // and accumulate the currents' terms. FP64-bound: 6 nt + 24 multiply-adds per
-// (pair, sample) and 26 per injection. The 1560-segment grid, 251 points, 64
-// samples, 4 injections: 58.8 ms by the rule per sample, 14.2 ms so (error of the
-// field against 64-bit quadrature 1.6e-13 -> 2.2e-15).
+// (pair, sample) and 20 per injection. The 1560-segment grid, 251 points, 64
+// samples, 4 injections: 58.8 ms by the rule per sample, 13.1 ms so (14.4 with the
+// vector potential's three components per pair; error of the field against 64-bit
+// quadrature 1.6e-13 -> 2.2e-15).
 constexpr int FS_E = 128;                 // pairs per tile, a thread each
 template <int NT>
 __global__ void __launch_bounds__(FS_THREADS) k_fields_series(SerArgs sa, int r0) {
@@ -469,6 +470,23 @@ __global__ void __launch_bounds__(FS_THREADS) k_fields_series(SerArgs sa, int r0
 #pragma unroll
         for (int c = 0; c < 3; ++c) { vec[r][c] = cz(0.0, 0.0); ef[r][c] = cz(0.0, 0.0); }
     }
+    // the vector potential of electrodes in a row of one length and direction D
+    // is summed as a multiple of D
+    double D[3] = {0.0, 0.0, 0.0};
+    double2 along[RMAX];
+#pragma unroll
+    for (int r = 0; r < RMAX; ++r) along[r] = cz(0.0, 0.0);
+    auto flush = [&]() {
+#pragma unroll
+        for (int r = 0; r < RMAX; ++r) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                vec[r][c].x = fma(along[r].x, D[c], vec[r][c].x);
+                vec[r][c].y = fma(along[r].y, D[c], vec[r][c].y);
+            }
+            along[r] = cz(0.0, 0.0);
+        }
+    };
     for (int e0 = e_begin; e0 < e_end; e0 += FS_E) {
         const int ne = min(FS_E, e_end - e0);
         __syncthreads();
@@ -500,6 +518,13 @@ __global__ void __launch_bounds__(FS_THREADS) k_fields_series(SerArgs sa, int r0
                 Bp = cscale(cmul(Bp, ex), q.iL);
             }
             if (q.bad) J1 = Ap = Bp = cz(nan(""), nan(""));
+            if ((a.want & WANT_VEC) && (__double_as_longlong(q.D[0]) != __double_as_longlong(D[0]) ||
+                                        __double_as_longlong(q.D[1]) != __double_as_longlong(D[1]) ||
+                                        __double_as_longlong(q.D[2]) != __double_as_longlong(D[2]))) {
+                flush();
+#pragma unroll
+                for (int c = 0; c < 3; ++c) D[c] = q.D[c];
+            }
             double2 F[3];                                   // the field of a unit current
             if (a.want & WANT_EF)
 #pragma unroll
@@ -519,18 +544,12 @@ __global__ void __launch_bounds__(FS_THREADS) k_fields_series(SerArgs sa, int r0
                 }
                 if (a.want & WANT_VEC) {
                     const double2 cl = a.cur_l[ci];
-                    if (cur_big(cl)) {
-                        const double2 cj = cmul(cl, J1);
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            vec[r][c].x = fma(cj.x, q.D[c], vec[r][c].x);
-                            vec[r][c].y = fma(cj.y, q.D[c], vec[r][c].y);
-                        }
-                    }
+                    if (cur_big(cl)) along[r] = cfma(cl, J1, along[r]);
                 }
             }
         }
     }
+    flush();
     // the electrode shares of a warp's lanes
     for (int o = G; o < 32; o <<= 1) {
 #pragma unroll
