@@ -354,3 +354,24 @@ def test_mixed_fill_touching_pairs_on_both_sides_of_their_series_limit(gpu_pkg, 
             for z, want in zip(got, gpu_fill(pkg, e, None, s, kappa[k])):
                 nz = spec & (np.abs(want) > 0)
                 assert elementwise(z[b][nz], want[nz]) < 1e-13
+
+
+@pytest.mark.parametrize("gap", [0.02, 0.1, 0.45, 0.55, 0.95, 1.05, 1.95, 2.05])
+@pytest.mark.parametrize("x", [0.05, 3.0, 12.0])
+def test_close_pairs_match_oracle(gpu_pkg, port, gap, x):
+    """Panels and orders on both sides of each ratio of distance to length, crossing and askew pairs of equal and unequal
+    lengths, within the series' reach and past it; oracle at 1e-10, entries at TOL."""
+    pkg = gpu_pkg
+    a = np.array([0.0, 0.0, -3.0])
+    for length, to in ((1.0, [0.0, 1.0, 0.0]), (0.4, [0.6, 0.0, 0.8]), (2.5, [0.8, 0.6, 0.0])):
+        c = a + [0.3, -0.2, gap]
+        e = np.stack([pkg.populate_electrode(a, a + [1.0, 0.0, 0.0], 5e-3),
+                      pkg.populate_electrode(c, c + length * np.array(to), 5e-3)])
+        gamma = x / (e[:, 9].max() * 17 / 16) * np.exp(0.25j * np.pi)
+        s, kappa = 1e5 + 1e6j, 0.01 + 1e-4j
+        got = [np.zeros(4, np.complex128) for _ in range(2)]
+        want = [np.zeros(4, np.complex128) for _ in range(2)]
+        assert pkg.calculate_impedances(*got, e, gamma, s, 1.0, kappa) == 0
+        assert port.calculate_impedances(*want, e, gamma, s, 1.0, kappa, req_abs=0.0, req_rel=1e-10) == 0
+        for g, w in zip(got, want):
+            assert elementwise(g, w) < TOL

@@ -432,10 +432,17 @@ struct SeriesView {
     double h, dmax;
 };
 
-__global__ void k_series_coef(const SampleCoef* __restrict__ coef, SeriesView v) {
+// The samples' constants: one row of CTAs the powers, a row per bucket the table.
+__global__ void k_series_tables(const SampleCoef* __restrict__ coef, SeriesView v) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= v.ns) return;
     const double2 g = coef[q].gamma;
+    if (blockIdx.y > 0) {
+        const int b = blockIdx.y - 1;
+        const double R = b * v.h;
+        v.tab[(long long)b * v.ns + q] = cexp_d(cz(-g.x * R, -g.y * R));
+        return;
+    }
     const double ga = sqrt(cabs2(g));
     const bool ok = ga * v.dmax <= SER_XMAX;
     v.ok[q] = ok;
@@ -449,14 +456,6 @@ __global__ void k_series_coef(const SampleCoef* __restrict__ coef, SeriesView v)
     }
 }
 
-__global__ void k_series_tab(const SampleCoef* __restrict__ coef, SeriesView v) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
-    if (q >= v.ns) return;
-    const double2 g = coef[q].gamma;
-    const double R = b * v.h;
-    v.tab[(long long)b * v.ns + q] = cexp_d(cz(-g.x * R, -g.y * R));
-}
-
 enum : int { SK_NONE = 0, SK_TENSOR = 1, SK_TOUCH = 2, SK_BAD = 3, SK_PAR = 4 };
 
 struct SeriesPk {
@@ -468,12 +467,28 @@ struct SeriesPk {
     int qm, npts;                // parallel: order on the middle piece (its panels are Ps); points in all
 };
 
+// Order of a panel pair `ratio` panel lengths apart, from 0.5 on: Gauss-Legendre
+// converges like rho^(-2q) with rho = 2 ratio + sqrt(4 ratio^2 + 1), so half a
+// length takes 20 points where two lengths take order_for's 8, but a quarter of the
+// panels: 90 points per squared distance instead of 256.
+TAGS_D int near_order(double ratio, double gl) {
+    if (ratio >= 2.0) return order_for(ratio, gl, true);
+    return min(QMAX, (ratio >= 1.0 ? 12 : 20) + (int)ceil(fmin(1.5 * gl, (double)QMAX)));
+}
+
+// Panels of a length at distance d: no longer than 2 d, nor, down to d / 2, than 8
+// / |gamma|, beyond which the order would run into QMAX.
+TAGS_D double near_panels(double len, double d, double ga) {
+    const double t = len / d;
+    return ceil(fmax(0.5 * t, fmin(2.0 * t, 0.125 * ga * len)));
+}
+
 // Parallel segments: the distance depends on u = t0 |dr| -+ t1 |ds| alone, and
 // the pairs of points at one u make up a trapezoid, rising over [0, s], level
 // over [s, l], falling over [l, s + l]. So the double integral is a single one
-// over three pieces, in panels no longer than half the distance, one order more
+// over three pieces, in panels no longer than twice the distance, one order more
 // than the tensor rule's for the weight's slope: 13 points instead of 25 for a
-// far pair of equal lengths, hundreds instead of tens of thousands for a wire
+// far pair of equal lengths, a hundred instead of tens of thousands for a wire
 // and its image. A level piece shorter than 1e-5 of the distance takes its
 // midpoint. Taken where the sender's deviation from the receiver's direction is
 // below 1e-15 of the distance (exactly zero along the axes) and no piece needs
@@ -492,7 +507,8 @@ TAGS_D void series_parallel(const Seg& S, const Seg& R, double d, double ga, Ser
     const double a2 = dot3(k.dr, k.dr);
     if (!(c2 <= 1e-30 * d * d * a2)) return;
     const double a = sqrt(a2), b = sqrt(dot3(k.ds, k.ds)), s = fmin(a, b), l = fmax(a, b);
-    const double p1 = ceil(2.0 * s / d), p2 = ceil(2.0 * (l - s) / d);
+    const bool far = 2.0 * l <= d;                          // one panel a piece
+    const double p1 = far ? 1.0 : near_panels(s, d, ga), p2 = far ? 1.0 : near_panels(l - s, d, ga);
     if (!(p1 <= 32.0 && p2 <= 32.0)) return;
     par /= a;
     k.h2 = 0.0;
@@ -505,9 +521,9 @@ TAGS_D void series_parallel(const Seg& S, const Seg& R, double d, double ga, Ser
     k.l = l;
     k.Pr = max(1, (int)p1);
     k.Ps = max(1, (int)p2);
-    const double lp = fmax(s / k.Pr, (l - s) / k.Ps);
+    const double lp = far ? fmax(s, l - s) : fmax(s / k.Pr, (l - s) / k.Ps);
     k.gl = ga * lp;
-    k.q = min(QMAX, order_for(d / lp, k.gl, true) + 1);
+    k.q = min(QMAX, near_order(d / lp, k.gl) + 1);
     k.qm = l == s ? 0 : l - s <= 1e-5 * d && ga * (l - s) <= 1e-6 ? 1 : k.q;
     k.npts = 2 * k.Pr * k.q + k.Ps * k.qm;
     k.kind = SK_PAR;
@@ -546,14 +562,18 @@ TAGS_D void series_classify(const Seg& S, const Seg& R, bool direct, double ga, 
     } else {
         const double dmin = seg_seg_dist(R.a, R.b, S.a, S.b);
         k.kind = dmin <= 1e-12 * lmax ? SK_BAD : SK_TENSOR;
-        // panels no longer than half the distance, each segment by its own
-        // length (the direct rule of k_fill_fp64 splits both by the longer)
+        // panels no longer than twice the distance, each segment by its own
+        // length (the direct rule of k_fill_fp64: half of it, by the longer)
         const double d = fmax(dmin, 1e-12 * lmax);
-        k.Pr = (int)fmin(32.0, fmax(1.0, ceil(2.0 * R.len / d)));
-        k.Ps = (int)fmin(32.0, fmax(1.0, ceil(2.0 * S.len / d)));
-        const double lp = fmax(R.len / k.Pr, S.len / k.Ps);
+        double lp = lmax;
+        k.Pr = k.Ps = 1;
+        if (!(2.0 * lmax <= d)) {
+            k.Pr = (int)fmin(32.0, fmax(1.0, near_panels(R.len, d, ga)));
+            k.Ps = (int)fmin(32.0, fmax(1.0, near_panels(S.len, d, ga)));
+            lp = fmax(R.len / k.Pr, S.len / k.Ps);
+        }
         k.gl = ga * lp;
-        k.q = order_for(dmin / lp, k.gl, true);
+        k.q = near_order(dmin / lp, k.gl);
         k.npts = k.Pr * k.Ps * k.q * k.q;
         if (k.kind == SK_TENSOR) series_parallel(S, R, d, ga, k);
     }
@@ -580,11 +600,14 @@ TAGS_D void group_transpose_sum(double (&acc)[NT], int g) {
 
 // The rule of one untouched record by nl lanes: f(r, weight / r) per point.
 // Parallel segments: the points of the rising and falling pieces, then the
-// level one's. Others: the tensor rule; the lanes share the points, or, a whole
-// warp with 32 panel pairs and more, the panel pairs, each at the order its own
-// distance needs (order_for's rule; only the closest need k.q), which is where
-// nearly all points of a finely split pair lie. The distance by rsqrt, 1 ulp,
-// which saves a root or a division of the point's ~20 instructions.
+// level one's. Others: the tensor rule, panel pair by panel pair, the lanes over
+// the points of each at the order its own distance needs (near_order's; the order
+// is chosen in FP32). The distance by rsqrt, 1 ulp, which saves a root or a
+// division of the point's ~20 instructions. With panels of half the closest distance
+// (order_for alone) 12 segments of 11 m past the reach took 5.85 ms against 2.48,
+// path voltages of 24 long segments 2.43 against 1.72, the drop-in chain at m = 100
+// 1.36 against 1.31; entries agree to 1e-15 down to distances of 1/16 of the length,
+// where 32 of the short panels end.
 template <class F>
 TAGS_D void rule_points(const SeriesPk& k, int lane, int nl, F f) {
     auto at = [&](double d2, double w) {
@@ -613,32 +636,29 @@ TAGS_D void rule_points(const SeriesPk& k, int lane, int nl, F f) {
         }
         at(d2, w * (hr * hs));
     };
-    if (nl == 32 && k.Pr * k.Ps >= 32) {
-        const double lr = sqrt(dot3(k.dr, k.dr)) * hr, ls = sqrt(dot3(k.ds, k.ds)) * hs, lp = fmax(lr, ls);
-        for (int pp = lane; pp < k.Pr * k.Ps; pp += 32) {
-            const int pi = pp / k.Ps, pj = pp - pi * k.Ps;
-            const double m0 = (pi + 0.5) * hr, m1 = (pj + 0.5) * hs;
-            double d2 = 0.0;
+    const int np = k.Pr * k.Ps;
+    for (int pp = 0; pp < np; ++pp) {
+        const int pi = pp / k.Ps, pj = pp - pi * k.Ps;
+        int q = k.q;
+        if (np > 1) {
+            const float h0 = 1.f / k.Pr, h1 = 1.f / k.Ps, m0 = (pi + 0.5f) * h0, m1 = (pj + 0.5f) * h1;
+            float d2 = 0.f, r2 = 0.f, s2 = 0.f;
             for (int c = 0; c < 3; ++c) {
-                const double d = k.o[c] + m0 * k.dr[c] - m1 * k.ds[c];
+                const float r = (float)k.dr[c], t = (float)k.ds[c], d = (float)k.o[c] + m0 * r - m1 * t;
                 d2 += d * d;
+                r2 += r * r;
+                s2 += t * t;
             }
-            const double ratio = (sqrt(d2) - 0.5 * (lr + ls)) / lp;     // at least that far apart
-            const int q = ratio >= 2.0 ? min(k.q, order_for(ratio, k.gl, true)) : k.q;
-            const double* x = g_glx + gl_off(q);
-            const double* w = g_glw + gl_off(q);
-            for (int qi = 0; qi < q; ++qi)
-                for (int qj = 0; qj < q; ++qj) point((pi + x[qi]) * hr, (pj + x[qj]) * hs, w[qi] * w[qj]);
+            const float lr = sqrtf(r2) * h0, ls = sqrtf(s2) * h1, lp = fmaxf(lr, ls);
+            const float ratio = 0.999f * (sqrtf(d2) - 0.5f * (lr + ls)) / lp;     // at least that far apart
+            if (ratio >= 1.f) q = min(q, near_order((double)ratio, k.gl));
         }
-        return;
-    }
-    const double* x = g_glx + gl_off(k.q);
-    const double* w = g_glw + gl_off(k.q);
-    const int qq = k.q * k.q, npts = k.Pr * k.Ps * qq;
-    for (int t = lane; t < npts; t += nl) {
-        const int pp = t / qq, u = t - pp * qq;
-        const int pi = pp / k.Ps, pj = pp - pi * k.Ps, qi = u / k.q, qj = u - qi * k.q;
-        point((pi + x[qi]) * hr, (pj + x[qj]) * hs, w[qi] * w[qj]);
+        const double* x = g_glx + gl_off(q);
+        const double* w = g_glw + gl_off(q);
+        for (int u = lane; u < q * q; u += nl) {
+            const int qi = u / q, qj = u - qi * q;
+            point((pi + x[qi]) * hr, (pj + x[qj]) * hs, w[qi] * w[qj]);
+        }
     }
 }
 
@@ -2453,9 +2473,8 @@ static SeriesView series_view(const SeriesGeo& g, void* ws, int ns) {
 
 static int series_tables(const SampleCoef* d_coef, const SeriesView& v, cudaStream_t st) {
     TAGS_CUDA_OK(cudaMemsetAsync(v.gmax, 0, 2 * sizeof(unsigned long long), st));     // and nfar
-    k_series_coef<<<(v.ns + 127) / 128, 128, 0, st>>>(d_coef, v);
-    k_series_tab<<<dim3((v.ns + 31) / 32, v.nbk), 32, 0, st>>>(d_coef, v);
-    tags_note_launch(2);
+    k_series_tables<<<dim3((v.ns + 31) / 32, v.nbk + 1), 32, 0, st>>>(d_coef, v);
+    tags_note_launch();
     TAGS_CUDA_OK(cudaGetLastError());
     return 0;
 }
