@@ -282,9 +282,10 @@ def run_reference(args):
 # starting 6 m outside the grid, four injections), here 251 points 0.3 m apart
 # across the benchmark grid at ground level; every Laplace sample of the set.
 FIELD_POINTS, FIELD_RHS, FIELD_STEP = 251, 4, 0.3
-# FP64 pipe operations one rule-node evaluation executes in k_fields
-# (potential, vector potential and field for four injections): (DFMA x 2 + DADD
-# + DMUL) per evaluation, from an ncu count of the kernel (see profiles/).
+# FP64 pipe operations one rule-node evaluation executes in k_fields, which
+# serves the samples past the moment series' reach (potential, vector potential
+# and field for four injections): (DFMA x 2 + DADD + DMUL) per evaluation, from an
+# ncu count of the kernel (see profiles/).
 FIELD_FP64_FLOPS_PER_EVAL = 196.9
 
 
@@ -391,13 +392,12 @@ def run_fields(args):
     roof = {"bound": "fp64", "kernel": "fields", "launches": f["launches"], "avg_launch_ms": f["ms"] / f["launches"],
             "evaluations_per_launch": evals / f["launches"], "evaluations_per_s": evals / dev_s,
             "unit": "TFLOP/s", "peak": fp64["peak"], "traffic": None}
-    if FIELD_FP64_FLOPS_PER_EVAL:
-        ach = evals * FIELD_FP64_FLOPS_PER_EVAL / dev_s / 1e12
-        roof.update({"achieved": ach, "frac": ach / fp64["peak"],
-                     "note": "executed FP64 flops (ncu count per rule-node evaluation x evaluations counted on "
-                             "the device) over the measured DFMA throughput of this pool's GB300"})
-    else:
-        roof.update({"achieved": None, "frac": None, "note": "FP64 operations per evaluation not yet counted"})
+    ach = (f["flops"] + evals * FIELD_FP64_FLOPS_PER_EVAL) / dev_s / 1e12
+    roof.update({"achieved": ach, "frac": ach / fp64["peak"],
+                 "note": "FP64 flops of the moment series' sums (2 x (6 terms + 24 + 20 per injection) per point, "
+                         "electrode and sample; the moments themselves left out), plus the samples past its reach (ncu "
+                         "count per rule-node evaluation x evaluations counted on the device), over the DFMA "
+                         "throughput measured in this run"})
     B_h2d = sum(2 * nb * FIELD_RHS * m * 16 + 2 * nb * 16 for _, nb, _, _ in steps) / len(steps)
     B_d2h = sum(7 * nb * FIELD_POINTS * FIELD_RHS * 16 for _, nb, _, _ in steps) / len(steps)
     line = {"metric": "field point-samples/s (1560-segment grid, 251-point line, 4 injections, 2048 samples)",
@@ -750,11 +750,11 @@ GPR_FIXTURE = os.path.join(ROOT, "tests", "golden", "gpr4.npz")
 
 
 def plain_fp64_record(pkg, elec, img, nodes, s_d, k_d, ie_d, centre, local, flush, steps=3, batch=8):
-    """The plain FP64 form (FP64 fill, LU with partial pivoting) timed the way
-    the mixed form is: device time from the plan's CUDA events, inputs in
-    HBM, L2 flushed between steps; `steps` steps of `batch` samples spread
-    over the band after one warm-up step (its cost does not depend on the
-    sample: no refinement)."""
+    """The plain FP64 form (FP64 fill, LDL^T in the static order, refinement)
+    timed the way the mixed form is: device time from the plan's CUDA events,
+    inputs in HBM, L2 flushed between steps; `steps` steps of `batch` samples
+    spread over the band after one warm-up step (its cost hardly depends on the
+    sample: one or two refinement steps)."""
     import torch
     n = nodes.shape[0]
     N = n + 2 * elec.shape[0]
@@ -794,9 +794,10 @@ def plain_fp64_record(pkg, elec, img, nodes, s_d, k_d, ie_d, centre, local, flus
     return {"value": steps * batch / dt, "unit": "solves/s", "steps": steps, "samples_per_step": batch,
             "ms_per_step": 1e3 * dt / steps, "step_ms": step_ms, "clocks": clk.summary(),
             "roofline": roof, "kernel_families": fams, "fp64_peak": fp64,
-            "note": "plain FP64 form of this library on the same workload: FP64 fill, FP64 LU with partial "
-                    "pivoting, device time from the plan's events, L2 flushed between steps; roofline and "
-                    "kernel_families from one more step launched kernel by kernel"}
+            "note": "plain FP64 form of this library on the same workload: FP64 fill, FP64 LDL^T with refinement, "
+                    "device time from the plan's events, L2 flushed between steps; roofline (lu_fp64_gemm: the trailing "
+                    "updates' complex flops, 8 per multiply-add, which three real products instead of four execute, so "
+                    "the fraction may pass 1) and kernel_families from one more step launched kernel by kernel"}
 
 
 def gpr_accuracy(pkg, plan, s_d, k_d, ie_d, centre, n, SB, sol_d, info_d, s, tmax, nt):

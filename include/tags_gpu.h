@@ -95,8 +95,9 @@ int fill_incidence_imm (tags_cdouble *wg, const Electrode *electrodes, size_t nu
 int fill_impedance_imm (tags_cdouble *wg, const tags_cdouble *zl, const tags_cdouble *zt,
                         size_t num_electrodes, size_t num_nodes);
 
-/* Solves W_G x = ie (W_G symmetric, lower half read); ie <- [U; I_L; I_T].
- * Returns 0, or k > 0 when the k-th pivot of the factorisation is exactly
+/* Solves W_G x = ie (W_G symmetric, lower half read); ie <- [U; I_L; I_T]. By
+ * an LDL^T in the order ZL, ZT, nodes with FP64 refinement, or, where that does
+ * not settle, by LU with partial pivoting. Returns 0, or k > 0 when the k-th pivot of the factorisation is exactly
  * zero (singular system). wg is left unchanged (the reference leaves its
  * factorisation there; its content is not part of the contract). */
 int solve_immittance (tags_cdouble *wg, tags_cdouble *ie, size_t num_electrodes, size_t num_nodes);
@@ -240,15 +241,16 @@ int tags_voltage_batch (const double *paths, size_t num_paths, const Electrode *
                         tags_cdouble *v);
 
 /* Node evaluations (rule node x sample) made by the field kernels on the
- * current device since the last reset: the unit of work of the post-processing
- * rules, for throughput reports. reset != 0 zeroes the counter after reading. */
+ * current device since the last reset: the unit of work of the rule that serves
+ * samples past the moment series' reach, for throughput reports (the series'
+ * operations are in the profile's `fields` family). reset != 0 zeroes the counter after reading. */
 int tags_fields_evaluations (unsigned long long *count, int reset);
 
 /* ---- Part 2: batched extension -------------------------------------------- */
 
 enum {
-    TAGS_PLAIN_FP64 = 0,  /* FP64 fill, FP64 LU with partial pivoting */
-    TAGS_MIXED = 1        /* FP32/FP64 fill, low-precision LU + FP64 refinement */
+    TAGS_PLAIN_FP64 = 0,  /* FP64 fill, FP64 LDL^T + refinement, pivoted LU where that does not settle */
+    TAGS_MIXED = 1        /* FP32/FP64 fill, low-precision LDL^T + FP64 refinement */
 };
 
 /* Error codes (negative) of the extension and of argument checks. */
@@ -488,7 +490,7 @@ int tags_debug_solve_path (int path);
 /* No counterpart in the reference. Caps the refinement steps of the mixed
  * form's passes (1 .. 40; 0 restores the default 40). A sample that has not
  * met its stopping rule after that many steps is re-solved by the plain FP64
- * path (partial pivoting), as one whose refinement stops converging; the
+ * path, as one whose refinement stops converging; the
  * run's stats count it in `fallbacks`. A cap of 1 sends every sample there
  * (the first correction is the whole solution), which tests that path. */
 int tags_plan_set_max_steps (tags_plan plan, int steps);

@@ -16,7 +16,9 @@
 // width in v, split further wherever |gamma| grows r by more than 1.5 across a
 // panel, integrate what is left with 8 nodes per panel; against 1e-14 adaptive
 // integrals over random geometries, frequencies and distances (1e-4 L to 5 L)
-// the rule stays within 1e-12 relative.
+// the rule stays within 1e-12 relative. Samples with |gamma| up to 2 / (L + 1/8 m) or
+// so share the rule's moments and cost a series each (k_fields_series); the
+// rule with an exponential per node (k_fields) serves the ones beyond.
 //
 // Path voltage. The reference integrates E . (p2 - p1) / |p2 - p1| over t in
 // [0, 1] with a cubature whose integrand is itself a field cubature per
@@ -850,7 +852,7 @@ void series_chunks(SerArgs* s, size_t part_cap) {
 
 // `direct`: samples past the series' reach are among these; `most`: the
 // series' largest number of terms (0: none of these samples takes it).
-int launch_fields(const SerArgs& sa, int most, bool direct, cudaStream_t st) {
+int launch_fields(const SerArgs& sa, int most, double madds, bool direct, cudaStream_t st) {
     const FieldArgs& base = sa.f;
     const int ngroups = (base.S + base.G - 1) / base.G;
     const long long items = (long long)base.P * ngroups * base.nchunk;
@@ -876,7 +878,8 @@ int launch_fields(const SerArgs& sa, int most, bool direct, cudaStream_t st) {
     }
     const long long n = (long long)base.S * base.P * base.R;
     k_fields_reduce<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(base);
-    tags_prof_end(TAGS_PROF_FIELDS, pf, st, 0.0, 0.0);
+    // the series' multiply-adds (k_fields counts its rule's evaluations itself)
+    tags_prof_end(TAGS_PROF_FIELDS, pf, st, 2.0 * madds * base.P * base.m, 0.0);
     tags_note_launch();
     TAGS_CUDA_OK(cudaGetLastError());
     return 0;
@@ -999,7 +1002,13 @@ int fields_run(const FieldsIn& in) {
         a.part = d_out + 7 * P * R * ns;
         a.nt = d_nt;
         a.spart = a.part + 7 * P * R * ns * (any_direct ? (size_t)nchunk : 0);
-        if (int e = launch_fields(sa, most, any_direct, st)) return e;
+        double madds = 0.0;                                  // per (point, electrode), as the series kernel's comment counts
+        const bool wv = (in.want & (WANT_VEC | WANT_EF)) != 0;
+        for (size_t k = s0; k < s0 + ns; ++k)
+            if (nt[k] > 0)
+                madds += (wv ? 6.0 : 2.0) * nt[k] + (wv ? 24.0 : 4.0) +
+                         (double)R * ((in.want & WANT_EF ? 12 : 0) + (in.want & WANT_VEC ? 4 : 0) + 4);
+        if (int e = launch_fields(sa, most, madds, any_direct, st)) return e;
         if (in.pot && (in.want & WANT_POT))
             TAGS_CUDA_OK(cudaMemcpyAsync(in.pot + s0 * P * R, a.pot, sizeof(double2) * P * R * ns,
                                          cudaMemcpyDeviceToHost, st));

@@ -1,18 +1,16 @@
-// Batched dense complex LU factorisation and triangular solves (CUDA cores).
+// Batched dense complex FP64 LU factorisation and triangular solves (CUDA cores).
 //
 // Replaces the reference's dense solve of the immittance system,
-// solve_immittance -> zsysv('L') (src/linalg.c:112-139). The plain FP64 form
-// uses LU with partial pivoting on the symmetrised W_G (row interchanges as in
-// LAPACK's getrf: pivot = first index of max |Re|+|Im|). The same kernels,
-// instantiated for complex FP32 and without pivoting, serve the mixed form's
-// statically ordered factorisation. Right-looking blocked algorithm with a
-// panel width NB: panel factorisation, row interchanges, triangular solve of
+// solve_immittance -> zsysv('L') (src/linalg.c:112-139), by LU with partial
+// pivoting on the symmetrised W_G (row interchanges as in LAPACK's getrf: pivot =
+// first index of max |Re|+|Im|): the allocation-free solve, and the systems that
+// the FP64 LDL^T in the static order (ldl64.cu) hands over because its check asks
+// for a pivot search. Right-looking blocked algorithm with a panel width NB: panel factorisation, row interchanges, triangular solve of
 // the block row, trailing update C -= L21 * U12.
 //
 // Layout: column-major, leading dimension ld, one matrix per blockIdx.z
 // (pointer + z * stride). ipiv is 0-based global row indices.
 #include <mutex>
-#include <type_traits>
 
 #include "tags_common.cuh"
 #include "tags_internal.h"
@@ -32,22 +30,8 @@ template <> struct Cx<double2> {
     static TAGS_D double2 inv(double2 a) { return cdiv(make_double2(1.0, 0.0), a); }
     static TAGS_D bool is_zero(double2 a) { return a.x == 0.0 && a.y == 0.0; }
 };
-template <> struct Cx<float2> {
-    using R = float;
-    static TAGS_D float2 zero() { return make_float2(0.f, 0.f); }
-    static TAGS_D float2 mul(float2 a, float2 b) { return fmulc(a, b); }
-    static TAGS_D float2 fma(float2 a, float2 b, float2 c) { return ffmac(a, b, c); }
-    static TAGS_D float2 sub(float2 a, float2 b) { return fsub(a, b); }
-    static TAGS_D float abs1(float2 a) { return fabsf(a.x) + fabsf(a.y); }
-    static TAGS_D float2 inv(float2 a) {
-        double2 r = cdiv(make_double2(1.0, 0.0), make_double2(a.x, a.y));
-        return make_float2((float)r.x, (float)r.y);
-    }
-    static TAGS_D bool is_zero(float2 a) { return a.x == 0.f && a.y == 0.f; }
-};
 // negation for the subtraction in the trailing update
 TAGS_D double2 negc(double2 a) { return make_double2(-a.x, -a.y); }
-TAGS_D float2 negc(float2 a) { return make_float2(-a.x, -a.y); }
 
 constexpr int PANEL_THREADS = 512;
 
@@ -332,11 +316,9 @@ int tags_lu_prepare() {
     static std::once_flag once;
     static int rc = 0;
     std::call_once(once, [] {
-        const int g64 = (int)(2 * NB * 64 * sizeof(double2)), g32 = (int)(2 * NB * 64 * sizeof(float2));
+        const int g64 = (int)(2 * NB * 64 * sizeof(double2));
         if (cudaFuncSetAttribute(k_gemm_update<double2, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, g64) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(k_gemm_update<float2, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, g32) !=
-                cudaSuccess)
+            cudaSuccess)
             rc = tags_fail(TAGS_E_CUDA, "cudaFuncSetAttribute(k_gemm_update) failed");
     });
     return rc;
@@ -366,7 +348,7 @@ int lu_impl(T* A, int n, long long ld, long long stride, int batch, int pivot, i
             k_trsm_row<T, NB><<<dim3((rest + 31) / 32, 1, batch), 256, 0, st>>>(A, n, ld, stride, j0, jb);
             tags_note_launch();
             dim3 g((rest + 63) / 64, (rest + 63) / 64, batch);
-            int pf = std::is_same<T, double2>::value ? tags_prof_begin(TAGS_PROF_LU64_GEMM, st) : -1;
+            int pf = tags_prof_begin(TAGS_PROF_LU64_GEMM, st);
             k_gemm_update<T, NB><<<g, 256, gsmem, st>>>(A, n, ld, stride, j0, jb);
             // rank-jb update of a rest x rest block: 8 rest^2 jb real flops
             tags_prof_end(TAGS_PROF_LU64_GEMM, pf, st, 8.0 * rest * (double)rest * jb * batch,
@@ -417,15 +399,7 @@ int tags_lu_z(double2* A, int n, long long ld, long long stride, int batch, int 
               cudaStream_t st) {
     return lu_impl<double2>(A, n, ld, stride, batch, pivot, ipiv, info, st);
 }
-int tags_lu_c(float2* A, int n, long long ld, long long stride, int batch, int pivot, int* ipiv, int* info,
-              cudaStream_t st) {
-    return lu_impl<float2>(A, n, ld, stride, batch, pivot, ipiv, info, st);
-}
 int tags_lu_solve_z(const double2* A, int n, long long ld, long long stride, int batch, const int* ipiv, double2* X,
                     int nrhs, long long ldx, long long xstride, cudaStream_t st) {
     return lu_solve_impl<double2>(A, n, ld, stride, batch, ipiv, X, nrhs, ldx, xstride, st);
-}
-int tags_lu_solve_c(const float2* A, int n, long long ld, long long stride, int batch, const int* ipiv, float2* X,
-                    int nrhs, long long ldx, long long xstride, cudaStream_t st) {
-    return lu_solve_impl<float2>(A, n, ld, stride, batch, ipiv, X, nrhs, ldx, xstride, st);
 }

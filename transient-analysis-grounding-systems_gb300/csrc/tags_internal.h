@@ -151,11 +151,7 @@ int tags_symmetrize_lower(double2* d_W, int N, long long ld, long long stride, i
 // lu.cu
 int tags_lu_z(double2* A, int n, long long ld, long long stride, int batch, int pivot, int* ipiv, int* info,
               cudaStream_t st);
-int tags_lu_c(float2* A, int n, long long ld, long long stride, int batch, int pivot, int* ipiv, int* info,
-              cudaStream_t st);
 int tags_lu_solve_z(const double2* A, int n, long long ld, long long stride, int batch, const int* ipiv, double2* X,
-                    int nrhs, long long ldx, long long xstride, cudaStream_t st);
-int tags_lu_solve_c(const float2* A, int n, long long ld, long long stride, int batch, const int* ipiv, float2* X,
                     int nrhs, long long ldx, long long xstride, cudaStream_t st);
 
 // inlt.cu
