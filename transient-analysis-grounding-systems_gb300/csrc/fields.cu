@@ -359,12 +359,14 @@ struct SerPair {
     int b, bad;
 };
 
-// Moments of one (point, electrode) pair by one thread: Gauss-Legendre in t
-// where the point is at least two lengths away (6 to 12 nodes by the distance),
-// else the sinh rule above in panels of at most 0.75.
+// Moments of one (point, electrode) pair by L lanes (g: this one), all of the
+// warp's groups together, `on` or not: Gauss-Legendre in t where the point is at
+// least two lengths away (6 to 12 nodes by the distance), else the sinh rule above
+// in panels of at most 0.75, up to ~1000 nodes, which one lane would take in a row.
 template <int NT>
 TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, double h, int nbk, const double* gx,
-                         const double* gw, SerPair& q, double* mom) {
+                         const double* gw, bool on, int g, int L, SerPair& out, double* mom) {
+    SerPair q;
     const double D[3] = {S.b[0] - S.a[0], S.b[1] - S.a[1], S.b[2] - S.a[2]};
     const double L2 = D[0] * D[0] + D[1] * D[1] + D[2] * D[2], Lg = sqrt(L2);
     const double w0[3] = {P0 - S.a[0], P1 - S.a[1], P2 - S.a[2]};
@@ -404,7 +406,7 @@ TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, double h
         const double ratio = dist * q.iL;
         const int o = ratio >= 16.0 ? 0 : ratio >= 8.0 ? 1 : ratio >= 4.0 ? 3 : 4;
         const int nq = o == 0 ? 6 : o == 1 ? 7 : o == 3 ? 9 : 12, off = o == 0 ? 0 : o == 1 ? 6 : o == 3 ? 21 : 30;
-        for (int i = 0; i < nq; ++i) {
+        for (int i = g; i < nq; i += L) {
             const double s = (gx[off + i] - u0) * Lg;
             node(s, fma(s, s, d2), gw[off + i]);
         }
@@ -417,13 +419,22 @@ TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, double h
             const double lo = split && side == 1 ? 0.0 : va, hi = split && side == 0 ? 0.0 : vb;
             const int np = max(1, (int)ceil(fmin((hi - lo) / 0.75, 64.0)));
             const double ph = (hi - lo) / np;
-            for (int p = 0; p < np; ++p)
-                for (int i = 0; i < 8; ++i) {
-                    const double v = lo + (p + gx[13 + i]) * ph, s = dp * sinh(v);
-                    node(s, fma(s, s, d2), gw[13 + i] * ph * (dp * q.iL) * cosh(v));
-                }
+            for (int t = g; t < 8 * np; t += L) {
+                const int p = t >> 3, i = t & 7;
+                const double v = lo + (p + gx[13 + i]) * ph, s = dp * sinh(v);
+                node(s, fma(s, s, d2), gw[13 + i] * ph * (dp * q.iL) * cosh(v));
+            }
         }
     }
+    for (int o = L >> 1; o > 0; o >>= 1)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            aN[n] += __shfl_xor_sync(0xffffffffu, aN[n], o);
+            aA[n] += __shfl_xor_sync(0xffffffffu, aA[n], o);
+            aB[n] += __shfl_xor_sync(0xffffffffu, aB[n], o);
+        }
+    if (!on || g != 0) return;
+    out = q;
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
         mom[n] = aN[n];
@@ -433,7 +444,8 @@ TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, double h
 }
 
 // A CTA per (point, electrode chunk, four sample groups at most): FS_E electrodes
-// at a time, a thread forms a pair's moments, then the warps (sample group x
+// at a time, a thread (or, with fewer electrodes, up to 32 lanes) forms a pair's
+// moments, then the warps (sample group x
 // share of the electrodes; lanes: G samples x 32 / G electrodes) sum the series
 // and accumulate the currents' terms. FP64-bound: 6 nt + 24 multiply-adds per
 // (pair, sample) and 20 per injection. The 1560-segment grid, 251 points, 64
@@ -492,10 +504,13 @@ __global__ void __launch_bounds__(FS_THREADS) k_fields_series(SerArgs sa, int r0
     for (int e0 = e_begin; e0 < e_end; e0 += FS_E) {
         const int ne = min(FS_E, e_end - e0);
         __syncthreads();
-        if (tid < ne) {
-            fser_moments<NT>(a.elec[e0 + tid], P0, P1, P2, sa.h, sa.nbk, gx, gw, pr[tid], mom + (size_t)tid * 3 * NT);
-            if (pr[tid].bad) raise_status(a.status, TAGS_ST_DEGENERATE_PAIR);
-        }
+        int L = 1;                                          // lanes per pair: a short tile shares out its nodes
+        while (2 * L * ne <= FS_THREADS && L < 32) L *= 2;
+        const int me = min(tid / L, ne - 1);
+        const bool on = tid < L * ne;
+        fser_moments<NT>(a.elec[e0 + me], P0, P1, P2, sa.h, sa.nbk, gx, gw, on, tid % L, L, pr[me],
+                         mom + (size_t)me * 3 * NT);
+        if (on && tid % L == 0 && pr[me].bad) raise_status(a.status, TAGS_ST_DEGENERATE_PAIR);
         __syncthreads();
         if (!valid) continue;
         for (int el = share * NS + sub; el < ne; el += nshare * NS) {
@@ -835,8 +850,8 @@ int series_terms(const SerGeo& g, zd gamma) {
     return std::min(n + 1, FS_NT);
 }
 
-// Electrode chunks of the series: CTAs for four per SM, at least 32
-// electrodes each, partial sums of at most part_cap bytes.
+// Electrode chunks of the series: CTAs for four per SM, at least 4 electrodes
+// each (a warp's lanes per pair then), partial sums of at most part_cap bytes.
 void series_chunks(SerArgs* s, size_t part_cap) {
     FieldArgs& a = s->f;
     const int ngroups = (a.S + a.G - 1) / a.G;
@@ -845,7 +860,7 @@ void series_chunks(SerArgs* s, size_t part_cap) {
     const size_t per = 7 * sizeof(double2) * a.P * a.R * (size_t)a.S * (4 / s->ngc);
     long long c = (152 * 4 + ctas - 1) / ctas;
     c = std::min<long long>(c, std::max<long long>(1, (long long)(part_cap / std::max<size_t>(per, 1))));
-    c = std::min<long long>(c, (a.m + 31) / 32);
+    c = std::min<long long>(c, (a.m + 3) / 4);
     s->echunk = (int)((a.m + c - 1) / c);
     a.schunk = (int)((a.m + s->echunk - 1) / s->echunk) * (4 / s->ngc);
 }
@@ -918,6 +933,14 @@ int fields_run(const FieldsIn& in) {
         nt[k] = series_terms(geo, zd(in.gamma[k].re, in.gamma[k].im));
         any_direct = any_direct || nt[k] == 0;
         any_series = any_series || nt[k] > 0;
+    }
+    // samples on both sides of the series' reach take both kernels one after the
+    // other; a call so small that either is bound by its own latency gives all
+    // samples to the rule (16 electrodes, 24 points, 3 samples: 0.69 ms by both,
+    // 0.61 by the rule; 90 electrodes, 76 points, 23 samples: 0.45 and 1.21)
+    if (any_direct && any_series && P * m * S <= 20000) {
+        std::fill(nt.begin(), nt.end(), 0);
+        any_series = false;
     }
     const int nchunk = any_direct ? field_chunks(P, cs, R, m, (size_t)1e9) : 1;
     auto series_args = [&](size_t ns) {
