@@ -107,7 +107,7 @@ int sym_solve(const tags_cdouble* z, const tags_cdouble* rhs, size_t m, size_t n
 // without pivoting (ldl64.cu), both blocks side by side; *done = 0 where its
 // check asks for the pivoted LU (nothing of the caller's is written then). One
 // pass of FP64 tiles instead of a CTA per 32 x 32 step for all right-hand
-// sides: 46.8 -> 2.3 ms for the examples' loop body at m = 220, n = 121 (FP64,
+// sides: 46.8 -> 2.1 ms for the examples' loop body at m = 220, n = 121 (FP64,
 // one refinement of every column; errors against 128-bit solves 2-4e-16, as the LU).
 int yla_ytb_ldl(tags_cdouble* yla, tags_cdouble* ytb, tags_cdouble* zl, tags_cdouble* zt, const tags_cdouble* a,
                 const tags_cdouble* b, size_t m, size_t n, cudaStream_t st, int* done) {

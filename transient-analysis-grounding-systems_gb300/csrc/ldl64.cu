@@ -14,8 +14,8 @@
 // is recovered by FP64 refinement against the untouched impedance blocks; a
 // sample whose corrections do not shrink to 1e-8 |x| (the next one would be
 // below FP64 rounding) is handed to the pivoted LU (lu.cu) by its caller.
-// Measured against that LU on GB300: 2 samples at m = 1560 714 -> 149 ms, 256
-// samples at m = 100 24.3 -> 6.7 ms, 100 samples at m = 10 0.66 -> 0.29 ms.
+// Measured against that LU on GB300: 2 samples at m = 1560 714 -> 120 ms, 256
+// samples at m = 100 24.3 -> 5.9 ms, 100 samples at m = 10 0.66 -> 0.25 ms.
 //
 // Layout: column-major N x N per sample, leading dimension ld. Lower triangle:
 // the matrix, then L; the strict upper triangle keeps U = D L^T of the panels
