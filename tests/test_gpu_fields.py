@@ -194,3 +194,10 @@ def test_field_series_and_its_limits_match_oracle(gpu_pkg, port, x, ns, nrhs, m,
                 # smallest normal number carries fewer than 53 bits on either side
                 for got, want in ((out["pot"][k, p, r], u), (out["vecpot"][k, p, r], va), (out["efield"][k, p, r], ve)):
                     assert np.max(np.abs(got - want)) <= TOL * np.max(np.abs(want)) + np.finfo(float).tiny
+
+
+@pytest.mark.parametrize("m,P,ns", [(1, 1, 1), (5, 1, 2), (63, 1, 1), (64, 1, 3), (130, 2, 40)])
+def test_field_of_few_points_and_many_electrodes_matches_oracle(gpu_pkg, port, m, P, ns):
+    """Lanes per pair from 32 down to 1, chunks summed by a thread or a warp; oracle at 1e-11, TOL of the largest
+    magnitude."""
+    test_field_series_and_its_limits_match_oracle(gpu_pkg, port, 0.05, ns, 2, m, P)

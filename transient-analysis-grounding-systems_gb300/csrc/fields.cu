@@ -597,10 +597,15 @@ __global__ void __launch_bounds__(FS_THREADS) k_fields_series(SerArgs sa, int r0
 
 // Sum of the electrode chunks and the scale factors: 1 / (4 pi kappa) for the
 // potential and field, mur mu0 / (4 pi) for the vector potential.
+// A thread per output, or a warp (lanes over the chunks) where few outputs have
+// many chunks each, which one thread would read one after the other (900
+// electrodes, 1 point, 2 samples: 0.75 -> 0.22 ms for the whole call).
+template <int W>
 __global__ void k_fields_reduce(FieldArgs a) {
     const long long n = (long long)a.S * a.P * a.R;
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, i = t / W;
+    const int lane = (int)(t % W);
+    if (i >= n) return;                                     // W = 32: the whole warp
     const int smp = (int)(i / ((long long)a.P * a.R));
     double2 v[7];
 #pragma unroll
@@ -608,10 +613,16 @@ __global__ void k_fields_reduce(FieldArgs a) {
     const bool ser = a.nt[smp] > 0;
     const double2* part = ser ? a.spart : a.part;
     const int nchunk = ser ? a.schunk : a.nchunk;
-    for (int ch = 0; ch < nchunk; ++ch) {
+    for (int ch = lane; ch < nchunk; ch += W) {
         const double2* q = part + ((long long)ch * n + i) * 7;
 #pragma unroll
         for (int c = 0; c < 7; ++c) v[c] = cadd(v[c], q[c]);
+    }
+    if (W > 1) {
+        for (int o = W / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int c = 0; c < 7; ++c) v[c] = cadd(v[c], shfl_xor2(v[c], o));
+        if (lane != 0) return;
     }
     const double2 i4pk = cdiv(cz(1.0, 0.0), cscale(a.kappa[smp], TAGS_FOUR_PI));
     const double u4pi = a.mur * TAGS_MU0 / TAGS_FOUR_PI;
@@ -892,7 +903,11 @@ int launch_fields(const SerArgs& sa, int most, double madds, bool direct, cudaSt
         TAGS_CUDA_OK(cudaGetLastError());
     }
     const long long n = (long long)base.S * base.P * base.R;
-    k_fields_reduce<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(base);
+    const int chunks = std::max(direct ? base.nchunk : 0, most > 0 ? base.schunk : 0);
+    if (chunks >= 16 && n <= 4864)                          // a warp each: 32 per SM
+        k_fields_reduce<32><<<(unsigned)((32 * n + 127) / 128), 128, 0, st>>>(base);
+    else
+        k_fields_reduce<1><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(base);
     // the series' multiply-adds (k_fields counts its rule's evaluations itself)
     tags_prof_end(TAGS_PROF_FIELDS, pf, st, 2.0 * madds * base.P * base.m, 0.0);
     tags_note_launch();
@@ -928,20 +943,24 @@ int fields_run(const FieldsIn& in) {
     // samples of the moment series, and those past its reach
     const SerGeo geo = series_geo(in.points, P, reinterpret_cast<const Seg*>(in.elec), m);
     std::vector<int> nt(S);
-    bool any_direct = false, any_series = false;
-    for (size_t k = 0; k < S; ++k) {
-        nt[k] = series_terms(geo, zd(in.gamma[k].re, in.gamma[k].im));
-        any_direct = any_direct || nt[k] == 0;
-        any_series = any_series || nt[k] > 0;
+    for (size_t k = 0; k < S; ++k) nt[k] = series_terms(geo, zd(in.gamma[k].re, in.gamma[k].im));
+    // a warp of the rule costs the same for one of its samples as for all, so a
+    // sample past the reach takes the warp's others along (42 electrodes, 126
+    // points, 40 samples: 1.89 ms with the others in the series, 1.56 with none)
+    for (size_t s0 = 0; s0 < S; s0 += cs) {
+        const size_t ns = std::min(cs, S - s0), G = (size_t)samples_per_warp(ns);
+        for (size_t g = s0; g < s0 + ns; g += G) {
+            const auto b = nt.begin() + g, e = nt.begin() + std::min(g + G, s0 + ns);
+            if (std::find(b, e, 0) != e) std::fill(b, e, 0);
+        }
     }
-    // samples on both sides of the series' reach take both kernels one after the
-    // other; a call so small that either is bound by its own latency gives all
-    // samples to the rule (16 electrodes, 24 points, 3 samples: 0.69 ms by both,
-    // 0.61 by the rule; 90 electrodes, 76 points, 23 samples: 0.45 and 1.21)
-    if (any_direct && any_series && P * m * S <= 20000) {
-        std::fill(nt.begin(), nt.end(), 0);
-        any_series = false;
-    }
+    // where the series' samples are so few that the rule, bound by its own latency,
+    // hardly notices them, it takes them all (its time grows by ~0.2 ms per 40,000
+    // of points x electrodes x samples, what the series takes at least)
+    const size_t far = (size_t)std::count(nt.begin(), nt.end(), 0);
+    if (far > 0 && P * m * (S - far) <= 40000) std::fill(nt.begin(), nt.end(), 0);
+    const bool any_direct = std::find(nt.begin(), nt.end(), 0) != nt.end();
+    const bool any_series = std::any_of(nt.begin(), nt.end(), [](int t) { return t > 0; });
     const int nchunk = any_direct ? field_chunks(P, cs, R, m, (size_t)1e9) : 1;
     auto series_args = [&](size_t ns) {
         SerArgs s{};
