@@ -154,3 +154,51 @@ def test_plain_plan_solves_on_clusters(gpu_pkg, m, ns):
     assert not info.any()
     for k in {0, ns - 1}:
         assert rel_err(sol[k], dense_solution(pkg, e, img, nodes, s[k], kappa[k], m // 2)) < TOL
+
+
+def refined_solution(w, b):
+    """Dense solve with the residual in extended precision."""
+    x = np.linalg.solve(w, b).astype(np.clongdouble)
+    wide = w.astype(np.clongdouble)
+    for _ in range(4):
+        x = x + np.linalg.solve(w, (b - wide @ x).astype(np.complex128))
+    return x
+
+
+@pytest.mark.parametrize("s", [1e-2, 1.0 + 10.0j, 1e2 + 1e2j, 8e4 + 1e3j, 8e4 + 1e6j])
+@pytest.mark.parametrize("sigma", [1e-6, 1e-4, 1e-2])
+@pytest.mark.parametrize("mesh", [2, 4])
+def test_currents_and_potentials_each_match_extended_precision(gpu_pkg, s, sigma, mesh):
+    """Potentials reach 1e4 V and more per ampere towards DC in resistive soil,
+    where a longitudinal current follows from a difference of potentials that
+    agree to 8 digits and more: the three blocks of the solution each against a
+    solve refined in extended precision, through the plan and solve_immittance.
+    Bound 1e-11 of the block's largest value: the solves' own 1e-15 or so and,
+    between the plan's fill and the drop-ins', entries that differ by 1e-15 in a
+    system whose impedance part has a condition number up to ~1e3."""
+    pkg = gpu_pkg
+    e, nodes = pkg.electrode_grid(mesh + 1, mesh + 1, 60.0, 60.0, 2, 2, 7e-3, -0.5)
+    img, inj = pkg.images(e), 5
+    m, n = len(e), len(nodes)
+    N = n + 2 * m
+    s = complex(s)
+    kappa = sigma + s * 10 * pkg.EPS0
+    zl, zt = np.zeros(m * m, np.complex128), np.zeros(m * m, np.complex128)
+    gamma, ref_t = pkg.medium(s, kappa)
+    assert pkg.calculate_impedances(zl, zt, e, gamma, s, 1.0, kappa) == 0
+    assert pkg.impedances_images(zl, zt, e, img, gamma, s, 1.0, kappa, 1.0, ref_t) == 0
+    wg = np.zeros(N * N, np.complex128)
+    assert pkg.fill_incidence_imm(wg, e, nodes) == 0
+    assert pkg.fill_impedance_imm(wg, zl, zt, m, n) == 0
+    w = np.tril(wg.reshape(N, N).T)
+    w = w + np.tril(w, -1).T
+    x = np.zeros(N, np.complex128)
+    x[inj] = 1.0
+    want = refined_solution(w, x)
+    assert pkg.solve_immittance(wg, x, m, n) == 0
+    sol, info, _ = pkg.hem_sweep(e, img, nodes, np.array([s]), np.array([kappa]), inj_node=inj)
+    assert not info.any()
+    for part in (slice(0, n), slice(n, n + m), slice(n + m, N)):
+        scale = np.abs(want[part]).max()
+        assert np.abs(x[part] - want[part]).max() <= 1e-11 * scale
+        assert np.abs(sol[0][part] - want[part]).max() <= 1e-11 * scale
