@@ -202,3 +202,39 @@ def test_currents_and_potentials_each_match_extended_precision(gpu_pkg, s, sigma
         scale = np.abs(want[part]).max()
         assert np.abs(x[part] - want[part]).max() <= 1e-11 * scale
         assert np.abs(sol[0][part] - want[part]).max() <= 1e-11 * scale
+
+
+@pytest.mark.parametrize("s", [1e-3, 0.31, 13.0])
+@pytest.mark.parametrize("length,m,sigma", [(1300.0, 15, 1.5e-7), (5.6, 74, 3.8e-2), (5.7, 95, 4.3e-5), (4.4, 62, 0.11),
+                                            (110.0, 81, 1.3e-3), (60.0, 130, 1e-3)])
+def test_refinement_goes_on_until_rounding(gpu_pkg, length, m, sigma, s):
+    """Real s towards DC: ZL is so small that the static order loses the ground
+    impedances' digits and refinement contracts by 1e-5 to 1e-3 only. Every
+    block of the plan's and solve_immittance's solution (one CTA per sample,
+    clusters, panels) against a solve refined in extended precision: a few N eps,
+    2e-13 for N up to 391."""
+    pkg = gpu_pkg
+    e, nodes = pkg.segment_electrode([0.0, 0.0, -0.5], [length, 0.0, -0.5], m, 5e-3)
+    img, inj, n = pkg.images(e), m // 3, m + 1
+    N = n + 2 * m
+    s = complex(s)
+    kappa = sigma + s * 10 * pkg.EPS0
+    zl, zt = np.zeros(m * m, np.complex128), np.zeros(m * m, np.complex128)
+    gamma, ref_t = pkg.medium(s, kappa)
+    assert pkg.calculate_impedances(zl, zt, e, gamma, s, 1.0, kappa) == 0
+    assert pkg.impedances_images(zl, zt, e, img, gamma, s, 1.0, kappa, 1.0, ref_t) == 0
+    wg = np.zeros(N * N, np.complex128)
+    assert pkg.fill_incidence_imm(wg, e, nodes) == 0
+    assert pkg.fill_impedance_imm(wg, zl, zt, m, n) == 0
+    w = np.tril(wg.reshape(N, N).T)
+    w = w + np.tril(w, -1).T
+    x = np.zeros(N, np.complex128)
+    x[inj] = 1.0
+    want = refined_solution(w, x)
+    assert pkg.solve_immittance(wg, x, m, n) == 0
+    sol, info, _ = pkg.hem_sweep(e, img, nodes, np.array([s]), np.array([kappa]), inj_node=inj)
+    assert not info.any()
+    for part in (slice(0, n), slice(n, n + m), slice(n + m, N)):
+        scale = np.abs(want[part]).max()
+        assert np.abs(x[part] - want[part]).max() <= 2e-13 * scale
+        assert np.abs(sol[0][part] - want[part]).max() <= 2e-13 * scale

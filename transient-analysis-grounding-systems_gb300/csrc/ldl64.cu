@@ -12,8 +12,8 @@
 // n = 1417). FP64 runs at two fused multiply-adds per clock and SM here, so
 // the flops are the time. What the missing pivot search may cost in accuracy
 // is recovered by FP64 refinement against the untouched impedance blocks; a
-// sample whose corrections do not shrink to 1e-8 |x| (the next one would be
-// below FP64 rounding) is handed to the pivoted LU (lu.cu) by its caller.
+// sample whose corrections do not shrink until the next one would be below FP64
+// rounding is handed to the pivoted LU (lu.cu) by its caller.
 // Measured against that LU on GB300: 2 samples at m = 1560 714 -> 120 ms, 256
 // samples at m = 100 24.3 -> 5.9 ms, 100 samples at m = 10 0.66 -> 0.25 ms.
 //
@@ -535,17 +535,24 @@ __global__ void k_ldl64_start(const double2* __restrict__ rhs, long long rstride
     X0[o] = cz(0.0, 0.0);
 }
 
+// The stopping rule, for the currents (amperes) and the potentials (volts), whose
+// sizes have nothing to do with one another, each by itself. A correction dn after
+// one of prev makes the next about dn^2 / prev; done when that is below 1e-16 of
+// the unknowns, xn. (By dn <= 1e-8 xn alone a contraction of 1e-4 stopped after two
+// refinements with 1e-12 left: 1200 random rods, wires and grids from |s| = 1e-4 / s
+// on were off by up to 9e-12, now by up to 2e-14, at the same times.)
+TAGS_D bool settled(double dn, double prev, double xn) { return dn <= 1e-8 * sqrt(prev) * sqrt(xn); }
+
 // x += dx and the stopping rule, one CTA per sample. Step 0's correction is x
-// itself. Later ones: dx <= 1e-8 |x| means a contraction below 1e-8, so the
-// next correction would be under FP64 rounding: done. A correction that did
-// not halve, or the last step's, leaves the sample to the pivoted LU.
+// itself. Unknowns below nc are currents. A correction that has not settled and
+// did not halve, or is the last step's, leaves the sample to the pivoted LU.
 __global__ void __launch_bounds__(256) k_ldl64_apply(const double2* __restrict__ S0, double2* __restrict__ X0, int N,
-                                                     int step, int last, int* __restrict__ active,
+                                                     int nc, int step, int last, int* __restrict__ active,
                                                      int* __restrict__ conv, double* __restrict__ prev) {
     const int b = blockIdx.x;
     if (!active[b]) return;
-    __shared__ double smx[2][8];
-    double dn = 0.0, xn = 0.0;
+    __shared__ double smx[4][8];
+    double mx[4] = {0.0, 0.0, 0.0, 0.0};                     // dx and x of the currents, of the potentials
     bool bad = false;
     for (int j = threadIdx.x; j < N; j += blockDim.x) {
         const long long o = (long long)N * b + j;
@@ -553,36 +560,40 @@ __global__ void __launch_bounds__(256) k_ldl64_apply(const double2* __restrict__
         X0[o] = x;
         const double a = cabs1(d), c = cabs1(x);
         bad = bad || !isfinite(a) || !isfinite(c);
-        dn = fmax(dn, a);
-        xn = fmax(xn, c);
+        if (j < nc) {
+            mx[0] = fmax(mx[0], a);
+            mx[1] = fmax(mx[1], c);
+        } else {
+            mx[2] = fmax(mx[2], a);
+            mx[3] = fmax(mx[3], c);
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        dn = fmax(dn, __shfl_xor_sync(0xffffffffu, dn, o));
-        xn = fmax(xn, __shfl_xor_sync(0xffffffffu, xn, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        smx[0][threadIdx.x >> 5] = dn;
-        smx[1][threadIdx.x >> 5] = xn;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        for (int o = 16; o > 0; o >>= 1) mx[q] = fmax(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], o));
+        if ((threadIdx.x & 31) == 0) smx[q][threadIdx.x >> 5] = mx[q];
     }
     const int anybad = __syncthreads_or(bad);
     if (threadIdx.x != 0) return;
-    for (int w = 1; w < 8; ++w) {
-        dn = fmax(dn, smx[0][w]);
-        xn = fmax(xn, smx[1][w]);
-    }
+    for (int w = 1; w < 8; ++w)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) mx[q] = fmax(mx[q], smx[q][w]);
     if (anybad) {
         active[b] = 0;
         return;
     }
     if (step > 0) {
-        if (dn <= 1e-8 * xn) {
-            conv[b] = 1;
-            active[b] = 0;
-        } else if (last || dn > 0.5 * prev[b]) {
-            active[b] = 0;
-        }
+        bool done = true, stuck = last != 0;
+        for (int q = 0; q < 2; ++q)
+            if (!settled(mx[2 * q], prev[2 * b + q], mx[2 * q + 1])) {
+                done = false;
+                stuck = stuck || mx[2 * q] > 0.5 * prev[2 * b + q];
+            }
+        if (done) conv[b] = 1;
+        if (done || stuck) active[b] = 0;
     }
-    prev[b] = dn;
+    prev[2 * b] = mx[0];
+    prev[2 * b + 1] = mx[2];
 }
 
 // Solutions to the original order; info 0, or the marker of a sample that
@@ -698,7 +709,7 @@ __global__ void __launch_bounds__(128) k_ldl64_small(const double2* __restrict__
     double2* A = reinterpret_cast<double2*>(smem_raw);     // (r, c) at c P + r
     double2* bv = A + (size_t)N * P;
     double2 *x = bv + N, *r = x + N, *dinv = r + N, *z = dinv + N;
-    __shared__ double smx[2][4];
+    __shared__ double smx[4][4];
     __shared__ int sstate;                                  // 0: go on, 1: done, 2: to the pivoted LU
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const double2* W = W0 + stride * b;
@@ -740,7 +751,7 @@ __global__ void __launch_bounds__(128) k_ldl64_small(const double2* __restrict__
         if (i > c) A[c * P + i] = cmul(A[c * P + i], dinv[c]);
     }
     __syncthreads();
-    double prev = 0.0;
+    double prev[2] = {0.0, 0.0};
     for (int step = 0; step < 4; ++step) {
         if (step > 0) {
             for (int i = tid; i < N; i += 128) {
@@ -778,32 +789,39 @@ __global__ void __launch_bounds__(128) k_ldl64_small(const double2* __restrict__
             }
         }
         __syncthreads();
-        double dn = 0.0, xn = 0.0;
+        double mx[4] = {0.0, 0.0, 0.0, 0.0};                 // dx and x of the currents, of the potentials
         bool bad = false;
         for (int i = tid; i < N; i += 128) {
             const double2 d = z[i], v = cadd(x[i], d);
             x[i] = v;
             bad = bad || !isfinite(cabs1(d)) || !isfinite(cabs1(v));
-            dn = fmax(dn, cabs1(d));
-            xn = fmax(xn, cabs1(v));
+            if (i < 2 * m) {
+                mx[0] = fmax(mx[0], cabs1(d));
+                mx[1] = fmax(mx[1], cabs1(v));
+            } else {
+                mx[2] = fmax(mx[2], cabs1(d));
+                mx[3] = fmax(mx[3], cabs1(v));
+            }
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            dn = fmax(dn, __shfl_xor_sync(0xffffffffu, dn, o));
-            xn = fmax(xn, __shfl_xor_sync(0xffffffffu, xn, o));
-        }
-        if (lane == 0) {
-            smx[0][warp] = dn;
-            smx[1][warp] = xn;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            for (int o = 16; o > 0; o >>= 1) mx[q] = fmax(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], o));
+            if (lane == 0) smx[q][warp] = mx[q];
         }
         const int anybad = __syncthreads_or(bad);
         if (tid == 0) {
-            dn = fmax(fmax(smx[0][0], smx[0][1]), fmax(smx[0][2], smx[0][3]));
-            xn = fmax(fmax(smx[1][0], smx[1][1]), fmax(smx[1][2], smx[1][3]));
-            sstate = 0;
-            if (anybad) sstate = 2;
-            else if (step > 0 && dn <= 1e-8 * xn) sstate = 1;
-            else if (step == 3 || (step > 0 && dn > 0.5 * prev)) sstate = 2;
-            prev = dn;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) mx[q] = fmax(fmax(smx[q][0], smx[q][1]), fmax(smx[q][2], smx[q][3]));
+            bool done = true, stuck = step == 3;
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                if (!settled(mx[2 * q], prev[q], mx[2 * q + 1])) {
+                    done = false;
+                    stuck = stuck || mx[2 * q] > 0.5 * prev[q];
+                }
+            sstate = anybad ? 2 : step == 0 ? 0 : done ? 1 : stuck ? 2 : 0;
+            prev[0] = mx[0];
+            prev[1] = mx[2];
         }
         __syncthreads();
         if (sstate) break;
@@ -1041,7 +1059,7 @@ Ws carve(void* p, int N, int batch) {
     w.r = w.x + (long long)N * batch;
     w.z = w.r + (long long)N * batch;
     w.prev = reinterpret_cast<double*>(w.z + (long long)N * batch);
-    w.active = reinterpret_cast<int*>(w.prev + batch);
+    w.active = reinterpret_cast<int*>(w.prev + 2 * batch);
     w.conv = w.active + batch;
     return w;
 }
@@ -1173,8 +1191,8 @@ int tags_ldl64_prepare() {
 }
 
 size_t tags_ldl64_workspace(int N, int batch) {
-    const size_t per = sizeof(double2) * (((size_t)(N + PB - 1) / PB + 2) * PB * PB + 4 * (size_t)N) + sizeof(double) +
-                       2 * sizeof(int);
+    const size_t per = sizeof(double2) * (((size_t)(N + PB - 1) / PB + 2) * PB * PB + 4 * (size_t)N) +
+                       2 * (sizeof(double) + sizeof(int));
     return per * batch + 64;
 }
 
@@ -1216,7 +1234,8 @@ int tags_ldl64_plan_solve(double2* W, const Incidence& inc, int m, int n, int nb
         }
         err = solve(W, N, N, NN, nb, m, w, step == 0 ? 2 * m : 0, st);
         if (err) break;
-        k_ldl64_apply<<<nb, 256, 0, st>>>(w.z, w.x, N, step, step + 1 == MAX_CORRECTIONS, w.active, w.conv, w.prev);
+        k_ldl64_apply<<<nb, 256, 0, st>>>(w.z, w.x, N, 2 * m, step, step + 1 == MAX_CORRECTIONS, w.active, w.conv,
+                                          w.prev);
         tags_note_launch();
     }
     if (err) return err;
@@ -1256,7 +1275,7 @@ int tags_ldl64_sym_solve(const double2* W, double2* A, int m, int n, void* ws, i
         }
         err = solve(A, N, N, 0, 1, zm, w, 0, st);
         if (err) break;
-        k_ldl64_apply<<<1, 256, 0, st>>>(w.z, w.x, N, step, step == 2, w.active, w.conv, w.prev);
+        k_ldl64_apply<<<1, 256, 0, st>>>(w.z, w.x, N, 2 * m, step, step == 2, w.active, w.conv, w.prev);
         tags_note_launch();
     }
     if (err) return err;
