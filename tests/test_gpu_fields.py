@@ -201,3 +201,53 @@ def test_field_of_few_points_and_many_electrodes_matches_oracle(gpu_pkg, port, m
     """Lanes per pair from 32 down to 1, chunks summed by a thread or a warp; oracle at 1e-11, TOL of the largest
     magnitude."""
     test_field_series_and_its_limits_match_oracle(gpu_pkg, port, 0.05, ns, 2, m, P)
+
+
+def fine_rule(point, e, gamma):
+    """The integrals of e^{-gamma r}/r and of (1 + gamma r) e^{-gamma r} / r^3 (point - position) over an electrode,
+    panels halving towards the point, 32 nodes each."""
+    a, b = e[:3], e[3:6]
+    x, w = np.polynomial.legendre.leggauss(32)
+    foot = np.clip((point - a) @ (b - a) / ((b - a) @ (b - a)), 0.0, 1.0)
+    edges = np.unique(np.clip(np.concatenate([[0.0, 1.0, foot], foot + 2.0 ** -np.arange(12), foot - 2.0 ** -np.arange(12)]),
+                              0.0, 1.0))
+    j, f = 0.0, np.zeros(3, np.complex128)
+    for lo, hi in zip(edges[:-1], edges[1:]):
+        t = lo + (hi - lo) * (x + 1) / 2
+        d = point - (a + t[:, None] * (b - a))
+        r = np.linalg.norm(d, axis=1)
+        ex = w * (hi - lo) / 2 * np.exp(-gamma * r)
+        j = j + (ex / r).sum()
+        f = f + ((ex * (1 + gamma * r) / r ** 3)[:, None] * d).sum(axis=0)
+    return j, f
+
+
+@pytest.mark.parametrize("x", [0.05, 0.36, 0.54, 0.6, 0.99, 1.1, 1.5, 1.99])
+@pytest.mark.parametrize("m", [1, 5, 70])
+def test_field_series_to_rounding_at_every_order(gpu_pkg, x, m):
+    """Points along the axis and abeam on both sides of every distance at which the series' rule changes its order, x =
+    |gamma| (L + L/8) / 2 up to the reach of 2: 1e-14 of the value (some ten roundings of the 24 terms' sum, whose
+    largest is e^2 times the first) and the rounding of the phase |gamma| r on either side. One electrode carries the
+    current, so that no two cancel."""
+    pkg = gpu_pkg
+    e, _ = pkg.segment_electrode([0.0, 0.0, -0.5], [1.0 * m, 0.0, -0.5], m, 7e-3)
+    gamma = x / 0.5625 * np.exp(0.25j * np.pi)
+    k = m // 2
+    mid = np.array([k + 0.5, 0.0, -0.5])
+    pts = []
+    for dist in (0.4, 1.9, 2.1, 3.9, 4.1, 7.9, 8.1, 15.9, 16.1, 20.0):
+        for turn in (0.0, 0.6, np.pi / 2):
+            step = np.array([np.cos(turn), np.sin(turn), 0.0])
+            pts.append(mid + (dist + 0.5 * abs(step[0])) * step + np.array([0.0, 1e-3 if turn == 0.0 else 0.0, 0.0]))
+    pts = np.array(pts)
+    if m > 1:
+        pts[:, 2] += 0.03                   # off the axis of the other electrodes
+    cur = np.zeros((1, 1, m), np.complex128)
+    cur[0, 0, k] = 1.0
+    out = pkg.fields_batch(pts, e, cur, cur, [gamma], [1.0 + 0j])
+    assert out["status"] == 0
+    for p, point in enumerate(pts):
+        j, f = fine_rule(point, e[k], gamma)
+        tol = 1e-14 + 2 * np.finfo(float).eps * abs(gamma) * (np.linalg.norm(point - mid) + 0.5)
+        assert abs(4 * np.pi * out["pot"][0, p, 0] - j) <= tol * abs(j)
+        assert np.abs(4 * np.pi * out["efield"][0, p, 0] - f).max() <= tol * np.abs(f).max()

@@ -327,6 +327,13 @@ TAGS_D bool cur_big(double2 c) {
 constexpr int FS_ORDERS[5] = {6, 7, 8, 9, 12};
 constexpr int FS_GL = 6 + 7 + 8 + 9 + 12;
 
+// The rule's orders from 16 and from 8 lengths away, as indices of FS_ORDERS: the
+// distance leaves 1/r and 1/r^3 with 6 and 7 nodes below 1e-15, but the moments
+// also carry e^{-gamma r} over the electrode, whose error at x = |gamma| dmax is
+// 8e-10 (x / 2)^12 with 6 nodes and 5e-12 (x / 2)^14 with 7 on the electrode's axis.
+// Each stays up to where that passes 1e-15 (6 nodes at every x: 6e-10 at x = 1.95).
+int fs_least_order(double x) { return x <= 0.55 ? 0 : x <= 1.0 ? 1 : 3; }
+
 __constant__ double c_fsx[FS_GL], c_fsw[FS_GL];   // nodes and weights on [0, 1], order by order
 
 struct SerArgs {
@@ -335,6 +342,8 @@ struct SerArgs {
     const double2* tab;     // [bucket][S]: e^{-gamma b h}
     double h;
     int nbk, ngc, echunk;   // buckets; sample groups per CTA (1, 2, 4); electrodes per CTA
+    int least;              // fs_least_order of the pass's largest |gamma| among the series' samples
+    double ga;              // that |gamma|
 };
 
 __global__ void k_fser_tables(const double2* __restrict__ gamma, const int* __restrict__ nt, int S, int nbk, double h,
@@ -361,10 +370,11 @@ struct SerPair {
 
 // Moments of one (point, electrode) pair by L lanes (g: this one), all of the
 // warp's groups together, `on` or not: Gauss-Legendre in t where the point is at
-// least two lengths away (6 to 12 nodes by the distance), else the sinh rule above
-// in panels of at most 0.75, up to ~1000 nodes, which one lane would take in a row.
+// least two lengths away (6 to 12 nodes by the distance and |gamma|), else the sinh
+// rule above in panels of at most 0.75 and, as in k_fields, 1.5 / |gamma| of r on
+// average, up to ~1000 nodes, which one lane would take in a row.
 template <int NT>
-TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, double h, int nbk, const double* gx,
+TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, const SerArgs& sa, const double* gx,
                          const double* gw, bool on, int g, int L, SerPair& out, double* mom) {
     SerPair q;
     const double D[3] = {S.b[0] - S.a[0], S.b[1] - S.a[1], S.b[2] - S.a[2]};
@@ -382,8 +392,8 @@ TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, double h
     const double uc = fmin(fmax(u0, 0.0), 1.0), du = (u0 - uc) * Lg;
     const double dist = sqrt(d2 + du * du);
     const double dm = (u0 - 0.5) * Lg, rc = sqrt(d2 + dm * dm);
-    q.b = min(nbk - 1, max(0, (int)rint(rc / h)));
-    const double R = q.b * h;
+    q.b = min(sa.nbk - 1, max(0, (int)rint(rc / sa.h)));
+    const double R = q.b * sa.h;
     double aN[NT], aA[NT], aB[NT];
 #pragma unroll
     for (int n = 0; n < NT; ++n) aN[n] = aA[n] = aB[n] = 0.0;
@@ -404,7 +414,7 @@ TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, double h
     q.bad = !(dist > 1e-12 * Lg) || !isfinite(rc);
     if (!q.bad && dist >= 2.0 * Lg) {
         const double ratio = dist * q.iL;
-        const int o = ratio >= 16.0 ? 0 : ratio >= 8.0 ? 1 : ratio >= 4.0 ? 3 : 4;
+        const int o = max(sa.least, ratio >= 16.0 ? 0 : ratio >= 8.0 ? 1 : ratio >= 4.0 ? 3 : 4);
         const int nq = o == 0 ? 6 : o == 1 ? 7 : o == 3 ? 9 : 12, off = o == 0 ? 0 : o == 1 ? 6 : o == 3 ? 21 : 30;
         for (int i = g; i < nq; i += L) {
             const double s = (gx[off + i] - u0) * Lg;
@@ -417,7 +427,9 @@ TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, double h
         const bool split = va < 0.0 && vb > 0.0;
         for (int side = 0; side < (split ? 2 : 1); ++side) {
             const double lo = split && side == 1 ? 0.0 : va, hi = split && side == 0 ? 0.0 : vb;
-            const int np = max(1, (int)ceil(fmin((hi - lo) / 0.75, 64.0)));
+            const double rl = dp * sinh(lo), rh = dp * sinh(hi);
+            const double dr = fabs(sqrt(fma(rh, rh, d2)) - sqrt(fma(rl, rl, d2)));
+            const int np = max(1, (int)ceil(fmin(fmax((hi - lo) / 0.75, sa.ga * dr / FC), 64.0)));
             const double ph = (hi - lo) / np;
             for (int t = g; t < 8 * np; t += L) {
                 const int p = t >> 3, i = t & 7;
@@ -508,8 +520,7 @@ __global__ void __launch_bounds__(FS_THREADS) k_fields_series(SerArgs sa, int r0
         while (2 * L * ne <= FS_THREADS && L < 32) L *= 2;
         const int me = min(tid / L, ne - 1);
         const bool on = tid < L * ne;
-        fser_moments<NT>(a.elec[e0 + me], P0, P1, P2, sa.h, sa.nbk, gx, gw, on, tid % L, L, pr[me],
-                         mom + (size_t)me * 3 * NT);
+        fser_moments<NT>(a.elec[e0 + me], P0, P1, P2, sa, gx, gw, on, tid % L, L, pr[me], mom + (size_t)me * 3 * NT);
         if (on && tid % L == 0 && pr[me].bad) raise_status(a.status, TAGS_ST_DEGENERATE_PAIR);
         __syncthreads();
         if (!valid) continue;
@@ -1018,6 +1029,9 @@ int fields_run(const FieldsIn& in) {
         int* d_nt = reinterpret_cast<int*>(tab + (size_t)geo.nbk * ns);
         TAGS_CUDA_OK(cudaMemcpyAsync(d_nt, nt.data() + s0, sizeof(int) * ns, cudaMemcpyHostToDevice, st));
         const int most = *std::max_element(nt.begin() + s0, nt.begin() + s0 + ns);
+        for (size_t k = s0; k < s0 + ns; ++k)
+            if (nt[k] > 0) sa.ga = std::max(sa.ga, std::abs(zd(in.gamma[k].re, in.gamma[k].im)));
+        sa.least = fs_least_order(sa.ga * geo.dmax);
         if (most > 0) {
             k_fser_tables<<<dim3((unsigned)((ns + 31) / 32), geo.nbk + 1), 32, 0, st>>>(d_gk, d_nt, (int)ns, geo.nbk,
                                                                                     geo.h, pw, tab);
