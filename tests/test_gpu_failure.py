@@ -165,3 +165,52 @@ def test_resolves_side_by_side_match_plain(gpu_pkg, m, ns):
         assert np.max(np.abs(sol - ref)) < 1e-10 * np.max(np.abs(ref))
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("m", [6, 40, 120])
+@pytest.mark.parametrize("value,kappa_value", [(complex(np.nan, 0.0), 0.01 + 1e-4j), (complex(0.0, 1e20), 0.01 + 1e-4j)])
+def test_samples_beside_an_invalid_one_are_solved(gpu_pkg, m, value, kappa_value):
+    """A plain run with an invalid sample fails, and its other samples are
+    solved all the same, those of s = 0 that need the pivoted LU among them, in
+    the pass of the invalid one and in later ones: equal to a run without it.
+    info holds 0 or a pivot's number, never an internal mark, also after a
+    geometry error."""
+    torch = pytest.importorskip("torch")
+    pkg = gpu_pkg
+    e, nodes = pkg.segment_electrode([0.0, 0.0, -0.5], [1.0 * m, 0.0, -0.5], m, 7e-3)
+    s = np.array([8e4 + 1e5j, 0.0, 8e4 + 1e6j, value, 0.0, 8e4 + 2e6j, 0.0])
+    kappa = np.where(s == 0.0, 0.01 + 0j, 0.01 + 1e-4j)
+    kappa[3] = kappa_value
+    good = np.array([0, 1, 2, 4, 5, 6])
+    want, info, _ = pkg.hem_sweep(e, pkg.images(e), nodes, s[good], kappa[good], inj_node=1)
+    assert not info.any()
+    pkg.lib().tags_gpu_set_quiet(1)
+    try:
+        for case in ("invalid sample", "geometry"):
+            es = e if case == "invalid sample" else np.concatenate([e, e[:1]])
+            for graphs in (True, False):
+                plan = pkg.Plan(es, pkg.images(es), nodes, pkg.PLAIN_FP64, 5, graphs)
+                s_d, k_d = (torch.from_numpy(v).cuda() for v in (s, kappa))
+                sol = torch.zeros((len(s), plan.N), dtype=torch.complex128, device="cuda")
+                got = torch.full((len(s),), 77, dtype=torch.int32, device="cuda")
+                try:
+                    with pytest.raises(RuntimeError):
+                        plan.run_device(s_d.data_ptr(), k_d.data_ptr(), len(s), 1.0, 0, 1, sol.data_ptr(), got.data_ptr())
+                finally:
+                    plan.close()
+                torch.cuda.synchronize()
+                assert not got.cpu().numpy()[good].any()
+                if case == "invalid sample":
+                    assert rel_err(sol.cpu().numpy()[good], want) < 1e-10
+        if np.isfinite(value):                      # a grid batch takes finite values only
+            jobs = [{"electrodes": e, "images": pkg.images(e), "nodes": nodes, "s": s, "kappa": kappa, "inj_node": 1}]
+            batch = pkg.GridBatch(jobs, precision=pkg.PLAIN_FP64)
+            try:
+                arr, keep, out = pkg._grid_jobs(jobs)
+                assert pkg.lib().tags_batch_run(batch.handle, arr, 1, None) == pkg.E_ARG
+            finally:
+                batch.close()
+            assert not out[0][1][good].any()
+            assert rel_err(out[0][0][good], want) < 1e-10
+    finally:
+        pkg.lib().tags_gpu_set_quiet(0)

@@ -400,7 +400,10 @@ extern "C" int tags_batch_run(tags_batch batch, const tags_grid_job* jobs, size_
                 if (e) return e;
             }
             TAGS_CUDA_OK(cudaStreamSynchronize(p->stream));
-        } else if (b->precision == TAGS_PLAIN_FP64 && !grid_status[q]) {
+        } else if (b->precision == TAGS_PLAIN_FP64 && (grid_status[q] & TAGS_ST_DEGENERATE_PAIR)) {
+            // every sample of the grid is NaN, as after a plan's run
+            TAGS_CUDA_OK(cudaMemset(g.d_info, 0, sizeof(int) * g.ns));
+        } else if (b->precision == TAGS_PLAIN_FP64) {
             // plain form: samples marked for the pivoted LU
             std::vector<int> si(g.ns);
             TAGS_CUDA_OK(cudaMemcpy(si.data(), g.d_info, sizeof(int) * g.ns, cudaMemcpyDeviceToHost));

@@ -342,15 +342,19 @@ int tags_plan_lu_one(tags_plan_s* p, int q, double2* W, int* ipiv, double2* x, i
 }
 
 // After a plain pass: samples marked for the pivoted LU are solved by it, one
-// by one in the first sample's matrix. A pass whose fill failed is left as it
-// is (the run reports the status).
+// by one in the first sample's matrix, whatever another sample's values brought
+// into the status. Only a geometry whose integrals diverge, which makes every
+// sample of the run NaN, is left as it is.
 static int finish_plain(tags_plan_s* p, int nb, cudaStream_t st) {
     std::vector<int> info(nb);
     int status = 0;
     TAGS_CUDA_OK(cudaMemcpyAsync(info.data(), p->d_info, sizeof(int) * nb, cudaMemcpyDeviceToHost, st));
     TAGS_CUDA_OK(cudaMemcpyAsync(&status, p->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     TAGS_CUDA_OK(cudaStreamSynchronize(st));
-    if (status) return 0;
+    if (status & TAGS_ST_DEGENERATE_PAIR) {
+        TAGS_CUDA_OK(cudaMemsetAsync(p->d_info, 0, sizeof(int) * nb, st));
+        return 0;
+    }
     for (int q = 0; q < nb; ++q) {
         if (info[q] != TAGS_INFO_RESOLVE) continue;
         double2* x = p->d_x + (size_t)q * p->N;
