@@ -251,3 +251,37 @@ def test_field_series_to_rounding_at_every_order(gpu_pkg, x, m):
         tol = 1e-14 + 2 * np.finfo(float).eps * abs(gamma) * (np.linalg.norm(point - mid) + 0.5)
         assert abs(4 * np.pi * out["pot"][0, p, 0] - j) <= tol * abs(j)
         assert np.abs(4 * np.pi * out["efield"][0, p, 0] - f).max() <= tol * np.abs(f).max()
+
+
+@pytest.mark.parametrize("dist,P,m", [(1000.0, 1, 10), (1000.0, 3, 1), (300.0, 40, 8), (30.0, 70, 4)])
+@pytest.mark.parametrize("ns", [1, 40, 130])
+def test_field_far_away_matches_fine_rule(gpu_pkg, dist, P, m, ns):
+    """Few pairs far apart, where most of the expansion centres between them are not used, and more pairs than centres:
+    exponentials formed per pair and from the table. Tolerance as in the test above, for m currents of one sign."""
+    pkg = gpu_pkg
+    e, _ = pkg.segment_electrode([0.0, 0.0, -0.5], [1.0 * m, 0.0, -0.5], m, 7e-3)
+    gamma = 0.02 * np.exp(0.25j * np.pi) * np.linspace(0.1, 1.0, ns)
+    pts = np.stack([np.linspace(dist, dist + 2.0, P), np.full(P, 0.3), np.zeros(P)], axis=1)
+    cur = np.ones((ns, 1, m), np.complex128)
+    out = pkg.fields_batch(pts, e, cur, cur, gamma, np.ones(ns, np.complex128))
+    assert out["status"] == 0
+    for k in {0, ns // 2, ns - 1}:
+        for p in {0, P - 1}:
+            j, f = (sum(v) for v in zip(*(fine_rule(pts[p], e[q], gamma[k]) for q in range(m))))
+            tol = 1e-14 + 2 * np.finfo(float).eps * abs(gamma[k]) * (dist + 2 + m)
+            assert abs(4 * np.pi * out["pot"][k, p, 0] - j) <= tol * abs(j)
+            assert np.abs(4 * np.pi * out["efield"][k, p, 0] - f).max() <= tol * np.abs(f).max()
+
+
+def test_field_memory_follows_the_work(gpu_pkg):
+    """A call of many samples and few pairs takes device memory for its samples, inputs and outputs, some 1 KB a sample
+    here, not for a table of every distance in between (64 KB a sample)."""
+    torch = pytest.importorskip("torch")
+    pkg = gpu_pkg
+    m, ns = 2, 200000
+    e, _ = pkg.segment_electrode([0.0, 0.0, -0.5], [1.0 * m, 0.0, -0.5], m, 7e-3)
+    cur = np.ones((ns, 1, m), np.complex128)
+    before = torch.cuda.mem_get_info()[0]
+    out = pkg.fields_batch([[1000.0, 0.0, 0.0]], e, cur, cur, np.full(ns, 0.01 + 0.01j), np.ones(ns, np.complex128))
+    assert out["status"] == 0 and np.ptp(out["pot"].real) == 0.0
+    assert before - torch.cuda.mem_get_info()[0] < 1 << 30

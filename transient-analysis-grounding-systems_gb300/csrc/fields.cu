@@ -339,13 +339,15 @@ __constant__ double c_fsx[FS_GL], c_fsw[FS_GL];   // nodes and weights on [0, 1]
 struct SerArgs {
     FieldArgs f;
     const double2* pw;      // [FS_NT][S]
-    const double2* tab;     // [bucket][S]: e^{-gamma b h}
+    const double2* tab;     // [bucket][S]: e^{-gamma b h} (null: formed per pair)
     double h;
     int nbk, ngc, echunk;   // buckets; sample groups per CTA (1, 2, 4); electrodes per CTA
     int least;              // fs_least_order of the pass's largest |gamma| among the series' samples
     double ga;              // that |gamma|
 };
 
+// The samples' constants: a row of CTAs per bucket of the table (nbk of them, none
+// where the pairs form theirs), one more for the powers.
 __global__ void k_fser_tables(const double2* __restrict__ gamma, const int* __restrict__ nt, int S, int nbk, double h,
                               double2* __restrict__ pw, double2* __restrict__ tab) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
@@ -463,9 +465,11 @@ TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, const Se
 // (pair, sample) and 20 per injection. The 1560-segment grid, 251 points, 64
 // samples, 4 injections: 58.8 ms by the rule per sample, 13.1 ms so (14.4 with the
 // vector potential's three components per pair; error of the field against 64-bit
-// quadrature 1.6e-13 -> 2.2e-15).
+// quadrature 1.6e-13 -> 2.2e-15). e^{-gamma R} comes from the table, or, where the
+// call has fewer pairs than the table has buckets, is formed per pair and sample
+// (TAB false): a point 1 km from ten electrodes needs 10 of 4002 buckets.
 constexpr int FS_E = 128;                 // pairs per tile, a thread each
-template <int NT>
+template <int NT, bool TAB>
 __global__ void __launch_bounds__(FS_THREADS) k_fields_series(SerArgs sa, int r0) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* mom = reinterpret_cast<double*>(smem_raw);              // [FS_E][3 NT]
@@ -485,6 +489,7 @@ __global__ void __launch_bounds__(FS_THREADS) k_fields_series(SerArgs sa, int r0
     const bool valid = grp < ngroups && smp < a.S && a.nt[smp] > 0;
     const int nt = __reduce_max_sync(0xffffffffu, valid ? a.nt[smp] : 0);
     const int nr = min(RMAX, a.R - r0);
+    const double2 gam = !TAB && valid ? a.gamma[smp] : cz(0.0, 0.0);
     const double P0 = a.pts[3 * p], P1 = a.pts[3 * p + 1], P2 = a.pts[3 * p + 2];
     const bool wv = (a.want & (WANT_VEC | WANT_EF)) != 0;
     const int e_begin = blockIdx.y * sa.echunk, e_end = min(a.m, e_begin + sa.echunk);
@@ -539,7 +544,9 @@ __global__ void __launch_bounds__(FS_THREADS) k_fields_series(SerArgs sa, int r0
                     Bp.y = fma(pn.y, mo[2 * NT + n], Bp.y);
                 }
             }
-            const double2 ex = sa.tab[(long long)q.b * a.S + smp];
+            double2 ex;
+            if (TAB) ex = sa.tab[(long long)q.b * a.S + smp];
+            else ex = cexp_d(cz(-gam.x * (q.b * sa.h), -gam.y * (q.b * sa.h)));
             J1 = cmul(J1, ex);
             if (wv) {
                 Ap = cmul(Ap, ex);
@@ -767,6 +774,14 @@ __global__ void k_voltage(const double* __restrict__ paths, int NL, const Seg* _
 bool g_tables_ready[64] = {};
 unsigned long long* g_evals[64] = {};   // per-device work counter
 
+// The instance for nt terms, and its shared memory.
+auto series_kernel(int nt, bool tab) {
+    if (nt <= 12) return tab ? k_fields_series<12, true> : k_fields_series<12, false>;
+    if (nt <= 16) return tab ? k_fields_series<16, true> : k_fields_series<16, false>;
+    return tab ? k_fields_series<FS_NT, true> : k_fields_series<FS_NT, false>;
+}
+size_t series_smem(int nt) { return FS_E * 3 * sizeof(double) * (nt <= 12 ? 12 : nt <= 16 ? 16 : FS_NT); }
+
 int fields_tables(int dev) {
     if (dev < 0 || dev >= 64) return TAGS_E_CUDA;
     if (g_tables_ready[dev]) return 0;
@@ -782,12 +797,11 @@ int fields_tables(int dev) {
     }
     TAGS_CUDA_OK(cudaMemcpyToSymbol(c_fsx, sx, sizeof(sx)));
     TAGS_CUDA_OK(cudaMemcpyToSymbol(c_fsw, sw, sizeof(sw)));
-    const int smem = FS_E * 3 * (int)sizeof(double);            // per term
-    if (cudaFuncSetAttribute(k_fields_series<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem * 12) != cudaSuccess ||
-        cudaFuncSetAttribute(k_fields_series<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem * 16) != cudaSuccess ||
-        cudaFuncSetAttribute(k_fields_series<FS_NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem * FS_NT) !=
-            cudaSuccess)
-        return tags_fail(TAGS_E_CUDA, "cudaFuncSetAttribute(k_fields_series) failed");
+    for (int nt : {12, 16, FS_NT})
+        for (bool tab : {true, false})
+            if (cudaFuncSetAttribute(series_kernel(nt, tab), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)series_smem(nt)) != cudaSuccess)
+                return tags_fail(TAGS_E_CUDA, "cudaFuncSetAttribute(k_fields_series) failed");
     TAGS_CUDA_OK(cudaMalloc(&g_evals[dev], sizeof(unsigned long long)));
     TAGS_CUDA_OK(cudaMemset(g_evals[dev], 0, sizeof(unsigned long long)));
     g_tables_ready[dev] = true;
@@ -900,10 +914,7 @@ int launch_fields(const SerArgs& sa, int most, double madds, bool direct, cudaSt
     if (most > 0) {
         const dim3 g((unsigned)base.P, (unsigned)(base.schunk / (4 / sa.ngc)), (unsigned)((ngroups + sa.ngc - 1) / sa.ngc));
         for (int r0 = 0; r0 < base.R; r0 += RMAX) {
-            const size_t smem = FS_E * 3 * sizeof(double);
-            if (most <= 12) k_fields_series<12><<<g, FS_THREADS, smem * 12, st>>>(sa, r0);
-            else if (most <= 16) k_fields_series<16><<<g, FS_THREADS, smem * 16, st>>>(sa, r0);
-            else k_fields_series<FS_NT><<<g, FS_THREADS, smem * FS_NT, st>>>(sa, r0);
+            series_kernel(most, sa.tab != nullptr)<<<g, FS_THREADS, series_smem(most), st>>>(sa, r0);
             tags_note_launch();
             TAGS_CUDA_OK(cudaGetLastError());
         }
@@ -949,10 +960,12 @@ int fields_run(const FieldsIn& in) {
     if (int e = fields_tables(c->device)) return e;
     cudaStream_t st = c->stream;
     const size_t P = in.P, m = in.m, R = in.R, S = in.S;
-    const size_t per_sample = sizeof(double2) * (4 * R * m + P * R * 7 + 2);
+    const SerGeo geo = series_geo(in.points, P, reinterpret_cast<const Seg*>(in.elec), m);
+    // a table of e^{-gamma b h} where the pairs are no fewer than its buckets
+    const size_t rows = (size_t)geo.nbk <= P * m ? (size_t)geo.nbk : 0;
+    const size_t per_sample = sizeof(double2) * (4 * R * m + P * R * 7 + 2 + FS_NT + rows) + sizeof(int);
     const size_t cs = chunk_samples(S, per_sample);
     // samples of the moment series, and those past its reach
-    const SerGeo geo = series_geo(in.points, P, reinterpret_cast<const Seg*>(in.elec), m);
     std::vector<int> nt(S);
     for (size_t k = 0; k < S; ++k) nt[k] = series_terms(geo, zd(in.gamma[k].re, in.gamma[k].im));
     // a warp of the rule costs the same for one of its samples as for all, so a
@@ -994,7 +1007,7 @@ int fields_run(const FieldsIn& in) {
     Seg* d_el = (Seg*)c->scratch(11, sizeof(Seg) * m + 16);
     double2* d_cur = (double2*)c->scratch(12, sizeof(double2) * 4 * R * m * cs + 16);
     double2* d_out = (double2*)c->scratch(13, sizeof(double2) * 7 * P * R * cs * (1 + parts) + 16);
-    double2* d_gk = (double2*)c->scratch(14, sizeof(double2) * ((2 + FS_NT + (size_t)geo.nbk) * cs) + sizeof(int) * cs + 16);
+    double2* d_gk = (double2*)c->scratch(14, sizeof(double2) * ((2 + FS_NT + rows) * cs) + sizeof(int) * cs + 16);
     if (!d_pts || !d_el || !d_cur || !d_out || !d_gk) return tags_fail(TAGS_E_NOMEM, "device allocation failed");
     TAGS_CUDA_OK(cudaMemcpyAsync(d_pts, in.points, sizeof(double) * 3 * P, cudaMemcpyHostToDevice, st));
     TAGS_CUDA_OK(cudaMemcpyAsync(d_el, in.elec, sizeof(Seg) * m, cudaMemcpyHostToDevice, st));
@@ -1026,20 +1039,20 @@ int fields_run(const FieldsIn& in) {
         FieldArgs& a = sa.f;
         double2* pw = d_gk + 2 * ns;
         double2* tab = pw + (size_t)FS_NT * ns;
-        int* d_nt = reinterpret_cast<int*>(tab + (size_t)geo.nbk * ns);
+        int* d_nt = reinterpret_cast<int*>(tab + rows * ns);
         TAGS_CUDA_OK(cudaMemcpyAsync(d_nt, nt.data() + s0, sizeof(int) * ns, cudaMemcpyHostToDevice, st));
         const int most = *std::max_element(nt.begin() + s0, nt.begin() + s0 + ns);
         for (size_t k = s0; k < s0 + ns; ++k)
             if (nt[k] > 0) sa.ga = std::max(sa.ga, std::abs(zd(in.gamma[k].re, in.gamma[k].im)));
         sa.least = fs_least_order(sa.ga * geo.dmax);
         if (most > 0) {
-            k_fser_tables<<<dim3((unsigned)((ns + 31) / 32), geo.nbk + 1), 32, 0, st>>>(d_gk, d_nt, (int)ns, geo.nbk,
-                                                                                    geo.h, pw, tab);
+            k_fser_tables<<<dim3((unsigned)((ns + 31) / 32), (unsigned)rows + 1), 32, 0, st>>>(
+                d_gk, d_nt, (int)ns, (int)rows, geo.h, pw, tab);
             tags_note_launch();
             TAGS_CUDA_OK(cudaGetLastError());
         }
         sa.pw = pw;
-        sa.tab = tab;
+        sa.tab = rows ? tab : nullptr;
         a.pts = d_pts;
         a.elec = d_el;
         a.cur_t = cur_t;
