@@ -543,6 +543,51 @@ __global__ void k_ldl64_start(const double2* __restrict__ rhs, long long rstride
 // on were off by up to 9e-12, now by up to 2e-14, at the same times.)
 TAGS_D bool settled(double dn, double prev, double xn) { return dn <= 1e-8 * sqrt(prev) * sqrt(xn); }
 
+// The rule's maxima of |Re| + |Im| as the values' upper words, which order as the
+// values do (to 2^-20) and need no FP64 instruction; an infinity or a NaN is at
+// least MAX_BAD. Of the currents' dx and x, then the potentials'.
+constexpr unsigned MAX_BAD = 0x7ff00000u;
+struct Maxima {
+    unsigned v[4] = {0, 0, 0, 0};
+    TAGS_D void take(bool current, double2 d, double2 x) {
+        const unsigned a = (unsigned)__double2hiint(cabs1(d)), c = (unsigned)__double2hiint(cabs1(x));
+        v[0] = max(v[0], current ? a : 0u);
+        v[1] = max(v[1], current ? c : 0u);
+        v[2] = max(v[2], current ? 0u : a);
+        v[3] = max(v[3], current ? 0u : c);
+    }
+    TAGS_D double value(int q) const { return __hiloint2double((int)v[q], 0); }
+    TAGS_D bool bad() const { return max(max(v[0], v[1]), max(v[2], v[3])) >= MAX_BAD; }
+};
+// Over a CTA of W warps; complete in thread 0. Ends with no barrier.
+template <int W>
+TAGS_D void maxima_reduce(Maxima& mx, unsigned (*sm)[W]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const unsigned r = __reduce_max_sync(0xffffffffu, mx.v[q]);
+        if ((threadIdx.x & 31) == 0) sm[q][threadIdx.x >> 5] = r;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        for (int w = 0; w < W; ++w) mx.v[q] = max(mx.v[q], sm[q][w]);
+}
+// What a step's maxima mean after corrections of prev (volts and amperes, updated):
+// 0 go on, 1 settled, 2 to the pivoted LU.
+TAGS_D int step_state(const Maxima& mx, int step, bool last, double* prev) {
+    bool done = true, stuck = last;
+    for (int q = 0; q < 2; ++q) {
+        const double dn = mx.value(2 * q);
+        if (step > 0 && !settled(dn, prev[q], mx.value(2 * q + 1))) {
+            done = false;
+            stuck = stuck || dn > 0.5 * prev[q];
+        }
+        prev[q] = dn;
+    }
+    return mx.bad() ? 2 : step == 0 ? 0 : done ? 1 : stuck ? 2 : 0;
+}
+
 // x += dx and the stopping rule, one CTA per sample. Step 0's correction is x
 // itself. Unknowns below nc are currents. A correction that has not settled and
 // did not halve, or is the last step's, leaves the sample to the pivoted LU.
@@ -551,49 +596,19 @@ __global__ void __launch_bounds__(256) k_ldl64_apply(const double2* __restrict__
                                                      int* __restrict__ conv, double* __restrict__ prev) {
     const int b = blockIdx.x;
     if (!active[b]) return;
-    __shared__ double smx[4][8];
-    double mx[4] = {0.0, 0.0, 0.0, 0.0};                     // dx and x of the currents, of the potentials
-    bool bad = false;
+    __shared__ unsigned smx[4][8];
+    Maxima mx;
     for (int j = threadIdx.x; j < N; j += blockDim.x) {
         const long long o = (long long)N * b + j;
         const double2 d = S0[o], x = cadd(X0[o], d);
         X0[o] = x;
-        const double a = cabs1(d), c = cabs1(x);
-        bad = bad || !isfinite(a) || !isfinite(c);
-        if (j < nc) {
-            mx[0] = fmax(mx[0], a);
-            mx[1] = fmax(mx[1], c);
-        } else {
-            mx[2] = fmax(mx[2], a);
-            mx[3] = fmax(mx[3], c);
-        }
+        mx.take(j < nc, d, x);
     }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        for (int o = 16; o > 0; o >>= 1) mx[q] = fmax(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], o));
-        if ((threadIdx.x & 31) == 0) smx[q][threadIdx.x >> 5] = mx[q];
-    }
-    const int anybad = __syncthreads_or(bad);
+    maxima_reduce<8>(mx, smx);
     if (threadIdx.x != 0) return;
-    for (int w = 1; w < 8; ++w)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) mx[q] = fmax(mx[q], smx[q][w]);
-    if (anybad) {
-        active[b] = 0;
-        return;
-    }
-    if (step > 0) {
-        bool done = true, stuck = last != 0;
-        for (int q = 0; q < 2; ++q)
-            if (!settled(mx[2 * q], prev[2 * b + q], mx[2 * q + 1])) {
-                done = false;
-                stuck = stuck || mx[2 * q] > 0.5 * prev[2 * b + q];
-            }
-        if (done) conv[b] = 1;
-        if (done || stuck) active[b] = 0;
-    }
-    prev[2 * b] = mx[0];
-    prev[2 * b + 1] = mx[2];
+    const int state = step_state(mx, step, last != 0, prev + 2 * b);
+    if (state == 1) conv[b] = 1;
+    if (state != 0) active[b] = 0;
 }
 
 // Solutions to the original order; info 0, or the marker of a sample that
@@ -709,7 +724,7 @@ __global__ void __launch_bounds__(128) k_ldl64_small(const double2* __restrict__
     double2* A = reinterpret_cast<double2*>(smem_raw);     // (r, c) at c P + r
     double2* bv = A + (size_t)N * P;
     double2 *x = bv + N, *r = x + N, *dinv = r + N, *z = dinv + N;
-    __shared__ double smx[4][4];
+    __shared__ unsigned smx[4][4];
     __shared__ int sstate;                                  // 0: go on, 1: done, 2: to the pivoted LU
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const double2* W = W0 + stride * b;
@@ -789,40 +804,14 @@ __global__ void __launch_bounds__(128) k_ldl64_small(const double2* __restrict__
             }
         }
         __syncthreads();
-        double mx[4] = {0.0, 0.0, 0.0, 0.0};                 // dx and x of the currents, of the potentials
-        bool bad = false;
+        Maxima mx;
         for (int i = tid; i < N; i += 128) {
             const double2 d = z[i], v = cadd(x[i], d);
             x[i] = v;
-            bad = bad || !isfinite(cabs1(d)) || !isfinite(cabs1(v));
-            if (i < 2 * m) {
-                mx[0] = fmax(mx[0], cabs1(d));
-                mx[1] = fmax(mx[1], cabs1(v));
-            } else {
-                mx[2] = fmax(mx[2], cabs1(d));
-                mx[3] = fmax(mx[3], cabs1(v));
-            }
+            mx.take(i < 2 * m, d, v);
         }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            for (int o = 16; o > 0; o >>= 1) mx[q] = fmax(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], o));
-            if (lane == 0) smx[q][warp] = mx[q];
-        }
-        const int anybad = __syncthreads_or(bad);
-        if (tid == 0) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) mx[q] = fmax(fmax(smx[q][0], smx[q][1]), fmax(smx[q][2], smx[q][3]));
-            bool done = true, stuck = step == 3;
-#pragma unroll
-            for (int q = 0; q < 2; ++q)
-                if (!settled(mx[2 * q], prev[q], mx[2 * q + 1])) {
-                    done = false;
-                    stuck = stuck || mx[2 * q] > 0.5 * prev[q];
-                }
-            sstate = anybad ? 2 : step == 0 ? 0 : done ? 1 : stuck ? 2 : 0;
-            prev[0] = mx[0];
-            prev[1] = mx[2];
-        }
+        maxima_reduce<4>(mx, smx);
+        if (tid == 0) sstate = step_state(mx, step, step == 3, prev);
         __syncthreads();
         if (sstate) break;
     }
@@ -860,8 +849,11 @@ __global__ void __launch_bounds__(128) k_ldl64_resid_full(const double2* __restr
     if (ip >= N) return;
     const double2* row = W + (long long)N * orig_index(ip, m, n);
     double2 cur = cz(0.0, 0.0), pot = cz(0.0, 0.0);
-    for (int j = lane; j < 2 * m; j += 32) cur = cfma(row[n + j], X[j], cur);
-    for (int j = lane; j < n; j += 32) pot = cfma(row[j], X[2 * m + j], pot);
+    for (int j = lane; j < N; j += 32) {
+        const double2 w = row[orig_index(j, m, n)], x = X[j];
+        if (j < 2 * m) cur = cfma(w, x, cur);
+        else pot = cfma(w, x, pot);
+    }
     for (int o = 16; o > 0; o >>= 1) {
         cur.x += __shfl_xor_sync(0xffffffffu, cur.x, o);
         cur.y += __shfl_xor_sync(0xffffffffu, cur.y, o);
