@@ -214,3 +214,30 @@ def test_samples_beside_an_invalid_one_are_solved(gpu_pkg, m, value, kappa_value
             assert rel_err(out[0][0][good], want) < 1e-10
     finally:
         pkg.lib().tags_gpu_set_quiet(0)
+
+
+@pytest.mark.parametrize("gap", [0.0, 700.0])
+def test_plain_plans_keep_to_the_share_of_memory_they_size_for(gpu_pkg, gap):
+    """Plans take at most 0.45 of the free memory for their samples and grid batches 0.6, the fill's tables included,
+    which for two segments far apart are 16 KB a sample beside a matrix of 1 KB."""
+    torch = pytest.importorskip("torch")
+    pkg = gpu_pkg
+    ends = [((gap * i, 0.3 * i, -0.5), (gap * i, 0.3 * i, -1.5)) for i in range(2)]
+    e = np.stack([pkg.populate_electrode(a, b, 7e-3) for a, b in ends])
+    nodes = np.array([p for pair in ends for p in pair])
+    s, budget = 8e4 + 2j * np.pi * np.linspace(1e3, 1e5, 60000), 1 << 30
+    kappa = np.full(len(s), 0.01 + 1e-4j)
+    jobs = [{"electrodes": e, "images": pkg.images(e), "nodes": nodes, "s": s, "kappa": kappa, "inj_node": 0}]
+    pkg.hem_sweep(e, pkg.images(e), nodes, s[:2], kappa[:2])
+    pkg.set_memory_budget(budget)
+    try:
+        for share, make in ((0.45, lambda: pkg.Plan(e, pkg.images(e), nodes, pkg.PLAIN_FP64, 60000)),
+                            (0.60, lambda: pkg.GridBatch(jobs, precision=pkg.PLAIN_FP64, max_batch=60000))):
+            before = torch.cuda.mem_get_info()[0]
+            held = make()
+            try:
+                assert before - torch.cuda.mem_get_info()[0] <= share * budget + (24 << 20)
+            finally:
+                held.close()
+    finally:
+        pkg.set_memory_budget(0)

@@ -1200,16 +1200,6 @@ extern "C" int tags_voltage_batch(const double* paths, size_t num_paths, const E
     if (!c) return tags_fail(TAGS_E_CUDA, "no usable CUDA device");
     if (int e = fields_tables(c->device)) return e;
     cudaStream_t st = c->stream;
-    const size_t cs =
-        std::min<size_t>(65535, chunk_samples(S, sizeof(double2) * (2 * R * m + NL * m + 3 * NL * R + 4)));
-    Seg* d_el = (Seg*)c->scratch(11, sizeof(Seg) * (m + NL) + 16);
-    double* d_paths = (double*)c->scratch(10, sizeof(double) * 6 * NL + 16);
-    double2* d_cur = (double2*)c->scratch(12, sizeof(double2) * 2 * R * m * cs + 16);
-    double2* d_jj = (double2*)c->scratch(13, sizeof(double2) * (NL * m + 3 * NL * R) * cs + 16);
-    double2* d_gk = (double2*)c->scratch(14, sizeof(double2) * 3 * cs + 16);
-    SampleCoef* d_coef = (SampleCoef*)c->scratch(15, sizeof(SampleCoef) * cs + 16);
-    if (!d_el || !d_paths || !d_cur || !d_jj || !d_gk || !d_coef)
-        return tags_fail(TAGS_E_NOMEM, "device allocation failed");
     // paths as segment records after the electrodes (radius 0)
     std::vector<Seg> segs(m + NL);
     if (m) memcpy(segs.data(), electrodes, sizeof(Seg) * m);
@@ -1227,6 +1217,16 @@ extern "C" int tags_voltage_batch(const double* paths, size_t num_paths, const E
         g.radius = 0.0;
     }
     const SeriesGeo geo = tags_series_geometry(segs[0].a, (int)(m + NL), nullptr, 0);
+    const size_t cs = std::min<size_t>(65535, chunk_samples(S, sizeof(double2) * (2 * R * m + NL * m + 3 * NL * R + 4) +
+                                                                   tags_series_workspace(geo, 1)));
+    Seg* d_el = (Seg*)c->scratch(11, sizeof(Seg) * (m + NL) + 16);
+    double* d_paths = (double*)c->scratch(10, sizeof(double) * 6 * NL + 16);
+    double2* d_cur = (double2*)c->scratch(12, sizeof(double2) * 2 * R * m * cs + 16);
+    double2* d_jj = (double2*)c->scratch(13, sizeof(double2) * (NL * m + 3 * NL * R) * cs + 16);
+    double2* d_gk = (double2*)c->scratch(14, sizeof(double2) * 3 * cs + 16);
+    SampleCoef* d_coef = (SampleCoef*)c->scratch(15, sizeof(SampleCoef) * cs + 16);
+    if (!d_el || !d_paths || !d_cur || !d_jj || !d_gk || !d_coef)
+        return tags_fail(TAGS_E_NOMEM, "device allocation failed");
     void* series = geo.nbk ? c->scratch(16, tags_series_workspace(geo, (int)cs)) : nullptr;
     TAGS_CUDA_OK(cudaMemcpyAsync(d_el, segs.data(), sizeof(Seg) * (m + NL), cudaMemcpyHostToDevice, st));
     TAGS_CUDA_OK(cudaMemcpyAsync(d_paths, paths, sizeof(double) * 6 * NL, cudaMemcpyHostToDevice, st));

@@ -82,13 +82,16 @@ static void batch_free(tags_batch_s* b) {
     delete b;
 }
 
-// Device bytes one resident sample of a plan needs (the estimate plan
+// Device bytes one resident sample of a job's plan needs (the estimate plan
 // creation uses to size its batch).
-static double bytes_per_sample(int m, int n, int precision) {
-    const double N = (double)n + 2.0 * m, NN = N * N;
-    return precision == TAGS_PLAIN_FP64 ? 16.0 * NN + 40.0 * N + (double)tags_ldl64_workspace((int)N, 1)
-                                        : 8.0 * NN + 32.0 * (double)m * m + 80.0 * N +
-                                              (double)tags_ldl_tc_workspace((int)N, 1);
+static double bytes_per_sample(const tags_grid_job& j, int precision) {
+    const int m = (int)j.num_electrodes, N = (int)j.num_nodes + 2 * m;
+    const double NN = (double)N * N;
+    if (precision != TAGS_PLAIN_FP64)
+        return 8.0 * NN + 32.0 * (double)m * m + 80.0 * N + (double)tags_ldl_tc_workspace(N, 1);
+    const SeriesGeo geo = tags_series_geometry(reinterpret_cast<const double*>(j.electrodes), m,
+                                               reinterpret_cast<const double*>(j.images), j.images ? m : 0);
+    return 16.0 * NN + 40.0 * N + (double)tags_ldl64_workspace(N, 1) + (double)tags_series_workspace(geo, 1);
 }
 
 // One capture of every grid's passes (see the file comment).
@@ -228,7 +231,7 @@ extern "C" int tags_batch_create(tags_batch* out, const tags_grid_job* jobs, siz
         const tags_grid_job& j = jobs[q];
         const double N = (double)j.num_nodes + 2.0 * j.num_electrodes;
         io += (double)j.ns * (16.0 * (N + 2.0 + (j.ie ? (double)j.num_nodes : 0.0)) + 4.0);
-        per[q] = bytes_per_sample((int)j.num_electrodes, (int)j.num_nodes, precision);
+        per[q] = bytes_per_sample(j, precision);
         res[q] = (long long)std::min<size_t>(j.ns, max_batch ? max_batch : 256);
     }
     const double budget = 0.6 * (double)freeb - io;

@@ -239,8 +239,11 @@ extern "C" int tags_plan_create(tags_plan* out, const Electrode* electrodes, con
     size_t freeb = 0;
     PLAN_CHECK(tags_free_memory(&freeb));
     const double NN = (double)N * (double)N;
+    if (precision == TAGS_PLAIN_FP64)
+        p->series = tags_series_geometry(p->h_elec.data(), p->m, p->h_img.data(), p->h_img.empty() ? 0 : p->m);
     double per = precision == TAGS_PLAIN_FP64
-                     ? 16.0 * NN + 40.0 * N + (double)tags_ldl64_workspace((int)N, 1)
+                     ? 16.0 * NN + 40.0 * N + (double)tags_ldl64_workspace((int)N, 1) +
+                           (double)tags_series_workspace(p->series, 1)
                      : 8.0 * NN + 32.0 * (double)p->m * p->m + 80.0 * N + (double)tags_ldl_tc_workspace((int)N, 1);
     long long cap = (long long)(0.45 * (double)freeb / per);
     long long b = max_batch ? (long long)max_batch : std::min<long long>(cap, 64);
@@ -254,7 +257,6 @@ extern "C" int tags_plan_create(tags_plan* out, const Electrode* electrodes, con
     if (precision == TAGS_PLAIN_FP64) {
         // one allocation: matrices, LDL^T workspace, the fill series' tables
         const size_t wb = sizeof(double2) * (size_t)NN * b, lb = (tags_ldl64_workspace(p->N, p->batch) + 255) / 256 * 256;
-        p->series = tags_series_geometry(p->h_elec.data(), p->m, p->h_img.data(), p->h_img.empty() ? 0 : p->m);
         PLAN_CHECK(cudaMalloc(&p->d_W, wb + lb + tags_series_workspace(p->series, p->batch)));
         p->d_ldl64 = reinterpret_cast<char*>(p->d_W) + wb;
         if (p->series.nbk) {
