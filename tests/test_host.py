@@ -275,6 +275,24 @@ def test_trailing_tile_list_leaves_out_the_zero_band(pkg):
     assert fn(-1, 0, 0, 0, 0, None, 0) == pkg.E_ARG
 
 
+def test_kernel_attributes_are_set_on_each_device():
+    """cudaFuncSetAttribute holds for the device that is current, so a process-wide once_flag around it leaves a second
+    device without: every such call is in a function that the per-device helper, or the per-device tables of the fields,
+    run. (One GPU at a time is at hand, so the sources are what can be checked.)"""
+    csrc = os.path.join(ROOT, "transient-analysis-grounding-systems_gb300", "csrc")
+    found = 0
+    for name in sorted(os.listdir(csrc)):
+        with open(os.path.join(csrc, name)) as f:
+            text = f.read()
+        if "cudaFuncSetAttribute(" not in text:
+            continue
+        found += 1
+        assert "tags_once_per_device(" in text or "g_tables_ready[dev]" in text, name
+        for body in re.findall(r"call_once\(.*?\n    \}\);", text, re.S):
+            assert "cudaFuncSetAttribute" not in body and "_attr<" not in body, name
+    assert found >= 5
+
+
 def test_bench_reference_arm_contract():
     """`bench.py --impl reference` (the CPU implementation of the path on the
     host cores) prints one JSON line carrying the bench contract's keys, with

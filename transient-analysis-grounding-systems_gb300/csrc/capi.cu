@@ -75,6 +75,16 @@ void tags_msg(const char* msg) {
 
 // ---- per-device context ------------------------------------------------------
 
+int tags_once_per_device(PerDevice& state, int (*setup)()) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return tags_fail(TAGS_E_CUDA, "no usable CUDA device");
+    std::lock_guard<std::mutex> lk(state.mu);
+    if (state.done[dev]) return 0;
+    const int err = setup();
+    state.done[dev] = err == 0;
+    return err;
+}
+
 DeviceCtx* tags_ctx() {
     static DeviceCtx ctxs[64];
     int dev = 0;

@@ -15,8 +15,6 @@
 // length that fits shared memory; the sums are radix by radix, so they are
 // shorter than the direct ones (nt = 4094: 2 + 23 + 89 terms instead of 2047)
 // and no less accurate.
-#include <mutex>
-
 #include "tags_common.cuh"
 #include "tags_internal.h"
 #include "../../include/tags_gpu.h"
@@ -367,14 +365,14 @@ int tags_launch_inlt(const double2* d_g, long long gseries, long long gk, const 
     const double c_fft = ceil(pairs / 152.0) * (double)nt * (5.0 * sum + 6.0 * FFT_LOW) / 2.0;
     const double c_direct = (double)nser * (double)nt * (double)ns * 3.0 / (2.0 * 152.0);
     if (nt <= FFT_NT_MAX && nt > 2 && c_fft < c_direct) {
-        static std::once_flag once;
-        static int rc = 0;
-        std::call_once(once, [] {
+        static PerDevice state;
+        const int err = tags_once_per_device(state, [] {
             if (cudaFuncSetAttribute(k_inlt_fft, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)(2 * FFT_NT_MAX * sizeof(double2))) != cudaSuccess)
-                rc = tags_fail(TAGS_E_CUDA, "cudaFuncSetAttribute(k_inlt_fft) failed");
+                return tags_fail(TAGS_E_CUDA, "cudaFuncSetAttribute(k_inlt_fft) failed");
+            return 0;
         });
-        if (rc) return rc;
+        if (err) return err;
         k_inlt_fft<<<(unsigned)((nser + 1) / 2), FFT_THREADS, 2 * sizeof(double2) * nt, st>>>(
             d_g, gseries, gk, sigma, scale, tw, (int)nt, plan, d_f, fseries, fj, nser);
         tags_note_launch();

@@ -27,7 +27,6 @@
 // workspace, so that a solve's diagonal step is a product (every CTA of a panel
 // launch factors the block itself, which saves a launch per panel).
 #include <algorithm>
-#include <mutex>
 
 #include "tags_common.cuh"
 #include "tags_internal.h"
@@ -1163,10 +1162,10 @@ constexpr int MAX_CORRECTIONS = 4;         // x itself and up to three refinemen
 
 }  // namespace
 
+// Kernel attributes, once per device, before any launch and any graph capture.
 int tags_ldl64_prepare() {
-    static std::once_flag once;
-    static int rc = 0;
-    std::call_once(once, [] {
+    static PerDevice state;
+    return tags_once_per_device(state, [] {
         if (cudaFuncSetAttribute(k_ldl64_mcols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MCOLS_SMEM) !=
                 cudaSuccess ||
             cudaFuncSetAttribute(k_ldl64_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1177,9 +1176,9 @@ int tags_ldl64_prepare() {
                                  (int)(6 * PB * 32 * sizeof(double))) != cudaSuccess ||
             cudaFuncSetAttribute(k_ldl64_solve_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(SOLVE_N_MAX * sizeof(double2))) != cudaSuccess)
-            rc = tags_fail(TAGS_E_CUDA, "cudaFuncSetAttribute(k_ldl64) failed");
+            return tags_fail(TAGS_E_CUDA, "cudaFuncSetAttribute(k_ldl64) failed");
+        return 0;
     });
-    return rc;
 }
 
 size_t tags_ldl64_workspace(int N, int batch) {

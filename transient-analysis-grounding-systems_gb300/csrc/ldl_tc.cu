@@ -1911,13 +1911,12 @@ static int launch_solve_cl(const float2* A, long long ld, long long mstride, int
     return 0;
 }
 
-// Kernel attributes and the tensor-map encoder, set once per process before
+// Kernel attributes and the tensor-map encoder, set once per device before
 // any launch (and so before any graph capture).
 int tags_ldl_tc_prepare() {
-    static std::once_flag once;
-    static int rc = 0;
-    std::call_once(once, [] {
-        rc = set_gemm_attr<2, 0>();
+    static PerDevice state;
+    return tags_once_per_device(state, [] {
+        int rc = set_gemm_attr<2, 0>();
         if (!rc) rc = set_gemm_attr<2, 1>();
         if (!rc) rc = set_gemm_attr<3, 0>();
         if (!rc) rc = set_gemm_attr<3, 1>();
@@ -1935,8 +1934,8 @@ int tags_ldl_tc_prepare() {
         if (!rc) rc = set_solve_cl_attr<8>();
         if (!rc) rc = set_solve_cl_attr<16>();
         if (!rc && !encode_fn()) rc = tags_fail(TAGS_E_CUDA, "cuTensorMapEncodeTiled is not available");
+        return rc;
     });
-    return rc;
 }
 
 template <int S, int MODE>

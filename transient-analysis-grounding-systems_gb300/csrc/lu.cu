@@ -10,8 +10,6 @@
 //
 // Layout: column-major, leading dimension ld, one matrix per blockIdx.z
 // (pointer + z * stride). ipiv is 0-based global row indices.
-#include <mutex>
-
 #include "tags_common.cuh"
 #include "tags_internal.h"
 #include "../../include/tags_gpu.h"
@@ -310,18 +308,17 @@ constexpr int NB = 32;
 
 }  // namespace
 
-// Kernel attributes of the LU, set once per process before any launch (and
-// so before any graph capture).
+// Kernel attributes of the LU, set once per device before any launch (and so
+// before any graph capture).
 int tags_lu_prepare() {
-    static std::once_flag once;
-    static int rc = 0;
-    std::call_once(once, [] {
+    static PerDevice state;
+    return tags_once_per_device(state, [] {
         const int g64 = (int)(2 * NB * 64 * sizeof(double2));
         if (cudaFuncSetAttribute(k_gemm_update<double2, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, g64) !=
             cudaSuccess)
-            rc = tags_fail(TAGS_E_CUDA, "cudaFuncSetAttribute(k_gemm_update) failed");
+            return tags_fail(TAGS_E_CUDA, "cudaFuncSetAttribute(k_gemm_update) failed");
+        return 0;
     });
-    return rc;
 }
 
 namespace {

@@ -6,6 +6,8 @@
 #include <nvtx3/nvToolsExt.h>
 #include <stdint.h>
 
+#include <mutex>
+
 // NVTX range over a host-side phase (fill, assemble, factor, refine, FP64
 // re-solve, INLT, a pass or a grid batch): pushed on construction, popped on
 // destruction. NVTX 3 is header-only; with no tool attached a push and a pop
@@ -105,6 +107,14 @@ int tags_launch_fill_mixed(const double* d_elec, const double* d_img, int m, voi
                            int nsamp, float2* d_zl, float2* d_zt, float2* d_zlo, float2* d_ztlo, long long bstride,
                            int has_img, const SpecialEntries& sp, const MomentFill& mf, int* d_status,
                            cudaStream_t st, float* rowpart = nullptr);
+// Runs setup once on each device (the calling thread's), not once in the process:
+// kernel attributes hold for the device that is current when they are set. A
+// setup that fails is run again by the next call.
+struct PerDevice {
+    std::mutex mu;
+    bool done[64] = {};
+};
+int tags_once_per_device(PerDevice& state, int (*setup)());
 // Geometry of the FP64 moment series over segment records (11 doubles each, on
 // the host): with it and a workspace for the samples of the launch, the
 // INTG_DOUBLE fill and the path integrals take their samples from per-launch
