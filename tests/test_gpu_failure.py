@@ -241,3 +241,25 @@ def test_plain_plans_keep_to_the_share_of_memory_they_size_for(gpu_pkg, gap):
                 held.close()
     finally:
         pkg.set_memory_budget(0)
+
+
+def test_path_voltages_without_room_for_their_tables(gpu_pkg):
+    """With too little device memory left for the pair integrals' tables (0.66 GB here) the call takes the rule per
+    sample, which needs none: the same voltages to the two rules' agreement of 1e-12, not an allocation error."""
+    torch = pytest.importorskip("torch")
+    pkg = gpu_pkg
+    e = np.stack([pkg.populate_electrode([700.0 * i, 0, -0.5], [700.0 * i, 0, -1.5], 7e-3) for i in range(2)])
+    ns = 40000
+    cur = np.ones((ns, 1, 2), np.complex128)
+    args = (np.array([[5.0, 1, 0, 6.0, 1, 0]]), e, cur, cur, np.full(ns, 0.01 + 0.01j), np.full(ns, 1e5j),
+            np.ones(ns, np.complex128))
+    few = [a if k < 2 else a[:3] for k, a in enumerate(args)]
+    want = pkg.voltage_batch(*few)
+    torch.cuda.empty_cache()
+    held = torch.empty(torch.cuda.mem_get_info()[0] - (400 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        got = pkg.voltage_batch(*args)
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    assert rel_err(got, np.broadcast_to(want[:1], got.shape)) < 1e-12

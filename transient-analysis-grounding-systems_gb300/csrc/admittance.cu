@@ -123,10 +123,7 @@ int yla_ytb_ldl(tags_cdouble* yla, tags_cdouble* ytb, tags_cdouble* zl, tags_cdo
     double2* d_Z = (double2*)c->scratch(6, sizeof(double2) * (2 * mm + 2 * mn + 1));
     double2* d_X = (double2*)c->scratch(7, sizeof(double2) * 2 * m * (n + m));
     void* ws = c->scratch(18, tags_ldl64_multi_workspace((int)m));
-    if (!d_Z || !d_X || !ws) {
-        cudaGetLastError();                                // no room: the LU needs less
-        return 0;
-    }
+    if (!d_Z || !d_X || !ws) return 0;                     // no room: the LU needs less
     double2* d_rhs = d_Z + 2 * mm;
     TAGS_CUDA_OK(cudaMemcpyAsync(d_Z, zl, sizeof(double2) * mm, cudaMemcpyHostToDevice, st));
     TAGS_CUDA_OK(cudaMemcpyAsync(d_Z + mm, zt, sizeof(double2) * mm, cudaMemcpyHostToDevice, st));

@@ -100,14 +100,20 @@ DeviceCtx* tags_ctx() {
     return &c;
 }
 
-// Grow-only device scratch owned by the context.
+// Grow-only device scratch owned by the context. Null where there is no room: the
+// caller reports that or goes on without, so the error does not stay behind for
+// the check of its next launch.
 void* DeviceCtx::scratch(int slot, size_t bytes) {
     if (bytes == 0) bytes = 16;
     if (scratch_bytes[slot] < bytes) {
         if (scratch_ptr[slot]) cudaFree(scratch_ptr[slot]);
         scratch_ptr[slot] = nullptr;
         scratch_bytes[slot] = 0;
-        if (cudaMalloc(&scratch_ptr[slot], bytes) != cudaSuccess) return nullptr;
+        if (cudaMalloc(&scratch_ptr[slot], bytes) != cudaSuccess) {
+            cudaGetLastError();
+            scratch_ptr[slot] = nullptr;
+            return nullptr;
+        }
         scratch_bytes[slot] = bytes;
     }
     return scratch_ptr[slot];
@@ -363,10 +369,7 @@ int tags_sym_solve_host(const tags_cdouble* w, tags_cdouble* x, size_t m, size_t
     double2* d_A = (double2*)c->scratch(17, sizeof(double2) * N * N);
     double2* d_x = (double2*)c->scratch(4, sizeof(double2) * N);
     void* ws = c->scratch(18, tags_ldl64_workspace((int)N, 1));
-    if (!d_W || !d_A || !d_x || !ws) {
-        cudaGetLastError();                              // no room for two matrices: the LU needs one
-        return 0;
-    }
+    if (!d_W || !d_A || !d_x || !ws) return 0;           // no room for two matrices: the LU needs one
     TAGS_CUDA_OK(cudaMemcpyAsync(d_W, w, sizeof(double2) * N * N, cudaMemcpyHostToDevice, st));
     TAGS_CUDA_OK(cudaMemcpyAsync(d_x, x, sizeof(double2) * N, cudaMemcpyHostToDevice, st));
     int err = tags_symmetrize_lower(d_W, (int)N, (long long)N, 0, 1, st);
