@@ -263,3 +263,31 @@ def test_path_voltages_without_room_for_their_tables(gpu_pkg):
         del held
         torch.cuda.empty_cache()
     assert rel_err(got, np.broadcast_to(want[:1], got.shape)) < 1e-12
+
+
+def test_resolves_buffer_grows_and_stays_when_it_cannot(gpu_pkg):
+    """The FP64 re-solves' buffer of a plan: taken for one sample, grown for more, and, with no device memory for a larger
+    one, kept as it is; the same solutions each time."""
+    torch = pytest.importorskip("torch")
+    pkg = gpu_pkg
+    m, ns = 250, 40                             # 9 MB a sample
+    e, nodes = pkg.segment_electrode([0.0, 0.0, -0.5], [1.0 * m, 0.0, -0.5], m, 7e-3)
+    s = 8e4 + 2j * np.pi * np.linspace(1e4, 5e6, ns)
+    kappa = 0.004 + s * 10 * pkg.EPS0
+    want, info, _ = pkg.hem_sweep(e, pkg.images(e), nodes, s, kappa, inj_node=1)
+    plan = pkg.Plan(e, pkg.images(e), nodes, pkg.MIXED, ns)
+    held = []
+    try:
+        plan.set_max_steps(1)
+        for take in (1, 3, 12, ns):
+            plan.run(s[:take], kappa[:take], inj_node=1)          # the pass's graph is built here
+            if take == 12:
+                torch.cuda.empty_cache()
+                held.append(torch.empty(torch.cuda.mem_get_info()[0] - (64 << 20), dtype=torch.uint8, device="cuda"))
+            sol, info, st = plan.run(s[:take], kappa[:take], inj_node=1)
+            assert st.fallbacks == take and not info.any()
+            assert np.max(np.abs(sol - want[:take])) < 1e-10 * np.max(np.abs(want))
+    finally:
+        plan.close()
+        held.clear()
+        torch.cuda.empty_cache()

@@ -380,10 +380,13 @@ extern "C" int tags_batch_run(tags_batch batch, const tags_grid_job* jobs, size_
                 }
             }
             // queued on the grid's own stream: the grids' re-solves, chains of
-            // small launches, run side by side
+            // small launches, run side by side. Their buffers stay with the batch,
+            // 2 GB between the grids (or one sample each).
             if (!failed[q].empty())
                 if (int e = tags_mixed_fallback_start(p, failed[q], g.d_s, g.d_k, b->mur, g.has_ie ? g.d_ie : nullptr,
-                                                      (int)g.inj, g.d_sol, g.d_info, p->stream))
+                                                      (int)g.inj, g.d_sol, g.d_info,
+                                                      std::min<size_t>((size_t)512 << 20, ((size_t)2 << 30) / njobs),
+                                                      p->stream))
                     return e;
         }
     }

@@ -702,32 +702,31 @@ size_t fb_bytes(const tags_plan_s* p, int cap, FbView* v) {
     return o;
 }
 
-// Room for up to `want` samples at a time: at most 64, 512 MB and an eighth of
-// the free memory, at least one. Kept with the plan, grown when more is asked.
-int fb_alloc(tags_plan_s* p, int want) {
+// Room for up to `want` samples at a time: at most 64, `most` bytes and an eighth
+// of the free memory, at least one. Kept with the plan, grown when more is asked;
+// the buffer that is there goes only when the larger one has been had.
+int fb_alloc(tags_plan_s* p, int want, size_t most) {
     want = std::min(want, 64);
     if (p->fb_cap >= want || (p->fb_cap > 0 && p->fb_full)) return 0;
     if (p->series.nbk == 0)
         p->series = tags_series_geometry(p->h_elec.data(), p->m, p->h_img.data(), p->h_img.empty() ? 0 : p->m);
     size_t freeb = 0;
     TAGS_CUDA_OK(tags_free_memory(&freeb));
-    const size_t one = fb_bytes(p, 1, nullptr), most = std::min<size_t>((size_t)512 << 20, freeb / 8);
-    const int cap = (int)std::max<size_t>(1, std::min<size_t>((size_t)want, most / one));
-    if (cap <= p->fb_cap) {
+    const size_t one = fb_bytes(p, 1, nullptr);
+    int cap = (int)std::max<size_t>(1, std::min<size_t>((size_t)want, std::min(most, freeb / 8) / one));
+    void* buf = nullptr;
+    for (; cap > p->fb_cap; cap /= 2) {
+        if (cudaMalloc(&buf, fb_bytes(p, cap, nullptr)) == cudaSuccess) break;
+        cudaGetLastError();
+        buf = nullptr;
+    }
+    if (!buf) {
         p->fb_full = 1;
-        return 0;
+        return p->fb_cap > 0 ? 0 : tags_fail(TAGS_E_NOMEM, "device allocation failed (FP64 fallback)");
     }
     if (p->d_fb) {
         TAGS_CUDA_OK(cudaStreamSynchronize(p->stream));
         TAGS_CUDA_OK(cudaFree(p->d_fb));
-        p->d_fb = nullptr;
-        p->d_series = nullptr;
-        p->series_ns = p->fb_cap = 0;
-    }
-    void* buf = nullptr;
-    if (cudaMalloc(&buf, fb_bytes(p, cap, nullptr)) != cudaSuccess) {
-        cudaGetLastError();
-        return tags_fail(TAGS_E_NOMEM, "device allocation failed (FP64 fallback)");
     }
     p->d_fb = buf;
     p->fb_cap = cap;
@@ -761,7 +760,7 @@ int fb_solve(tags_plan_s* p, const FbView& v, int nf, double2* x, int* info, cud
 static int fallback_plain(tags_plan_s* p, const std::vector<int>& idx, cudaStream_t st) {
     TagsRange range("tags FP64 re-solve");
     const size_t N = p->N;
-    if (int e = fb_alloc(p, (int)idx.size())) return e;
+    if (int e = fb_alloc(p, (int)idx.size(), (size_t)512 << 20)) return e;
     FbView v;
     fb_bytes(p, p->fb_cap, &v);
     const double2* bvec = p->d_r + (size_t)p->batch * N;
@@ -787,9 +786,10 @@ int tags_plan_rhs(tags_plan_s* p, double2* d_X, const double2* d_ie, int inj_nod
 int tags_plan_coef(tags_plan_s* p, const double2* d_s, const double2* d_kappa, double mur, int nb, cudaStream_t st);
 
 int tags_mixed_fallback_start(tags_plan_s* p, const std::vector<int>& idx, const double2* d_s, const double2* d_kappa,
-                              double mur, const double2* d_ie, int inj_node, double2* x, int* info, cudaStream_t st) {
+                              double mur, const double2* d_ie, int inj_node, double2* x, int* info, size_t most,
+                              cudaStream_t st) {
     const size_t N = p->N;
-    if (int e = fb_alloc(p, (int)idx.size())) return e;
+    if (int e = fb_alloc(p, (int)idx.size(), most)) return e;
     FbView v;
     fb_bytes(p, p->fb_cap, &v);
     for (size_t k0 = 0; k0 < idx.size(); k0 += std::min(p->fb_cap, p->batch)) {

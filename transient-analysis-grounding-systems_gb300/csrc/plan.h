@@ -135,10 +135,12 @@ int tags_mixed_ir_step(tags_plan_s* p, int nb, cudaStream_t st, cudaGraphConditi
 int tags_mixed_finish(tags_plan_s* p, int nb, cudaStream_t st, int* h_iters, double* h_berr, int* h_conv,
                       int* h_steps);
 // Plain FP64 re-solves of samples idx of a sweep (inputs and outputs on the
-// device, sample by sample), queued on st; info TAGS_INFO_RESOLVE asks for
-// tags_mixed_fallback_lu of that sample (its own inputs and outputs).
+// device, sample by sample), queued on st, as many at a time as `most` bytes
+// hold; info TAGS_INFO_RESOLVE asks for tags_mixed_fallback_lu of that sample
+// (its own inputs and outputs).
 int tags_mixed_fallback_start(tags_plan_s* p, const std::vector<int>& idx, const double2* d_s, const double2* d_kappa,
-                              double mur, const double2* d_ie, int inj_node, double2* x, int* info, cudaStream_t st);
+                              double mur, const double2* d_ie, int inj_node, double2* x, int* info, size_t most,
+                              cudaStream_t st);
 int tags_mixed_fallback_lu(tags_plan_s* p, const double2* d_s, const double2* d_kappa, double mur, const double2* d_ie,
                            int inj_node, double2* x_out, int* info_out, cudaStream_t st);
 // While-node after the work captured so far on `st` (condition 1 at launch);
