@@ -861,7 +861,7 @@ def main():
     ap.add_argument("--panels", type=int, default=0, help="mixed form: panels per trailing update, 1..6 (0 = plan default)")
     ap.add_argument("--split", type=int, default=0, help="mixed-form split: 3 bf16x3, 2 bf16x2, 16 fp16x2 (0 = plan default)")
     ap.add_argument("--solve-path", type=int, default=-1,
-                    help="triangular solves: 0 per block, 1 one CTA per sample, 2/4/8 clusters (-1 = default)")
+                    help="triangular solves: 0 per block, 1 one CTA per sample, 2/4/8/16 clusters (-1 = default)")
     ap.add_argument("--ref-steps", type=int, default=4, help="cap on timed steps of the reference arm")
     ap.add_argument("--first-batch", type=int, default=0,
                     help="batch of samples the warm-up and timed steps start from (0 = the whole job in order)")

@@ -478,13 +478,13 @@ int tags_debug_tri_tiles (int M, int zlo, int zhi, int planes, int planes_band, 
 /* No counterpart in the reference. Test hook (process-wide, for passes and
  * graphs built afterwards): how the mixed form's triangular solves run.
  * 0: block by block (two kernels per 128-row block and sweep); 1: one CTA per
- * sample with x in shared memory; 2, 4, 8: a cluster of that many CTAs per
- * sample, x spread over their shared memory; -1 (default): the largest of
- * 16 and 8 with G x samples per pass <= SMs / 2, else of 4 and 2 with
- * G x samples <= SMs, else one CTA
- * per sample. Paths 1..8
- * need x in shared memory (N up to about 25000) and otherwise run block by
- * block. All form every sum in the same order and give identical results. */
+ * sample with x in shared memory; 2, 4, 8, 16: a cluster of that many CTAs per
+ * sample, x spread over their shared memory (16 is refused where the device has
+ * no room for such a cluster); -1 (default): the largest of 16 and 8 with G x
+ * samples per pass <= SMs / 2, else of 4 and 2 with G x samples <= SMs, else one
+ * CTA per sample. Paths 1..16 need x in shared memory (N up to about 25000) and
+ * otherwise run block by block. All form every sum in the same order and give
+ * identical results. */
 int tags_debug_solve_path (int path);
 
 /* No counterpart in the reference. Caps the refinement steps of the mixed

@@ -144,3 +144,30 @@ def test_solve_paths_are_identical(gpu_pkg, N, zl_m):
         out[path] = x
     for path in (1, 2, 4, 8):
         assert np.array_equal(out[path], out[0]), path
+
+
+@pytest.mark.parametrize("N,zl_m", [(60, 0), (517, 0), (1000, 300), (1500, 400), (2305, 700)])
+@pytest.mark.parametrize("nb", [1, 4, 5, 10])
+def test_solves_on_clusters_of_sixteen_are_identical(gpu_pkg, N, zl_m, nb):
+    """Clusters of 16 CTAs per sample, what the default takes for up to four samples, and the default itself (16, 8 and 4
+    CTAs for these counts) against the solve block by block, three times over: every sum in the same order."""
+    fn = gpu_pkg.lib().tags_debug_ldl_solve
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
+                   ctypes.c_int]
+    fn.restype = ctypes.c_int
+    rng = np.random.default_rng(N + 7 * zl_m)
+    mats = np.stack([_banded_sym(rng, N, zl_m, 3.0 + q % 2) for q in range(nb)])
+    rhs = rng.standard_normal((nb, N)) + 1j * rng.standard_normal((nb, N))
+    flat = np.ascontiguousarray(np.transpose(mats, (0, 2, 1))).astype(np.complex128)
+    out = []
+    for path in (0, 16, -1, 16, -1, 16, -1):
+        buf, x = flat.copy(), rhs.copy()
+        assert gpu_pkg.lib().tags_debug_solve_path(path) == 0
+        try:
+            code = fn(buf.ctypes.data, x.ctypes.data, N, nb, 16, zl_m, 4)
+        finally:
+            gpu_pkg.lib().tags_debug_solve_path(-1)
+        assert code == 0, gpu_pkg.last_error()
+        out.append(x)
+    for x in out[1:]:
+        assert np.array_equal(x, out[0])

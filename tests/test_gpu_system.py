@@ -441,6 +441,31 @@ def test_solve_paths_match_in_plans(gpu_pkg, count, per_pass):
     assert np.max(np.abs(out[0][0][:, 0] - gd["u0"][idx]) / np.abs(gd["u0"][idx])) < 1e-6
 
 
+@pytest.mark.parametrize("per_pass", [1, 2, 4, 5, 9])
+def test_solve_paths_match_in_plans_of_few_samples(gpu_pkg, per_pass):
+    """Passes of 1 to 9 samples, whose solves run on clusters of 16 and 8 CTAs by default, three times over, and of 16
+    throughout: the solutions and refinement counts of one CTA per sample, bit for bit, and no sample re-solved."""
+    pkg = gpu_pkg
+    gd = golden("grid2.npz")
+    e, nodes = gd["elec"], gd["nodes"]
+    idx = np.linspace(0, len(gd["s"]) - 1, 2 * per_pass + 1).astype(int)
+    s, kappa = gd["s"][idx], gd["kappa"][idx]
+    ie = np.zeros((len(idx), nodes.shape[0]), np.complex128)
+    ie[:, 0] = gd["inj_s"][idx]
+    out = []
+    for path in (1, -1, -1, -1, 16):
+        assert pkg.lib().tags_debug_solve_path(path) == 0
+        try:
+            sol, info, st = pkg.hem_sweep(e, pkg.images(e), nodes, s, kappa, ie=ie, precision=pkg.MIXED,
+                                          max_batch=per_pass)
+        finally:
+            pkg.lib().tags_debug_solve_path(-1)
+        assert np.all(info == 0) and st.fallbacks == 0
+        out.append((sol, st.max_iterations))
+    for sol, it in out[1:]:
+        assert np.array_equal(sol, out[0][0]) and it == out[0][1]
+
+
 @pytest.mark.parametrize("nt", [3, 4, 5, 17, 96, 128, 255, 338, 1009, 2046, 4094, 6561, 7001])
 def test_many_series_inverse_laplace_matches_numpy(gpu_pkg, nt):
     """Enough series for the mixed-radix transform (odd counts leave a single

@@ -1401,7 +1401,7 @@ __global__ void k_diag_scale(const float2* __restrict__ A0, long long ld, long l
 }
 
 // How the triangular solves run (tags_debug_solve_path): 0 the per-block
-// kernels; 1 k_ldl_solve_cta (one CTA per sample); 2, 4, 8 k_ldl_solve_cl
+// kernels; 1 k_ldl_solve_cta (one CTA per sample); 2, 4, 8, 16 k_ldl_solve_cl
 // (a cluster of that many CTAs per sample); -1 (default) the largest of the
 // cluster sizes 16 and 8 with G x samples <= SMs / 2 and all clusters resident,
 // else of 4 and 2 with G x samples <= SMs, else one CTA per sample: with
@@ -2287,8 +2287,13 @@ extern "C" int tags_debug_tri_tiles(int M, int zlo, int zhi, int planes, int pla
 }
 
 extern "C" int tags_debug_solve_path(int path) {
-    if (path != -1 && path != 0 && path != 1 && path != 2 && path != 4 && path != 8)
-        return tags_fail(TAGS_E_ARG, "tags_debug_solve_path: -1, 0, 1, 2, 4 or 8");
+    if (path != -1 && path != 0 && path != 1 && path != 2 && path != 4 && path != 8 && path != 16)
+        return tags_fail(TAGS_E_ARG, "tags_debug_solve_path: -1, 0, 1, 2, 4, 8 or 16");
+    if (path == 16) {
+        // more CTAs than a cluster is promised to have room for
+        if (int e = tags_ldl_tc_prepare()) return e;
+        if (!g_solve_cl_ok[16]) return tags_fail(TAGS_E_ARG, "tags_debug_solve_path: no cluster of 16 on this device");
+    }
     g_solve_path = path;
     return 0;
 }
