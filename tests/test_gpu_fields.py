@@ -285,3 +285,68 @@ def test_field_memory_follows_the_work(gpu_pkg):
     out = pkg.fields_batch([[1000.0, 0.0, 0.0]], e, cur, cur, np.full(ns, 0.01 + 0.01j), np.ones(ns, np.complex128))
     assert out["status"] == 0 and np.ptp(out["pot"].real) == 0.0
     assert before - torch.cuda.mem_get_info()[0] < 1 << 30
+
+
+def check_against_fine_rule(out, pts, e, il, it, gamma, samples, points):
+    """Potential, vector potential and field of the given samples and points to 1e-12 of the summed magnitudes."""
+    for k in samples:
+        for p in points:
+            pairs = [fine_rule(pts[p], seg, gamma[k]) for seg in e]
+            j = np.array([v[0] for v in pairs])
+            f = np.array([v[1] for v in pairs])
+            d = e[:, 3:6] - e[:, :3]
+            for r in range(il.shape[1]):
+                for got, want, size in (
+                        (4 * np.pi * out["pot"][k, p, r], it[k, r] @ j, np.abs(it[k, r]) @ np.abs(j)),
+                        (1e7 * out["vecpot"][k, p, r], (il[k, r] * j) @ d, np.abs(il[k, r] * j) @ np.abs(d).max(axis=1)),
+                        (4 * np.pi * out["efield"][k, p, r], it[k, r] @ f, np.abs(it[k, r]) @ np.abs(f).max(axis=1))):
+                    assert np.max(np.abs(got - want)) <= 1e-12 * size
+
+
+@pytest.mark.parametrize("ns,far", [(80, (40,)), (96, (3, 95)), (70, (66,)), (200, (130, 131))])
+def test_field_call_with_both_kernels_matches_fine_rule(gpu_pkg, ns, far):
+    """Some groups of 32 samples hold one past the series' reach and take the rule per sample, the others the series, in
+    one call with a partial last group and five injections. The evaluations counted are those of calls of the former
+    groups alone, so both kernels had their part."""
+    pkg = gpu_pkg
+    rng = np.random.default_rng(ns)
+    m, P, R = 40, 36, 5
+    e, _ = pkg.segment_electrode([0.0, 0.0, -0.5], [1.0 * m, 0.0, -0.5], m, 7e-3)
+    pts = np.stack([np.linspace(-0.3, 50.0, P), np.full(P, 0.2), np.linspace(0.0, 3.0, P) - 0.4], axis=1)
+    gamma = 0.9 / 0.5625 * np.exp(0.25j * np.pi) * np.linspace(0.2, 1.0, ns)
+    gamma[list(far)] *= 10 / np.abs(gamma[list(far)])
+    il, it = (rng.standard_normal((ns, R, m)) + 1j * rng.standard_normal((ns, R, m)) for _ in range(2))
+    kappa = np.ones(ns, np.complex128)
+    pkg.fields_evaluations(reset=True)
+    out = pkg.fields_batch(pts, e, il, it, gamma, kappa)
+    together = pkg.fields_evaluations(reset=True)
+    assert out["status"] == 0
+    rule = sorted({f // 32 for f in far})
+    for g in rule:
+        take = slice(32 * g, min(ns, 32 * g + 32))
+        # alone, a last group of fewer is shared out differently (G samples per warp), but evaluates the same nodes
+        alone = pkg.fields_batch(pts, e, il[take], it[take], gamma[take], kappa[take])
+        assert rel(alone["efield"], out["efield"][take]) < 1e-12
+    assert 0 < pkg.fields_evaluations(reset=True) == together
+    check_against_fine_rule(out, pts, e, il, it, gamma, sorted({0, ns - 1, far[0], far[0] - 1, 32 * (far[0] // 32) - 1}),
+                            (0, P - 1))
+
+
+def rel(a, b):
+    return float(np.max(np.abs(a - b)) / np.max(np.abs(b)))
+
+
+@pytest.mark.parametrize("x", [0.04, 0.085, 0.1, 0.3, 0.36, 0.38, 1.2])
+@pytest.mark.parametrize("ns,m", [(5, 3), (40, 33)])
+def test_field_series_of_many_samples_at_every_term_count(gpu_pkg, x, ns, m):
+    """Calls of several samples whose largest needs up to 12, 16 and 24 terms (x = 0.09 and 0.37 part them)."""
+    pkg = gpu_pkg
+    rng = np.random.default_rng(m)
+    e, _ = pkg.segment_electrode([0.0, 0.0, -0.5], [1.0 * m, 0.0, -0.5], m, 7e-3)
+    pts = np.stack([np.linspace(-0.3, 1.4 * m, 6), np.full(6, 0.2), np.linspace(0.0, 3.0, 6) - 0.4], axis=1)
+    gamma = x / 0.5625 * np.exp(0.25j * np.pi) * np.linspace(0.2, 1.0, ns)
+    il, it = (rng.standard_normal((ns, 5, m)) + 1j * rng.standard_normal((ns, 5, m)) for _ in range(2))
+    pkg.fields_evaluations(reset=True)
+    out = pkg.fields_batch(pts, e, il, it, gamma, np.ones(ns, np.complex128))
+    assert out["status"] == 0 and pkg.fields_evaluations() == 0
+    check_against_fine_rule(out, pts, e, il, it, gamma, {0, ns // 2, ns - 1}, (0, 2, 5))

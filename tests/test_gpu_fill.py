@@ -375,3 +375,28 @@ def test_close_pairs_match_oracle(gpu_pkg, port, gap, x):
         assert port.calculate_impedances(*want, e, gamma, s, 1.0, kappa, req_abs=0.0, req_rel=1e-10) == 0
         for g, w in zip(got, want):
             assert elementwise(g, w) < TOL
+
+
+@pytest.mark.parametrize("m", [2, 17])
+@pytest.mark.parametrize("x", [0.05, 0.19, 0.21, 0.25, 0.57, 0.6])
+def test_fill_series_on_both_sides_of_its_term_counts_match_oracle(gpu_pkg, port, m, x):
+    """Moments of 12, 16 and 32 terms near the reach of each (x = 0.20 and 0.58), direct and image kinds; as above."""
+    test_fill_series_and_its_limits_match_oracle(gpu_pkg, port, m, x)
+
+
+@pytest.mark.parametrize("x", [0.05, 0.19, 0.25, 0.57, 0.6])
+def test_fill_terms_by_four_lanes_match_whole_warps(gpu_pkg, x):
+    """The instances of 12, 16 and 32 terms with four lanes per record (10011 pairs) against whole warps (the first 20
+    segments alone), near the reach of each; sums of up to 64 terms of one sign in another order, 1e-13."""
+    pkg = gpu_pkg
+    e = bent_wire(pkg, 141)
+    gamma = x / (e[:, 9].max() * 17 / 16) * np.exp(0.25j * np.pi)
+    s, kappa = 1e5 + 1e6j, 0.01 + 1e-4j
+    out = []
+    for k in (len(e), 20):
+        z = [np.zeros(k * k, np.complex128) for _ in range(2)]
+        assert pkg.calculate_impedances(*z, e[:k], gamma, s, 1.0, kappa) == 0
+        out.append([np.tril(v.reshape(k, k).T)[:20, :20] for v in z])
+    for a, b in zip(*out):
+        nz = b != 0
+        assert np.array_equal(a != 0, nz) and elementwise(a[nz], b[nz]) < 1e-13

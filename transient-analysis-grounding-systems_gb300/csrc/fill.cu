@@ -408,8 +408,8 @@ __global__ void __launch_bounds__(128) k_path_pairs(const double* __restrict__ e
 // exponential (~130) per sample, and a sample 2 nt + 20 per pair. Pairs
 // sharing an endpoint: the radial part of the Duffy rule in closed form,
 // \int_0^1 (t rho - R)^n dt = g_n / (n + 1), g_n = sum_i (rho - R)^i (-R)^(n-i).
-// Terms: x^nt / nt! <= 1e-17 at x = max |gamma| dmax (16 up to x ~ 0.75, else
-// 32, which reach x = 3.5, where the sum's largest term is e^3.5 of N_0 and
+// Terms: x^nt / nt! <= 1e-17 at x = max |gamma| dmax (moments of 12 up to x = 0.2, of
+// 16 up to x = 0.58, else of 32, which reach x = 3.5, where the sum's largest term is e^3.5 of N_0 and
 // the rounding ~1e-14 of the entry). Samples beyond that keep an exponential per
 // point (k_fill_far).
 // Measured on GB300 against the direct rule for every sample: the plain form's
