@@ -80,7 +80,7 @@ int sym_solve(const tags_cdouble* z, const tags_cdouble* rhs, size_t m, size_t n
     if (!d_Z || !d_X || !d_ipiv) return tags_fail(TAGS_E_NOMEM, "device allocation failed");
     TAGS_CUDA_OK(cudaMemcpyAsync(d_Z, z, sizeof(double2) * m * m, cudaMemcpyHostToDevice, st));
     int err = tags_symmetrize_lower(d_Z, (int)m, (long long)m, 0, 1, st);
-    if (!err) err = tags_lu_z(d_Z, (int)m, (long long)m, 0, 1, 1, d_ipiv, d_ipiv + m, st);
+    if (!err) err = tags_lu_z(d_Z, (int)m, (long long)m, 0, 1, d_ipiv, d_ipiv + m, st);
     if (err) return err;
     int info = 0;
     TAGS_CUDA_OK(cudaMemcpyAsync(&info, d_ipiv + m, sizeof(int), cudaMemcpyDeviceToHost, st));

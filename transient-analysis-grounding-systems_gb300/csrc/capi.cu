@@ -405,7 +405,7 @@ extern "C" int solve_immittance(tags_cdouble* wg, tags_cdouble* ie, size_t num_e
     TAGS_CUDA_OK(cudaMemcpyAsync(d_x, ie, sizeof(double2) * N, cudaMemcpyHostToDevice, st));
     int err = tags_symmetrize_lower(d_W, (int)N, (long long)N, 0, 1, st);
     if (err) return err;
-    err = tags_lu_z(d_W, (int)N, (long long)N, 0, 1, 1, d_ipiv, d_ipiv + N, st);
+    err = tags_lu_z(d_W, (int)N, (long long)N, 0, 1, d_ipiv, d_ipiv + N, st);
     if (err) return err;
     int info = 0;
     TAGS_CUDA_OK(cudaMemcpyAsync(&info, d_ipiv + N, sizeof(int), cudaMemcpyDeviceToHost, st));

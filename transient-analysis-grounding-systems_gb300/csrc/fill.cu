@@ -296,12 +296,19 @@ TAGS_D void pair_index(long long p, int m, int& i, int& k) {
     k = ii + (int)(p - (long long)ii * (2LL * m - ii + 1) / 2);
 }
 
-TAGS_D void store(double2* base, long long idx, double2 v, bool acc) {
-    if (acc) {
-        double2 o = base[idx];
-        base[idx] = cadd(o, v);
-    } else {
-        base[idx] = v;
+// The entry (k, i) of sample s to its places.
+TAGS_D void store_entry(const FillOut& out, int s, int i, int k, double2 zl, double2 zt, int* status) {
+    if (!isfinite(zl.x + zl.y + zt.x + zt.y)) raise_status(status, TAGS_ST_NONFINITE);
+    zl = cscale(zl, out.sign);
+    zt = cscale(zt, out.sign);
+    const long long bs = out.batch_stride * s;
+    if (out.zl) {
+        out.zl[bs + out.row0_l + k + out.ld * (out.col0_l + i)] = zl;
+        if (out.mirror && k != i) out.zl[bs + out.row0_l + i + out.ld * (out.col0_l + k)] = zl;
+    }
+    if (out.zt) {
+        out.zt[bs + out.row0_t + k + out.ld * (out.col0_t + i)] = zt;
+        if (out.mirror && k != i) out.zt[bs + out.row0_t + i + out.ld * (out.col0_t + k)] = zt;
     }
 }
 
@@ -356,20 +363,7 @@ __global__ void __launch_bounds__(128) k_fill_fp64(const double* __restrict__ el
         zt = cadd(zt, cmul(cscale(cTi, 1.0 / (S.len * R.len)), intg));
         if (cost > TAGS_DBL_EPSILON) zl = cadd(zl, cscale(cmul(cLi, intg), cost / (S.len * R.len)));
     }
-    if (!isfinite(zl.x + zl.y + zt.x + zt.y)) raise_status(status, TAGS_ST_NONFINITE);
-    const bool acc = out.accumulate != 0;
-    const double sg = out.sign;
-    zl = cscale(zl, sg);
-    zt = cscale(zt, sg);
-    const long long bs = out.batch_stride * smp;
-    if (out.zl) {
-        store(out.zl + bs, (long long)(out.row0_l + k) + out.ld * (out.col0_l + i), zl, acc);
-        if (out.mirror && k != i) store(out.zl + bs, (long long)(out.row0_l + i) + out.ld * (out.col0_l + k), zl, acc);
-    }
-    if (out.zt) {
-        store(out.zt + bs, (long long)(out.row0_t + k) + out.ld * (out.col0_t + i), zt, acc);
-        if (out.mirror && k != i) store(out.zt + bs, (long long)(out.row0_t + i) + out.ld * (out.col0_t + k), zt, acc);
-    }
+    store_entry(out, smp, i, k, zl, zt, status);
 }
 
 // Path/electrode double integrals for the path voltage: thread per
@@ -781,23 +775,6 @@ TAGS_D double2 direct_integral(const SeriesPk& k, double2 g, int lane) {
         a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
     }
     return a;
-}
-
-// The entry (k, i) of sample s to its places.
-TAGS_D void store_entry(const FillOut& out, int s, int i, int k, double2 zl, double2 zt, int* status) {
-    if (!isfinite(zl.x + zl.y + zt.x + zt.y)) raise_status(status, TAGS_ST_NONFINITE);
-    const bool accum = out.accumulate != 0;
-    zl = cscale(zl, out.sign);
-    zt = cscale(zt, out.sign);
-    const long long bs = out.batch_stride * s;
-    if (out.zl) {
-        store(out.zl + bs, (long long)(out.row0_l + k) + out.ld * (out.col0_l + i), zl, accum);
-        if (out.mirror && k != i) store(out.zl + bs, (long long)(out.row0_l + i) + out.ld * (out.col0_l + k), zl, accum);
-    }
-    if (out.zt) {
-        store(out.zt + bs, (long long)(out.row0_t + k) + out.ld * (out.col0_t + i), zt, accum);
-        if (out.mirror && k != i) store(out.zt + bs, (long long)(out.row0_t + i) + out.ld * (out.col0_t + k), zt, accum);
-    }
 }
 
 // The entries of the samples past the series' reach (long segments at high
@@ -2313,16 +2290,7 @@ __global__ void k_mhem_fp64(const double* __restrict__ elec, const double* __res
         zl = cadd(zl, cmul(cmul(e2, pot[2 * mm + e]), c.cLi));
         zt = cadd(zt, cmul(cmul(e2, pot[3 * mm + e]), c.cTi));
     }
-    if (!isfinite(zl.x + zl.y + zt.x + zt.y)) raise_status(status, TAGS_ST_NONFINITE);
-    zl = cscale(zl, out.sign);
-    zt = cscale(zt, out.sign);
-    const long long bs = out.batch_stride * smp;
-    store(out.zl + bs, (long long)(out.row0_l + k) + out.ld * (out.col0_l + i), zl, out.accumulate != 0);
-    store(out.zt + bs, (long long)(out.row0_t + k) + out.ld * (out.col0_t + i), zt, out.accumulate != 0);
-    if (out.mirror && k != i) {
-        store(out.zl + bs, (long long)(out.row0_l + i) + out.ld * (out.col0_l + k), zl, out.accumulate != 0);
-        store(out.zt + bs, (long long)(out.row0_t + i) + out.ld * (out.col0_t + k), zt, out.accumulate != 0);
-    }
+    store_entry(out, smp, i, k, zl, zt, status);
 }
 
 constexpr int MIX_SG = 4;   // samples per thread of the mHEM rescale

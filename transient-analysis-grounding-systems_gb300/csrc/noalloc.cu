@@ -74,7 +74,7 @@ extern "C" int tags_solve_immittance_noalloc(tags_cdouble* d_wg, tags_cdouble* d
     // factorise the caller's W_G in place (the reference's zsysv also
     // overwrites it), lower half read as in zsysv('L')
     int err = tags_symmetrize_lower(W, n, (long long)N, 0, 1, st);
-    if (!err) err = tags_lu_z(W, n, (long long)N, 0, 1, 1, ipiv, info_d, st);
+    if (!err) err = tags_lu_z(W, n, (long long)N, 0, 1, ipiv, info_d, st);
     if (err) return err;
     int info = 0;
     TAGS_CUDA_OK(cudaMemcpyAsync(&info, info_d, sizeof(int), cudaMemcpyDeviceToHost, st));

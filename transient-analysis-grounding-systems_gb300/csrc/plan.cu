@@ -339,7 +339,7 @@ int tags_plan_lu_one(tags_plan_s* p, int q, double2* W, int* ipiv, double2* x, i
     out.sign = -1.0;
     out.mirror = 1;
     err = tags_plan_fill_fp64(p, p->d_coef + q, 1, out, st);
-    if (!err) err = tags_lu_z(W, (int)N, N, NN, 1, 1, ipiv, info, st);
+    if (!err) err = tags_lu_z(W, (int)N, N, NN, 1, ipiv, info, st);
     return err ? err : tags_lu_solve_z(W, (int)N, N, NN, 1, ipiv, x, 1, N, N, st);
 }
 

@@ -52,7 +52,6 @@ struct FillOut {
     int row0_l, col0_l, row0_t, col0_t;
     double sign;
     int mirror;
-    int accumulate;
 };
 
 int tags_fill_tables_init();
@@ -159,8 +158,7 @@ int tags_wg_impedance(double2* d_W, long long ld, const double2* d_zl, const dou
 int tags_symmetrize_lower(double2* d_W, int N, long long ld, long long stride, int batch, cudaStream_t st);
 
 // lu.cu
-int tags_lu_z(double2* A, int n, long long ld, long long stride, int batch, int pivot, int* ipiv, int* info,
-              cudaStream_t st);
+int tags_lu_z(double2* A, int n, long long ld, long long stride, int batch, int* ipiv, int* info, cudaStream_t st);
 int tags_lu_solve_z(const double2* A, int n, long long ld, long long stride, int batch, const int* ipiv, double2* X,
                     int nrhs, long long ldx, long long xstride, cudaStream_t st);
 
