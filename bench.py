@@ -796,8 +796,8 @@ def plain_fp64_record(pkg, elec, img, nodes, s_d, k_d, ie_d, centre, local, flus
             "roofline": roof, "kernel_families": fams, "fp64_peak": fp64,
             "note": "plain FP64 form of this library on the same workload: FP64 fill, FP64 LDL^T with refinement, "
                     "device time from the plan's events, L2 flushed between steps; roofline (lu_fp64_gemm: the trailing "
-                    "updates' complex flops, 8 per multiply-add, which three real products instead of four execute, so "
-                    "the fraction may pass 1) and kernel_families from one more step launched kernel by kernel"}
+                    "updates' executed flops, 6 per complex multiply-add: three real products) and kernel_families "
+                    "from one more step launched kernel by kernel"}
 
 
 def gpr_accuracy(pkg, plan, s_d, k_d, ie_d, centre, n, SB, sol_d, info_d, s, tmax, nt):

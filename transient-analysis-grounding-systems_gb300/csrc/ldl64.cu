@@ -1105,7 +1105,8 @@ int factor(double2* A, int N, long long ld, long long stride, int nb, int m, con
         else
             k_ldl64_update<16, 1><<<dim3((unsigned)(t16 * (t16 + 1) / 2), nb), 256, 6 * PB * 16 * sizeof(double), st>>>(
                 A, ld, stride, q);
-        tags_prof_end(TAGS_PROF_LU64_GEMM, pf, st, 4.0 * q.cnt * (q.cnt + 1.0) * q.jb * nb,
+        // the three real products' flops, 6 per complex multiply-add
+        tags_prof_end(TAGS_PROF_LU64_GEMM, pf, st, 3.0 * q.cnt * (q.cnt + 1.0) * q.jb * nb,
                       (16.0 * q.cnt * (q.cnt + 1.0) + 32.0 * q.cnt * q.jb) * nb);
         tags_note_launch();
     }
