@@ -85,6 +85,18 @@ int tags_once_per_device(PerDevice& state, int (*setup)()) {
     return err;
 }
 
+int tags_num_sms() {
+    static std::atomic<int> sms[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 152;
+    int n = sms[dev].load();
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 152;
+        sms[dev].store(n);
+    }
+    return n;
+}
+
 DeviceCtx* tags_ctx() {
     static DeviceCtx ctxs[64];
     int dev = 0;

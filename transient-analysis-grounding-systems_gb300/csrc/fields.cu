@@ -828,7 +828,7 @@ inline double2 D2(tags_cdouble v) { return make_double2(v.re, v.im); }
 int field_chunks(size_t P, size_t ns, size_t R, size_t m, size_t part_cap) {
     const size_t G = (size_t)samples_per_warp(ns);
     const size_t warps = P * ((ns + G - 1) / G);
-    const size_t target = 152 * 8 * 6;
+    const size_t target = (size_t)tags_num_sms() * 8 * 6;
     size_t c = warps ? (target + warps - 1) / warps : 1;
     c = std::min<size_t>(c, std::max<size_t>(1, m / 16));
     c = std::min<size_t>(c, 64);
@@ -894,7 +894,7 @@ void series_chunks(SerArgs* s, size_t part_cap) {
     s->ngc = ngroups >= 3 ? 4 : ngroups;
     const long long ctas = (long long)a.P * ((ngroups + s->ngc - 1) / s->ngc);
     const size_t per = 7 * sizeof(double2) * a.P * a.R * (size_t)a.S * (4 / s->ngc);
-    long long c = (152 * 4 + ctas - 1) / ctas;
+    long long c = (tags_num_sms() * 4 + ctas - 1) / ctas;
     c = std::min<long long>(c, std::max<long long>(1, (long long)(part_cap / std::max<size_t>(per, 1))));
     c = std::min<long long>(c, (a.m + 3) / 4);
     s->echunk = (int)((a.m + c - 1) / c);
@@ -926,7 +926,7 @@ int launch_fields(const SerArgs& sa, int most, double madds, bool direct, cudaSt
     }
     const long long n = (long long)base.S * base.P * base.R;
     const int chunks = std::max(direct ? base.nchunk : 0, most > 0 ? base.schunk : 0);
-    if (chunks >= 16 && n <= 4864)                          // a warp each: 32 per SM
+    if (chunks >= 16 && n <= 32 * tags_num_sms())           // a warp each
         k_fields_reduce<32><<<(unsigned)((32 * n + 127) / 128), 128, 0, st>>>(base);
     else
         k_fields_reduce<1><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(base);
@@ -1020,7 +1020,7 @@ int fields_run(const FieldsIn& in) {
         double2* cur_t = d_cur + 2 * nc;      // transposed [m][R][ns]
         double2* cur_l = d_cur + 3 * nc;
         const bool need_t = (in.want & (WANT_POT | WANT_EF)) != 0, need_l = (in.want & WANT_VEC) != 0;
-        const int tb = 256, tg = (int)std::min<size_t>((nc + tb - 1) / tb, 152 * 16);
+        const int tb = 256, tg = (int)std::min<size_t>((nc + tb - 1) / tb, (size_t)tags_num_sms() * 16);
         if (need_t) {
             TAGS_CUDA_OK(cudaMemcpyAsync(raw_t, in.it + s0 * R * m, sizeof(double2) * nc, cudaMemcpyHostToDevice, st));
             k_cur_transpose<<<tg, tb, 0, st>>>(raw_t, cur_t, (int)ns, (int)R, (int)m);
@@ -1155,7 +1155,7 @@ extern "C" int tags_gpd_mhem_batch(const double* points, size_t num_points, cons
     for (size_t s0 = 0; s0 < S; s0 += cs) {
         const size_t ns = std::min(cs, S - s0), nc = R * m * ns;
         TAGS_CUDA_OK(cudaMemcpyAsync(d_cur, it + s0 * R * m, sizeof(double2) * nc, cudaMemcpyHostToDevice, st));
-        const int tb = 256, tg = (int)std::min<size_t>((nc + tb - 1) / tb, 152 * 16);
+        const int tb = 256, tg = (int)std::min<size_t>((nc + tb - 1) / tb, (size_t)tags_num_sms() * 16);
         k_cur_transpose<<<tg, tb, 0, st>>>(d_cur, d_cur + nc, (int)ns, (int)R, (int)m);
         tags_note_launch();
         TAGS_CUDA_OK(cudaGetLastError());
@@ -1239,7 +1239,7 @@ extern "C" int tags_voltage_batch(const double* paths, size_t num_paths, const E
         double2* d_v = d_u + 2 * NL * R * ns;
         if (m) {
             TAGS_CUDA_OK(cudaMemcpyAsync(d_cur, il + s0 * R * m, sizeof(double2) * nc, cudaMemcpyHostToDevice, st));
-            const int tb = 256, tg = (int)std::min<size_t>((nc + tb - 1) / tb, 152 * 16);
+            const int tb = 256, tg = (int)std::min<size_t>((nc + tb - 1) / tb, (size_t)tags_num_sms() * 16);
             k_cur_transpose<<<tg, tb, 0, st>>>(d_cur, cur_l, (int)ns, (int)R, (int)m);
             tags_note_launch();
             TAGS_CUDA_OK(cudaGetLastError());

@@ -2449,13 +2449,13 @@ static int series_tables(const SampleCoef* d_coef, const SeriesView& v, cudaStre
 
 // CTAs of the kernels for the samples past the reach: four per SM at most.
 static unsigned far_ctas(long long pairs, int ns) {
-    return (unsigned)std::min<long long>(608, (pairs * ns + SER_THREADS / 32 - 1) / (SER_THREADS / 32));
+    return (unsigned)std::min<long long>(4 * tags_num_sms(), (pairs * ns + SER_THREADS / 32 - 1) / (SER_THREADS / 32));
 }
 
 // Records per CTA: up to `most`, fewer while the grid would leave SMs idle.
 static int series_tile(long long n, int most) {
     int t = most;
-    while (t > 2 && (n + t - 1) / t < 608) t /= 2;
+    while (t > 2 && (n + t - 1) / t < 4 * tags_num_sms()) t /= 2;
     return t;
 }
 

@@ -356,14 +356,15 @@ int tags_launch_inlt(const double2* d_g, long long gseries, long long gk, const 
     k_inlt_tables<<<(unsigned)((nt + 127) / 128), 128, 0, st>>>(d_s, ns, nt, tmax, filter, sigma, scale);
     tags_note_launch();
     // SM cycles of either way (two FP64 multiply-adds per clock and SM): the
-    // transform keeps a CTA's SM for nt (5 sum r + 6 FFT_LOW) / 2 and runs 152 pairs at a
+    // transform keeps a CTA's SM for nt (5 sum r + 6 FFT_LOW) / 2 and runs a pair per SM at a
     // time, the direct sums take three operations a term on all SMs. nt = 4094:
     // one series 60 us direct, the transform ~1.4 ms for up to 304.
     int sum = 0;
     const FftPlan plan = nt <= FFT_NT_MAX ? fft_plan((int)nt, &sum) : FftPlan{};
     const double pairs = 0.5 * (double)(nser + 1);
-    const double c_fft = ceil(pairs / 152.0) * (double)nt * (5.0 * sum + 6.0 * FFT_LOW) / 2.0;
-    const double c_direct = (double)nser * (double)nt * (double)ns * 3.0 / (2.0 * 152.0);
+    const double sms = tags_num_sms();
+    const double c_fft = ceil(pairs / sms) * (double)nt * (5.0 * sum + 6.0 * FFT_LOW) / 2.0;
+    const double c_direct = (double)nser * (double)nt * (double)ns * 3.0 / (2.0 * sms);
     if (nt <= FFT_NT_MAX && nt > 2 && c_fft < c_direct) {
         static PerDevice state;
         const int err = tags_once_per_device(state, [] {

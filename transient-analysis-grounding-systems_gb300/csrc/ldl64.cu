@@ -1062,6 +1062,7 @@ constexpr int SOLVE_N_MAX = 14000;        // 16 B per unknown in the one-CTA sol
 // least FP64 instructions per warp: 690 for a CTA's block and 576, 320 or 192
 // per group of 32, 16 or 8 rows.
 int panel_split(int rows, int nb, int& lpr, int& passes) {
+    const int sms = tags_num_sms();
     long long best = -1;
     int ctas = 1;
     for (int l = 4, ins = 576; l <= 16; l *= 2, ins = l == 8 ? 320 : 192)
@@ -1069,7 +1070,7 @@ int panel_split(int rows, int nb, int& lpr, int& passes) {
             const int groups = (rows * l + 127) / 128, c = (groups + ps - 1) / ps;
             if (c == last) continue;                       // as many CTAs with fewer passes
             last = c;
-            const long long cost = ((long long)nb * c + 151) / 152 * (690 + ins * ps);
+            const long long cost = ((long long)nb * c + sms - 1) / sms * (690 + ins * ps);
             if (best < 0 || cost < best) {
                 best = cost;
                 lpr = l;
@@ -1081,7 +1082,7 @@ int panel_split(int rows, int nb, int& lpr, int& passes) {
 }
 
 int factor(double2* A, int N, long long ld, long long stride, int nb, int m, const Ws& w, cudaStream_t st) {
-    const int P = panel_count(N, m);
+    const int P = panel_count(N, m), sms = tags_num_sms();
     for (int p = 0; p < P; ++p) {
         const Panel q = panel_at(p, N, m);
         int lpr, passes;
@@ -1096,10 +1097,10 @@ int factor(double2* A, int N, long long ld, long long stride, int nb, int m, con
         // tile rows) and fills the SMs
         pf = tags_prof_begin(TAGS_PROF_LU64_GEMM, st);
         const long long t64 = (q.cnt + 63) / 64, t32 = (q.cnt + 31) / 32, t16 = (q.cnt + 15) / 16;
-        if (t64 >= 10 && t64 * (t64 + 1) / 2 * nb >= 608)
+        if (t64 >= 10 && t64 * (t64 + 1) / 2 * nb >= 4 * sms)
             k_ldl64_update<64, 4><<<dim3((unsigned)(t64 * (t64 + 1) / 2), nb), 256, 6 * PB * 64 * sizeof(double), st>>>(
                 A, ld, stride, q);
-        else if (t32 >= 10 && t32 * (t32 + 1) / 2 * nb >= 304)
+        else if (t32 >= 10 && t32 * (t32 + 1) / 2 * nb >= 2 * sms)
             k_ldl64_update<32, 2><<<dim3((unsigned)(t32 * (t32 + 1) / 2), nb), 256, 6 * PB * 32 * sizeof(double), st>>>(
                 A, ld, stride, q);
         else
@@ -1122,7 +1123,7 @@ int solve(const double2* A, int N, long long ld, long long stride, int nb, int m
     int p0 = 0;
     while (p0 + 1 < P && panel_at(p0, N, m).base <= lead) ++p0;
     int pf = tags_prof_begin(TAGS_PROF_LU64_OTHER, st);
-    if (N > 64 && N <= SCL_N && nb <= (N <= 320 ? 38 : 19)) {
+    if (N > 64 && N <= SCL_N && nb <= tags_num_sms() / SCL_G * (N <= 320 ? 2 : 1)) {
         k_ldl64_solve_cl<<<dim3(SCL_G, nb), 128, scl_smem(N), st>>>(A, ld, stride, N, m, w.linv, w.wstride, w.r, w.z, p0,
                                                                     w.active);
         tags_prof_end(TAGS_PROF_LU64_OTHER, pf, st, 0.0, 0.0);
@@ -1298,10 +1299,11 @@ int tags_ldl64_multi_solve(const double2* Z, const double2* rhs, int M, int n, i
     TAGS_CUDA_OK(cudaMemcpyAsync(A, Z, sizeof(double2) * MM * nb, cudaMemcpyDeviceToDevice, st));
     if (int e = factor(A, M, M, MM, nb, 0, w, st)) return e;
     // as many columns per CTA as leave the busiest SM the least to do
+    const int sms = tags_num_sms();
     int ct = 1;
     long long best = 0;
     for (int t = 1; t <= MCOLS_MAX && mcols_smem(M, t) <= MCOLS_SMEM; ++t) {
-        const long long ctas = (long long)((R + t - 1) / t) * nb, cost = (ctas + 151) / 152 * t;
+        const long long ctas = (long long)((R + t - 1) / t) * nb, cost = (ctas + sms - 1) / sms * t;
         if (t == 1 || cost <= best) {
             best = cost;
             ct = t;

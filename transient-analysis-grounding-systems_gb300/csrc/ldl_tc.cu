@@ -1809,16 +1809,6 @@ static float2* linv32_of(void* ws, int N, int batch_cap) {
     return dinv + 2LL * TB * batch_cap;
 }
 
-static int num_sms() {
-    static int n = 0;
-    if (!n) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 132;
-    }
-    return n;
-}
-
 template <int S, int MODE>
 static int set_gemm_attr() {
     TAGS_CUDA_OK(cudaFuncSetAttribute(k_gemm_tc<S, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1941,7 +1931,7 @@ int tags_ldl_tc_prepare() {
 template <int S, int MODE>
 static int launch_gemm_m(const CUtensorMap& mA, const CUtensorMap& mB, const GemmArgs& g, cudaStream_t st) {
     const int total = g.tiles * g.nb;
-    const int grid = total < num_sms() ? total : num_sms();
+    const int grid = total < tags_num_sms() ? total : tags_num_sms();
     if (grid <= 0) return 0;
     k_gemm_tc<S, MODE><<<grid, GEMM_THREADS, GemmCfg<S>::SMEM, st>>>(mA, mB, g);
     tags_note_launch();
@@ -2002,7 +1992,7 @@ int tags_ldl_solve_c(const float2* A, int N, long long ld, long long mstride, in
     if (path < 0) {
         path = 1;
         for (int G = 16; G >= 2; G /= 2)
-            if ((long long)nb * G <= (G > 4 ? num_sms() / 2 : num_sms()) && g_solve_cl_ok[G] >= (G > 4 ? nb : 1)) {
+            if ((long long)nb * G <= (G > 4 ? tags_num_sms() / 2 : tags_num_sms()) && g_solve_cl_ok[G] >= (G > 4 ? nb : 1)) {
                 path = G;
                 break;
             }
@@ -2022,7 +2012,7 @@ int tags_ldl_solve_c(const float2* A, int N, long long ld, long long mstride, in
                             : launch_solve_cl<16>(A, ld, mstride, N, L32, ls, x, xstride, zl_m, active, lead_step,
                                                   lead_zero, nb, smem, st);
         } else {
-            const int few = split ? num_sms() / 4 : 0;
+            const int few = split ? tags_num_sms() / 4 : 0;
             k_ldl_solve_cta<<<nb, SOLVE_THREADS, smem, st>>>(A, ld, mstride, N, L32, ls, x, xstride, zl_m, active,
                                                              lead_step, lead_zero, split ? nact : nullptr, few);
             tags_note_launch();

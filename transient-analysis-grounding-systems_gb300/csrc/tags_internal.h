@@ -114,6 +114,7 @@ struct PerDevice {
     bool done[64] = {};
 };
 int tags_once_per_device(PerDevice& state, int (*setup)());
+int tags_num_sms();      // SMs of the calling thread's device
 // Geometry of the FP64 moment series over segment records (11 doubles each, on
 // the host): with it and a workspace for the samples of the launch, the
 // INTG_DOUBLE fill and the path integrals take their samples from per-launch
