@@ -333,6 +333,10 @@ constexpr int FS_GL = 6 + 7 + 8 + 9 + 12;
 // 8e-10 (x / 2)^12 with 6 nodes and 5e-12 (x / 2)^14 with 7 on the electrode's axis.
 // Each stays up to where that passes 1e-15 (6 nodes at every x: 6e-10 at x = 1.95).
 int fs_least_order(double x) { return x <= 0.55 ? 0 : x <= 1.0 ? 1 : 3; }
+// Panels of the near points per unit of v, for the same reason: 3000 random points
+// within two lengths stay within 7e-14 (1e-15 in the median) with panels of 0.75 at x =
+// 1, 6e-15 with 0.5 at 1.5 and 4e-15 with 0.375 at 2, where 0.75 gives up to 1e-12.
+double fs_panels(double x) { return 1.0 / (x <= 1.0 ? 0.75 : x <= 1.5 ? 0.5 : 0.375); }
 
 __constant__ double c_fsx[FS_GL], c_fsw[FS_GL];   // nodes and weights on [0, 1], order by order
 
@@ -342,8 +346,8 @@ struct SerArgs {
     const double2* tab;     // [bucket][S]: e^{-gamma b h} (null: formed per pair)
     double h;
     int nbk, ngc, echunk;   // buckets; sample groups per CTA (1, 2, 4); electrodes per CTA
-    int least;              // fs_least_order of the pass's largest |gamma| among the series' samples
-    double ga;              // that |gamma|
+    int least;              // fs_least_order and fs_panels of the largest |gamma| among the series' samples
+    double panels;
 };
 
 // The samples' constants: a row of CTAs per bucket of the table (nbk of them, none
@@ -373,8 +377,8 @@ struct SerPair {
 // Moments of one (point, electrode) pair by L lanes (g: this one), all of the
 // warp's groups together, `on` or not: Gauss-Legendre in t where the point is at
 // least two lengths away (6 to 12 nodes by the distance and |gamma|), else the sinh
-// rule above in panels of at most 0.75 and, as in k_fields, 1.5 / |gamma| of r on
-// average, up to ~1000 nodes, which one lane would take in a row.
+// rule above in panels of 0.75 down to 0.375, up to ~1000 nodes, which one lane
+// would take in a row.
 template <int NT>
 TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, const SerArgs& sa, const double* gx,
                          const double* gw, bool on, int g, int L, SerPair& out, double* mom) {
@@ -429,9 +433,7 @@ TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, const Se
         const bool split = va < 0.0 && vb > 0.0;
         for (int side = 0; side < (split ? 2 : 1); ++side) {
             const double lo = split && side == 1 ? 0.0 : va, hi = split && side == 0 ? 0.0 : vb;
-            const double rl = dp * sinh(lo), rh = dp * sinh(hi);
-            const double dr = fabs(sqrt(fma(rh, rh, d2)) - sqrt(fma(rl, rl, d2)));
-            const int np = max(1, (int)ceil(fmin(fmax((hi - lo) / 0.75, sa.ga * dr / FC), 64.0)));
+            const int np = max(1, (int)ceil(fmin((hi - lo) * sa.panels, 64.0)));
             const double ph = (hi - lo) / np;
             for (int t = g; t < 8 * np; t += L) {
                 const int p = t >> 3, i = t & 7;
@@ -961,8 +963,11 @@ int fields_run(const FieldsIn& in) {
     cudaStream_t st = c->stream;
     const size_t P = in.P, m = in.m, R = in.R, S = in.S;
     const SerGeo geo = series_geo(in.points, P, reinterpret_cast<const Seg*>(in.elec), m);
-    // a table of e^{-gamma b h} where the pairs are no fewer than its buckets
-    const size_t rows = (size_t)geo.nbk <= P * m ? (size_t)geo.nbk : 0;
+    // a table of e^{-gamma b h} where the pairs are no fewer than its buckets, or the
+    // whole table is one warp per SM quarter (5 points, 24 electrodes, one sample: 160 us
+    // with it, 166 with an exponential per pair)
+    const bool few = (size_t)geo.nbk * S <= 32 * 4 * (size_t)tags_num_sms();
+    const size_t rows = few || (size_t)geo.nbk <= P * m ? (size_t)geo.nbk : 0;
     const size_t per_sample = sizeof(double2) * (4 * R * m + P * R * 7 + 2 + FS_NT + rows) + sizeof(int);
     const size_t cs = chunk_samples(S, per_sample);
     // samples of the moment series, and those past its reach
@@ -1042,9 +1047,11 @@ int fields_run(const FieldsIn& in) {
         int* d_nt = reinterpret_cast<int*>(tab + rows * ns);
         TAGS_CUDA_OK(cudaMemcpyAsync(d_nt, nt.data() + s0, sizeof(int) * ns, cudaMemcpyHostToDevice, st));
         const int most = *std::max_element(nt.begin() + s0, nt.begin() + s0 + ns);
+        double x = 0.0;
         for (size_t k = s0; k < s0 + ns; ++k)
-            if (nt[k] > 0) sa.ga = std::max(sa.ga, std::abs(zd(in.gamma[k].re, in.gamma[k].im)));
-        sa.least = fs_least_order(sa.ga * geo.dmax);
+            if (nt[k] > 0) x = std::max(x, std::abs(zd(in.gamma[k].re, in.gamma[k].im)) * geo.dmax);
+        sa.least = fs_least_order(x);
+        sa.panels = fs_panels(x);
         if (most > 0) {
             k_fser_tables<<<dim3((unsigned)((ns + 31) / 32), (unsigned)rows + 1), 32, 0, st>>>(
                 d_gk, d_nt, (int)ns, (int)rows, geo.h, pw, tab);
