@@ -396,16 +396,16 @@ __global__ void __launch_bounds__(128) k_path_pairs(const double* __restrict__ e
 //   J(gamma) = e^{-gamma R} sum_n (-gamma)^n / n! N_n,   N_n = \int\int (r - R)^n / r dt0 dt1,
 // about R = b h, the multiple of h nearest the midpoint distance (pairs sharing
 // an endpoint: nearest (L_i + L_k) / 2), so |r - R| <= Lmax + h / 2 = dmax. The
-// moments are geometry only: one pass over the points of the direct rule (the
-// same panels; the order of the pass's largest |gamma|) serves all samples.
+// moments are geometry only: one pass over the points of a fixed rule (panels and
+// order by the distance and the pass's largest |gamma|) serves all samples.
 // A point costs ~25 + 2 nt FP64 operations once instead of a complex
 // exponential (~130) per sample, and a sample 2 nt + 20 per pair. Pairs
 // sharing an endpoint: the radial part of the Duffy rule in closed form,
 // \int_0^1 (t rho - R)^n dt = g_n / (n + 1), g_n = sum_i (rho - R)^i (-R)^(n-i).
 // Terms: x^nt / nt! <= 1e-17 at x = max |gamma| dmax (moments of 12 up to x = 0.2, of
-// 16 up to x = 0.58, else of 32, which reach x = 3.5, where the sum's largest term is e^3.5 of N_0 and
-// the rounding ~1e-14 of the entry). Samples beyond that keep an exponential per
-// point (k_fill_far).
+// 16 up to x = 0.58, else of 32, which reach x = 3.5, where the sum's largest term
+// is e^3.5 of N_0 and the rounding stays below 1e-14 of the entry). Samples beyond
+// that keep an exponential per point (k_fill_far).
 // Measured on GB300 against the direct rule for every sample: the plain form's
 // pass of 256 samples at m = 100 217 -> 24.3 ms, 100 samples at m = 10 3.50 ->
 // 0.66 ms, one sample at m = 100 through the drop-ins 11.9 -> 6.7 ms (the fill
