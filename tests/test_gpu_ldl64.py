@@ -238,3 +238,44 @@ def test_refinement_goes_on_until_rounding(gpu_pkg, length, m, sigma, s):
         scale = np.abs(want[part]).max()
         assert np.abs(x[part] - want[part]).max() <= 2e-13 * scale
         assert np.abs(sol[0][part] - want[part]).max() <= 2e-13 * scale
+
+
+@pytest.mark.parametrize("m", [15, 74, 130])
+@pytest.mark.parametrize("kind", ["s = 0", "sub-hertz", "both and usual ones"])
+@pytest.mark.parametrize("graphs", [True, False])
+def test_hard_samples_are_solved_side_by_side(gpu_pkg, m, kind, graphs):
+    """Samples that need more corrections than a pass makes, or the pivoted LU, go through those together, in plans (two
+    passes, the second shorter) and in a grid batch: launches that do not grow with their number (a LU takes four per 32
+    unknowns and two sweeps of two; the structured solve four a correction, up to 32 unknowns a launch in its sweeps),
+    and every sample against the same solved alone."""
+    pkg = gpu_pkg
+    e, nodes = pkg.segment_electrode([0.0, 0.0, -0.5], [0.08 * m, 0.0, -0.5], m, 5e-3)
+    img, ns = pkg.images(e), 60
+    N = 3 * m + 1
+    hard = 2j * np.pi * np.logspace(-2, 0, ns)
+    s = {"s = 0": np.zeros(ns, np.complex128), "sub-hertz": hard,
+         "both and usual ones": np.where(np.arange(ns) % 3 == 0, 0.0, np.where(np.arange(ns) % 3 == 1, hard, 8e4 + 1e5j))}[kind]
+    kappa = np.full(ns, 1e-4 + 0j)
+    plan = pkg.Plan(e, img, nodes, pkg.PLAIN_FP64, 40, graphs)
+    try:
+        plan.run(s, kappa, inj_node=2)                      # graphs built
+        before = pkg.launch_count()
+        sol, info, _ = plan.run(s, kappa, inj_node=2)
+        launches = pkg.launch_count() - before
+        assert not info.any()
+        panels = (N + 31) // 32 + 2
+        assert launches <= 2 * (60 + panels * (2 + 14 * 2 + 2 + 8))
+        for k in (0, 1, 2, 39, 40, 59):
+            alone, info, _ = plan.run(s[k:k + 1], kappa[k:k + 1], inj_node=2)
+            assert not info.any()
+            for part in (slice(0, m + 1), slice(m + 1, 2 * m + 1), slice(2 * m + 1, N)):
+                assert np.abs(sol[k][part] - alone[0][part]).max() <= 2e-13 * np.abs(alone[0][part]).max()
+    finally:
+        plan.close()
+    if graphs:
+        jobs = [{"electrodes": e, "images": img, "nodes": nodes, "s": s, "kappa": kappa, "inj_node": 2}]
+        (got, info), = pkg.solve_batch(jobs, precision=pkg.PLAIN_FP64)
+        assert not info.any()
+        for part in (slice(0, m + 1), slice(m + 1, 2 * m + 1), slice(2 * m + 1, N)):
+            scale = np.abs(sol[:, part]).max(axis=1)
+            assert (np.abs(got[:, part] - sol[:, part]).max(axis=1) <= 2e-13 * scale).all()

@@ -384,12 +384,9 @@ int tags_sym_solve_host(const tags_cdouble* w, tags_cdouble* x, size_t m, size_t
     if (!d_W || !d_A || !d_x || !ws) return 0;           // no room for two matrices: the LU needs one
     TAGS_CUDA_OK(cudaMemcpyAsync(d_W, w, sizeof(double2) * N * N, cudaMemcpyHostToDevice, st));
     TAGS_CUDA_OK(cudaMemcpyAsync(d_x, x, sizeof(double2) * N, cudaMemcpyHostToDevice, st));
-    int err = tags_symmetrize_lower(d_W, (int)N, (long long)N, 0, 1, st);
-    if (!err) err = tags_ldl64_sym_solve(d_W, d_A, (int)m, (int)n, ws, c->status, d_x, c->status + 1, st);
+    int err = tags_symmetrize_lower(d_W, (int)N, (long long)N, 0, 1, st), info = 0;
+    if (!err) err = tags_ldl64_sym_solve(d_W, d_A, (int)m, (int)n, ws, c->status, d_x, &info, st);
     if (err) return err;
-    int info = 0;
-    TAGS_CUDA_OK(cudaMemcpyAsync(&info, c->status + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-    TAGS_CUDA_OK(cudaStreamSynchronize(st));
     if (info != 0) return 0;
     TAGS_CUDA_OK(cudaMemcpyAsync(x, d_x, sizeof(double2) * N, cudaMemcpyDeviceToHost, st));
     TAGS_CUDA_OK(cudaStreamSynchronize(st));

@@ -330,8 +330,13 @@ extern "C" int tags_batch_run(tags_batch batch, const tags_grid_job* jobs, size_
     acc.split = b->precision == TAGS_PLAIN_FP64 ? 0 : TAGS_SPLIT_F16;
     long long launched = b->launches_fixed;
     int first_err = 0, all_status = 0;
-    std::vector<std::vector<int>> failed(njobs);          // per grid: samples for the FP64 re-solve
-    std::vector<int> grid_status(njobs, 0);
+    // per grid: samples for the FP64 re-solve, and for the pivoted LU. The grids'
+    // buffers for them stay with the batch, 2 GB between them or one sample each.
+    std::vector<std::vector<int>> failed(njobs), pivoted(njobs);
+    const size_t most = std::min<size_t>((size_t)512 << 20, ((size_t)2 << 30) / njobs);
+    auto sweep = [&](const GridSlot& g) {
+        return ResolveSweep{g.d_s, g.d_k, g.has_ie ? g.d_ie : nullptr, b->mur, (int)g.inj};
+    };
     for (size_t q = 0; q < njobs; ++q) {
         const tags_grid_job& j = jobs[q];
         GridSlot& g = b->grids[q];
@@ -341,7 +346,6 @@ extern "C" int tags_batch_run(tags_batch batch, const tags_grid_job* jobs, size_
         int gst = 0;
         TAGS_CUDA_OK(cudaMemcpy(&gst, p->d_status, sizeof(int), cudaMemcpyDeviceToHost));
         all_status |= gst;
-        grid_status[q] = gst;
         if (b->precision != TAGS_PLAIN_FP64 && !gst) {
             const int bc = p->batch;
             std::vector<int> si((size_t)g.passes * (3 * bc + 2)), se(2 * (size_t)g.passes);
@@ -379,53 +383,49 @@ extern "C" int tags_batch_run(tags_batch batch, const tags_grid_job* jobs, size_
                     failed[q].push_back(k0 + s);
                 }
             }
-            // queued on the grid's own stream: the grids' re-solves, chains of
-            // small launches, run side by side. Their buffers stay with the batch,
-            // 2 GB between the grids (or one sample each).
-            if (!failed[q].empty())
-                if (int e = tags_mixed_fallback_start(p, failed[q], g.d_s, g.d_k, b->mur, g.has_ie ? g.d_ie : nullptr,
-                                                      (int)g.inj, g.d_sol, g.d_info,
-                                                      std::min<size_t>((size_t)512 << 20, ((size_t)2 << 30) / njobs),
-                                                      p->stream))
-                    return e;
+        } else if (gst & TAGS_ST_DEGENERATE_PAIR) {
+            // plain form: every sample of the grid is NaN, as after a plan's run
+            if (b->precision == TAGS_PLAIN_FP64) TAGS_CUDA_OK(cudaMemset(g.d_info, 0, sizeof(int) * g.ns));
+        } else if (b->precision == TAGS_PLAIN_FP64) {
+            std::vector<int> si(g.ns);
+            TAGS_CUDA_OK(cudaMemcpy(si.data(), g.d_info, sizeof(int) * g.ns, cudaMemcpyDeviceToHost));
+            for (int k = 0; k < g.ns; ++k) {
+                if (si[k] == TAGS_INFO_MORE) failed[q].push_back(k);
+                if (si[k] == TAGS_INFO_RESOLVE) pivoted[q].push_back(k);
+            }
         }
+        // queued on the grid's own stream: the grids' re-solves, chains of small
+        // launches, run side by side
+        const int steps = b->precision == TAGS_PLAIN_FP64 ? TAGS_RESOLVE_STEPS : TAGS_FIRST_STEPS;
+        if (int e = tags_resolve_sweep_ldl(p, failed[q], sweep(g), steps, g.d_sol, g.d_info, most, p->stream)) return e;
+    }
+    // what those ask for next: further corrections, grid by grid in rounds, then the
+    // pivoted LU
+    for (bool more = true; more;) {
+        more = false;
+        for (size_t q = 0; q < njobs; ++q) {
+            if (failed[q].empty()) continue;
+            GridSlot& g = b->grids[q];
+            TAGS_CUDA_OK(cudaStreamSynchronize(g.plan->stream));
+            std::vector<int> si(g.ns), rest;
+            TAGS_CUDA_OK(cudaMemcpy(si.data(), g.d_info, sizeof(int) * g.ns, cudaMemcpyDeviceToHost));
+            for (int k : failed[q]) {
+                if (si[k] == TAGS_INFO_MORE) rest.push_back(k);
+                if (si[k] == TAGS_INFO_RESOLVE) pivoted[q].push_back(k);
+            }
+            failed[q] = rest;
+            if (int e = tags_resolve_sweep_more(g.plan, rest, sweep(g), g.d_sol, g.d_info, most, g.plan->stream)) return e;
+            more = more || !rest.empty();
+        }
+    }
+    for (size_t q = 0; q < njobs; ++q) {
+        GridSlot& g = b->grids[q];
+        if (int e = tags_resolve_sweep_lu(g.plan, pivoted[q], sweep(g), g.d_sol, g.d_info, most, g.plan->stream)) return e;
     }
     for (size_t q = 0; q < njobs; ++q) {
         const tags_grid_job& j = jobs[q];
         GridSlot& g = b->grids[q];
-        tags_plan_s* p = g.plan;
-        if (!failed[q].empty()) {
-            TAGS_CUDA_OK(cudaStreamSynchronize(p->stream));
-            std::vector<int> si(g.ns);
-            TAGS_CUDA_OK(cudaMemcpy(si.data(), g.d_info, sizeof(int) * g.ns, cudaMemcpyDeviceToHost));
-            for (int k : failed[q]) {
-                if (si[k] != TAGS_INFO_RESOLVE) continue;
-                int e = tags_mixed_fallback_lu(p, g.d_s + k, g.d_k + k, b->mur,
-                                               g.has_ie ? g.d_ie + (size_t)k * g.n : nullptr, (int)g.inj,
-                                               g.d_sol + (size_t)k * g.N, g.d_info + k, p->stream);
-                if (e) return e;
-            }
-            TAGS_CUDA_OK(cudaStreamSynchronize(p->stream));
-        } else if (b->precision == TAGS_PLAIN_FP64 && (grid_status[q] & TAGS_ST_DEGENERATE_PAIR)) {
-            // every sample of the grid is NaN, as after a plan's run
-            TAGS_CUDA_OK(cudaMemset(g.d_info, 0, sizeof(int) * g.ns));
-        } else if (b->precision == TAGS_PLAIN_FP64) {
-            // plain form: samples marked for the pivoted LU
-            std::vector<int> si(g.ns);
-            TAGS_CUDA_OK(cudaMemcpy(si.data(), g.d_info, sizeof(int) * g.ns, cudaMemcpyDeviceToHost));
-            for (int k = 0; k < g.ns; ++k) {
-                if (si[k] != TAGS_INFO_RESOLVE) continue;
-                if (!p->d_ipiv) TAGS_CUDA_OK(cudaMalloc(&p->d_ipiv, sizeof(int) * (p->N + 1)));
-                int e = tags_plan_coef(p, g.d_s + k, g.d_k + k, b->mur, 1, p->stream);
-                if (!e) e = tags_plan_rhs(p, p->d_x, g.has_ie ? g.d_ie + (size_t)k * g.n : nullptr, (int)g.inj, 1, p->stream);
-                if (!e) e = tags_plan_lu_one(p, 0, p->d_W, p->d_ipiv, p->d_x, p->d_info, p->stream);
-                if (e) return e;
-                TAGS_CUDA_OK(cudaMemcpyAsync(g.d_sol + (size_t)k * g.N, p->d_x, sizeof(double2) * g.N,
-                                             cudaMemcpyDeviceToDevice, p->stream));
-                TAGS_CUDA_OK(cudaMemcpyAsync(g.d_info + k, p->d_info, sizeof(int), cudaMemcpyDeviceToDevice, p->stream));
-            }
-            TAGS_CUDA_OK(cudaStreamSynchronize(p->stream));
-        }
+        if (!pivoted[q].empty()) TAGS_CUDA_OK(cudaStreamSynchronize(g.plan->stream));
         if (j.sol)
             TAGS_CUDA_OK(cudaMemcpy(j.sol, g.d_sol, sizeof(double2) * (size_t)g.ns * g.N, cudaMemcpyDeviceToHost));
         if (j.info) {

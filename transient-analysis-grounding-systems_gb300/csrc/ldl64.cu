@@ -610,21 +610,16 @@ __global__ void __launch_bounds__(256) k_ldl64_apply(const double2* __restrict__
     if (state != 0) active[b] = 0;
 }
 
-// Solutions to the original order; info 0, or the marker of a sample that
-// needs the pivoted LU.
-__global__ void k_ldl64_out(const double2* __restrict__ X0, int m, int n, const int* __restrict__ conv,
-                            double2* __restrict__ out, long long ostride, int* __restrict__ info) {
+// Solutions to the original order; info 0, or the mark of a sample that needs more
+// corrections (its last one still contracted) or the pivoted LU.
+__global__ void k_ldl64_out(const double2* __restrict__ X0, int m, int n, const int* __restrict__ active,
+                            const int* __restrict__ conv, double2* __restrict__ out, long long ostride,
+                            int* __restrict__ info) {
     const int N = n + 2 * m, b = blockIdx.y;
     const int ip = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ip == 0) info[b] = conv[b] ? 0 : TAGS_INFO_RESOLVE;
+    if (ip == 0) info[b] = conv[b] ? 0 : active[b] ? TAGS_INFO_MORE : TAGS_INFO_RESOLVE;
     if (ip >= N) return;
     out[ostride * b + orig_index(ip, m, n)] = X0[(long long)N * b + ip];
-}
-
-// The saved right-hand side of one sample back to the original order.
-__global__ void k_ldl64_rhs_back(const double2* __restrict__ B, int m, int n, double2* __restrict__ out) {
-    const int ip = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ip < n + 2 * m) out[orig_index(ip, m, n)] = B[ip];
 }
 
 // ---- the plan's system: impedance blocks in the coupling blocks, sparse incidence
@@ -766,7 +761,7 @@ __global__ void __launch_bounds__(128) k_ldl64_small(const double2* __restrict__
     }
     __syncthreads();
     double prev[2] = {0.0, 0.0};
-    for (int step = 0; step < 4; ++step) {
+    for (int step = 0; step < TAGS_RESOLVE_STEPS; ++step) {
         if (step > 0) {
             for (int i = tid; i < N; i += 128) {
                 double2 a = cz(0.0, 0.0), u = cz(0.0, 0.0);
@@ -810,7 +805,7 @@ __global__ void __launch_bounds__(128) k_ldl64_small(const double2* __restrict__
             mx.take(i < 2 * m, d, v);
         }
         maxima_reduce<4>(mx, smx);
-        if (tid == 0) sstate = step_state(mx, step, step == 3, prev);
+        if (tid == 0) sstate = step_state(mx, step, step + 1 == TAGS_RESOLVE_STEPS, prev);
         __syncthreads();
         if (sstate) break;
     }
@@ -1160,8 +1155,6 @@ int solve(const double2* A, int N, long long ld, long long stride, int nb, int m
     return 0;
 }
 
-constexpr int MAX_CORRECTIONS = 4;         // x itself and up to three refinements
-
 }  // namespace
 
 // Kernel attributes, once per device, before any launch and any graph capture.
@@ -1203,8 +1196,30 @@ FillOut tags_ldl64_fill_out(double2* W, int m, int n) {
     return out;
 }
 
+// Corrections [from, to) of the plan's system, then the solutions and info.
+static int corrections(const double2* W, const Incidence& inc, int m, int n, int nb, const Ws& w, int from, int to,
+                       double2* x, int* info, cudaStream_t st) {
+    const int N = n + 2 * m;
+    const long long NN = (long long)N * N;
+    for (int step = from; step < to; ++step) {
+        if (step > 0) {
+            k_ldl64_resid_z<<<dim3((m + 63) / 64, 2, nb), 64, 0, st>>>(W, N, NN, inc, m, n, w.b, w.x, w.r, w.active);
+            k_ldl64_resid_nodes<<<dim3((n + 127) / 128, nb), 128, 0, st>>>(inc, m, n, w.b, w.x, w.r, w.active);
+            tags_note_launch(2);
+        }
+        if (int e = solve(W, N, N, NN, nb, m, w, step == 0 ? 2 * m : 0, st)) return e;
+        k_ldl64_apply<<<nb, 256, 0, st>>>(w.z, w.x, N, 2 * m, step, step + 1 == TAGS_RESOLVE_STEPS, w.active, w.conv,
+                                          w.prev);
+        tags_note_launch();
+    }
+    k_ldl64_out<<<dim3((N + 127) / 128, nb), 128, 0, st>>>(w.x, m, n, w.active, w.conv, x, N, info);
+    tags_note_launch();
+    TAGS_CUDA_OK(cudaGetLastError());
+    return 0;
+}
+
 int tags_ldl64_plan_solve(double2* W, const Incidence& inc, int m, int n, int nb, int batch, void* ws,
-                          const double2* rhs, double2* x, int* info, cudaStream_t st) {
+                          const double2* rhs, double2* x, int* info, int steps, cudaStream_t st) {
     if (int e = tags_ldl64_prepare()) return e;
     const int N = n + 2 * m;
     const long long NN = (long long)N * N;
@@ -1218,64 +1233,54 @@ int tags_ldl64_plan_solve(double2* W, const Incidence& inc, int m, int n, int nb
     k_ldl64_start<<<dim3((N + 127) / 128, nb), 128, 0, st>>>(rhs, N, m, n, w.b, w.r, w.x, w.active, w.conv);
     k_ldl64_build<<<dim3(N, nb), 128, 0, st>>>(W, N, NN, inc, m, n);
     tags_note_launch(2);
-    int err = factor(W, N, N, NN, nb, m, w, st);
-    for (int step = 0; step < MAX_CORRECTIONS && !err; ++step) {
-        if (step > 0) {
-            k_ldl64_resid_z<<<dim3((m + 63) / 64, 2, nb), 64, 0, st>>>(W, N, NN, inc, m, n, w.b, w.x, w.r, w.active);
-            k_ldl64_resid_nodes<<<dim3((n + 127) / 128, nb), 128, 0, st>>>(inc, m, n, w.b, w.x, w.r, w.active);
-            tags_note_launch(2);
-        }
-        err = solve(W, N, N, NN, nb, m, w, step == 0 ? 2 * m : 0, st);
-        if (err) break;
-        k_ldl64_apply<<<nb, 256, 0, st>>>(w.z, w.x, N, 2 * m, step, step + 1 == MAX_CORRECTIONS, w.active, w.conv,
-                                          w.prev);
-        tags_note_launch();
-    }
-    if (err) return err;
-    k_ldl64_out<<<dim3((N + 127) / 128, nb), 128, 0, st>>>(w.x, m, n, w.conv, x, N, info);
-    tags_note_launch();
-    TAGS_CUDA_OK(cudaGetLastError());
-    return 0;
+    const int err = factor(W, N, N, NN, nb, m, w, st);
+    return err ? err : corrections(W, inc, m, n, nb, w, 0, steps, x, info, st);
 }
 
-int tags_ldl64_saved_rhs(void* ws, int m, int n, int batch, int q, double2* out, cudaStream_t st) {
-    const int N = n + 2 * m;
-    const Ws w = carve(ws, N, batch);
-    k_ldl64_rhs_back<<<(N + 127) / 128, 128, 0, st>>>(w.b + (long long)N * q, m, n, out);
-    tags_note_launch();
-    TAGS_CUDA_OK(cudaGetLastError());
-    return 0;
+int tags_ldl64_plan_more(const double2* W, const Incidence& inc, int m, int n, int nb, int batch, void* ws, int* step,
+                         double2* x, int* info, cudaStream_t st) {
+    const int from = *step;
+    *step = std::min(from + 2, TAGS_RESOLVE_STEPS);
+    return corrections(W, inc, m, n, nb, carve(ws, n + 2 * m, batch), from, *step, x, info, st);
 }
 
-int tags_ldl64_sym_solve(const double2* W, double2* A, int m, int n, void* ws, int* d_flag, double2* x, int* info,
+const double2* tags_ldl64_saved_rhs(void* ws, int N, int batch) { return carve(ws, N, batch).b; }
+
+int tags_ldl64_sym_solve(const double2* W, double2* A, int m, int n, void* ws, int* d_words, double2* x, int* info,
                          cudaStream_t st) {
     if (int e = tags_ldl64_prepare()) return e;
     const int N = n + 2 * m;
     const Ws w = carve(ws, N, 1);
-    TAGS_CUDA_OK(cudaMemsetAsync(d_flag, 0, sizeof(int), st));
+    TAGS_CUDA_OK(cudaMemsetAsync(d_words, 0, sizeof(int), st));
     k_ldl64_start<<<dim3((N + 127) / 128, 1), 128, 0, st>>>(x, N, m, n, w.b, w.r, w.x, w.active, w.conv);
-    k_ldl64_permute<<<dim3(N, (N + 127) / 128), 128, 0, st>>>(W, A, m, n, d_flag);
+    k_ldl64_permute<<<dim3(N, (N + 127) / 128), 128, 0, st>>>(W, A, m, n, d_words);
     tags_note_launch(2);
     int coupled = 0;
-    TAGS_CUDA_OK(cudaMemcpyAsync(&coupled, d_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    TAGS_CUDA_OK(cudaMemcpyAsync(&coupled, d_words, sizeof(int), cudaMemcpyDeviceToHost, st));
     TAGS_CUDA_OK(cudaStreamSynchronize(st));
     const int zm = coupled ? 0 : m;          // the structure skipped by the elimination, if it is there
     int err = factor(A, N, N, 0, 1, zm, w, st);
-    for (int step = 0; step < 3 && !err; ++step) {
-        if (step > 0) {
-            k_ldl64_resid_full<<<(N + 3) / 4, 128, 0, st>>>(W, m, n, w.b, w.x, w.r, w.active);
+    // three corrections, and where they still contract without having settled, more
+    *info = TAGS_INFO_MORE;
+    for (int step = 0; *info == TAGS_INFO_MORE && !err;) {
+        for (const int end = step == 0 ? 3 : TAGS_RESOLVE_STEPS; step < end && !err; ++step) {
+            if (step > 0) {
+                k_ldl64_resid_full<<<(N + 3) / 4, 128, 0, st>>>(W, m, n, w.b, w.x, w.r, w.active);
+                tags_note_launch();
+            }
+            err = solve(A, N, N, 0, 1, zm, w, 0, st);
+            if (err) return err;
+            k_ldl64_apply<<<1, 256, 0, st>>>(w.z, w.x, N, 2 * m, step, step + 1 == TAGS_RESOLVE_STEPS, w.active, w.conv,
+                                             w.prev);
             tags_note_launch();
         }
-        err = solve(A, N, N, 0, 1, zm, w, 0, st);
-        if (err) break;
-        k_ldl64_apply<<<1, 256, 0, st>>>(w.z, w.x, N, 2 * m, step, step == 2, w.active, w.conv, w.prev);
+        k_ldl64_out<<<dim3((N + 127) / 128, 1), 128, 0, st>>>(w.x, m, n, w.active, w.conv, x, N, d_words + 1);
         tags_note_launch();
+        TAGS_CUDA_OK(cudaGetLastError());
+        TAGS_CUDA_OK(cudaMemcpyAsync(info, d_words + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+        TAGS_CUDA_OK(cudaStreamSynchronize(st));
     }
-    if (err) return err;
-    k_ldl64_out<<<dim3((N + 127) / 128, 1), 128, 0, st>>>(w.x, m, n, w.conv, x, N, info);
-    tags_note_launch();
-    TAGS_CUDA_OK(cudaGetLastError());
-    return 0;
+    return err;
 }
 
 bool tags_ldl64_multi_fits(int M) { return mcols_smem(M, 1) <= MCOLS_SMEM; }

@@ -626,200 +626,6 @@ int tags_mixed_free(tags_plan_s* p) {
     return 0;
 }
 
-// ---- FP64 re-solves of samples that did not converge -----------------------------
-
-namespace {
-
-// Inputs of the samples idx[0..) side by side: their coefficients and
-// right-hand sides (a plan's pass).
-__global__ void k_fb_gather(const int* __restrict__ idx, const SampleCoef* __restrict__ coef,
-                            const double2* __restrict__ rhs, int N, SampleCoef* __restrict__ coef_out,
-                            double2* __restrict__ rhs_out) {
-    const int b = blockIdx.y, q = idx[b], r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r == 0) coef_out[b] = coef[q];
-    if (r < N) rhs_out[(size_t)b * N + r] = rhs[(size_t)q * N + r];
-}
-
-// The same from a sweep's arrays (a grid batch): s and kappa, and the
-// right-hand sides [ie; 0; 0] or a unit current at inj.
-__global__ void k_fb_inputs(const int* __restrict__ idx, const double2* __restrict__ s,
-                            const double2* __restrict__ kappa, const double2* __restrict__ ie, int inj, int n, int N,
-                            double2* __restrict__ s_out, double2* __restrict__ kappa_out,
-                            double2* __restrict__ rhs_out) {
-    const int b = blockIdx.y, q = idx[b], r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r == 0) {
-        s_out[b] = s[q];
-        kappa_out[b] = kappa[q];
-    }
-    if (r >= N) return;
-    double2 v = make_double2(0.0, 0.0);
-    if (r < n) {
-        if (ie) v = ie[(size_t)q * n + r];
-        else if (r == inj) v = make_double2(1.0, 0.0);
-    }
-    rhs_out[(size_t)b * N + r] = v;
-}
-
-__global__ void k_fb_scatter(const int* __restrict__ idx, const double2* __restrict__ x, const int* __restrict__ info,
-                             int N, double2* __restrict__ x_out, int* __restrict__ info_out) {
-    const int b = blockIdx.y, q = idx[b], r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r == 0) info_out[q] = info[b];
-    if (r < N) x_out[(size_t)q * N + r] = x[(size_t)b * N + r];
-}
-
-// The re-solves' buffers in p->d_fb, for fb_cap samples at a time.
-struct FbView {
-    double2* W;          // matrices (the pivoted LU of one sample too)
-    char* ldl;
-    char* series;
-    SampleCoef* coef;
-    double2 *sk, *rhs;   // s and kappa (2 cap), right-hand sides and solutions (cap x N)
-    int *info, *idx, *ipiv;
-};
-
-size_t up256(size_t v) { return (v + 255) / 256 * 256; }
-
-size_t fb_bytes(const tags_plan_s* p, int cap, FbView* v) {
-    const size_t N = p->N;
-    char* b = reinterpret_cast<char*>(p->d_fb);
-    size_t o = 0;
-    auto take = [&](size_t bytes) {
-        char* r = b ? b + o : nullptr;
-        o += up256(bytes);
-        return r;
-    };
-    FbView w;
-    w.W = reinterpret_cast<double2*>(take(sizeof(double2) * N * N * cap));
-    w.ldl = take(tags_ldl64_workspace((int)N, cap));
-    w.series = take(tags_series_workspace(p->series, cap));
-    w.coef = reinterpret_cast<SampleCoef*>(take(sizeof(SampleCoef) * cap));
-    w.sk = reinterpret_cast<double2*>(take(sizeof(double2) * 2 * cap));
-    w.rhs = reinterpret_cast<double2*>(take(sizeof(double2) * N * cap));
-    w.info = reinterpret_cast<int*>(take(sizeof(int) * cap));
-    w.idx = reinterpret_cast<int*>(take(sizeof(int) * cap));
-    w.ipiv = reinterpret_cast<int*>(take(sizeof(int) * (N + 1)));
-    if (v) *v = w;
-    return o;
-}
-
-// Room for up to `want` samples at a time: at most 64, `most` bytes and an eighth
-// of the free memory, at least one. Kept with the plan, grown when more is asked;
-// the buffer that is there goes only when the larger one has been had.
-int fb_alloc(tags_plan_s* p, int want, size_t most) {
-    want = std::min(want, 64);
-    if (p->fb_cap >= want || (p->fb_cap > 0 && p->fb_full)) return 0;
-    if (p->series.nbk == 0)
-        p->series = tags_series_geometry(p->h_elec.data(), p->m, p->h_img.data(), p->h_img.empty() ? 0 : p->m);
-    size_t freeb = 0;
-    TAGS_CUDA_OK(tags_free_memory(&freeb));
-    const size_t one = fb_bytes(p, 1, nullptr);
-    int cap = (int)std::max<size_t>(1, std::min<size_t>((size_t)want, std::min(most, freeb / 8) / one));
-    void* buf = nullptr;
-    for (; cap > p->fb_cap; cap /= 2) {
-        if (cudaMalloc(&buf, fb_bytes(p, cap, nullptr)) == cudaSuccess) break;
-        cudaGetLastError();
-        buf = nullptr;
-    }
-    if (!buf) {
-        p->fb_full = 1;
-        return p->fb_cap > 0 ? 0 : tags_fail(TAGS_E_NOMEM, "device allocation failed (FP64 fallback)");
-    }
-    if (p->d_fb) {
-        TAGS_CUDA_OK(cudaStreamSynchronize(p->stream));
-        TAGS_CUDA_OK(cudaFree(p->d_fb));
-    }
-    p->d_fb = buf;
-    p->fb_cap = cap;
-    p->fb_full = cap < want;
-    FbView v;
-    fb_bytes(p, cap, &v);
-    if (p->series.nbk) {
-        p->d_series = v.series;
-        p->series_ns = cap;
-    }
-    return 0;
-}
-
-// The samples whose inputs are in v.coef and v.rhs [0, nf): the structured
-// LDL^T (ldl64.cu), solutions and info to sample idx[..] of x and info.
-int fb_solve(tags_plan_s* p, const FbView& v, int nf, double2* x, int* info, cudaStream_t st) {
-    int err = tags_plan_fill_fp64(p, v.coef, nf, tags_ldl64_fill_out(v.W, p->m, p->n), st);
-    if (!err) err = tags_ldl64_plan_solve(v.W, p->inc, p->m, p->n, nf, p->fb_cap, v.ldl, v.rhs, v.rhs, v.info, st);
-    if (err) return err;
-    k_fb_scatter<<<dim3((p->N + 255) / 256, nf), 256, 0, st>>>(v.idx, v.rhs, v.info, p->N, x, info);
-    tags_note_launch();
-    TAGS_CUDA_OK(cudaGetLastError());
-    return 0;
-}
-
-}  // namespace
-
-// Re-solve samples `idx` of the current pass in plain FP64, side by side: the
-// structured LDL^T with refinement, and where that does not converge the LU
-// with partial pivoting.
-static int fallback_plain(tags_plan_s* p, const std::vector<int>& idx, cudaStream_t st) {
-    TagsRange range("tags FP64 re-solve");
-    const size_t N = p->N;
-    if (int e = fb_alloc(p, (int)idx.size(), (size_t)512 << 20)) return e;
-    FbView v;
-    fb_bytes(p, p->fb_cap, &v);
-    const double2* bvec = p->d_r + (size_t)p->batch * N;
-    for (size_t k0 = 0; k0 < idx.size(); k0 += p->fb_cap) {
-        const int nf = (int)std::min<size_t>(p->fb_cap, idx.size() - k0);
-        TAGS_CUDA_OK(cudaMemcpyAsync(v.idx, idx.data() + k0, sizeof(int) * nf, cudaMemcpyHostToDevice, st));
-        k_fb_gather<<<dim3((unsigned)((N + 255) / 256), nf), 256, 0, st>>>(v.idx, p->d_coef, bvec, (int)N, v.coef, v.rhs);
-        tags_note_launch();
-        if (int e = fb_solve(p, v, nf, p->d_x, p->d_info, st)) return e;
-    }
-    std::vector<int> info(p->batch);
-    TAGS_CUDA_OK(cudaMemcpyAsync(info.data(), p->d_info, sizeof(int) * p->batch, cudaMemcpyDeviceToHost, st));
-    TAGS_CUDA_OK(cudaStreamSynchronize(st));
-    for (int q : idx) {
-        if (info[q] != TAGS_INFO_RESOLVE) continue;
-        TAGS_CUDA_OK(cudaMemcpyAsync(p->d_x + q * N, bvec + q * N, sizeof(double2) * N, cudaMemcpyDeviceToDevice, st));
-        if (int e = tags_plan_lu_one(p, q, v.W, v.ipiv, p->d_x + q * N, p->d_info + q, st)) return e;
-    }
-    return 0;
-}
-
-int tags_plan_rhs(tags_plan_s* p, double2* d_X, const double2* d_ie, int inj_node, int nb, cudaStream_t st);
-int tags_plan_coef(tags_plan_s* p, const double2* d_s, const double2* d_kappa, double mur, int nb, cudaStream_t st);
-
-int tags_mixed_fallback_start(tags_plan_s* p, const std::vector<int>& idx, const double2* d_s, const double2* d_kappa,
-                              double mur, const double2* d_ie, int inj_node, double2* x, int* info, size_t most,
-                              cudaStream_t st) {
-    const size_t N = p->N;
-    if (int e = fb_alloc(p, (int)idx.size(), most)) return e;
-    FbView v;
-    fb_bytes(p, p->fb_cap, &v);
-    for (size_t k0 = 0; k0 < idx.size(); k0 += std::min(p->fb_cap, p->batch)) {
-        const int nf = (int)std::min<size_t>(std::min(p->fb_cap, p->batch), idx.size() - k0);
-        TAGS_CUDA_OK(cudaMemcpyAsync(v.idx, idx.data() + k0, sizeof(int) * nf, cudaMemcpyHostToDevice, st));
-        k_fb_inputs<<<dim3((unsigned)((N + 255) / 256), nf), 256, 0, st>>>(v.idx, d_s, d_kappa, d_ie, inj_node, p->n,
-                                                                        (int)N, v.sk, v.sk + p->fb_cap, v.rhs);
-        tags_note_launch();
-        int err = tags_plan_coef(p, v.sk, v.sk + p->fb_cap, mur, nf, st);
-        if (err) return err;
-        TAGS_CUDA_OK(cudaMemcpyAsync(v.coef, p->d_coef, sizeof(SampleCoef) * nf, cudaMemcpyDeviceToDevice, st));
-        err = fb_solve(p, v, nf, x, info, st);
-        if (err) return err;
-    }
-    return 0;
-}
-
-int tags_mixed_fallback_lu(tags_plan_s* p, const double2* d_s, const double2* d_kappa, double mur, const double2* d_ie,
-                           int inj_node, double2* x_out, int* info_out, cudaStream_t st) {
-    FbView v;
-    fb_bytes(p, p->fb_cap, &v);
-    int err = tags_plan_coef(p, d_s, d_kappa, mur, 1, st);          // coefficients in slot 0
-    if (!err) err = tags_plan_rhs(p, v.rhs, d_ie, inj_node, 1, st);
-    if (!err) err = tags_plan_lu_one(p, 0, v.W, v.ipiv, v.rhs, v.info, st);
-    if (err) return err;
-    TAGS_CUDA_OK(cudaMemcpyAsync(x_out, v.rhs, sizeof(double2) * p->N, cudaMemcpyDeviceToDevice, st));
-    TAGS_CUDA_OK(cudaMemcpyAsync(info_out, v.info, sizeof(int), cudaMemcpyDeviceToDevice, st));
-    return 0;
-}
-
 // ---- one pass of nb samples, in four stages -------------------------------------
 // The right-hand side b is in d_x when a pass starts (written by the plan).
 
@@ -972,7 +778,8 @@ int tags_mixed_finish(tags_plan_s* p, int nb, cudaStream_t st, int* h_iters, dou
         h_berr[q] = ird[2 * b + q];
         if (!h_conv[q]) failed.push_back(q);
     }
-    return failed.empty() ? 0 : fallback_plain(p, failed, st);
+    const ResolveInputs in{p->d_coef, p->d_r + (size_t)p->batch * p->N, 0};
+    return tags_resolve_pass(p, failed, {}, in, p->d_x, p->d_info, st);
 }
 
 int tags_plan_coef(tags_plan_s* p, const double2* d_s, const double2* d_kappa, double mur, int nb, cudaStream_t st);

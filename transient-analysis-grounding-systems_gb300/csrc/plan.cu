@@ -160,7 +160,7 @@ static void plan_free(tags_plan_s* p) {
     if (!p) return;
     cudaSetDevice(p->device);
     if (p->stream) cudaStreamSynchronize(p->stream);
-    void* ptrs[] = {p->d_elec, p->d_img, p->d_cond, p->d_coef, p->d_status, p->d_info, p->d_ipiv, p->d_W, p->d_x,
+    void* ptrs[] = {p->d_elec, p->d_img, p->d_cond, p->d_coef, p->d_status, p->d_info, p->d_W, p->d_x,
                     p->inc.node_ptr, p->inc.node_seg, p->inc.node_a, p->inc.seg_ptr, p->inc.seg_node, p->inc.seg_a};
     for (void* q : ptrs)
         if (q) cudaFree(q);
@@ -312,41 +312,20 @@ extern "C" int tags_plan_set_fill(tags_plan plan, int integration_type) {
 
 // Plain FP64 pass over nb samples whose coefficients and right-hand sides are
 // already in p->d_coef and p->d_x: fill, LDL^T in the static order, refinement.
-// info of a sample that needs the pivoted LU is TAGS_INFO_RESOLVE
-// (tags_plan_finish_plain).
+// info of a sample that needs more steps or the pivoted LU says so (finish_plain).
 int tags_plan_run_plain(tags_plan_s* p, const double2*, int nb, cudaStream_t st) {
     TagsRange range("tags fill");
     int err = tags_plan_fill_fp64(p, p->d_coef, nb, tags_ldl64_fill_out(p->d_W, p->m, p->n), st);
     if (err) return err;
     range.next("tags factor");
-    return tags_ldl64_plan_solve(p->d_W, p->inc, p->m, p->n, nb, p->batch, p->d_ldl64, p->d_x, p->d_x, p->d_info, st);
+    return tags_ldl64_plan_solve(p->d_W, p->inc, p->m, p->n, nb, p->batch, p->d_ldl64, p->d_x, p->d_x, p->d_info,
+                                 TAGS_PASS_STEPS, st);
 }
 
-// W_G of sample q's coefficients, its LU with partial pivoting and the solve.
-int tags_plan_lu_one(tags_plan_s* p, int q, double2* W, int* ipiv, double2* x, int* info, cudaStream_t st) {
-    const long long N = p->N, NN = N * N;
-    TagsRange range("tags FP64 re-solve");
-    TAGS_CUDA_OK(cudaMemsetAsync(W, 0, sizeof(double2) * NN, st));
-    int err = tags_wg_incidence(W, N, NN, 1, p->d_cond, p->n, p->m, st);
-    if (err) return err;
-    FillOut out{};
-    out.zl = W;
-    out.zt = W;
-    out.ld = N;
-    out.batch_stride = NN;
-    out.row0_l = out.col0_l = p->n;
-    out.row0_t = out.col0_t = p->n + p->m;
-    out.sign = -1.0;
-    out.mirror = 1;
-    err = tags_plan_fill_fp64(p, p->d_coef + q, 1, out, st);
-    if (!err) err = tags_lu_z(W, (int)N, N, NN, 1, ipiv, info, st);
-    return err ? err : tags_lu_solve_z(W, (int)N, N, NN, 1, ipiv, x, 1, N, N, st);
-}
-
-// After a plain pass: samples marked for the pivoted LU are solved by it, one
-// by one in the first sample's matrix, whatever another sample's values brought
-// into the status. Only a geometry whose integrals diverge, which makes every
-// sample of the run NaN, is left as it is.
+// After a plain pass: its samples marked for more refinement or for the pivoted
+// LU are solved side by side, whatever another sample's values brought into the
+// status. Only a geometry whose integrals diverge, which makes every sample of the
+// run NaN, is left as it is.
 static int finish_plain(tags_plan_s* p, int nb, cudaStream_t st) {
     std::vector<int> info(nb);
     int status = 0;
@@ -357,15 +336,18 @@ static int finish_plain(tags_plan_s* p, int nb, cudaStream_t st) {
         TAGS_CUDA_OK(cudaMemsetAsync(p->d_info, 0, sizeof(int) * nb, st));
         return 0;
     }
-    for (int q = 0; q < nb; ++q) {
-        if (info[q] != TAGS_INFO_RESOLVE) continue;
-        double2* x = p->d_x + (size_t)q * p->N;
-        if (!p->d_ipiv) TAGS_CUDA_OK(cudaMalloc(&p->d_ipiv, sizeof(int) * (p->N + 1)));
-        int err = tags_ldl64_saved_rhs(p->d_ldl64, p->m, p->n, p->batch, q, x, st);
-        if (!err) err = tags_plan_lu_one(p, q, p->d_W, p->d_ipiv, x, p->d_info + q, st);
-        if (err) return err;
+    // corrections go on where the pass left them
+    for (int step = TAGS_PASS_STEPS; std::find(info.begin(), info.end(), TAGS_INFO_MORE) != info.end();) {
+        if (int e = tags_ldl64_plan_more(p->d_W, p->inc, p->m, p->n, nb, p->batch, p->d_ldl64, &step, p->d_x, p->d_info, st))
+            return e;
+        TAGS_CUDA_OK(cudaMemcpyAsync(info.data(), p->d_info, sizeof(int) * nb, cudaMemcpyDeviceToHost, st));
+        TAGS_CUDA_OK(cudaStreamSynchronize(st));
     }
-    return 0;
+    std::vector<int> lu;
+    for (int q = 0; q < nb; ++q)
+        if (info[q] == TAGS_INFO_RESOLVE) lu.push_back(q);
+    const ResolveInputs in{p->d_coef, tags_ldl64_saved_rhs(p->d_ldl64, p->N, p->batch), 2 * p->m};
+    return tags_resolve_pass(p, {}, lu, in, p->d_x, p->d_info, st);
 }
 
 // ---- graph passes ------------------------------------------------------------------

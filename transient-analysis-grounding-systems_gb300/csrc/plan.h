@@ -54,7 +54,6 @@ struct tags_plan_s {
     SampleCoef* d_coef = nullptr;   // batch
     int* d_status = nullptr;        // 4 words
     int* d_info = nullptr;          // batch
-    int* d_ipiv = nullptr;          // N + 1 (pivoted LU of one sample, allocated with the first)
     double2* d_W = nullptr;         // plain: batch x N x N
     void* d_ldl64 = nullptr;        // plain: workspace of the FP64 LDL^T (part of d_W)
     SeriesGeo series;               // FP64 fill from per-pass moments (fill.cu) and its workspace,
@@ -111,6 +110,8 @@ struct tags_plan_s {
     size_t stage_bytes = 0;
     void* d_fb = nullptr;           // FP64 re-solves of fb_cap samples at a time (allocated with the first)
     int fb_cap = 0, fb_full = 0;    // fb_full: no room for more
+    int fb_run = 0, fb_step = 0;    // samples of the LDL^T run whose state it holds (0: not all that were asked for)
+                                    // and the number of its next correction
     // host copy of the geometry (11 doubles per segment; nodes 3 per node), so
     // a twin plan can be built from it
     std::vector<double> h_elec, h_img, h_nodes;
@@ -134,34 +135,61 @@ int tags_mixed_ir_setup(tags_plan_s* p, int nb, cudaStream_t st);
 int tags_mixed_ir_step(tags_plan_s* p, int nb, cudaStream_t st, cudaGraphConditionalHandle cond, int set_cond);
 int tags_mixed_finish(tags_plan_s* p, int nb, cudaStream_t st, int* h_iters, double* h_berr, int* h_conv,
                       int* h_steps);
-// Plain FP64 re-solves of samples idx of a sweep (inputs and outputs on the
-// device, sample by sample), queued on st, as many at a time as `most` bytes
-// hold; info TAGS_INFO_RESOLVE asks for tags_mixed_fallback_lu of that sample
-// (its own inputs and outputs).
-int tags_mixed_fallback_start(tags_plan_s* p, const std::vector<int>& idx, const double2* d_s, const double2* d_kappa,
-                              double mur, const double2* d_ie, int inj_node, double2* x, int* info, size_t most,
-                              cudaStream_t st);
-int tags_mixed_fallback_lu(tags_plan_s* p, const double2* d_s, const double2* d_kappa, double mur, const double2* d_ie,
-                           int inj_node, double2* x_out, int* info_out, cudaStream_t st);
+// resolve.cu: FP64 re-solves of a pass's samples, x and info sample by sample: `first` by
+// the structured LDL^T and what that asks for, `lu` by the pivoted LU. Inputs of sample
+// q: coef[q] and rhs[q N ..], in the original order or (currents_first = 2m) the static
+// one.
+struct ResolveInputs {
+    const SampleCoef* coef;
+    const double2* rhs;
+    int currents_first;
+};
+int tags_resolve_pass(tags_plan_s* p, const std::vector<int>& first, const std::vector<int>& lu, const ResolveInputs& in,
+                      double2* x, int* info, cudaStream_t st);
+// The stages of the same for samples of a sweep whose inputs lie on the device sample
+// by sample, queued on st, as many samples at a time as `most` bytes hold; info after
+// one asks for the next: the structured LDL^T of samples `first`, the next corrections
+// of those of them in `more` (again while info asks for it), the pivoted LU.
+struct ResolveSweep {
+    const double2 *s, *kappa, *ie;   // ie null: a unit current at inj
+    double mur;
+    int inj;
+};
+int tags_resolve_sweep_ldl(tags_plan_s* p, const std::vector<int>& first, const ResolveSweep& in, int steps, double2* x,
+                           int* info, size_t most, cudaStream_t st);
+int tags_resolve_sweep_more(tags_plan_s* p, const std::vector<int>& more, const ResolveSweep& in, double2* x, int* info,
+                            size_t most, cudaStream_t st);
+int tags_resolve_sweep_lu(tags_plan_s* p, const std::vector<int>& idx, const ResolveSweep& in, double2* x, int* info,
+                          size_t most, cudaStream_t st);
 // While-node after the work captured so far on `st` (condition 1 at launch);
 // its body graph is returned for a separate capture.
 int tags_plan_add_while_node(cudaStream_t st, cudaGraphConditionalHandle* cond, cudaGraph_t* body);
-// ldl64.cu: FP64 LDL^T in the static order with refinement (plain form). A
-// sample whose corrections do not shrink gets info = TAGS_INFO_RESOLVE: its
-// caller solves it by the pivoted LU.
-constexpr int TAGS_INFO_RESOLVE = -1000000;
+// ldl64.cu: FP64 LDL^T in the static order with refinement (plain form). A sample
+// whose corrections do not shrink, or are not finite, gets info = TAGS_INFO_RESOLVE:
+// its caller solves it by the pivoted LU. One that was still contracting when its
+// steps ran out gets TAGS_INFO_MORE: its caller goes on with it, up to
+// TAGS_RESOLVE_STEPS, after which it is TAGS_INFO_RESOLVE. A captured pass makes
+// TAGS_PASS_STEPS (a launch that finds no sample active costs ~2 us), a re-solve
+// TAGS_FIRST_STEPS before its host looks.
+constexpr int TAGS_INFO_RESOLVE = -1000000, TAGS_INFO_MORE = -1000001;
+constexpr int TAGS_PASS_STEPS = 4, TAGS_FIRST_STEPS = 3, TAGS_RESOLVE_STEPS = 10;
 int tags_ldl64_prepare();
 size_t tags_ldl64_workspace(int N, int batch);
 // where the fill of a pass writes ZL and ZT inside W (n + 2m square per sample)
 FillOut tags_ldl64_fill_out(double2* W, int m, int n);
 // after that fill: x (original order, may be rhs) = W^-1 rhs for nb samples
 int tags_ldl64_plan_solve(double2* W, const Incidence& inc, int m, int n, int nb, int batch, void* ws,
-                          const double2* rhs, double2* x, int* info, cudaStream_t st);
-// the right-hand side of sample q of the last solve, in the original order
-int tags_ldl64_saved_rhs(void* ws, int m, int n, int batch, int q, double2* out, cudaStream_t st);
+                          const double2* rhs, double2* x, int* info, int steps, cudaStream_t st);
+// the next two corrections, from number *step on (moved on), of the last solve, whose W
+// and ws are as it left them (N > 64: smaller systems never ask for more)
+int tags_ldl64_plan_more(const double2* W, const Incidence& inc, int m, int n, int nb, int batch, void* ws, int* step,
+                         double2* x, int* info, cudaStream_t st);
+// the right-hand sides of the last solve (batch x N, static order)
+const double2* tags_ldl64_saved_rhs(void* ws, int N, int batch);
 // one full symmetric matrix W (original order, kept), A of the same size for
-// the factors, x the right-hand side and the solution; *d_flag is scratch
-int tags_ldl64_sym_solve(const double2* W, double2* A, int m, int n, void* ws, int* d_flag, double2* x, int* info,
+// the factors, x the right-hand side and the solution, *info on the host; d_words:
+// two scratch words
+int tags_ldl64_sym_solve(const double2* W, double2* A, int m, int n, void* ws, int* d_words, double2* x, int* info,
                          cudaStream_t st);
 // nb full symmetric matrices Z (M x M): X = Z^-1 [rhs, I] (M x (n + M) each;
 // rhs M x n). *d_bad is raised when a check of the result finds it less
@@ -174,6 +202,3 @@ int tags_ldl64_multi_solve(const double2* Z, const double2* rhs, int M, int n, i
 // tags_ldl64_sym_solve; *done = 0 (x as it was) where the pivoted LU is wanted.
 // The caller holds the drop-in lock.
 int tags_sym_solve_host(const tags_cdouble* w, tags_cdouble* x, size_t m, size_t n, int* done);
-// the pivoted LU of one sample from the plan's coefficients slot q into W
-// (N x N), right-hand side and solution in x, info on the device
-int tags_plan_lu_one(tags_plan_s* p, int q, double2* W, int* ipiv, double2* x, int* info, cudaStream_t st);
