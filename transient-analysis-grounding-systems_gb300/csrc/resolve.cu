@@ -4,10 +4,10 @@
 // stages, each over all the samples that need it: the structured LDL^T with a pass's
 // corrections, up to TAGS_RESOLVE_STEPS of them, and the LU with partial pivoting
 // (lu.cu).
-// Refinement that still contracts is cheaper than the LU (64 samples of a 74-segment
-// wire at s = 0.01 .. 1 Hz: 2.8 against 19 ms), and the LU's serial panels cost a
-// batch little more than one sample: 64 samples at s = 0 66 -> 3.6 ms (N = 46) and
-// 433 -> 53 ms (N = 285) against one LU after the other.
+// Refinement that still contracts is cheaper than the LU (64 samples at 0.01 .. 1 Hz,
+// 100 segments in 1e-4 S/m: 2.7 ms in all, 60 by the LU alone), and the LU's serial
+// panels cost a batch little more than one sample: 64 samples at s = 0 66 -> 1.3 ms (N =
+// 46) and 433 -> 11.6 ms (N = 285) against one LU after the other.
 #include <algorithm>
 #include <vector>
 
