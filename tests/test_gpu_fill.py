@@ -400,3 +400,9 @@ def test_fill_terms_by_four_lanes_match_whole_warps(gpu_pkg, x):
     for a, b in zip(*out):
         nz = b != 0
         assert np.array_equal(a != 0, nz) and elementwise(a[nz], b[nz]) < 1e-13
+
+
+@pytest.mark.parametrize("x", [0.9, 1.65, 1.75])
+def test_fill_of_24_terms_by_four_lanes_matches_whole_warps(gpu_pkg, x):
+    """The same on both sides of the 24-term instance's reach (x = 1.7)."""
+    test_fill_terms_by_four_lanes_match_whole_warps(gpu_pkg, x)

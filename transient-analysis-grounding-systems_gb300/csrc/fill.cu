@@ -402,10 +402,12 @@ __global__ void __launch_bounds__(128) k_path_pairs(const double* __restrict__ e
 // exponential (~130) per sample, and a sample 2 nt + 20 per pair. Pairs
 // sharing an endpoint: the radial part of the Duffy rule in closed form,
 // \int_0^1 (t rho - R)^n dt = g_n / (n + 1), g_n = sum_i (rho - R)^i (-R)^(n-i).
-// Terms: x^nt / nt! <= 1e-17 at x = max |gamma| dmax (moments of 12 up to x = 0.2, of
-// 16 up to x = 0.58, else of 32, which reach x = 3.5, where the sum's largest term
-// is e^3.5 of N_0 and the rounding stays below 1e-14 of the entry). Samples beyond
-// that keep an exponential per point (k_fill_far).
+// Terms: x^nt / nt! <= 1e-17 at x = max |gamma| dmax: moments of 12 up to x = 0.2, of
+// 16 up to x = 0.58, of 24 up to x = 1.7 (four lanes per record, where many pairs make
+// the moments count: one sample of 1560 segments through the drop-ins at x = 0.66 30.6
+// -> 27.3 ms, 28.8 by the direct rule), else of 32, which reach x = 3.5, where the sum's
+// largest term is e^3.5 of N_0 and the rounding stays below 1e-14 of the entry. Samples
+// beyond that keep an exponential per point (k_fill_far).
 // Measured on GB300 against the direct rule for every sample: the plain form's
 // pass of 256 samples at m = 100 217 -> 24.3 ms, 100 samples at m = 10 3.50 ->
 // 0.66 ms, one sample at m = 100 through the drop-ins 11.9 -> 6.7 ms (the fill
@@ -719,7 +721,7 @@ TAGS_D void cta_moments(const SeriesPk* pk, int nrec, double (*mom)[SER_NT], int
         const bool on = r < nrec && (pk[r].kind == SK_TENSOR || pk[r].kind == SK_PAR) && pk[r].npts <= SER_SHORT;
         series_moments<NT, L>(pk[on ? r : 0], on, tid % L, mom[r]);
     }
-    constexpr int NW = NT == 12 ? 16 : NT;
+    constexpr int NW = NT == 12 ? 16 : NT == 24 ? 32 : NT;
     for (int r = tid >> 5; r < nrec; r += SER_THREADS / 32)
         if (pk[r].kind == SK_TOUCH ||
             ((pk[r].kind == SK_TENSOR || pk[r].kind == SK_PAR) && (L == 32 || pk[r].npts > SER_SHORT)))
@@ -730,6 +732,7 @@ template <int L>
 TAGS_D void cta_moments_of(int nt, const SeriesPk* pk, int nrec, double (*mom)[SER_NT], int tid) {
     if (L == 4 && nt <= 12) cta_moments<12, 4>(pk, nrec, mom, tid);
     else if (nt <= 16) cta_moments<16, L>(pk, nrec, mom, tid);
+    else if (L == 4 && nt <= 24) cta_moments<24, 4>(pk, nrec, mom, tid);
     else cta_moments<32, L>(pk, nrec, mom, tid);
 }
 
