@@ -22,13 +22,12 @@
 
 namespace {
 
-__global__ void k_twiddles(double2* __restrict__ tw, long long nt) {
-    long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= nt) return;
+// The nt-th root number q of unity: angle 2 pi q / nt in [0, 2 pi); sincospi keeps it
+// exact at the quadrants.
+TAGS_D double2 root_of_unity(long long q, long long nt) {
     double s, c;
-    // angle 2 pi q / nt in [0, 2 pi); sincospi keeps it exact at the quadrants
     sincospi(2.0 * (double)q / (double)nt, &s, &c);
-    tw[q] = make_double2(c, s);
+    return make_double2(c, s);
 }
 
 __device__ double window(int filter, double w, double omega) {
@@ -42,12 +41,14 @@ __device__ double window(int filter, double w, double omega) {
     }
 }
 
-// sigma_k of the samples and the output scale e^{c t_j} / (nt dt), once per call.
+// The roots of unity, sigma_k of the samples and the output scale e^{c t_j} / (nt dt),
+// once per call.
 __global__ void k_inlt_tables(const double2* __restrict__ s, long long ns, long long nt, double tmax, int filter,
-                              double* __restrict__ sigma, double* __restrict__ scale) {
+                              double2* __restrict__ tw, double* __restrict__ sigma, double* __restrict__ scale) {
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q < ns) sigma[q] = window(filter, s[q].y, s[ns - 1].y);
     if (q < nt) {
+        tw[q] = root_of_unity(q, nt);
         const double dt = tmax / (double)(nt - 1);
         scale[q] = exp(s[0].x * (double)q * dt) / ((double)nt * dt);
     }
@@ -297,10 +298,12 @@ FftPlan fft_plan(int nt, int* sum) {
 
 // ---- forward -------------------------------------------------------------------
 
-// The damped samples f[j] dt e^{-c t_j}, once per call.
-__global__ void k_nlt_damp(const double* __restrict__ f, long long nt, double tmax, double* __restrict__ v) {
+// The roots of unity and the damped samples f[j] dt e^{-c t_j}, once per call.
+__global__ void k_nlt_damp(const double* __restrict__ f, long long nt, double tmax, double2* __restrict__ tw,
+                           double* __restrict__ v) {
     const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= nt) return;
+    tw[j] = root_of_unity(j, nt);
     const double c = log((double)nt * (double)nt) / tmax, dt = tmax / (double)(nt - 1);
     v[j] = f[j] * dt * exp(-c * (double)j * dt);
 }
@@ -334,13 +337,6 @@ __global__ void __launch_bounds__(32 * DIR_PARTS) k_nlt(const double* __restrict
     g[k] = make_double2(re, im);
 }
 
-int twiddles(double2* d_tw, long long nt, cudaStream_t st) {
-    k_twiddles<<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(d_tw, nt);
-    tags_note_launch();
-    TAGS_CUDA_OK(cudaGetLastError());
-    return 0;
-}
-
 }  // namespace
 
 size_t tags_inlt_workspace(long long nt) { return (sizeof(double2) + 2 * sizeof(double)) * (size_t)nt + 64; }
@@ -352,8 +348,7 @@ int tags_launch_inlt(const double2* d_g, long long gseries, long long gk, const 
     double2* tw = reinterpret_cast<double2*>(ws);
     double* scale = reinterpret_cast<double*>(tw + nt);
     double* sigma = scale + nt;                                // ns <= nt values
-    if (int e = twiddles(tw, nt, st)) return e;
-    k_inlt_tables<<<(unsigned)((nt + 127) / 128), 128, 0, st>>>(d_s, ns, nt, tmax, filter, sigma, scale);
+    k_inlt_tables<<<(unsigned)((nt + 127) / 128), 128, 0, st>>>(d_s, ns, nt, tmax, filter, tw, sigma, scale);
     tags_note_launch();
     // SM cycles of either way (two FP64 multiply-adds per clock and SM): the
     // transform keeps a CTA's SM for nt (5 sum r + 6 FFT_LOW) / 2 and runs a pair per SM at a
@@ -392,8 +387,7 @@ int tags_launch_inlt(const double2* d_g, long long gseries, long long gk, const 
 int tags_launch_nlt(const double* d_f, long long nt, void* ws, double tmax, double2* d_g, cudaStream_t st) {
     double2* tw = reinterpret_cast<double2*>(ws);
     double* v = reinterpret_cast<double*>(tw + nt);
-    if (int e = twiddles(tw, nt, st)) return e;
-    k_nlt_damp<<<(unsigned)((nt + 127) / 128), 128, 0, st>>>(d_f, nt, tmax, v);
+    k_nlt_damp<<<(unsigned)((nt + 127) / 128), 128, 0, st>>>(d_f, nt, tmax, tw, v);
     k_nlt<<<(unsigned)((nt / 2 + 1 + 31) / 32), 32 * DIR_PARTS, 0, st>>>(v, nt, tw, d_g);
     tags_note_launch(2);
     TAGS_CUDA_OK(cudaGetLastError());
