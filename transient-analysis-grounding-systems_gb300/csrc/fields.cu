@@ -1020,23 +1020,28 @@ int fields_run(const FieldsIn& in) {
     for (size_t s0 = 0; s0 < S; s0 += cs) {
         const size_t ns = std::min(cs, S - s0);
         const size_t nc = R * m * ns;
+        const bool turn = !((ns == 1) + (R == 1) + (m == 1) >= 2);    // else the transposed array is the same
         double2* raw_t = d_cur;               // [ns][R][m] as given
         double2* raw_l = d_cur + nc;
-        double2* cur_t = d_cur + 2 * nc;      // transposed [m][R][ns]
-        double2* cur_l = d_cur + 3 * nc;
+        double2* cur_t = turn ? d_cur + 2 * nc : raw_t;      // transposed [m][R][ns]
+        double2* cur_l = turn ? d_cur + 3 * nc : raw_l;
         const bool need_t = (in.want & (WANT_POT | WANT_EF)) != 0, need_l = (in.want & WANT_VEC) != 0;
         const int tb = 256, tg = (int)std::min<size_t>((nc + tb - 1) / tb, (size_t)tags_num_sms() * 16);
         if (need_t) {
             TAGS_CUDA_OK(cudaMemcpyAsync(raw_t, in.it + s0 * R * m, sizeof(double2) * nc, cudaMemcpyHostToDevice, st));
-            k_cur_transpose<<<tg, tb, 0, st>>>(raw_t, cur_t, (int)ns, (int)R, (int)m);
-            tags_note_launch();
-            TAGS_CUDA_OK(cudaGetLastError());
+            if (turn) {
+                k_cur_transpose<<<tg, tb, 0, st>>>(raw_t, cur_t, (int)ns, (int)R, (int)m);
+                tags_note_launch();
+                TAGS_CUDA_OK(cudaGetLastError());
+            }
         }
         if (need_l) {
             TAGS_CUDA_OK(cudaMemcpyAsync(raw_l, in.il + s0 * R * m, sizeof(double2) * nc, cudaMemcpyHostToDevice, st));
-            k_cur_transpose<<<tg, tb, 0, st>>>(raw_l, cur_l, (int)ns, (int)R, (int)m);
-            tags_note_launch();
-            TAGS_CUDA_OK(cudaGetLastError());
+            if (turn) {
+                k_cur_transpose<<<tg, tb, 0, st>>>(raw_l, cur_l, (int)ns, (int)R, (int)m);
+                tags_note_launch();
+                TAGS_CUDA_OK(cudaGetLastError());
+            }
         }
         TAGS_CUDA_OK(cudaMemcpyAsync(d_gk, in.gamma + s0, sizeof(double2) * ns, cudaMemcpyHostToDevice, st));
         TAGS_CUDA_OK(cudaMemcpyAsync(d_gk + ns, in.kappa + s0, sizeof(double2) * ns, cudaMemcpyHostToDevice, st));
