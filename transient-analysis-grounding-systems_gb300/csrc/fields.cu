@@ -327,16 +327,20 @@ TAGS_D bool cur_big(double2 c) {
 constexpr int FS_ORDERS[5] = {6, 7, 8, 9, 12};
 constexpr int FS_GL = 6 + 7 + 8 + 9 + 12;
 
-// The rule's orders from 16 and from 8 lengths away, as indices of FS_ORDERS: the
-// distance leaves 1/r and 1/r^3 with 6 and 7 nodes below 1e-15, but the moments
-// also carry e^{-gamma r} over the electrode, whose error at x = |gamma| dmax is
-// 8e-10 (x / 2)^12 with 6 nodes and 5e-12 (x / 2)^14 with 7 on the electrode's axis.
-// Each stays up to where that passes 1e-15 (6 nodes at every x: 6e-10 at x = 1.95).
-int fs_least_order(double x) { return x <= 0.55 ? 0 : x <= 1.0 ? 1 : 3; }
+// The rule's least order, as an index of FS_ORDERS, at y = |gamma| times half the range
+// of r over the electrode, y2 / s2 = y^2: the distance leaves 1/r and 1/r^3 with 6 nodes
+// from 16 and 7 from 8 lengths on below 1e-15, but the moments also carry e^{-gamma r},
+// whose error is 3e-9 (y / 2)^12 with 6 nodes, 2e-11 (y / 2)^14 with 7 and 1e-13 (y / 2)^16
+// with 8. Each stays up to where that passes 1e-15 to 4e-15 (6 nodes throughout: 6e-10 at the
+// series' reach on the electrode's axis).
+TAGS_D int fs_least_order(double y2, double s2) {
+    return y2 <= 0.24 * s2 ? 0 : y2 <= 0.7 * s2 ? 1 : y2 <= 1.8 * s2 ? 2 : 3;
+}
 // Panels of the near points per unit of v, for the same reason: 3000 random points
-// within two lengths stay within 7e-14 (1e-15 in the median) with panels of 0.75 at x =
-// 1, 6e-15 with 0.5 at 1.5 and 4e-15 with 0.375 at 2, where 0.75 gives up to 1e-12.
-double fs_panels(double x) { return 1.0 / (x <= 1.0 ? 0.75 : x <= 1.5 ? 0.5 : 0.375); }
+// within two lengths stay within 8e-14 (6e-16 in the median; 5e-14 for x near 0) with
+// panels of 0.75 at x = 1.1, 5e-15 with 0.6 at 1.25, 6e-15 with 0.5 at 1.5 and 4e-15 with
+// 0.375 at 2, where 0.75 gives up to 1e-12.
+double fs_panels(double x) { return 1.0 / (x <= 1.1 ? 0.75 : x <= 1.25 ? 0.6 : x <= 1.5 ? 0.5 : 0.375); }
 
 __constant__ double c_fsx[FS_GL], c_fsw[FS_GL];   // nodes and weights on [0, 1], order by order
 
@@ -346,8 +350,7 @@ struct SerArgs {
     const double2* tab;     // [bucket][S]: e^{-gamma b h} (null: formed per pair)
     double h;
     int nbk, ngc, echunk;   // buckets; sample groups per CTA (1, 2, 4); electrodes per CTA
-    int least;              // fs_least_order and fs_panels of the largest |gamma| among the series' samples
-    double panels;
+    double ga2, panels;     // a quarter of the largest |gamma|^2 among the series' samples, and its fs_panels
 };
 
 // The samples' constants: a row of CTAs per bucket of the table (nbk of them, none
@@ -420,8 +423,10 @@ TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, const Se
     q.bad = !(dist > 1e-12 * Lg) || !isfinite(rc);
     if (!q.bad && dist >= 2.0 * Lg) {
         const double ratio = dist * q.iL;
-        const int o = max(sa.least, ratio >= 16.0 ? 0 : ratio >= 8.0 ? 1 : ratio >= 4.0 ? 3 : 4);
-        const int nq = o == 0 ? 6 : o == 1 ? 7 : o == 3 ? 9 : 12, off = o == 0 ? 0 : o == 1 ? 6 : o == 3 ? 21 : 30;
+        // r grows by L |dm| / rc over the electrode
+        const int o = max(fs_least_order(sa.ga2 * L2 * (dm * dm), fma(dm, dm, d2)),
+                          ratio >= 16.0 ? 0 : ratio >= 8.0 ? 1 : ratio >= 4.0 ? 3 : 4);
+        const int nq = o == 4 ? 12 : 6 + o, off = o == 4 ? 30 : 6 * o + o * (o - 1) / 2;
         for (int i = g; i < nq; i += L) {
             const double s = (gx[off + i] - u0) * Lg;
             node(s, fma(s, s, d2), gw[off + i]);
@@ -1052,11 +1057,11 @@ int fields_run(const FieldsIn& in) {
         int* d_nt = reinterpret_cast<int*>(tab + rows * ns);
         TAGS_CUDA_OK(cudaMemcpyAsync(d_nt, nt.data() + s0, sizeof(int) * ns, cudaMemcpyHostToDevice, st));
         const int most = *std::max_element(nt.begin() + s0, nt.begin() + s0 + ns);
-        double x = 0.0;
+        double ga = 0.0;
         for (size_t k = s0; k < s0 + ns; ++k)
-            if (nt[k] > 0) x = std::max(x, std::abs(zd(in.gamma[k].re, in.gamma[k].im)) * geo.dmax);
-        sa.least = fs_least_order(x);
-        sa.panels = fs_panels(x);
+            if (nt[k] > 0) ga = std::max(ga, std::abs(zd(in.gamma[k].re, in.gamma[k].im)));
+        sa.ga2 = 0.25 * ga * ga;
+        sa.panels = fs_panels(ga * geo.dmax);
         if (most > 0) {
             k_fser_tables<<<dim3((unsigned)((ns + 31) / 32), (unsigned)rows + 1), 32, 0, st>>>(
                 d_gk, d_nt, (int)ns, (int)rows, geo.h, pw, tab);
