@@ -324,8 +324,8 @@ TAGS_D bool cur_big(double2 c) {
     if (hy >= lim && hy < 0x7ff00000 && hx < 0x7ff00000) return true;
     return cabs2(c) >= 0x1.fffffffffffffp-105;      // the squares whose root rounds to 2^-52 or more
 }
-constexpr int FS_ORDERS[5] = {6, 7, 8, 9, 12};
-constexpr int FS_GL = 6 + 7 + 8 + 9 + 12;
+constexpr int FS_ORDERS[6] = {6, 7, 8, 9, 10, 12};
+constexpr int FS_GL = 6 + 7 + 8 + 9 + 10 + 12, FS_8 = 6 + 7, FS_10 = 6 + 7 + 8 + 9;
 
 // The rule's least order, as an index of FS_ORDERS, at y = |gamma| times half the range
 // of r over the electrode, y2 / s2 = y^2: the distance leaves 1/r and 1/r^3 with 6 nodes
@@ -336,12 +336,6 @@ constexpr int FS_GL = 6 + 7 + 8 + 9 + 12;
 TAGS_D int fs_least_order(double y2, double s2) {
     return y2 <= 0.24 * s2 ? 0 : y2 <= 0.7 * s2 ? 1 : y2 <= 1.8 * s2 ? 2 : 3;
 }
-// Panels of the near points per unit of v, for the same reason: 3000 random points
-// within two lengths stay within 8e-14 (6e-16 in the median; 5e-14 for x near 0) with
-// panels of 0.75 at x = 1.1, 5e-15 with 0.6 at 1.25, 6e-15 with 0.5 at 1.5 and 4e-15 with
-// 0.375 at 2, where 0.75 gives up to 1e-12.
-double fs_panels(double x) { return 1.0 / (x <= 1.1 ? 0.75 : x <= 1.25 ? 0.6 : x <= 1.5 ? 0.5 : 0.375); }
-
 __constant__ double c_fsx[FS_GL], c_fsw[FS_GL];   // nodes and weights on [0, 1], order by order
 
 struct SerArgs {
@@ -350,7 +344,8 @@ struct SerArgs {
     const double2* tab;     // [bucket][S]: e^{-gamma b h} (null: formed per pair)
     double h;
     int nbk, ngc, echunk;   // buckets; sample groups per CTA (1, 2, 4); electrodes per CTA
-    double ga2, panels;     // a quarter of the largest |gamma|^2 among the series' samples, and its fs_panels
+    double ga2;             // a quarter of the largest |gamma|^2 among the series' samples
+    int near;               // nodes per panel of the near points' rule: 8 or 10
 };
 
 // The samples' constants: a row of CTAs per bucket of the table (nbk of them, none
@@ -380,8 +375,11 @@ struct SerPair {
 // Moments of one (point, electrode) pair by L lanes (g: this one), all of the
 // warp's groups together, `on` or not: Gauss-Legendre in t where the point is at
 // least two lengths away (6 to 12 nodes by the distance and |gamma|), else the sinh
-// rule above in panels of 0.75 down to 0.375, up to ~1000 nodes, which one lane
-// would take in a row.
+// rule above, up to ~400 nodes, which one lane would take in a row: panels of 0.75 with
+// 8 nodes, or of one with 10 where e^{-gamma r} asks for them (x > 1.1). 3000 random
+// points within two lengths, 25 nodes each on average either way, stay within 8e-14 (6e-16
+// in the median) and 4e-15; 8 nodes at x = 2: 1e-12. With 10 throughout, pairs of few
+// lanes take a second round for one panel: path voltages of 40 paths 0.90 -> 0.92 ms.
 template <int NT>
 TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, const SerArgs& sa, const double* gx,
                          const double* gw, bool on, int g, int L, SerPair& out, double* mom) {
@@ -425,8 +423,8 @@ TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, const Se
         const double ratio = dist * q.iL;
         // r grows by L |dm| / rc over the electrode
         const int o = max(fs_least_order(sa.ga2 * L2 * (dm * dm), fma(dm, dm, d2)),
-                          ratio >= 16.0 ? 0 : ratio >= 8.0 ? 1 : ratio >= 4.0 ? 3 : 4);
-        const int nq = o == 4 ? 12 : 6 + o, off = o == 4 ? 30 : 6 * o + o * (o - 1) / 2;
+                          ratio >= 16.0 ? 0 : ratio >= 8.0 ? 1 : ratio >= 4.0 ? 3 : 5);
+        const int nq = o == 5 ? 12 : 6 + o, off = o == 5 ? 40 : 6 * o + o * (o - 1) / 2;
         for (int i = g; i < nq; i += L) {
             const double s = (gx[off + i] - u0) * Lg;
             node(s, fma(s, s, d2), gw[off + i]);
@@ -434,16 +432,18 @@ TAGS_D void fser_moments(const Seg& S, double P0, double P1, double P2, const Se
     } else if (!q.bad) {
         const double d = sqrt(d2), dp = fmax(d, 1e-6 * Lg);
         const double va = asinh(-u0 * Lg / dp), vb = asinh((1.0 - u0) * Lg / dp);
+        const int nn = sa.near, off = nn == 8 ? FS_8 : FS_10, inv = nn == 8 ? 8193 : 6554;
+        const double wide = nn == 8 ? 1.0 / 0.75 : 1.0;
         // panels on either side of the foot, or one range
         const bool split = va < 0.0 && vb > 0.0;
         for (int side = 0; side < (split ? 2 : 1); ++side) {
             const double lo = split && side == 1 ? 0.0 : va, hi = split && side == 0 ? 0.0 : vb;
-            const int np = max(1, (int)ceil(fmin((hi - lo) * sa.panels, 64.0)));
+            const int np = max(1, (int)ceil(fmin((hi - lo) * wide, 64.0)));
             const double ph = (hi - lo) / np;
-            for (int t = g; t < 8 * np; t += L) {
-                const int p = t >> 3, i = t & 7;
-                const double v = lo + (p + gx[13 + i]) * ph, s = dp * sinh(v);
-                node(s, fma(s, s, d2), gw[13 + i] * ph * (dp * q.iL) * cosh(v));
+            for (int t = g; t < nn * np; t += L) {
+                const int p = (t * inv) >> 16, i = off + t - nn * p;        // p = t / nn up to 64 panels
+                const double v = lo + (p + gx[i]) * ph, s = dp * sinh(v);
+                node(s, fma(s, s, d2), gw[i] * ph * (dp * q.iL) * cosh(v));
             }
         }
     }
@@ -1061,7 +1061,7 @@ int fields_run(const FieldsIn& in) {
         for (size_t k = s0; k < s0 + ns; ++k)
             if (nt[k] > 0) ga = std::max(ga, std::abs(zd(in.gamma[k].re, in.gamma[k].im)));
         sa.ga2 = 0.25 * ga * ga;
-        sa.panels = fs_panels(ga * geo.dmax);
+        sa.near = ga * geo.dmax <= 1.1 ? 8 : 10;
         if (most > 0) {
             k_fser_tables<<<dim3((unsigned)((ns + 31) / 32), (unsigned)rows + 1), 32, 0, st>>>(
                 d_gk, d_nt, (int)ns, (int)rows, geo.h, pw, tab);
